@@ -151,6 +151,7 @@ struct g5b_engine {
     MoePlan plan;
     float *xm, *inv_head, *logits, *am_v;
     int   *am_i, *am_out;
+    void  *sample_buf = nullptr;
     void  *flush_buf = nullptr; size_t flush_bytes = 0;
     cudaEvent_t prof_ev[PROF_SLOTS + 1];
     float prof_ms[PROF_SLOTS];
@@ -735,7 +736,8 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         CU(cudaHostGetDevicePointer((void **)&e->err_dev, hp, 0));
     }
     if (walloc(e, &e->xm, N * E) || walloc(e, &e->inv_head, N) || walloc(e, &e->logits, N * (size_t)c.vocab) ||
-        walloc(e, &e->am_v, N * 64) || walloc(e, &e->am_i, N * 64) || walloc(e, &e->am_out, (size_t)e->cap + N)) return -1;
+        walloc(e, &e->am_v, N * 64) || walloc(e, &e->am_i, N * 64) || walloc(e, &e->am_out, (size_t)e->cap + N) ||
+        e->dalloc(&e->sample_buf, sample_scratch_bytes(c.vocab))) return -1;
     if (e->mtp && (walloc(e, &e->mtp_h, ((size_t)e->cap + N) * E) || walloc(e, &e->mtp_cat, N * 2 * E) ||
                    walloc(e, &e->mtp_x, N * E))) return -1;
     CU(cudaStreamSynchronize(e->st));
@@ -1361,7 +1363,7 @@ extern "C" int g5b_engine_decode_sampled(g5b_engine *e, int first, int n, float 
         const int rc = forward_device(e, e->ids_dev + i, 1, false, nullptr, nullptr);
         if (rc) { e->cached = start; return -1; }
         // the step counter of the draw is the position the token will occupy
-        sample_token(e->st, e->ids_dev + i + 1, e->logits, e->logits + e->c.vocab, e->c.vocab, temperature, top_p, seed,
+        sample_token(e->st, e->ids_dev + i + 1, e->logits, e->sample_buf, e->c.vocab, temperature, top_p, seed,
                      (uint64_t)(start + i + 1));
     }
     e->cached = start;
@@ -2070,7 +2072,7 @@ extern "C" int g5b_sample_host(const float *logits, int V, float temperature, fl
     if (with_device(device, &st)) return -1;
     if (V < 1 || !(temperature > 0.f) || !(top_p > 0.f)) return fail("sampling needs a vocabulary, temperature > 0 and top_p > 0");
     Tmp t;
-    float *ld = (float *)t.up(logits, (size_t)V * 4), *pd = (float *)t.up(nullptr, (size_t)V * 4);
+    float *ld = (float *)t.up(logits, (size_t)V * 4), *pd = (float *)t.up(nullptr, sample_scratch_bytes(V));
     int *od = (int *)t.up(nullptr, 4);
     if (!ld || !pd || !od) return fail("out of device memory");
     sample_token(st, od, ld, pd, V, temperature, top_p, seed, step);

@@ -92,3 +92,17 @@ def test_sampled_decode_loop(gpu_lib):
     b = eng.decode_sampled(int(a[-1]), 5, 0.9, 0.8, 99)
     assert np.array_equal(np.concatenate([a, b]), toks)
     eng.close()
+
+
+@pytest.mark.parametrize("V", [1, 2, 1023, 1025, 2049, 40000, 1048577])
+def test_sampler_at_the_edges_of_its_ranges(gpu_lib, V):
+    """Vocabularies around the sampler's ranges of 1024 tokens, and more tokens than 1024 such ranges; logits with
+    many exact ties, so that whole groups of tokens stand on the nucleus threshold."""
+    rng = np.random.default_rng(V)
+    for top_p in (0.02, 0.6, 0.97, 1.0):
+        for ties in (False, True):
+            logits = (2.0 * rng.standard_normal(V)).astype(np.float32)
+            if ties:
+                logits = np.round(logits)
+            seed, step = int(rng.integers(1, 1 << 40)), int(rng.integers(0, 4096))
+            assert pkg.sample_host(logits, 0.9, top_p, seed, step) == sample_restated(logits, 0.9, top_p, seed, step), (top_p, ties)
