@@ -43,6 +43,7 @@ constexpr size_t EP_FLAG_BYTES = 1024;   // exchange region: the ranks' step wor
 constexpr int EP_HEAD_WORD0 = 64;        // words [64, 64 + 5 x 8): the vocabulary-split head's (value, index) slots of two parities and its arrival counters (up to 8 ranks)
 constexpr int MLA_PART_TOKENS = 4;     // tokens whose attention partial sums are held at once
 constexpr int CHUNK = 64;       // positions one pass of a layer works on (the reference's MoE chunk, glm53f_ops.c:988)
+constexpr int TC_MIN_T = 2;     // positions from which the projections go to the tensor cores
 constexpr int PROF_SLOTS = 8;
 
 struct Layer {
@@ -61,7 +62,7 @@ struct Layer {
     DMat   router;
     float *bias = nullptr;
     uint8_t *expert_slab = nullptr;
-    size_t   expert_stride = 0;
+    size_t   expert_mat = 0, expert_stride = 0;
     int      expert_dt = -1;
     std::vector<ExpertW> table;          // n_local routed + 1 shared (host mirror)
     std::vector<uint8_t> have;           // [n_local][3]
@@ -164,6 +165,11 @@ struct g5b_engine {
         CU(cudaMemsetAsync(*p, 0, bytes, st));
         owned.push_back(*p);
         return 0;
+    }
+    void drop(void *p)
+    {
+        for (size_t i = 0; i < owned.size(); i++)
+            if (owned[i] == p) { cudaFree(p); owned.erase(owned.begin() + (long)i); return; }
     }
 };
 
@@ -435,12 +441,15 @@ static int ensure_expert_slab(g5b_engine *e, Layer &w, int dt)
         sc = up256((size_t)((c.moe_inter + br - 1) / br) * ((c.hidden + bc - 1) / bc) * 4) * 2 +
              up256((size_t)((c.hidden + br - 1) / br) * ((c.moe_inter + bc - 1) / bc) * 4);
     }
+    w.expert_mat = mat;
     w.expert_stride = 3 * mat + sc;
     w.expert_dt = dt;
-    if (e->dalloc((void **)&w.expert_slab, w.expert_stride * (size_t)e->n_local)) return -1;
+    // (the last place is the shared expert's: finalize moves it here, so that one tensor map covers them all)
+    const int places = e->n_local + (c.n_shared == 1 ? 1 : 0);
+    if (e->dalloc((void **)&w.expert_slab, w.expert_stride * (size_t)places)) return -1;
     w.table.assign((size_t)e->n_local + 1, ExpertW{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr});
     w.have.assign((size_t)e->n_local * 3, 0);
-    for (int i = 0; i < e->n_local; i++) {
+    for (int i = 0; i < places; i++) {
         uint8_t *base = w.expert_slab + (size_t)i * w.expert_stride;
         ExpertW &x = w.table[i];
         x.gate = base; x.up = base + mat; x.down = base + 2 * mat;
@@ -671,10 +680,22 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
                 for (int k = 0; k < 3; k++)
                     if (!w.have[(size_t)i * 3 + k])
                         return fail("layer %d: routed expert %d is incomplete", l, e->n_local0 + i);
-            if (c.n_shared == 1 && w.sh_gate.dt == w.expert_dt) {
-                ExpertW &s = w.table[e->n_local];
-                s.gate = (const uint8_t *)w.sh_gate.w; s.up = (const uint8_t *)w.sh_up.w; s.down = (const uint8_t *)w.sh_down.w;
-                s.gate_s = w.sh_gate.s; s.up_s = w.sh_up.s; s.down_s = w.sh_down.s;
+            if (c.n_shared == 1 && w.sh_gate.dt == w.expert_dt && w.sh_up.dt == w.expert_dt && w.sh_down.dt == w.expert_dt) {
+                // into the slab, behind the routed experts; its own allocations are given back
+                const ExpertW &s = w.table[e->n_local];
+                auto move = [&](DMat &m, const uint8_t *codes, const float *scales) -> int {
+                    if (!m.loaded()) return 0;
+                    if (copy_in(e, (void *)codes, m.w, m.bytes(), 1)) return -1;
+                    e->drop(m.w);
+                    m.w = (void *)codes;
+                    if (m.s) {
+                        if (copy_in(e, (void *)scales, m.s, (size_t)((m.rows + m.br - 1) / m.br) * m.scols * 4, 1)) return -1;
+                        e->drop(m.s);
+                        m.s = (float *)scales;
+                    }
+                    return 0;
+                };
+                if (move(w.sh_gate, s.gate, s.gate_s) || move(w.sh_up, s.up, s.up_s) || move(w.sh_down, s.down, s.down_s)) return -1;
             }
             if (walloc(e, &w.table_dev, w.table.size())) return -1;
             CU(cudaMemcpyAsync(w.table_dev, w.table.data(), w.table.size() * sizeof(ExpertW), cudaMemcpyHostToDevice, e->st));
@@ -719,13 +740,14 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
     const size_t pairs = N * K + N;
     if (walloc(e, &e->rscore, N * c.n_experts) || walloc(e, &e->rw, N * K) || walloc(e, &e->ridx, N * K) ||
         walloc(e, &e->act, pairs * (I > SI ? I : SI)) || walloc(e, &e->contrib, pairs * E) ||
-        walloc(e, &e->gu, N * 2 * DI) || walloc(e, &e->dact, N * DI) || walloc(e, &e->xinv, N) ||
+        walloc(e, &e->gu, N * 2 * DI) || walloc(e, &e->dact, N * DI) || walloc(e, &e->xinv, pairs) ||
         walloc(e, &e->hc_part, N * 32 * (MIX + 1)) || walloc(e, &e->hc_count, N) ||
-        e->dalloc(&e->xterms, N * 2 * E * 2)) return -1;
+        e->dalloc(&e->xterms, pairs * 2 * E * 2)) return -1;
     e->plan.max_slots = (int)((N * K < (size_t)e->n_local ? N * K : (size_t)e->n_local) + 1);
     e->plan.max_pairs = (int)pairs;
     if (walloc(e, &e->plan.n_slots, 1) || walloc(e, &e->plan.slot_expert, e->plan.max_slots) ||
         walloc(e, &e->plan.slot_off, e->plan.max_slots) || walloc(e, &e->plan.slot_cnt, e->plan.max_slots) ||
+        walloc(e, &e->plan.slot_tile0, e->plan.max_slots + 1) || walloc(e, &e->plan.n_pairs, 1) ||
         walloc(e, &e->plan.pair_tok, pairs) || walloc(e, &e->plan.pair_dst, pairs)) return -1;
     if (walloc(e, &e->counter, CHUNK + 4) || walloc(e, &e->tile_done, E / 32 + 1) || walloc(e, &e->grid_sync, 2)) return -1;
     {
@@ -764,6 +786,14 @@ static MoeShape moe_shape(const g5b_engine *e, const Layer &w)
     s.n_local0 = e->n_local0; s.n_local = e->n_local;
     s.limit = c.swiglu_limit; s.routed_scale = c.routed_scale; s.norm_topk = c.norm_topk;
     return s;
+}
+
+static ExpertSlab expert_slab(const g5b_engine *e, const Layer &w)
+{
+    const g5b_config &c = e->c;
+    const int br = c.fp8_block_r > 0 ? c.fp8_block_r : 1, bc = c.fp8_block_c > 0 ? c.fp8_block_c : 1;
+    return ExpertSlab{w.expert_slab, w.expert_mat, w.expert_stride, up256((size_t)((c.moe_inter + br - 1) / br) * ((c.hidden + bc - 1) / bc) * 4),
+                      e->n_local + (c.n_shared == 1 ? 1 : 0)};
 }
 
 static void prof_mark(g5b_engine *e, int slot)
@@ -815,9 +845,9 @@ static int run_moe_seq_split(g5b_engine *e, Layer &w, const float *x, int n, flo
         const float *xg = all + (size_t)g0 * c.hidden;
         router_plan(e->st, e->ridx, e->rw, e->rscore, xg, c.hidden, w.router.w, w.router.dt, w.bias, m, s, e->plan,
                     with_shared ? 1 : 0, e->counter, last ? me * n - g0 : 0, last ? n : 0);
-        if (e->expert_path >= 1 && moe_mma_batch_supported(s, m)) {
-            moe_mma_batch_gateup(e->st, e->act, e->xterms, e->xinv, xg, c.hidden, w.table_dev, e->plan, m, s, e->err_dev);
-            moe_mma_batch_down(e->st, e->contrib, e->act, w.table_dev, e->plan, m, s, e->err_dev);
+        if (e->expert_path >= 1 && tc_moe_takes(e->tc, s, m)) {
+            if (tc_moe_run(e->tc, e->st, e->contrib, e->act, e->xterms, e->xinv, xg, c.hidden, expert_slab(e, w), e->plan, m, s))
+                return fail("the expert kernels could not be launched");
         } else {
             moe_gateup(e->st, e->act, xg, c.hidden, w.table_dev, e->plan, m, s);
             moe_down(e->st, e->contrib, e->act, w.table_dev, e->plan, m, s);
@@ -890,11 +920,10 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
         prof_collect(e, 4);
         return 0;
     }
-    if (e->expert_path >= 1 && (shared_in_plan || !with_shared) && moe_mma_batch_supported(s, n)) {
-        // batches: the tensor-core pipeline with four tokens per weight stage
-        moe_mma_batch_gateup(e->st, e->act, e->xterms, e->xinv, x, c.hidden, w.table_dev, e->plan, n, s, e->err_dev);
-        prof_mark(e, 2);
-        moe_mma_batch_down(e->st, e->contrib, e->act, w.table_dev, e->plan, n, s, e->err_dev);
+    if (e->expert_path >= 1 && (shared_in_plan || !with_shared) && tc_moe_takes(e->tc, s, n)) {
+        if (tc_moe_run(e->tc, e->st, e->contrib, e->act, e->xterms, e->xinv, x, c.hidden, expert_slab(e, w), e->plan, n, s))
+            return fail("the expert kernels could not be launched");
+        prof_mark(e, 2);                          // (gate/up and down are not told apart here)
         prof_mark(e, 3);
     } else {
         moe_gateup(e->st, e->act, x, c.hidden, w.table_dev, e->plan, n, s);
@@ -951,15 +980,14 @@ static void prefetch_beside(g5b_engine *e, const DMat &m)
 // once; the rest (few rows, odd shapes) to the one-token kernel in one launch.
 static int proj_batch(g5b_engine *e, const GemvSeg *segs, int n, int T, bool early)
 {
-    if (T < 8 || !e->tc || e->tensor_gemm == 0) { gemv_batch(e->st, segs, n, T, early); return 0; }
-    tc_gemm_new_input(e->tc);
-    GemvSeg rest[GEMV_MAX_SEG];
-    int nr = 0;
+    if (T < TC_MIN_T || !e->tc || e->tensor_gemm == 0) { gemv_batch(e->st, segs, n, T, early); return 0; }
+    GemvSeg tc[GEMV_MAX_SEG], rest[GEMV_MAX_SEG];
+    int nt = 0, nr = 0;
     for (int i = 0; i < n; i++) {
-        if (tc_gemm_takes(e->tc, segs[i], T)) {
-            if (tc_gemm_run(e->tc, e->st, segs[i], T)) return fail("the tensor-core projection could not be launched");
-        } else rest[nr++] = segs[i];
+        if (tc_gemm_takes(e->tc, segs[i], T)) tc[nt++] = segs[i];
+        else rest[nr++] = segs[i];
     }
+    if (nt && tc_gemm_run(e->tc, e->st, tc, nt, T)) return fail("the tensor-core projection could not be launched");
     if (nr) gemv_batch(e->st, rest, nr, T);
     return 0;
 }
@@ -1201,6 +1229,7 @@ static int check_device_error(g5b_engine *e)
         // the grid-wide counters and tile counters of the interrupted launch are unusable: start over
         cudaMemsetAsync(e->grid_sync, 0, 2 * sizeof(unsigned long long), e->st);
         cudaMemsetAsync(e->tile_done, 0, ((size_t)e->c.hidden / 32 + 1) * sizeof(int), e->st);
+        tc_gemm_recover(e->tc, e->st);
         if (e->ep_arrive) cudaMemsetAsync(e->ep_arrive, 0, sizeof(int), e->st);
         cudaStreamSynchronize(e->st);
         e->grid_launches = 0;

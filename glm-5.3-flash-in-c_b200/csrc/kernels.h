@@ -65,17 +65,17 @@ inline void gemv(cudaStream_t st, const DMat &m, const float *x, int ldx, float 
     gemv_batch(st, &s, 1, T);
 }
 
-// ---- tc_gemm.cu ---------------------------------------------------------------------------
-// FP8 block-scaled (128 x 128 blocks) and BF16 matrices times 8..64 positions on tcgen05 tensor
-// cores, weights streamed once by TMA; activations as exact 16-bit term sums. Segments that share
-// an input reuse its terms within one burst of calls; tc_gemm_new_input forgets them (call it
-// whenever the input buffers get new contents). err: where a bounded wait that ran out is recorded.
+// ---- tc_stream.cu -------------------------------------------------------------------------
+// FP8 block-scaled (128 x 128 blocks) and BF16 matrices times 2..64 positions on tcgen05 tensor
+// cores, weights streamed once by TMA; activations as exact 16-bit term sums. Matrices of one format and
+// width go out in one launch. err: where a bounded wait that ran out is recorded (tc_gemm_recover after it).
+constexpr int TC_TILE_ROWS = 32;          // rows of one expert that a weight tile is multiplied with at once
 struct TcGemm;
 TcGemm *tc_gemm_create(int max_c, int *err);
 void tc_gemm_free(TcGemm *g);
-void tc_gemm_new_input(TcGemm *g);
+void tc_gemm_recover(TcGemm *g, cudaStream_t st);
 bool tc_gemm_takes(const TcGemm *g, const GemvSeg &s, int T);
-int  tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg &s, int T);
+int  tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg *segs, int n, int T);
 
 // ---- elementwise.cu -----------------------------------------------------------------------
 void rms_factor(cudaStream_t st, const float *x, int n, int ld, int rows, float eps, float *inv);
@@ -138,6 +138,8 @@ struct MoePlan {          // device arrays describing which expert multiplies wh
     int *slot_cnt;        // [max_slots] pairs of the slot
     int *pair_tok;        // [max_pairs] activation row of the pair
     int *pair_dst;        // [max_pairs] row of the contribution buffer the pair writes
+    int *slot_tile0;      // [max_slots + 1] first token tile of the slot (tiles of at most TC_TILE_ROWS pairs)
+    int *n_pairs;         // [1] pairs of all slots
     int  max_slots, max_pairs;
 };
 struct MoeShape {
@@ -158,13 +160,17 @@ void moe_mma_gateup(cudaStream_t st, void *act_terms, const float *x, const Expe
 void moe_mma_down(cudaStream_t st, float *out, float *contrib, const void *act_terms, const float *w,
                   const ExpertW *experts, const MoePlan &p, const MoeShape &s, int with_shared, int *tile_done,
                   int *err);
-// Batches of 2..64 tokens on the same pipeline, four tokens per weight stage (moe_mma_batch.cu).
-// xterms: scratch for [T][2][E] F16, xinv: [T] floats. Contributions only; the caller combines.
-bool moe_mma_batch_supported(const MoeShape &s, int T);
-void moe_mma_batch_gateup(cudaStream_t st, void *act_terms, void *xterms, float *xinv, const float *x, int ldx,
-                          const ExpertW *experts, const MoePlan &p, int T, const MoeShape &s, int *err);
-void moe_mma_batch_down(cudaStream_t st, float *contrib, const void *act_terms, const ExpertW *experts,
-                        const MoePlan &p, int T, const MoeShape &s, int *err);
+// Batches: the experts' matrices streamed past the rows that chose them (tc_stream.cu), gate/up with the
+// clamped SwiGLU, then down. act, xterms: scratch for F16 terms [2][max_pairs][I] and [2][max_pairs][E], xinv:
+// [max_pairs]. Contributions only; the caller combines.
+struct ExpertSlab {       // a layer's experts in one allocation: expert i's gate | up | down codes at base + i * stride, `mat` bytes apart
+    const uint8_t *base;   // (then the scales: gate | up | down, scale_gate bytes each for the first two)
+    size_t mat, stride, scale_gate;
+    int count;
+};
+bool tc_moe_takes(const TcGemm *g, const MoeShape &s, int T);
+int  tc_moe_run(TcGemm *g, cudaStream_t st, float *contrib, void *act, void *xterms, float *xinv, const float *x, int ldx,
+                const ExpertSlab &w, const MoePlan &p, int T, const MoeShape &s);
 // The whole batch-1 layer (router, top-k, experts, combine) as one cooperative kernel
 // (moe_decode.cu). `sync` holds two device counters that only grow; `launches` is the host's count of
 // launches so far on them. Returns -1 when the cooperative launch is refused.

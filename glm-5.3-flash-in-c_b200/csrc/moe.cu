@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
 {
     __shared__ int sidx_buf[RT_MAX_TOKENS * G5B_MAX_TOPK];
     __shared__ int cnt[G5B_MAX_EXPERTS], off[G5B_MAX_EXPERTS];
-    __shared__ int psum[RT_WARPS * 32], ssum[RT_WARPS * 32];
+    __shared__ int psum[RT_WARPS * 32], ssum[RT_WARPS * 32], tsum[RT_WARPS * 32];
     __shared__ int is_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int e = blockIdx.x * RT_WARPS + warp, t = blockIdx.y;
@@ -181,28 +181,29 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     }
     __syncthreads();
     const int per = (a.n_local + nth - 1) / nth;              // consecutive experts per thread
-    int pairs = 0, slots = 0;
+    int pairs = 0, slots = 0, tiles = 0;
     for (int k = 0; k < per; k++) {
         const int le = tid * per + k;
-        if (le < a.n_local && cnt[le]) { pairs += cnt[le]; slots++; }
+        if (le < a.n_local && cnt[le]) { pairs += cnt[le]; slots++; tiles += (cnt[le] + TC_TILE_ROWS - 1) / TC_TILE_ROWS; }
     }
-    psum[tid] = pairs; ssum[tid] = slots;
+    psum[tid] = pairs; ssum[tid] = slots; tsum[tid] = tiles;
     __syncthreads();
     for (int o = 1; o < nth; o <<= 1) {                       // inclusive scans over the threads
-        const int pv = tid >= o ? psum[tid - o] : 0, sv = tid >= o ? ssum[tid - o] : 0;
+        const int pv = tid >= o ? psum[tid - o] : 0, sv = tid >= o ? ssum[tid - o] : 0, tv = tid >= o ? tsum[tid - o] : 0;
         __syncthreads();
-        psum[tid] += pv; ssum[tid] += sv;
+        psum[tid] += pv; ssum[tid] += sv; tsum[tid] += tv;
         __syncthreads();
     }
-    int pbase = psum[tid] - pairs, sbase = ssum[tid] - slots;
-    const int total_pairs = psum[nth - 1], total_slots = ssum[nth - 1];
+    int pbase = psum[tid] - pairs, sbase = ssum[tid] - slots, tbase = tsum[tid] - tiles;
+    const int total_pairs = psum[nth - 1], total_slots = ssum[nth - 1], total_tiles = tsum[nth - 1];
     for (int k = 0; k < per; k++) {
         const int le = tid * per + k;
         if (le >= a.n_local) break;
         off[le] = pbase;
         if (cnt[le]) {
             a.p.slot_expert[sbase] = le; a.p.slot_off[sbase] = pbase; a.p.slot_cnt[sbase] = cnt[le];
-            pbase += cnt[le]; sbase++;
+            a.p.slot_tile0[sbase] = tbase;
+            pbase += cnt[le]; sbase++; tbase += (cnt[le] + TC_TILE_ROWS - 1) / TC_TILE_ROWS;
         }
     }
     __syncthreads();
@@ -220,7 +221,12 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
         if (tid == 0) { a.p.slot_expert[total_slots] = a.n_local; a.p.slot_off[total_slots] = total_pairs; a.p.slot_cnt[total_slots] = a.sh_n; }
         for (int tt = tid; tt < a.sh_n; tt += nth) { a.p.pair_tok[total_pairs + tt] = a.sh_t0 + tt; a.p.pair_dst[total_pairs + tt] = n + a.sh_t0 + tt; }
     }
-    if (tid == 0) *a.p.n_slots = total_slots + (shared ? 1 : 0);
+    if (tid == 0) {
+        a.p.slot_tile0[total_slots] = total_tiles;
+        if (shared) a.p.slot_tile0[total_slots + 1] = total_tiles + (a.sh_n + TC_TILE_ROWS - 1) / TC_TILE_ROWS;
+        *a.p.n_slots = total_slots + (shared ? 1 : 0);
+        *a.p.n_pairs = total_pairs + (shared ? a.sh_n : 0);
+    }
 }
 
 // p may be null-planned (p.n_slots == nullptr) when only the routing is wanted.

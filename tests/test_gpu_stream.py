@@ -1,0 +1,49 @@
+"""The tensor-core streaming kernels (csrc/tc_stream.cu) at the sizes where their tiles end: rows of W that do
+not fill a 128-row tile, columns that do not fill a unit (256 FP8 / 128 BF16), 2..64 positions around the multiples
+of 8 and the step from one to two groups of 32 rows, matrices of one unit, and experts with few and with many rows."""
+import numpy as np
+import pytest
+
+import common
+import synth
+
+pkg = synth.pkg
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("hidden,inter", [(128, 128), (384, 256), (1152, 640)])
+def test_projections_at_the_edges_of_tiles(gpu_lib, hidden, inter):
+    """Dense gate (inter x hidden) and down (hidden x inter) in FP8, b_proj (few rows) and o_proj in BF16, against FP64."""
+    c = synth.tiny_spec().cfg.copy()
+    c.n_layers, c.hidden, c.dense_inter, c.kda_heads = 1, hidden, inter, 3
+    spec = synth.Spec(c, [0], [1], with_head=False)
+    tensors = synth.make_model(spec, seed=3, recipe="spread")
+    eng, _ = common.build_models(spec, tensors, 64, oracle=False, options={"allow_partial": 1})
+    rng = np.random.default_rng(4)
+    for name in ("mlp.gate_proj", "mlp.down_proj", "self_attn.q_proj", "self_attn.b_proj", "self_attn.o_proj"):
+        full = f"layers.0.{name}.weight"
+        arr, dt, sc = tensors[full]
+        if dt == pkg.DT_FP8:
+            w = synth.E4M3_TABLE[arr].astype(np.float64) * np.repeat(np.repeat(sc, 128, 0), 128, 1)[:arr.shape[0], :arr.shape[1]]
+        else:
+            w = (arr.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+        x = (rng.standard_normal((64, w.shape[1])) * np.exp2(rng.integers(-8, 9, (64, 1)))).astype(np.float32)
+        for T in (2, 7, 8, 9, 31, 32, 33, 40, 63, 64):
+            got, want = eng.op_matvec(full, x[:T]), x[:T].astype(np.float64) @ w.T
+            scale = np.abs(want).max(axis=1, keepdims=True) + 1e-30
+            assert np.max(np.abs(got - want) / scale) < 2e-6, (name, T)
+    eng.close()
+
+
+@pytest.mark.parametrize("T", [2, 9, 31, 33, 64])
+def test_experts_with_few_and_with_many_rows(gpu_lib, binding, T):
+    """Four experts of which every token takes two and the shared one: slots of up to T rows, cut into tiles of 32."""
+    c = synth.tiny_spec().cfg.copy()
+    c.n_layers, c.n_experts, c.topk, c.moe_inter, c.hidden = 1, 4, 2, 384, 256
+    spec = synth.Spec(c, [0], [0], with_head=False)
+    tensors = synth.make_model(spec, seed=8, recipe="spread")
+    eng, orc = common.build_models(spec, tensors, 64, binding, options={"allow_partial": 1})
+    x = np.random.default_rng(T).standard_normal((T, c.hidden)).astype(np.float32)
+    assert common.rel_err(eng.op_moe(0, x), orc.op_moe(0, x)) < 1e-5
+    assert common.rel_err(eng.op_moe(0, x, False), orc.op_moe(0, x, False)) < 1e-5
+    eng.close(); orc.close()
