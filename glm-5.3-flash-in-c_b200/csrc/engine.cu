@@ -42,7 +42,12 @@ void set_last_error(const char *msg) { snprintf(g_err, sizeof g_err, "%s", msg);
 constexpr size_t EP_FLAG_BYTES = 1024;   // exchange region: the ranks' step words, then the row buffers
 constexpr int EP_HEAD_WORD0 = 64;        // words [64, 64 + 5 x 8): the vocabulary-split head's (value, index) slots of two parities and its arrival counters (up to 8 ranks)
 constexpr int MLA_PART_TOKENS = 4;     // tokens whose attention partial sums are held at once
-constexpr int CHUNK = 64;       // positions one pass of a layer works on (the reference's MoE chunk, glm53f_ops.c:988)
+constexpr int CHUNK = 64;       // positions of a batch step, of a device op, of one pass of the attention core and the head
+                                // (the reference's MoE chunk, glm53f_ops.c:988)
+// Positions one pass of a layer works on: a prompt goes through a layer in passes this long, so that the weights are
+// read once per pass. 2048 positions fill the tensor cores (a routed expert then has about 60 of them) and take 2.3 GB
+// of work buffers at full size; engines with short sessions keep fewer (host ops may still bring that many rows).
+constexpr int PASS_MAX = 2048, PASS_MIN = 256;
 constexpr int TC_MIN_T = 2;     // positions from which the projections go to the tensor cores
 constexpr int PROF_SLOTS = 8;
 
@@ -108,13 +113,15 @@ struct g5b_engine {
     int last_T = 0;                              // positions of the last forward call (rows of mtp_h in use)
     float *enorm = nullptr, *hnorm = nullptr, *head_norm = nullptr;
     DMat eh;
-    float *mtp_h = nullptr;                      // [cap + CHUNK][hidden]: stream means of the positions of the last forward call
-    float *mtp_cat = nullptr, *mtp_x = nullptr;  // [CHUNK][2 hidden], [CHUNK][hidden]
+    float *mtp_h = nullptr;                      // [cap + pass][hidden]: stream means of the positions of the last forward call
+    float *mtp_cat = nullptr, *mtp_x = nullptr;  // [pass][2 hidden], [pass][hidden]
     std::vector<float *> kda_snap;               // speculative decode: per layer, the current sequence's KDA state as it was
     bool snap_first = false;                     // after the first position of the two-position pass in flight
     int seq_split = 0;                           // option "sequence_split": every rank runs its own sequences, MoE layers
                                                  // gather the ranks' tokens and send contribution rows home
     int *ep_arrive = nullptr;
+    int pass = CHUNK;                            // positions one pass of a layer works on
+    int pick0 = 0;                               // first row of the most recent MoE pass's last CHUNK (g5b_engine_last_picks)
     int ep_wait_ms = 5000;                       // wall-clock limit of a wait for the other ranks (option "ep_wait_ms")
     bool dirty = false;                          // a call failed half-way: session state is undefined until reset
     int latent_bf16 = 0, profile = 0, partial = 0, expert_path = 2;
@@ -130,7 +137,7 @@ struct g5b_engine {
     float *norm = nullptr;
     std::vector<void *> owned;
 
-    // work buffers (CHUNK positions)
+    // work buffers (`pass` positions; the attention core's and the head's CHUNK)
     float *h = nullptr; size_t h_tokens = 0;
     int   *ids_dev = nullptr; size_t ids_cap = 0;
     float *inv0, *inv1, *mix, *xc, *xn, *y, *post, *comb;
@@ -714,7 +721,9 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
             if (walloc(e, &w.kda_state, e->n_seq * e->kda_seq)) return -1;
         }
     }
-    const size_t N = CHUNK, E = c.hidden, M = c.hc_mult, MIX = (2 + M) * M;
+    // (the ranks of an expert-parallel group exchange buffers of CHUNK positions)
+    e->pass = e->ep_size > 1 ? CHUNK : e->cap <= PASS_MIN ? PASS_MIN : e->cap >= PASS_MAX ? PASS_MAX : (e->cap + CHUNK - 1) / CHUNK * CHUNK;
+    const size_t N = (size_t)e->pass, NA = CHUNK, E = c.hidden, M = c.hc_mult, MIX = (2 + M) * M;
     const size_t P = (size_t)c.kda_heads * c.kda_head_dim, D = c.kda_head_dim;
     const size_t H = c.mla_heads, KL = c.kv_lora, stride = (size_t)c.index_topk + c.index_kpool;
     const size_t K = c.topk, I = c.moe_inter, SI = (size_t)c.moe_inter * c.n_shared;
@@ -730,11 +739,11 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
     if (walloc(e, &e->mq_raw, N * c.q_lora) || walloc(e, &e->mct, N * KL) || walloc(e, &e->mwk, N * c.index_dim) ||
         walloc(e, &e->mgate, N * c.index_dim) || walloc(e, &e->mwp, N * c.index_heads) ||
         walloc(e, &e->mq, N * H * c.qk_nope) || walloc(e, &e->mqidx, N * (size_t)c.index_heads * c.index_dim) ||
-        walloc(e, &e->mcb, N * H * KL) || walloc(e, &e->macc, N * H * c.v_head) ||
-        walloc(e, &e->mscore, N * ((size_t)e->cap / c.index_kpool + 1)) || walloc(e, &e->minvq, N) ||
-        walloc(e, &e->mqa, N * H * KL) || walloc(e, &e->mdsc, N * H * stride) ||
-        walloc(e, &e->msel, N * stride) || walloc(e, &e->mnsel, N) ||
-        walloc(e, &e->mstats, N * H * 2) || walloc(e, &e->mcount, N * H) ||
+        walloc(e, &e->mcb, NA * H * KL) || walloc(e, &e->macc, N * H * c.v_head) ||
+        walloc(e, &e->mscore, NA * ((size_t)e->cap / c.index_kpool + 1)) || walloc(e, &e->minvq, N) ||
+        walloc(e, &e->mqa, NA * H * KL) || walloc(e, &e->mdsc, NA * H * stride) ||
+        walloc(e, &e->msel, NA * stride) || walloc(e, &e->mnsel, NA) ||
+        walloc(e, &e->mstats, NA * H * 2) || walloc(e, &e->mcount, NA * H) ||
         walloc(e, &e->mpart, (size_t)MLA_PART_TOKENS * H * ((stride + 31) / 32) * KL)) return -1;
     e->mpart_bytes = (size_t)MLA_PART_TOKENS * H * ((stride + 31) / 32) * KL * sizeof(double);
     const size_t pairs = N * K + N;
@@ -757,8 +766,8 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         e->err_host = hp;
         CU(cudaHostGetDevicePointer((void **)&e->err_dev, hp, 0));
     }
-    if (walloc(e, &e->xm, N * E) || walloc(e, &e->inv_head, N) || walloc(e, &e->logits, N * (size_t)c.vocab) ||
-        walloc(e, &e->am_v, N * 64) || walloc(e, &e->am_i, N * 64) || walloc(e, &e->am_out, (size_t)e->cap + N) ||
+    if (walloc(e, &e->xm, NA * E) || walloc(e, &e->inv_head, NA) || walloc(e, &e->logits, NA * (size_t)c.vocab) ||
+        walloc(e, &e->am_v, NA * 64) || walloc(e, &e->am_i, NA * 64) || walloc(e, &e->am_out, (size_t)e->cap + NA) ||
         e->dalloc(&e->sample_buf, sample_scratch_bytes(c.vocab))) return -1;
     if (e->mtp && (walloc(e, &e->mtp_h, ((size_t)e->cap + N) * E) || walloc(e, &e->mtp_cat, N * 2 * E) ||
                    walloc(e, &e->mtp_x, N * E))) return -1;
@@ -768,7 +777,7 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         int max_c = e->mtp ? 2 * c.hidden : c.hidden;
         for (int v : {P, c.q_lora, c.kv_lora, c.kda_head_dim, c.mla_heads * c.v_head}) max_c = v > max_c ? v : max_c;
         for (int v : {c.dense_inter, c.moe_inter * c.n_shared}) max_c = v > max_c ? v : max_c;
-        e->tc = tc_gemm_create(max_c, e->err_dev);
+        e->tc = tc_gemm_create(max_c, e->pass, e->err_dev);
         if (!e->tc) return fail("the tensor-core projection path could not be set up (tensor-map encoder or scratch)");
     }
     e->cached_seq.assign((size_t)e->n_seq, 0);
@@ -871,6 +880,7 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
     if (e->ep_size > 1 && !e->ep_connected)
         return fail("expert-parallel engine: connect the ranks (g5b_engine_ep_connect) before running a MoE layer");
     const MoeShape s = moe_shape(e, w);
+    e->pick0 = (n - 1) / CHUNK * CHUNK;
     if (e->seq_split && e->ep_size > 1) return run_moe_seq_split(e, w, x, n, out, with_shared, s);
     const bool shared_in_plan = with_shared && c.n_shared == 1 && w.sh_gate.dt == s.dt;
     const bool one_gpu_decode = e->ep_size == 1 && (shared_in_plan || !with_shared);
@@ -1033,7 +1043,7 @@ static int run_kda(g5b_engine *e, Layer &w, const float *x, int n, float *out, b
         return fail("this layer's KDA weights were not loaded");
     const bool ts = kda_heads_split(e, w);
     const int Hl = ts ? H / e->ep_size : H, h0 = ts ? e->ep_rank * Hl : 0, Pl = Hl * D, p0 = h0 * D;
-    float *lrf = e->klr, *lrg = e->klr + (size_t)CHUNK * D;
+    float *lrf = e->klr, *lrg = e->klr + (size_t)e->pass * D;
     GemvSeg a[6] = {make_seg(row_slice(w.kq, p0, Pl), x, E, e->kq + p0, P), make_seg(row_slice(w.kk, p0, Pl), x, E, e->kk + p0, P),
                     make_seg(row_slice(w.kv, p0, Pl), x, E, e->kv + p0, P), make_seg(row_slice(w.kb, h0, Hl), x, E, e->kbraw + h0, H),
                     make_seg(w.f_a, x, E, lrf, D), make_seg(w.g_a, x, E, lrg, D)};
@@ -1137,25 +1147,30 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
     GemvSeg b[2] = {make_seg(qb, e->mq_raw, c.q_lora, e->mq, Hl * c.qk_nope, e->minvq, w.q_a_norm),
                     make_seg(w.wq_b, e->mq_raw, c.q_lora, e->mqidx, c.index_heads * c.index_dim, e->minvq, w.q_a_norm)};
     if (proj_batch(e, b, 2, n, true)) return -1;
+    // The attention core takes CHUNK positions at a time.
     // The indexer (pool scores, top-k, expansion: two latency-bound kernels) and the absorption of
     // W_k into the query need nothing from each other: the absorption runs on the side stream
     // meanwhile and the main stream takes it back before the scores.
-    bool forked = false, join = false;
-    if (e->side && e->side_ev && e->side_done && cudaEventRecord(e->side_ev, e->st) == cudaSuccess &&
-        cudaStreamWaitEvent(e->side, e->side_ev, 0) == cudaSuccess) {
-        mla_absorb(e->side, e->mqa, e->mq, kvb, n, sl);
-        forked = true;
-        join = cudaEventRecord(e->side_done, e->side) == cudaSuccess;
-        if (!join) cudaStreamSynchronize(e->side);
+    for (int t0 = 0; t0 < n; t0 += CHUNK) {
+        const int nt = n - t0 < CHUNK ? n - t0 : CHUNK, at = batch ? cached : cached + t0;
+        const float *mq = e->mq + (size_t)t0 * Hl * c.qk_nope;
+        bool forked = false, join = false;
+        if (e->side && e->side_ev && e->side_done && cudaEventRecord(e->side_ev, e->st) == cudaSuccess &&
+            cudaStreamWaitEvent(e->side, e->side_ev, 0) == cudaSuccess) {
+            mla_absorb(e->side, e->mqa, mq, kvb, nt, sl);
+            forked = true;
+            join = cudaEventRecord(e->side_done, e->side) == cudaSuccess;
+            if (!join) cudaStreamSynchronize(e->side);
+        }
+        dsa_select(e->st, e->msel, e->mnsel, ist, e->mqidx + (size_t)t0 * c.index_heads * c.index_dim, e->mwp + (size_t)t0 * c.index_heads, e->mscore, nt, at, s);
+        if (!forked) mla_absorb(e->st, e->mqa, mq, kvb, nt, sl);
+        else if (join && cudaStreamWaitEvent(e->st, e->side_done, 0) != cudaSuccess) cudaStreamSynchronize(e->side);
+        if (flash)
+            mla_attend_flash(e->st, e->mcb, e->mqa, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf);
+        else
+            mla_attend(e->st, e->mcb, e->mqa, lat, e->msel, e->mnsel, e->mdsc, e->mpart, e->mstats, e->mcount, MLA_PART_TOKENS, nt, at, sl);
+        mla_vout(e->st, e->macc + (size_t)t0 * Hl * c.v_head, e->mcb, kvb, nt, sl);
     }
-    dsa_select(e->st, e->msel, e->mnsel, ist, e->mqidx, e->mwp, e->mscore, n, cached, s);
-    if (!forked) mla_absorb(e->st, e->mqa, e->mq, kvb, n, sl);
-    else if (join && cudaStreamWaitEvent(e->st, e->side_done, 0) != cudaSuccess) cudaStreamSynchronize(e->side);
-    if (flash)
-        mla_attend_flash(e->st, e->mcb, e->mqa, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, n, cached, sf);
-    else
-        mla_attend(e->st, e->mcb, e->mqa, lat, e->msel, e->mnsel, e->mdsc, e->mpart, e->mstats, e->mcount, MLA_PART_TOKENS, n, cached, sl);
-    mla_vout(e->st, e->macc, e->mcb, kvb, n, sl);
     if (ms) {
         GemvSeg o = make_seg(col_slice(w.mo, h0 * s.vh, Hl * s.vh), e->macc, Hl * c.v_head, e->ts_part, E);
         if (proj_batch(e, &o, 1, n, true)) return -1;
@@ -1186,7 +1201,7 @@ static void flush_hc_post(g5b_engine *e)
     e->post_h = nullptr;
 }
 
-// One decoder layer over n <= CHUNK positions (reference: glm53f_decoder_layer,
+// One decoder layer over n <= e->pass positions (reference: glm53f_decoder_layer,
 // src/core/glm53f_ops.c:1400-1433).
 static int run_layer(g5b_engine *e, int l, float *h, int n, int cached, bool batch = false)
 {
@@ -1279,14 +1294,14 @@ static int forward_device(g5b_engine *e, const int *ids_dev, int T, bool all_pos
     e->post_h = nullptr;                              // nothing is owed from a call that failed half-way
     embed_rows(e->st, e->h, e->embed, ids_dev, T, M);
     for (int l = 0; l < c.n_layers; l++)
-        for (int t0 = 0; t0 < T; t0 += CHUNK) {
-            const int n = T - t0 < CHUNK ? T - t0 : CHUNK;
+        for (int t0 = 0; t0 < T; t0 += e->pass) {
+            const int n = T - t0 < e->pass ? T - t0 : e->pass;
             if (run_layer(e, l, e->h + (size_t)t0 * M * E, n, batch ? e->cached : e->cached + t0, batch)) return -1;
         }
     flush_hc_post(e);
     // with the MTP layer open every position's stream mean is kept, row t of this call
     // (src/model/glm53f_model.c:460-468)
-    if (e->mtp && (size_t)T <= (size_t)e->cap + CHUNK) { head_mean(e->st, e->mtp_h, e->h, T, M, E); e->last_T = T; }
+    if (e->mtp && (size_t)T <= (size_t)e->cap + e->pass) { head_mean(e->st, e->mtp_h, e->h, T, M, E); e->last_T = T; }
     const int first = all_positions ? 0 : T - 1;
     for (int t0 = first; t0 < T; t0 += CHUNK) {
         const int n = T - t0 < CHUNK ? T - t0 : CHUNK;
@@ -1603,14 +1618,14 @@ struct Staged {
     }
 };
 
-// Ops accept any T >= 1: the host entry points walk it in CHUNK-sized pieces.
+// Ops accept any T >= 1: the host entry points walk it in pieces of e->pass rows.
 static int check_op(g5b_engine *e, int layer, int T)
 {
     if (T < 1) return fail("ops take at least one position, got %d", T);
     return check_layer(e, layer, 1);
 }
 
-#define FOR_CHUNKS(T) for (int t0 = 0, n_ = 0; (n_ = (T) - t0 < CHUNK ? (T) - t0 : CHUNK), t0 < (T); t0 += CHUNK)
+#define FOR_CHUNKS(T) for (int t0 = 0, n_ = 0; (n_ = (T) - t0 < e->pass ? (T) - t0 : e->pass), t0 < (T); t0 += e->pass)
 
 // glm53f_mtp_feed (src/model/glm53f_mtp.c:100-144) on the MTP layer's own caches and position
 // count: x = eh_proj([RMSNorm(embed(next), enorm), RMSNorm(h, hnorm)]); x += MLA(RMSNorm(x,
@@ -1626,7 +1641,7 @@ static int mtp_feed_rows(g5b_engine *e, const float *h, const float *h_dev, cons
     const int E = c.hidden;
     if (T < 1) return fail("mtp_feed needs at least one position");
     if (e->mtp_cached + T > e->cap) return fail("%d + %d MTP positions exceed the capacity %d", e->mtp_cached, T, e->cap);
-    if (!h && T > e->cap + CHUNK) return fail("no kept hidden states for %d positions", T);
+    if (!h && T > e->cap + e->pass) return fail("no kept hidden states for %d positions", T);
     for (int t = 0; t < T; t++)
         if (next_ids[t] < 0 || next_ids[t] >= c.vocab) return fail("token id %d outside the vocabulary", next_ids[t]);
     if (!e->embed.loaded() || !e->lm_head.loaded() || !e->eh.loaded() || !e->enorm || !e->hnorm || !e->head_norm)
@@ -1646,8 +1661,8 @@ static int mtp_feed_rows(g5b_engine *e, const float *h, const float *h_dev, cons
         if (!xo) return fail("out of device memory");
     }
     e->post_h = nullptr;
-    for (int t0 = 0; t0 < T; t0 += CHUNK) {
-        const int n = T - t0 < CHUNK ? T - t0 : CHUNK;
+    for (int t0 = 0; t0 < T; t0 += e->pass) {
+        const int n = T - t0 < e->pass ? T - t0 : e->pass;
         float *cat = e->mtp_cat, *x = e->mtp_x;
         embed_rows(e->st, cat, e->embed, e->ids_dev + t0, n, 2);                 // both halves; the second is replaced
         CU(cudaMemcpy2DAsync(cat + E, (size_t)2 * E * 4, hd + (size_t)t0 * E, (size_t)E * 4, (size_t)E * 4, (size_t)n,
@@ -1770,7 +1785,7 @@ extern "C" int g5b_mtp_feed(g5b_engine *e, const float *h, const int *next_ids, 
 extern "C" int g5b_mtp_hidden(g5b_engine *e, int first, int T, float *dst)
 {
     if (!e || !e->finalized || !e->mtp) return fail("the MTP layer is not enabled");
-    if (first < 0 || T < 1 || first + T > e->cap + CHUNK) return fail("rows outside the kept hidden states");
+    if (first < 0 || T < 1 || first + T > e->cap + e->pass) return fail("rows outside the kept hidden states");
     CU(cudaSetDevice(e->device));
     CU(cudaMemcpyAsync(dst, e->mtp_h + (size_t)first * e->c.hidden, (size_t)T * e->c.hidden * 4, cudaMemcpyDeviceToHost, e->st));
     CU(cudaStreamSynchronize(e->st));
@@ -1849,8 +1864,9 @@ extern "C" int g5b_engine_last_picks(g5b_engine *e, int T, int *idx, float *w)
     if (T < 1 || T > CHUNK) return fail("last_picks covers 1..%d positions", CHUNK);
     CU(cudaSetDevice(e->device));
     const size_t n = (size_t)T * e->c.topk;
-    if (idx) CU(cudaMemcpyAsync(idx, e->ridx, n * 4, cudaMemcpyDeviceToHost, e->st));
-    if (w)   CU(cudaMemcpyAsync(w, e->rw, n * 4, cudaMemcpyDeviceToHost, e->st));
+    const size_t at = (size_t)e->pick0 * e->c.topk;
+    if (idx) CU(cudaMemcpyAsync(idx, e->ridx + at, n * 4, cudaMemcpyDeviceToHost, e->st));
+    if (w)   CU(cudaMemcpyAsync(w, e->rw + at, n * 4, cudaMemcpyDeviceToHost, e->st));
     CU(cudaStreamSynchronize(e->st));
     return 0;
 }
@@ -1885,11 +1901,11 @@ extern "C" int g5b_op_mla(g5b_engine *e, int layer, const float *x, int T, int c
         })) return -1;
     if (n_sel_out) {
         int ns = 0;
-        CU(cudaMemcpyAsync(&ns, e->mnsel + last_n - 1, 4, cudaMemcpyDeviceToHost, e->st));
+        CU(cudaMemcpyAsync(&ns, e->mnsel + (last_n - 1) % CHUNK, 4, cudaMemcpyDeviceToHost, e->st));
         CU(cudaStreamSynchronize(e->st));
         *n_sel_out = ns;
         if (sel_out && ns > 0) {
-            CU(cudaMemcpyAsync(sel_out, e->msel + (size_t)(last_n - 1) * (e->c.index_topk + e->c.index_kpool),
+            CU(cudaMemcpyAsync(sel_out, e->msel + (size_t)((last_n - 1) % CHUNK) * (e->c.index_topk + e->c.index_kpool),
                                (size_t)ns * 4, cudaMemcpyDeviceToHost, e->st));
             CU(cudaStreamSynchronize(e->st));
         }

@@ -66,12 +66,12 @@ inline void gemv(cudaStream_t st, const DMat &m, const float *x, int ldx, float 
 }
 
 // ---- tc_stream.cu -------------------------------------------------------------------------
-// FP8 block-scaled (128 x 128 blocks) and BF16 matrices times 2..64 positions on tcgen05 tensor
+// FP8 block-scaled (128 x 128 blocks) and BF16 matrices times 2 positions or more on tcgen05 tensor
 // cores, weights streamed once by TMA; activations as exact 16-bit term sums. Matrices of one format and
 // width go out in one launch. err: where a bounded wait that ran out is recorded (tc_gemm_recover after it).
 constexpr int TC_TILE_ROWS = 32;          // rows of one expert that a weight tile is multiplied with at once
 struct TcGemm;
-TcGemm *tc_gemm_create(int max_c, int *err);
+TcGemm *tc_gemm_create(int max_c, int max_t, int *err);      // widest input, most positions
 void tc_gemm_free(TcGemm *g);
 void tc_gemm_recover(TcGemm *g, cudaStream_t st);
 bool tc_gemm_takes(const TcGemm *g, const GemvSeg &s, int T);

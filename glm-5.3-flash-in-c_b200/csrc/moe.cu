@@ -229,14 +229,73 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     }
 }
 
+// The same grouping for more tokens than one router launch takes: one CTA, the expert ids read from memory.
+constexpr int PLAN_THREADS = 1024;
+__global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, int T, int K, int n_local0, int n_local, int with_shared, MoePlan p)
+{
+    __shared__ int cnt[G5B_MAX_EXPERTS], off[G5B_MAX_EXPERTS];
+    __shared__ int wsum[3][PLAN_THREADS / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = T * K;
+    cnt[tid] = 0;
+    __syncthreads();
+    for (int i = tid; i < n; i += PLAN_THREADS) {
+        const int le = idx[i] - n_local0;
+        if (le >= 0 && le < n_local) atomicAdd(&cnt[le], 1);
+    }
+    __syncthreads();
+    const int mine = tid < n_local ? cnt[tid] : 0;            // one expert per thread (at most G5B_MAX_EXPERTS of them)
+    int v[3] = {mine, mine > 0, (mine + TC_TILE_ROWS - 1) / TC_TILE_ROWS}, own[3];
+    for (int k = 0; k < 3; k++) {
+        own[k] = v[k];
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v[k], o); if (lane >= o) v[k] += u; }
+        if (lane == 31) wsum[k][warp] = v[k];
+    }
+    __syncthreads();
+    int total[3];
+    for (int k = 0; k < 3; k++) {
+        int before = 0, all = 0;
+        for (int w = 0; w < PLAN_THREADS / 32; w++) { if (w < warp) before += wsum[k][w]; all += wsum[k][w]; }
+        v[k] += before - own[k];                              // exclusive
+        total[k] = all;
+    }
+    if (mine) {
+        p.slot_expert[v[1]] = tid; p.slot_off[v[1]] = v[0]; p.slot_cnt[v[1]] = mine; p.slot_tile0[v[1]] = v[2];
+    }
+    off[tid] = v[0];
+    __syncthreads();
+    cnt[tid] = 0;                                             // reused as the write cursor of each expert
+    __syncthreads();
+    for (int i = tid; i < n; i += PLAN_THREADS) {
+        const int le = idx[i] - n_local0;
+        if (le < 0 || le >= n_local) continue;
+        const int pos = off[le] + atomicAdd(&cnt[le], 1);
+        p.pair_tok[pos] = i / K;
+        p.pair_dst[pos] = i;
+    }
+    if (with_shared)
+        for (int t = tid; t < T; t += PLAN_THREADS) { p.pair_tok[total[0] + t] = t; p.pair_dst[total[0] + t] = n + t; }
+    if (tid == 0) {
+        if (with_shared) { p.slot_expert[total[1]] = n_local; p.slot_off[total[1]] = total[0]; p.slot_cnt[total[1]] = T; }
+        p.slot_tile0[total[1]] = total[2];
+        if (with_shared) p.slot_tile0[total[1] + 1] = total[2] + (T + TC_TILE_ROWS - 1) / TC_TILE_ROWS;
+        *p.n_slots = total[1] + (with_shared ? 1 : 0);
+        *p.n_pairs = total[0] + (with_shared ? T : 0);
+    }
+}
+
 // p may be null-planned (p.n_slots == nullptr) when only the routing is wanted.
 void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float *x, int ldx, const void *gate,
                  int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &p, int with_shared,
                  int *counter, int shared_t0, int shared_n)
 {
-    RouterArgs a{idx, w, score, x, ldx, gate, gate_dt, bias, s.NE, s.E, s.K, T, s.norm_topk, s.routed_scale,
-                 p, s.n_local0, s.n_local, with_shared, counter, shared_t0, shared_n < 0 ? T : shared_n};
-    G5B_LAUNCH(router_kernel, dim3((s.NE + RT_WARPS - 1) / RT_WARPS, T), RT_WARPS * 32, 0, st, a);
+    const bool one = T <= RT_MAX_TOKENS;
+    for (int t0 = 0; t0 < T; t0 += RT_MAX_TOKENS) {
+        const int n = T - t0 < RT_MAX_TOKENS ? T - t0 : RT_MAX_TOKENS;
+        RouterArgs a{idx + (size_t)t0 * s.K, w + (size_t)t0 * s.K, score + (size_t)t0 * s.NE, x + (size_t)t0 * ldx, ldx, gate, gate_dt, bias, s.NE, s.E, s.K, n,
+                     s.norm_topk, s.routed_scale, one ? p : MoePlan{}, s.n_local0, s.n_local, with_shared, counter, shared_t0, shared_n < 0 ? n : shared_n};
+        G5B_LAUNCH(router_kernel, dim3((s.NE + RT_WARPS - 1) / RT_WARPS, n), RT_WARPS * 32, 0, st, a);
+    }
+    if (!one && p.n_slots) G5B_LAUNCH(moe_plan_kernel, 1, PLAN_THREADS, 0, st, idx, T, s.K, s.n_local0, s.n_local, with_shared, p);
 }
 
 // ----------------------------------------------------------------- experts ----

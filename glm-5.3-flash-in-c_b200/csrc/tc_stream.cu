@@ -64,7 +64,8 @@ struct TsArgs {
     int n_seg, tiles;          // projections: tiles of all matrices
     int KB;                    // units per tile
     int blocks;                // FP8: 128-column blocks per row (2 KB, or one less)
-    int T, n, plane;           // rows, rows rounded up to 8; rows between the terms' planes
+    int T, n, plane;           // rows, rows of the largest tile (a multiple of 8); rows between the terms' planes
+    int nt;                    // projections: tiles of n rows that T rows make
     // experts
     const uint8_t *scales;     // expert 0's scales of the matrix (gate/up: of the gate); the up projection's lie up_off on
     size_t scale_stride, up_off;
@@ -93,12 +94,19 @@ struct TsPlan { const int *tile0, *off, *cnt, *exp; int slots; };
 template <int MODE>
 struct TsCursor {
     int which, rt, row0, np, n;
-    int slot, tt, nt, rows, cnt;
+    int slot, tt, nt, rows, cnt;               // (projections: row0 = the matrix's first terms row + tt * n)
     __device__ __forceinline__ void rows_of_tile(const TsPlan &p)
     {
         const int left = cnt - tt * rows;
         row0 = p.off[slot] + tt * rows;
         np = left < rows ? left : rows;
+        n = (np + 7) & ~7;
+    }
+    __device__ __forceinline__ void columns(const TsArgs &a)
+    {
+        const int left = a.T - tt * a.n;
+        row0 = a.seg[which].xrow + tt * a.n;
+        np = left < a.n ? left : a.n;
         n = (np + 7) & ~7;
     }
     __device__ __forceinline__ void enter(const TsPlan &p)
@@ -110,7 +118,9 @@ struct TsCursor {
         if (MODE == TS_DENSE) {
             which = 0;
             for (int i = 1; i < a.n_seg; i++) if (tile >= a.seg[i].tile0) which = i;
-            rt = tile - a.seg[which].tile0; row0 = a.seg[which].xrow; np = a.T; n = a.n;
+            const int local = tile - a.seg[which].tile0;
+            rt = local / a.nt; tt = local - rt * a.nt;
+            columns(a);
         } else {
             int lo = 0, hi = p.slots - 1;                     // the last slot whose first tile is not beyond this one
             while (lo < hi) { const int mid = (lo + hi + 1) >> 1; if (p.tile0[mid] * a.RT <= tile) lo = mid; else hi = mid - 1; }
@@ -124,8 +134,9 @@ struct TsCursor {
     __device__ __forceinline__ void next(const TsArgs &a, const TsPlan &p)      // (may step past the last tile: not used then)
     {
         if (MODE == TS_DENSE) {
-            rt++;
-            if (which + 1 < a.n_seg && rt == a.seg[which + 1].tile0 - a.seg[which].tile0) { which++; rt = 0; row0 = a.seg[which].xrow; }
+            if (++tt == a.nt) { tt = 0; rt++; }
+            if (tt == 0 && which + 1 < a.n_seg && rt * a.nt == a.seg[which + 1].tile0 - a.seg[which].tile0) { which++; rt = 0; }
+            columns(a);
         } else {
             if (++tt == nt) { tt = 0; rt++; }
             if (rt == a.RT) {
@@ -157,7 +168,7 @@ struct TsEpi {
             dst0 = lane < t.np ? __ldcg(a.p.pair_dst + t.row0 + lane) : 0;
             dst1 = lane + 32 < t.np ? __ldcg(a.p.pair_dst + t.row0 + lane + 32) : 0;
         } else {
-            const float *iv = MODE == TS_DENSE ? a.seg[t.which].inv : a.xinv + t.row0;
+            const float *iv = MODE == TS_DENSE ? a.seg[t.which].inv + t.tt * a.n : a.xinv + t.row0;
             inv0 = lane < t.np ? __ldcg(iv + lane) : 0.f;
             inv1 = lane + 32 < t.np ? __ldcg(iv + lane + 32) : 0.f;
         }
@@ -178,7 +189,7 @@ __device__ __forceinline__ void ts_store(const TsArgs &a, const TsCursor<MODE> &
     if (MODE == TS_DENSE) {
         const TsSeg &sg = a.seg[t.which];
         const int c = tid & 127;
-        float *y = sg.y + t.rt * 128 + c;
+        float *y = sg.y + (size_t)t.tt * a.n * sg.ldy + t.rt * 128 + c;
         const bool live = t.rt * 128 + c < sg.R;              // (rows of a ragged last tile beyond R do not exist)
 #pragma unroll 2
         for (int r = r0 + (tid >> 7); r < r0 + nr; r += 2) {
@@ -600,9 +611,8 @@ __global__ void __launch_bounds__(TS_BF16_THREADS, 1) tc_stream_bf16_kernel(cons
     } else if (warp == 9) {
         if (elect_one()) {
             int s = 0, fp = 0, c = 0;
-            const int N = (3 * a.n + 15) & ~15;
-            const uint32_t idesc = tc_idesc(1, N);
             TS_WALK(t, {
+                const uint32_t idesc = tc_idesc(1, (3 * t.n + 15) & ~15);
                 for (int kb = kb0; kb < kb1; kb++) {
                     const bool fresh = kb == kb0 || kb % TS_SEG_UNITS == 0;
                     if (fresh && c >= 2 && !(ok = mbar_wait(&acc_empty[c & 1], (uint32_t)(c / 2 - 1) & 1, a.err, 44))) break;
@@ -624,11 +634,11 @@ __global__ void __launch_bounds__(TS_BF16_THREADS, 1) tc_stream_bf16_kernel(cons
         __syncwarp();
     } else {
         const int quarter = warp & 3, eg = warp >> 2, e0 = eg * TS_EN, row = quarter * 32 + lane;
-        const int np = a.T - e0 < 0 ? 0 : a.T - e0 < TS_EN ? a.T - e0 : TS_EN;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
         const TsEpi<false, MODE> ep{};
         int c = 0;
         TS_WALK(t, {
+            const int np = t.np - e0 < 0 ? 0 : t.np - e0 < TS_EN ? t.np - e0 : TS_EN;
             float acc[TS_EN];
 #pragma unroll
             for (int i = 0; i < TS_EN; i++) acc[i] = 0.f;
@@ -784,11 +794,12 @@ bool tc_encode(CUtensorMap *m, const void *base, CUtensorMapDataType dt, int elt
 }
 
 struct TcGemm {
-    void *terms = nullptr;          // [2 inputs][3 terms][64][max_c] 16-bit
-    float *inv = nullptr;           // [2][64]
+    void *terms = nullptr;          // 16-bit values: [inputs][terms][plane][columns]
+    size_t terms_n = 0;             // how many fit
+    float *inv = nullptr;           // [2][plane]
     float *part = nullptr;          // partial results of the CTAs
     int *cnt = nullptr;             // units done per tile
-    int max_c = 0, ctas = 0;
+    int max_c = 0, max_t = 0, ctas = 0;
     int *err = nullptr;
     // maps by (pointer, kind, rows, columns, pitch or inputs, box)
     std::map<std::tuple<const void *, int, size_t, size_t, size_t, int>, CUtensorMap> maps;
@@ -796,19 +807,21 @@ struct TcGemm {
 };
 constexpr int TS_CNT = 1 << 16;     // tiles of one launch at most
 
-TcGemm *tc_gemm_create(int max_c, int *err)
+TcGemm *tc_gemm_create(int max_c, int max_t, int *err)
 {
     if (!encode_fn()) return nullptr;
     TcGemm *g = new TcGemm;
     g->max_c = max_c; g->err = err; g->ctas = dev_sms();
-    if (cudaMalloc(&g->terms, (size_t)2 * 3 * TS_N * max_c * 2) != cudaSuccess || cudaMalloc((void **)&g->inv, 2 * TS_N * 4) != cudaSuccess ||
+    g->max_t = max_t > TS_N ? max_t : TS_N;
+    g->terms_n = (size_t)3 * (g->max_t > 2 * TS_N ? g->max_t : 2 * TS_N) * max_c;
+    if (cudaMalloc(&g->terms, g->terms_n * 2) != cudaSuccess || cudaMalloc((void **)&g->inv, (size_t)2 * g->max_t * 4) != cudaSuccess ||
         cudaMalloc((void **)&g->part, (size_t)g->ctas * 2 * TS_N * 128 * 4) != cudaSuccess ||
         cudaMalloc((void **)&g->cnt, TS_CNT * 4) != cudaSuccess) {
         cudaGetLastError();
         tc_gemm_free(g);
         return nullptr;
     }
-    cudaMemset(g->terms, 0, (size_t)2 * 3 * TS_N * max_c * 2);
+    cudaMemset(g->terms, 0, g->terms_n * 2);
     cudaMemset(g->cnt, 0, TS_CNT * 4);
     cudaStreamSynchronize(nullptr);      // the engine's streams do not wait for the default stream
     return g;
@@ -894,10 +907,10 @@ static SmemGrant grant_dense, grant_gateup, grant_down, grant_bf16;
 
 bool tc_gemm_takes(const TcGemm *g, const GemvSeg &s, int T)
 {
-    if (!g || T < 2 || T > TS_N || s.C > g->max_c || s.R < 16) return false;
+    if (!g || T < 2 || T > g->max_t || s.C > g->max_c || s.R < 16) return false;
     if ((reinterpret_cast<uintptr_t>(s.W) & 15) || (((size_t)s.ldw * (s.dt == DT_FP8 ? 1 : 2)) & 15)) return false;
     if ((reinterpret_cast<uintptr_t>(s.x) & 15) || (s.ldx & 3) || (s.xw && (reinterpret_cast<uintptr_t>(s.xw) & 15))) return false;
-    if ((s.R + 127) / 128 > TS_CNT / TS_MAX_SEG) return false;
+    if ((s.R + 127) / 128 * ((T + 31) / 32) > TS_CNT / TS_MAX_SEG) return false;
     if (s.dt == DT_FP8) return s.C % 128 == 0 && s.br == 128 && s.bc == 128 && s.S != nullptr;
     if (s.dt == DT_BF16) return s.C % 64 == 0;
     return false;
@@ -915,23 +928,25 @@ int tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg *segs, int n, int T)
         TsArgs a{};
         TsSplit sp{};
         int ins = 0;
-        a.T = T; a.n = (T + 7) & ~7; a.plane = TS_N; a.KB = (C + (fp8 ? 255 : 127)) / (fp8 ? 256 : 128); a.blocks = C / 128;
+        const int plane = T <= TS_N ? TS_N : g->max_t;         // (two layouts only: the maps are kept)
+        const int most = fp8 && T > TS_N ? TS_EN : TS_N;        // rows per tile
+        a.T = T; a.n = T < most ? (T + 7) & ~7 : most; a.nt = (T + a.n - 1) / a.n; a.plane = plane; a.KB = (C + (fp8 ? 255 : 127)) / (fp8 ? 256 : 128); a.blocks = C / 128;
         for (int i = first; i < n && a.n_seg < TS_MAX_SEG; i++) {
             const GemvSeg &s = segs[i];
             if (done[i] || (s.dt == DT_FP8) != fp8 || s.C != C) continue;
             int k = 0;
             while (k < ins && !(sp.in[k].x == s.x && sp.in[k].xinv == s.xinv && sp.in[k].xw == s.xw && sp.in[k].ldx == s.ldx)) k++;
-            if (k == 2) continue;
+            if (k == 2 || (size_t)(k + 1) * terms * plane * C > g->terms_n) continue;
             if (k == ins) sp.in[ins++] = TsSplitIn{s.x, s.xinv, s.xw, s.ldx};
             const CUtensorMap *w = w_map(g, s.W, fp8, (size_t)s.R, (size_t)C, (size_t)s.ldw);
             if (!w) return -1;
             m.w[a.n_seg] = *w;
-            a.seg[a.n_seg++] = TsSeg{s.S, g->inv + k * TS_N, s.y, s.scols, s.R, s.ldy, a.tiles, k * terms * TS_N};
-            a.tiles += (s.R + 127) / 128;
+            a.seg[a.n_seg++] = TsSeg{s.S, g->inv + (size_t)k * plane, s.y, s.scols, s.R, s.ldy, a.tiles, k * terms * plane};
+            a.tiles += (s.R + 127) / 128 * a.nt;
             done[i] = true;
         }
-        if (!x_maps(g, m, g->terms, fp8, TS_N, (size_t)C, 2)) return -1;
-        sp.terms = g->terms; sp.inv = g->inv; sp.C = C; sp.plane = TS_N;
+        if (!x_maps(g, m, g->terms, fp8, (size_t)plane, (size_t)C, ins)) return -1;
+        sp.terms = g->terms; sp.inv = g->inv; sp.C = C; sp.plane = plane;
         if (fp8) G5B_LAUNCH_PDL(tc_split_kernel<true>, dim3(T, ins), dim3(512), 0, st, sp);
         else     G5B_LAUNCH_PDL(tc_split_kernel<false>, dim3(T, ins), dim3(512), 0, st, sp);
         a.part = g->part; a.cnt = g->cnt; a.err = g->err;
@@ -948,7 +963,7 @@ int tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg *segs, int n, int T)
 // ------------------------------------------------------------------ routed experts ----
 bool tc_moe_takes(const TcGemm *g, const MoeShape &s, int T)
 {
-    if (!g || T < 1 || T > TS_N || s.dt != DT_FP8 || s.br != 128 || s.bc != 128 || s.E % 128 || s.I % 128) return false;
+    if (!g || T < 1 || T > g->max_t || s.dt != DT_FP8 || s.br != 128 || s.bc != 128 || s.E % 128 || s.I % 128) return false;
     if (!(s.limit > 0.f) || s.limit * s.limit > 60000.f) return false;                  // activations must fit F16
     const int slots = (T * s.K < s.n_local ? T * s.K : s.n_local) + 1;
     return (long)(slots + (T * s.K + T) / TC_TILE_ROWS) * (s.I / 64 > s.E / 128 ? s.I / 64 : s.E / 128) <= TS_CNT;

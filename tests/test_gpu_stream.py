@@ -35,7 +35,7 @@ def test_projections_at_the_edges_of_tiles(gpu_lib, hidden, inter):
     eng.close()
 
 
-@pytest.mark.parametrize("T", [2, 9, 31, 33, 64])
+@pytest.mark.parametrize("T", [2, 9, 31, 33, 64, 65, 300])
 def test_experts_with_few_and_with_many_rows(gpu_lib, binding, T):
     """Four experts of which every token takes two and the shared one: slots of up to T rows, cut into tiles of 32."""
     c = synth.tiny_spec().cfg.copy()
@@ -46,4 +46,17 @@ def test_experts_with_few_and_with_many_rows(gpu_lib, binding, T):
     x = np.random.default_rng(T).standard_normal((T, c.hidden)).astype(np.float32)
     assert common.rel_err(eng.op_moe(0, x), orc.op_moe(0, x)) < 1e-5
     assert common.rel_err(eng.op_moe(0, x, False), orc.op_moe(0, x, False)) < 1e-5
+    eng.close(); orc.close()
+
+
+def test_prompt_of_several_attention_chunks(gpu_lib, binding):
+    """A prompt longer than the 64 positions of the attention core and the router, then decode steps on its state."""
+    spec = synth.tiny_spec()
+    tensors = synth.make_model(spec, seed=31, recipe="spread")
+    eng, orc = common.build_models(spec, tensors, 300, binding)
+    ids = np.random.default_rng(6).integers(0, spec.cfg.vocab, 270).astype(np.int32)
+    g, w = eng.forward(ids)[0], orc.forward(ids)[0]
+    for tok in (3, 77):
+        assert common.rel_err(g, w) < 1e-3 and int(g.argmax()) == int(w.argmax())
+        g, w = eng.forward([tok])[0], orc.forward([tok])[0]
     eng.close(); orc.close()
