@@ -735,7 +735,7 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         walloc(e, &e->kz, N * P) || walloc(e, &e->kgb, N * P) || walloc(e, &e->ko, N * P) ||
         walloc(e, &e->kbraw, N * c.kda_heads) || walloc(e, &e->klr, N * 2 * D) ||
         walloc(e, &e->kscr.qn, N * P) || walloc(e, &e->kscr.kn, N * P) || walloc(e, &e->kscr.vn, N * P) ||
-        walloc(e, &e->kscr.al, N * P) || walloc(e, &e->kscr.beta, N * c.kda_heads)) return -1;
+        walloc(e, &e->kscr.al, N * P) || walloc(e, &e->kscr.beta, N * c.kda_heads * 2)) return -1;
     if (walloc(e, &e->mq_raw, N * c.q_lora) || walloc(e, &e->mct, N * KL) || walloc(e, &e->mwk, N * c.index_dim) ||
         walloc(e, &e->mgate, N * c.index_dim) || walloc(e, &e->mwp, N * c.index_heads) ||
         walloc(e, &e->mq, N * H * c.qk_nope) || walloc(e, &e->mqidx, N * (size_t)c.index_heads * c.index_dim) ||
@@ -1059,7 +1059,7 @@ static int run_kda(g5b_engine *e, Layer &w, const float *x, int n, float *out, b
     if (n == 1 && !ts) prefetch_beside(e, w.ko);        // the recurrence below leaves half the SMs and all of HBM idle
     if (batch)
         kda_core(e->st, e->ko, e->kq, e->kk, e->kv, e->kz, e->kbraw, e->kgb, w.q_conv, w.k_conv, w.v_conv,
-                 w.A_log, w.dt_bias, w.o_norm, w.kda_state, 1, ks, n, e->kda_seq, nullptr, h0, Hl);
+                 w.A_log, w.dt_bias, w.o_norm, w.kda_state, 1, ks, n, e->kda_seq, nullptr, h0, Hl, nullptr, 0, &e->kscr);
     else
         kda_core(e->st, e->ko, e->kq, e->kk, e->kv, e->kz, e->kbraw, e->kgb, w.q_conv, w.k_conv, w.v_conv,
                  w.A_log, w.dt_bias, w.o_norm, w.kda_state + (size_t)e->cur_seq * e->kda_seq, n, ks, 1, 0,

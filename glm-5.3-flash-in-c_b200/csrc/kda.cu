@@ -216,160 +216,254 @@ __global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaAr
     }
 }
 
-// Several positions of one sequence (prefill chunks, the two-position pass of speculative decode).
-// Run position by position, the kernel above spends its time in what does NOT depend on the
-// previous position: three convolutions with an exactly rounded SiLU, the gate's exactly rounded
-// sigmoid and exponential, the l2norm sums in FP64 - about 8 us per position for a head, 0.5 ms for a
-// chunk of 64. Here that part runs for all positions at once (kda_prep_kernel: one CTA per head and
-// position) into scratch rows, and only the state update walks the positions (kda_scan_kernel: one
-// CTA per head, the state column in registers, eight positions' vectors in shared memory at a time,
-// their output norms reduced together). Every value is computed by the same operations in the
-// same order as in kda_core_kernel, so the results are bit-identical.
+// Several positions of one sequence (prompts, the two-position pass of speculative decode), or one position each of
+// many sequences. What does not depend on the previous position - three convolutions with SiLU, the gate, the
+// l2norm sums - runs for all positions at once (kda_prep_kernel, a warp per position and head); the state update
+// alone walks the positions (kda_scan_kernel); the output's norm and gate follow for all positions at once
+// (kda_out_kernel).
+//
+// The scan: the columns of the state are independent of each other, so a head's 128 are dealt to four CTAs, and a
+// column to PARTS lanes of 128 / PARTS rows each, in registers. Both products of a position are taken with the
+// decayed state, o = q.(aS) + (q.k) u, so that one round of shuffles serves them and the next position waits for u
+// alone; the positions' vectors arrive by asynchronous copies, 8 positions ahead. What bounds it over many positions
+// is that chain (shared loads, sums, three shuffles): eight lanes to a column then. Over one position of many
+// sequences it is the state's memory traffic, and four lanes to a column read it in whole 32-byte sectors.
+// (One CTA per head and one thread per column, sums in one chain of 128: 2.6 us per position, 5.2 ms for 2048.)
+// The sums of a column are taken in parts with four accumulators each, products fused.
 struct KdaPrep {
     KdaArgs a;
-    float *qn, *kn, *vn, *al, *beta;        // [T][P] normalised q (scaled), normalised k, v, exp(gate); [T][H] beta
+    float *qn, *kn, *vn, *al, *beta;        // [rows][P] normalised q (scaled), normalised k, v, exp(gate); [rows][H][2] beta, q.k
+    int heads;                              // of this launch
 };
 
-template <int DS>
-__global__ void __launch_bounds__(DS) kda_prep_kernel(const KdaPrep p)
+// A warp takes KDA_RUN positions of one head: the convolution weights stay in registers, the taps come as vectors.
+// Bound by its 0.5 GB of memory traffic at 2048 positions of 64 heads (82 us). KW: the width of the convolution, 0 for
+// one known at run time only.
+constexpr int KDA_RUN = 8;
+template <int DS, int KW>
+__global__ void __launch_bounds__(256) kda_prep_kernel(const KdaPrep p)
 {
-    __shared__ double red[32];
+    pdl_trigger();
     const KdaArgs &a = p.a;
-    constexpr int D = DS;
-    const int h = a.head0 + blockIdx.x, t = blockIdx.y, d = threadIdx.x;
-    const int P = a.H * D, K = a.K, hist = K - 1;
-    const int ch = h * D + d;
-    const float *cs = a.state + (size_t)a.H * D * D;
+    constexpr int D = DS, C = DS / 32;      // channels per lane
+    struct alignas(4 * C) Vec { float v[C]; };
+    const int lane = threadIdx.x & 31, runs = (a.T + KDA_RUN - 1) / KDA_RUN, seq = blockIdx.y / runs, t0 = (blockIdx.y - seq * runs) * KDA_RUN;
+    const int hl = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (hl >= p.heads) { pdl_wait(); return; }
+    const int h = a.head0 + hl, P = a.H * D, K = KW ? KW : a.K, hist = K - 1, ch = h * D + lane * C;
+    const float *cs = a.state + (size_t)seq * a.seq_stride + (size_t)a.H * D * D;
+    const float *const xs[3] = {a.q, a.k, a.v}, *const ws[3] = {a.q_conv, a.k_conv, a.v_conv};
+    float w[3][C][KW ? KW : 1], dt[C];
+#pragma unroll
+    for (int i = 0; i < C; i++) {
+        dt[i] = a.dt_bias[ch + i];
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int j = 0; j < KW; j++) w[c][i][j] = ws[c][(size_t)(ch + i) * KW + j];
+    }
+    const float ea = expf_host(a.A_log[h]), qscale = 1.0f / sqrtf((float)D);
     pdl_wait();
-    // the K - 1 inputs before position t: earlier rows of this call, or the carried history (oldest first)
-    auto conv = [&](const float *x, const float *w, const float *past) {
-        float acc = __fmul_rn(w[(size_t)ch * K + hist], x[(size_t)t * P + ch]);
-        for (int j = 0; j < hist; j++) {
-            const int tt = t - hist + j;
-            const float v = tt >= 0 ? x[(size_t)tt * P + ch] : past[(size_t)ch * hist + (hist + tt)];
-            acc = mul_add_unfused(w[(size_t)ch * K + j], v, acc);
+    for (int t = t0; t < a.T && t < t0 + KDA_RUN; t++) {
+        const int rr = seq * a.T + t;
+        float y[3][C];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            // the K - 1 inputs before position t: earlier rows of this call, or the carried history (oldest first)
+            const float *x = xs[c] + (size_t)rr * P + ch, *past = cs + (size_t)c * P * hist + (size_t)ch * hist;
+            auto tap = [&](int i, int j) { return KW ? w[c][i][KW ? j : 0] : ws[c][(size_t)(ch + i) * K + j]; };
+            const Vec now = *reinterpret_cast<const Vec *>(x);
+#pragma unroll
+            for (int i = 0; i < C; i++) y[c][i] = __fmul_rn(tap(i, hist), now.v[i]);
+#pragma unroll
+            for (int j = 0; j < (KW ? KW - 1 : hist); j++) {
+                const int tt = t - hist + j;
+                Vec old;
+                if (tt >= 0) old = *reinterpret_cast<const Vec *>(x - (size_t)(hist - j) * P);
+                else
+#pragma unroll
+                    for (int i = 0; i < C; i++) old.v[i] = past[(size_t)i * hist + (hist + tt)];
+#pragma unroll
+                for (int i = 0; i < C; i++) y[c][i] = mul_add_unfused(tap(i, j), old.v[i], y[c][i]);
+            }
+#pragma unroll
+            for (int i = 0; i < C; i++) y[c][i] = __fmul_rn(y[c][i], sigmoid_near(y[c][i]));
         }
-        return __fmul_rn(acc, sigmoid_host(acc));
-    };
-    const float qv = conv(a.q, a.q_conv, cs);
-    const float kv = conv(a.k, a.k_conv, cs + (size_t)P * hist);
-    const float vv = conv(a.v, a.v_conv, cs + (size_t)2 * P * hist);
-    const double qq = block_sum((double)qv * (double)qv, red);
-    const double kk = block_sum((double)kv * (double)kv, red);
-    const float qinv = (float)(1.0 / sqrt(qq + (double)1e-6f));
-    const float kinv = (float)(1.0 / sqrt(kk + (double)1e-6f));
-    const size_t off = (size_t)t * P + ch;
-    p.qn[off] = __fmul_rn(__fmul_rn(qv, qinv), 1.0f / sqrtf((float)D));
-    p.kn[off] = __fmul_rn(kv, kinv);
-    p.vn[off] = vv;
-    const float ea = expf_host(a.A_log[h]);
-    const float g = __fmul_rn(a.gate_lb, sigmoid_host(__fmul_rn(ea, __fadd_rn(a.z[off], a.dt_bias[ch]))));
-    p.al[off] = expf_host(g);
-    if (d == 0) p.beta[(size_t)t * a.H + h] = sigmoid_host(a.braw[(size_t)t * a.H + h]);
+        // l2norm: divide by sqrt(sum of squares + 1e-6), sums in FP64 (glm53f_ops.c:661-667)
+        double qq = 0.0, kk = 0.0, qk = 0.0;
+#pragma unroll
+        for (int i = 0; i < C; i++) {
+            qq += (double)y[0][i] * (double)y[0][i];
+            kk += (double)y[1][i] * (double)y[1][i];
+        }
+        qq = warp_sum(qq); kk = warp_sum(kk);
+        const float qinv = (float)(1.0 / sqrt(qq + (double)1e-6f)), kinv = (float)(1.0 / sqrt(kk + (double)1e-6f));
+        const size_t off = (size_t)rr * P + ch;
+        const Vec z = *reinterpret_cast<const Vec *>(a.z + off);
+        Vec qn, kn, vn, al;
+#pragma unroll
+        for (int i = 0; i < C; i++) {
+            qn.v[i] = __fmul_rn(__fmul_rn(y[0][i], qinv), qscale);
+            kn.v[i] = __fmul_rn(y[1][i], kinv);
+            vn.v[i] = y[2][i];
+            al.v[i] = expf_near(__fmul_rn(a.gate_lb, sigmoid_near(__fmul_rn(ea, __fadd_rn(z.v[i], dt[i])))));
+            qk += (double)qn.v[i] * (double)kn.v[i];
+        }
+        qk = warp_sum(qk);
+        *reinterpret_cast<Vec *>(p.qn + off) = qn;
+        *reinterpret_cast<Vec *>(p.kn + off) = kn;
+        *reinterpret_cast<Vec *>(p.vn + off) = vn;
+        *reinterpret_cast<Vec *>(p.al + off) = al;
+        if (lane == 0) *reinterpret_cast<float2 *>(p.beta + ((size_t)rr * a.H + h) * 2) = make_float2(sigmoid_near(a.braw[(size_t)rr * a.H + h]), (float)qk);
+    }
 }
 
-constexpr int KDA_TB = 8;
-template <int DS>
-__global__ void __launch_bounds__(DS) kda_scan_kernel(const KdaPrep p)
+// Two floats side by side: one instruction for both (products and sums fused).
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float x, float y) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y)); return r; }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ float f2_sum(F2 a) { float x, y; asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); return __fadd_rn(x, y); }
+
+constexpr int KDA_TB = 8, KDA_COLS = 32;
+template <int DS, int PARTS>
+__global__ void __launch_bounds__(32 * PARTS) kda_scan_kernel(const KdaPrep p)
 {
-    constexpr int NW = DS / 32, D = DS;
-    __shared__ __align__(16) float sQ[KDA_TB][DS], sK[KDA_TB][DS], sAl[KDA_TB][DS];
-    __shared__ float sV[KDA_TB][DS], sO[KDA_TB][DS], sBeta[KDA_TB];
-    __shared__ double redo[KDA_TB][NW];
+    pdl_trigger();
+    constexpr int D = DS, R = DS / PARTS, PART = R + 4, NT = KDA_COLS * PARTS;   // rows per lane; their stride in shared memory (other banks)
+    __shared__ __align__(16) float vec[2][KDA_TB][3][PARTS * PART];      // decay, k, q
+    __shared__ __align__(16) float sv[2][KDA_TB][KDA_COLS];
+    __shared__ float2 sb[2][KDA_TB];
     const KdaArgs &a = p.a;
-    const int h = a.head0 + blockIdx.x, d = threadIdx.x, lane = d & 31, wid = d >> 5;
-    const int P = a.H * D, K = a.K, hist = K - 1;
-    const int ch = h * D + d;
-    float *S = a.state + (size_t)h * D * D;
-    float *cs = a.state + (size_t)a.H * D * D;
-    float sreg[DS];
-#pragma unroll
-    for (int i = 0; i < DS; i++) sreg[i] = S[(size_t)i * DS + d];
-    const float onw = a.o_norm[d];
+    const int groups = D / KDA_COLS, hl = blockIdx.x / groups, h = a.head0 + hl, col0 = (blockIdx.x % groups) * KDA_COLS, seq = blockIdx.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane / (32 / PARTS), col = col0 + warp * (32 / PARTS) + lane % (32 / PARTS);
+    const int P = a.H * D, hist = a.K - 1, row0 = seq * a.T;
+    float *state = a.state + (size_t)seq * a.seq_stride;
+    float *S = state + (size_t)h * D * D + (size_t)part * R * D + col;
     pdl_wait();
-    for (int t0 = 0; t0 < a.T; t0 += KDA_TB) {
+    auto fetch = [&](int t0, int buf) {
         const int nt = a.T - t0 < KDA_TB ? a.T - t0 : KDA_TB;
-#pragma unroll
-        for (int j = 0; j < KDA_TB; j++) {
-            if (j < nt) {
-                const size_t off = (size_t)(t0 + j) * P + ch;
-                sQ[j][d] = p.qn[off]; sK[j][d] = p.kn[off]; sAl[j][d] = p.al[off];
-                sV[j][d] = p.vn[off];
-                if (d == 0) sBeta[j] = p.beta[(size_t)(t0 + j) * a.H + h];
-            }
+        constexpr int Q = D / 4;                                     // 16-byte pieces of a vector
+        for (int i = threadIdx.x; i < nt * 3 * Q; i += NT) {
+            const int j = i / (3 * Q), w = (i / Q) % 3, c = i % Q;
+            const float *src = (w == 0 ? p.al : w == 1 ? p.kn : p.qn) + (size_t)(row0 + t0 + j) * P + h * D + c * 4;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&vec[buf][j][w][(c * 4 / R) * PART + (c * 4) % R]);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
         }
-        __syncthreads();
-        // the recurrence: this thread's column of the state through nt positions, no barrier inside
-#pragma unroll 1
+        for (int i = threadIdx.x; i < nt * (KDA_COLS / 4); i += NT) {
+            const int j = i / (KDA_COLS / 4), c = i % (KDA_COLS / 4);
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sv[buf][j][c * 4]);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(p.vn + (size_t)(row0 + t0 + j) * P + h * D + col0 + c * 4) : "memory");
+        }
+        if (threadIdx.x < nt) sb[buf][threadIdx.x] = __ldcg(reinterpret_cast<const float2 *>(p.beta) + (size_t)(row0 + t0 + threadIdx.x) * a.H + h);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0, 0);
+    F2 s[R / 2];
+#pragma unroll
+    for (int i = 0; i < R / 2; i++) s[i] = f2(S[(size_t)(2 * i) * D], S[(size_t)(2 * i + 1) * D]);
+    int buf = 0;
+    for (int t0 = 0; t0 < a.T; t0 += KDA_TB, buf ^= 1) {
+        const int nt = a.T - t0 < KDA_TB ? a.T - t0 : KDA_TB;
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();                                             // this group's vectors are there, the other buffer is free
+        if (t0 + KDA_TB < a.T) fetch(t0 + KDA_TB, buf ^ 1);
+#pragma unroll 2
         for (int j = 0; j < nt; j++) {
-            {
-                float u = 0.f, o1 = 0.f;
-                // (the vectors are read four elements at a time: every lane reads the same address, a broadcast)
-                const float4 *al4 = reinterpret_cast<const float4 *>(sAl[j]), *k4 = reinterpret_cast<const float4 *>(sK[j]),
-                             *q4 = reinterpret_cast<const float4 *>(sQ[j]);
+            const float4 *al4 = reinterpret_cast<const float4 *>(&vec[buf][j][0][part * PART]), *k4 = reinterpret_cast<const float4 *>(&vec[buf][j][1][part * PART]),
+                         *q4 = reinterpret_cast<const float4 *>(&vec[buf][j][2][part * PART]);
+            F2 u0 = f2(0.f, 0.f), u1 = u0, o0 = u0, o1 = u0, k[R / 2];
 #pragma unroll
-                for (int i = 0; i < DS; i += 4) {
-                    const float4 al = al4[i / 4], kk = k4[i / 4];
-                    sreg[i] = __fmul_rn(sreg[i], al.x);         u = __fadd_rn(u, __fmul_rn(sreg[i], kk.x));
-                    sreg[i + 1] = __fmul_rn(sreg[i + 1], al.y); u = __fadd_rn(u, __fmul_rn(sreg[i + 1], kk.y));
-                    sreg[i + 2] = __fmul_rn(sreg[i + 2], al.z); u = __fadd_rn(u, __fmul_rn(sreg[i + 2], kk.z));
-                    sreg[i + 3] = __fmul_rn(sreg[i + 3], al.w); u = __fadd_rn(u, __fmul_rn(sreg[i + 3], kk.w));
-                }
-                u = __fmul_rn(__fsub_rn(sV[j][d], u), sBeta[j]);
+            for (int i = 0; i < R / 4; i++) {
+                const float4 al = al4[i], kk = k4[i], q = q4[i];
+                k[2 * i] = f2(kk.x, kk.y); k[2 * i + 1] = f2(kk.z, kk.w);
+                s[2 * i] = f2_mul(s[2 * i], f2(al.x, al.y));
+                s[2 * i + 1] = f2_mul(s[2 * i + 1], f2(al.z, al.w));
+                u0 = f2_fma(s[2 * i], k[2 * i], u0);
+                u1 = f2_fma(s[2 * i + 1], k[2 * i + 1], u1);
+                o0 = f2_fma(s[2 * i], f2(q.x, q.y), o0);
+                o1 = f2_fma(s[2 * i + 1], f2(q.z, q.w), o1);
+            }
+            float u = __fadd_rn(f2_sum(u0), f2_sum(u1)), o = __fadd_rn(f2_sum(o0), f2_sum(o1));
 #pragma unroll
-                for (int i = 0; i < DS; i += 4) {
-                    const float4 kk = k4[i / 4], qq = q4[i / 4];
-                    sreg[i] = __fadd_rn(sreg[i], __fmul_rn(kk.x, u));         o1 = __fadd_rn(o1, __fmul_rn(sreg[i], qq.x));
-                    sreg[i + 1] = __fadd_rn(sreg[i + 1], __fmul_rn(kk.y, u)); o1 = __fadd_rn(o1, __fmul_rn(sreg[i + 1], qq.y));
-                    sreg[i + 2] = __fadd_rn(sreg[i + 2], __fmul_rn(kk.z, u)); o1 = __fadd_rn(o1, __fmul_rn(sreg[i + 2], qq.z));
-                    sreg[i + 3] = __fadd_rn(sreg[i + 3], __fmul_rn(kk.w, u)); o1 = __fadd_rn(o1, __fmul_rn(sreg[i + 3], qq.w));
-                }
-                sO[j][d] = o1;
-                if (a.snap && t0 + j == a.snap_after) {
-                    float *Sn = a.snap + (size_t)h * D * D;
+            for (int m = 32 / PARTS; m < 32; m <<= 1) {
+                u = __fadd_rn(u, __shfl_xor_sync(0xffffffffu, u, m));
+                o = __fadd_rn(o, __shfl_xor_sync(0xffffffffu, o, m));
+            }
+            const float2 b = sb[buf][j];
+            u = __fmul_rn(__fsub_rn(sv[buf][j][col - col0], u), b.x);
+            const F2 uu = f2(u, u);
 #pragma unroll
-                    for (int i = 0; i < DS; i++) Sn[(size_t)i * DS + d] = sreg[i];
+            for (int i = 0; i < R / 2; i++) s[i] = f2_fma(k[i], uu, s[i]);
+            if (part == 0) a.o[(size_t)(row0 + t0 + j) * P + h * D + col] = __fmaf_rn(b.y, u, o);
+            if (a.snap && t0 + j == a.snap_after) {
+                float *Sn = a.snap + (size_t)h * D * D + (size_t)part * R * D + col;
+#pragma unroll
+                for (int i = 0; i < R / 2; i++) {
+                    float x, y;
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s[i].v));
+                    Sn[(size_t)(2 * i) * D] = x; Sn[(size_t)(2 * i + 1) * D] = y;
                 }
             }
         }
-        // per-head RMSNorm with weight and the output gate of the nt positions, their sums reduced together
-        // (the warp tree and warp order of block_sum)
-#pragma unroll
-        for (int j = 0; j < KDA_TB; j++) {
-            const double woo = warp_sum(j < nt ? (double)sO[j][d] * (double)sO[j][d] : 0.0);
-            if (lane == 0) redo[j][wid] = woo;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < KDA_TB; j++) {
-            if (j < nt) {
-                double oo = 0.0;
-#pragma unroll
-                for (int w = 0; w < NW; w++) oo += redo[j][w];
-                const size_t off = (size_t)(t0 + j) * P + ch;
-                const float inv = (float)(1.0 / sqrt(oo / (double)D + (double)a.rms_eps));
-                const float n = __fmul_rn(onw, __fmul_rn(sO[j][d], inv));
-                a.o[off] = __fmul_rn(n, sigmoid_host(a.gb[off]));
-            }
-        }
-        __syncthreads();                                          // the vectors are rewritten by the next group
     }
 #pragma unroll
-    for (int i = 0; i < DS; i++) S[(size_t)i * DS + d] = sreg[i];
-    // the convolution histories: the K - 1 inputs before position `upto` (the call's rows, older ones from the old history)
+    for (int i = 0; i < R / 2; i++) {
+        float x, y;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s[i].v));
+        S[(size_t)(2 * i) * D] = x; S[(size_t)(2 * i + 1) * D] = y;
+    }
+    // the convolution histories of this CTA's channels: the K - 1 inputs before position `upto` (the call's rows, older
+    // ones from the old history, which the preparation has read)
+    float *cs = state + (size_t)a.H * D * D;
     auto histories = [&](float *dst, int upto) {
         const float *src[3] = {a.q, a.k, a.v};
-        for (int part = 0; part < 3; part++) {
+        for (int i = threadIdx.x; i < 3 * KDA_COLS; i += NT) {
+            const int w = i / KDA_COLS, ch = h * D + col0 + i % KDA_COLS;
             float nv[16];
             for (int j = 0; j < hist; j++) {
                 const int tt = upto - hist + j;
-                nv[j] = tt >= 0 ? src[part][(size_t)tt * P + ch] : cs[(size_t)part * P * hist + (size_t)ch * hist + (hist + tt)];
+                nv[j] = tt >= 0 ? src[w][(size_t)(row0 + tt) * P + ch] : cs[(size_t)w * P * hist + (size_t)ch * hist + (hist + tt)];
             }
-            for (int j = 0; j < hist; j++) dst[(size_t)part * P * hist + (size_t)ch * hist + j] = nv[j];
+            for (int j = 0; j < hist; j++) dst[(size_t)w * P * hist + (size_t)ch * hist + j] = nv[j];
         }
     };
-    if (a.snap && a.snap_after + 1 <= a.T) histories(a.snap + (size_t)a.H * D * D, a.snap_after + 1);   // before cs changes
+    if (a.snap && a.snap_after + 1 <= a.T) histories(a.snap + (size_t)a.H * D * D, a.snap_after + 1);   // before cs changes (each channel by one thread)
     histories(cs, a.T);
+}
+
+// Per-head RMSNorm with weight, then the sigmoid output gate (glm53f_ops.c:748-752), in place; a warp per row and head.
+template <int DS>
+__global__ void __launch_bounds__(256) kda_out_kernel(const KdaArgs a, int heads)
+{
+    pdl_trigger();
+    constexpr int D = DS, C = DS / 32;
+    const int lane = threadIdx.x & 31, hl = blockIdx.x * 8 + (threadIdx.x >> 5);
+    pdl_wait();
+    if (hl >= heads) return;
+    const int h = a.head0 + hl;
+    const size_t off = (size_t)blockIdx.y * a.H * D + h * D + lane * C;
+    float o[C];
+    double oo = 0.0;
+#pragma unroll
+    for (int i = 0; i < C; i++) { o[i] = a.o[off + i]; oo += (double)o[i] * (double)o[i]; }
+    oo = warp_sum(oo);
+    const float inv = (float)(1.0 / sqrt(oo / (double)D + (double)a.rms_eps));
+#pragma unroll
+    for (int i = 0; i < C; i++)
+        a.o[off + i] = __fmul_rn(__fmul_rn(a.o_norm[lane * C + i], __fmul_rn(o[i], inv)), sigmoid_near(a.gb[off + i]));
+}
+
+template <int DS>
+static void kda_rows(cudaStream_t st, const KdaArgs &a, const KdaScratch &x, int heads, int n_seq)
+{
+    KdaPrep p{a, x.qn, x.kn, x.vn, x.al, x.beta, heads};
+    const dim3 pg((heads + 7) / 8, (a.T + KDA_RUN - 1) / KDA_RUN * n_seq), sg(heads * (DS / KDA_COLS), n_seq);
+    if (a.K == 4) G5B_LAUNCH_PDL((kda_prep_kernel<DS, 4>), pg, dim3(256), 0, st, p);
+    else          G5B_LAUNCH_PDL((kda_prep_kernel<DS, 0>), pg, dim3(256), 0, st, p);
+    if (a.T > 1) G5B_LAUNCH_PDL((kda_scan_kernel<DS, 8>), sg, dim3(256), 0, st, p);
+    else         G5B_LAUNCH_PDL((kda_scan_kernel<DS, 4>), sg, dim3(128), 0, st, p);
+    G5B_LAUNCH_PDL(kda_out_kernel<DS>, dim3((heads + 7) / 8, a.T * n_seq), dim3(256), 0, st, a, heads);
 }
 
 void kda_core(cudaStream_t st, float *o, const float *q, const float *k, const float *v, const float *z,
@@ -385,17 +479,9 @@ void kda_core(cudaStream_t st, float *o, const float *q, const float *k, const f
               fused ? lr->lrf : nullptr, fused ? lr->lrg : nullptr, snap, snap_after};
     const dim3 grid(heads > 0 ? heads : s.H, n_seq < 1 ? 1 : n_seq);
     const size_t smem = fused ? (size_t)2 * s.D * (2 * s.D + 16) : 0;
-    if (T > 1 && n_seq <= 1 && scratch && s.K <= 17 && (s.D == 128 || s.D == 64)) {
-        // several positions: everything that does not depend on the previous position first, in parallel
-        KdaPrep p{a, scratch->qn, scratch->kn, scratch->vn, scratch->al, scratch->beta};
-        const dim3 pgrid(grid.x, T);
-        if (s.D == 128) {
-            G5B_LAUNCH_PDL(kda_prep_kernel<128>, pgrid, dim3(128), 0, st, p);
-            G5B_LAUNCH(kda_scan_kernel<128>, dim3(grid.x), dim3(128), 0, st, p);
-        } else {
-            G5B_LAUNCH(kda_prep_kernel<64>, pgrid, dim3(64), 0, st, p);
-            G5B_LAUNCH(kda_scan_kernel<64>, dim3(grid.x), dim3(64), 0, st, p);
-        }
+    if (T * grid.y > 1 && scratch && s.K <= 17 && (s.D == 128 || s.D == 64)) {
+        if (s.D == 128) kda_rows<128>(st, a, *scratch, (int)grid.x, (int)grid.y);
+        else            kda_rows<64>(st, a, *scratch, (int)grid.x, (int)grid.y);
         return;
     }
     if (s.D == 128) {
