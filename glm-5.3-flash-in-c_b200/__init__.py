@@ -276,13 +276,13 @@ class FlatModel:
         return h
 
     def op_kda(self, layer, x):
-        x = _f32(x); out = np.zeros_like(x)
+        x = _f32(x); out = np.empty_like(x)
         if self._fn("op_kda")(self.handle, layer, x.ctypes.data, x.shape[0], out.ctypes.data) != 0:
             self._err("op_kda")
         return out
 
     def op_mla(self, layer, x, cached):
-        x = _f32(x); out = np.zeros_like(x)
+        x = _f32(x); out = np.empty_like(x)
         sel = np.zeros(self.cfg.index_topk + self.cfg.index_kpool, np.int32)
         n = C.c_int(0)
         if self._fn("op_mla")(self.handle, layer, x.ctypes.data, x.shape[0], cached, out.ctypes.data,
@@ -298,14 +298,14 @@ class FlatModel:
         return idx, w
 
     def op_moe(self, layer, x, with_shared=True):
-        x = _f32(x); out = np.zeros_like(x)
+        x = _f32(x); out = np.empty_like(x)
         if self._fn("op_moe")(self.handle, layer, x.ctypes.data, x.shape[0], out.ctypes.data,
                               1 if with_shared else 0) != 0:
             self._err("op_moe")
         return out
 
     def op_mlp(self, layer, x):
-        x = _f32(x); out = np.zeros_like(x)
+        x = _f32(x); out = np.empty_like(x)
         if self._fn("op_mlp")(self.handle, layer, x.ctypes.data, x.shape[0], out.ctypes.data) != 0:
             self._err("op_mlp")
         return out

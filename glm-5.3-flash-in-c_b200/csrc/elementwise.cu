@@ -340,4 +340,33 @@ void l2_prefetch(cudaStream_t st, const void *p, size_t bytes)
     G5B_LAUNCH(l2_prefetch_kernel, blocks < 1 ? 1 : blocks, 128, 0, st, static_cast<const uint8_t *>(p), bytes);
 }
 
+// Rows of mapped host memory to the device.
+__global__ void __launch_bounds__(256) host_rows_kernel(float4 *dst, const float4 *src, size_t n)
+{
+    pdl_trigger();
+    const size_t i = (size_t)blockIdx.x * 256 + threadIdx.x;
+    const float4 v = i < n ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    pdl_wait();
+    if (i < n) dst[i] = v;
+}
+void host_rows(cudaStream_t st, float *dst, const float *src, size_t n)
+{
+    G5B_LAUNCH_PDL(host_rows_kernel, dim3((unsigned)((n / 4 + 255) / 256)), dim3(256), 0, st, reinterpret_cast<float4 *>(dst),
+                   reinterpret_cast<const float4 *>(src), n / 4);
+}
+
+// [size, list] of a selection (size < 0: every visible position, no list).
+__global__ void __launch_bounds__(512) selection_out_kernel(int *dst, const int *nsel, const int *sel)
+{
+    pdl_trigger();
+    pdl_wait();
+    const int n = *nsel;
+    if (threadIdx.x == 0) dst[0] = n;
+    for (int i = threadIdx.x; i < n; i += 512) dst[1 + i] = sel[i];
+}
+void selection_out(cudaStream_t st, int *dst, const int *nsel, const int *sel)
+{
+    G5B_LAUNCH_PDL(selection_out_kernel, dim3(1), dim3(512), 0, st, dst, nsel, sel);
+}
+
 }  // namespace g5b

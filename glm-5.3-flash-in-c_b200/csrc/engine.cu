@@ -126,6 +126,9 @@ struct g5b_engine {
     bool dirty = false;                          // a call failed half-way: session state is undefined until reset
     int latent_bf16 = 0, profile = 0, partial = 0, expert_path = 2;
     unsigned long long *grid_sync = nullptr, grid_launches = 0;
+    float *io_in = nullptr, *io_in_dev = nullptr;   // staging rows of the host-buffer ops: io_rows in, then io_rows out
+    size_t io_rows = 0;
+    int *io_sel = nullptr, *io_sel_dev = nullptr;   // mapped: the size and the list of an attention op's selection
     int *counter = nullptr, *tile_done = nullptr, *err_dev = nullptr;
     volatile int *err_host = nullptr;   // mapped host memory: kernels record a timed-out wait here
     cudaStream_t st = nullptr;
@@ -1536,6 +1539,8 @@ extern "C" void g5b_engine_free(g5b_engine *e)
     if (e->ids_dev) cudaFree(e->ids_dev);
     if (e->flush_buf) cudaFree(e->flush_buf);
     if (e->err_host) cudaFreeHost((void *)e->err_host);
+    if (e->io_in) cudaFreeHost(e->io_in);
+    if (e->io_sel) cudaFreeHost(e->io_sel);
     for (int i = 0; i <= PROF_SLOTS; i++) cudaEventDestroy(e->prof_ev[i]);
     if (e->side) { cudaStreamSynchronize(e->side); cudaStreamDestroy(e->side); }
     if (e->side_ev) cudaEventDestroy(e->side_ev);
@@ -1793,32 +1798,74 @@ extern "C" int g5b_mtp_hidden(g5b_engine *e, int first, int T, float *dst)
 }
 
 
-// Host buffers through the engine's own staging rows (no allocation per call): copy a piece in,
-// run, copy the result out; one wait at the end. With pinned host memory the copies overlap the
-// kernels of the neighbouring pieces.
-// `direct_out`: the op's last kernel writes every output element exactly once with plain stores.
-// If the caller's buffer is pinned and mapped, that kernel then writes straight into it (16 KB per
-// token over PCIe as posted writes, visible once the stream has drained) and the copy engine's
-// turn after the kernel - about 6 us of a 90 us call at batch 1 - is saved.
+// Rows of mapped host memory to the device by a kernel, not the copy engine: handing over between the copy engine and a
+// kernel costs a few microseconds, which is a tenth of a one-row call. PCIe is as fast either way; beyond
+// HOST_KERNEL_BYTES the copies run in slices beside the host's own copy into the staging rows.
+constexpr size_t HOST_KERNEL_BYTES = (size_t)128 << 10, HOST_SLICE = (size_t)128 << 10;
+static float *mapped_on_device(const void *p)
+{
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost) return static_cast<float *>(at.devicePointer);
+    cudaGetLastError();
+    return nullptr;
+}
+
+// Pinned, mapped staging rows for calls on ordinary host memory: as many as the largest call so far, at most one pass's.
+static bool ensure_io(g5b_engine *e, size_t rows)
+{
+    if (rows <= e->io_rows) return true;
+    if (e->io_in) cudaFreeHost(e->io_in);
+    e->io_in = nullptr; e->io_rows = 0;
+    const size_t n = rows * e->c.hidden;
+    void *p = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&p, 2 * n * sizeof(float), cudaHostAllocMapped) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (cudaHostGetDevicePointer(&d, p, 0) != cudaSuccess) { cudaGetLastError(); cudaFreeHost(p); return false; }
+    e->io_in = static_cast<float *>(p); e->io_in_dev = static_cast<float *>(d);
+    e->io_rows = rows;
+    return true;
+}
+
+// Host buffers in, host buffers out; the engine's own rows in between (no allocation per call once the staging rows
+// are there). Ordinary memory goes through pinned staging rows: the driver's own staging of a pageable copy blocks
+// the host, 10 us for one row and 0.2 ms for 64.
+// `direct_out`: the op's last kernel writes every output element exactly once with plain stores. It then writes
+// straight into mapped host memory (the caller's if that is pinned, else the staging rows; posted writes over PCIe,
+// visible once the stream has drained) and the copy engine's turn after the kernel is saved.
 template <typename F>
 static int host_op(g5b_engine *e, const float *x, int T, float *out, F &&run, bool direct_out = false)
 {
-    const size_t E = e->c.hidden;
-    float *out_dev = nullptr;
-    if (direct_out) {
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, out) == cudaSuccess && at.type == cudaMemoryTypeHost && at.devicePointer)
-            out_dev = static_cast<float *>(at.devicePointer);
-        else
-            cudaGetLastError();
-    }
+    const size_t E = e->c.hidden, rows = (size_t)(T < e->pass ? T : e->pass);
+    const float *x_dev = mapped_on_device(x);
+    float *out_dev = mapped_on_device(out);
+    const bool staged = (x_dev && out_dev) || ensure_io(e, rows);
+    float *io_out = e->io_in ? e->io_in + e->io_rows * E : nullptr, *io_out_dev = e->io_in ? e->io_in_dev + e->io_rows * E : nullptr;
     FOR_CHUNKS(T) {
-        CU(cudaMemcpyAsync(e->xn, x + t0 * E, n_ * E * 4, cudaMemcpyHostToDevice, e->st));
-        if (run(e->xn, n_, out_dev ? out_dev + t0 * E : e->y, t0)) {
+        const size_t bytes = n_ * E * 4;
+        const float *src = x + t0 * E, *src_dev = x_dev ? x_dev + t0 * E : staged ? e->io_in_dev : nullptr;
+        const bool via = !x_dev && staged;                           // through the staging rows
+        if (src_dev && bytes <= HOST_KERNEL_BYTES && E % 4 == 0 && ((uintptr_t)src_dev & 15) == 0) {
+            if (via) memcpy(e->io_in, src, bytes);
+            host_rows(e->st, e->xn, src_dev, bytes / 4);
+        } else if (via) {
+            for (size_t o = 0; o < bytes; o += HOST_SLICE) {
+                const size_t nb = bytes - o < HOST_SLICE ? bytes - o : HOST_SLICE;
+                memcpy(reinterpret_cast<char *>(e->io_in) + o, reinterpret_cast<const char *>(src) + o, nb);
+                CU(cudaMemcpyAsync(reinterpret_cast<char *>(e->xn) + o, reinterpret_cast<char *>(e->io_in) + o, nb, cudaMemcpyHostToDevice, e->st));
+            }
+        } else
+            CU(cudaMemcpyAsync(e->xn, src, bytes, cudaMemcpyHostToDevice, e->st));
+        float *od = !direct_out ? e->y : out_dev ? out_dev + t0 * E : staged ? io_out_dev : e->y;
+        if (run(e->xn, n_, od, t0)) {
             cudaStreamSynchronize(e->st);            // copies on the caller's buffers must not outlive the call
             return -1;
         }
-        if (!out_dev) CU(cudaMemcpyAsync(out + t0 * E, e->y, n_ * E * 4, cudaMemcpyDeviceToHost, e->st));
+        const bool back = !out_dev && staged;
+        if (od == e->y) CU(cudaMemcpyAsync(back ? io_out : out + t0 * E, e->y, bytes, cudaMemcpyDeviceToHost, e->st));
+        if (back) {
+            CU(cudaStreamSynchronize(e->st));
+            memcpy(out + t0 * E, io_out, bytes);
+        } else if (via)
+            CU(cudaStreamSynchronize(e->st));                        // the staging rows are filled again
     }
     CU(cudaStreamSynchronize(e->st));
     CU(cudaGetLastError());
@@ -1877,7 +1924,7 @@ extern "C" int g5b_op_mlp(g5b_engine *e, int layer, const float *x, int T, float
     if (!e->L[layer].is_dense) return fail("layer %d is a MoE layer", layer);
     return host_op(e, x, T, out, [&](const float *xd, int n, float *od, int) {
         return run_mlp(e, e->L[layer], xd, n, od);
-    });
+    }, e->ep_size <= 1);
 }
 
 extern "C" int g5b_op_kda(g5b_engine *e, int layer, const float *x, int T, float *out)
@@ -1886,7 +1933,7 @@ extern "C" int g5b_op_kda(g5b_engine *e, int layer, const float *x, int T, float
     if (e->L[layer].is_mla) return fail("layer %d is an MLA layer", layer);
     return host_op(e, x, T, out, [&](const float *xd, int n, float *od, int) {
         return run_kda(e, e->L[layer], xd, n, od);
-    });
+    }, e->ep_size <= 1);
 }
 
 extern "C" int g5b_op_mla(g5b_engine *e, int layer, const float *x, int T, int cached, float *out,
@@ -1894,21 +1941,24 @@ extern "C" int g5b_op_mla(g5b_engine *e, int layer, const float *x, int T, int c
 {
     if (check_op(e, layer, T)) return -1;
     if (!e->L[layer].is_mla) return fail("layer %d is a KDA layer", layer);
-    int last_n = 0;
+    // the last position's selection goes to the host beside the result, not by copies and waits of its own
+    const int most = e->c.index_topk + e->c.index_kpool;
+    if (n_sel_out && !e->io_sel) {
+        void *p = nullptr, *d = nullptr;
+        CU(cudaHostAlloc(&p, (size_t)(most + 1) * sizeof(int), cudaHostAllocMapped));
+        e->io_sel = static_cast<int *>(p);
+        CU(cudaHostGetDevicePointer(&d, p, 0));
+        e->io_sel_dev = static_cast<int *>(d);
+    }
     if (host_op(e, x, T, out, [&](const float *xd, int n, float *od, int t0) {
-            last_n = n;
-            return run_mla(e, e->L[layer], xd, n, cached + t0, od);
-        })) return -1;
+            if (run_mla(e, e->L[layer], xd, n, cached + t0, od)) return -1;
+            const int at = (n - 1) % CHUNK;
+            if (n_sel_out && t0 + n == T) selection_out(e->st, e->io_sel_dev, e->mnsel + at, e->msel + (size_t)at * most);
+            return 0;
+        }, e->ep_size <= 1)) return -1;
     if (n_sel_out) {
-        int ns = 0;
-        CU(cudaMemcpyAsync(&ns, e->mnsel + (last_n - 1) % CHUNK, 4, cudaMemcpyDeviceToHost, e->st));
-        CU(cudaStreamSynchronize(e->st));
-        *n_sel_out = ns;
-        if (sel_out && ns > 0) {
-            CU(cudaMemcpyAsync(sel_out, e->msel + (size_t)((last_n - 1) % CHUNK) * (e->c.index_topk + e->c.index_kpool),
-                               (size_t)ns * 4, cudaMemcpyDeviceToHost, e->st));
-            CU(cudaStreamSynchronize(e->st));
-        }
+        *n_sel_out = e->io_sel[0];
+        if (sel_out && e->io_sel[0] > 0) memcpy(sel_out, e->io_sel + 1, (size_t)e->io_sel[0] * sizeof(int));
     }
     return 0;
 }

@@ -78,6 +78,8 @@ bool tc_gemm_takes(const TcGemm *g, const GemvSeg &s, int T);
 int  tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg *segs, int n, int T);
 
 // ---- elementwise.cu -----------------------------------------------------------------------
+void host_rows(cudaStream_t st, float *dst, const float *src, size_t n);          // n: a multiple of 4, both 16-byte aligned
+void selection_out(cudaStream_t st, int *dst, const int *nsel, const int *sel);
 void rms_factor(cudaStream_t st, const float *x, int n, int ld, int rows, float eps, float *inv);
 void rms_apply(cudaStream_t st, float *y, const float *x, const float *w, const float *inv, int n,
                int ld, int rows);
