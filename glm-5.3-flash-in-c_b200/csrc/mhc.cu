@@ -559,6 +559,177 @@ __global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCC_THREADS) 
     cluster_wait();
 }
 
+// ---- the same site for many positions (four streams): one CTA per position, three at a time on an SM.
+// A cluster finishes one position sooner, but only 37 fit the GPU at once and each is a chain of latencies: 45 us for 64
+// positions, 1197 us for 2048. What bounds many positions is arithmetic - (2 + M) M products per stream element, ten
+// FP32 instructions each to carry the sums like FP64: 31,000 cycles per position and SM, 223 us for 2048 - so the chains of one
+// position (exponentials, Sinkhorn, norms) run beside the products of the others. Measured: 453 us for 2048 positions.
+// The streams stay in shared memory; a thread takes every 256th piece of eight elements and six mixer rows at a time.
+constexpr int HCR_THREADS = 256, HCR_ROWS = 6, HCR_M = 4, HCR_MIX = (2 + HCR_M) * HCR_M;
+constexpr size_t HCR_MAX_SMEM = (size_t)200 << 10;
+
+__device__ __forceinline__ void acc2_merge(Acc2 &a, float s, float c)
+{
+    acc2_add(a, s);
+    a.c = __fadd_rn(a.c, c);
+}
+__device__ __forceinline__ Acc2 acc2_warp_sum(Acc2 a)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float s = __shfl_xor_sync(0xffffffffu, a.s, o), c = __shfl_xor_sync(0xffffffffu, a.c, o);
+        acc2_merge(a, s, c);
+    }
+    return a;
+}
+
+__global__ void __launch_bounds__(HCR_THREADS, 3) hc_pre_rows_kernel(const HcFused a)
+{
+    extern __shared__ __align__(16) float hs[];                  // [4][E]; the collapsed vector later takes the first E
+    __shared__ double part[HCR_THREADS / 32][HCR_MIX + 1], dots[HCR_MIX + 1], pre[HCR_M], red[HCR_THREADS / 32];
+    __shared__ float mx[HCR_MIX];
+    constexpr int M = HCR_M, MM = M * M, MIX = HCR_MIX, NWARPS = HCR_THREADS / 32;
+    pdl_trigger();
+    const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = a.E, ME = M * E;
+    float *ht = a.h + (size_t)t * ME;
+    const double eps = (double)a.hc_eps;
+    pdl_wait();
+
+    Acc2 sq;
+    if (a.y) {
+        // the pending hc_post of the previous site, as in the kernel above
+        float cb[MM], po[M];
+#pragma unroll
+        for (int i = 0; i < MM; i++) cb[i] = __ldcg(a.comb + (size_t)t * MM + i);
+#pragma unroll
+        for (int i = 0; i < M; i++) po[i] = __ldcg(a.post + (size_t)t * M + i);
+        for (int d = tid * 2; d < E; d += HCR_THREADS * 2) {
+            const float2 yv = *reinterpret_cast<const float2 *>(a.y + (size_t)t * E + d);
+            float2 hv[M];
+#pragma unroll
+            for (int i = 0; i < M; i++) hv[i] = *reinterpret_cast<const float2 *>(ht + (size_t)i * E + d);
+#pragma unroll
+            for (int j = 0; j < M; j++) {
+                Acc2 s0, s1;
+                acc2_fma(s0, po[j], yv.x);
+                acc2_fma(s1, po[j], yv.y);
+#pragma unroll
+                for (int i = 0; i < M; i++) { acc2_fma(s0, cb[i * M + j], hv[i].x); acc2_fma(s1, cb[i * M + j], hv[i].y); }
+                const float2 nv = make_float2(acc2_f32(s0), acc2_f32(s1));
+                *reinterpret_cast<float2 *>(hs + j * E + d) = nv;
+                *reinterpret_cast<float2 *>(ht + (size_t)j * E + d) = nv;
+                acc2_fma(sq, nv.x, nv.x);
+                acc2_fma(sq, nv.y, nv.y);
+            }
+        }
+    } else {
+        for (int i = tid * 4; i < ME; i += HCR_THREADS * 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(ht + i);
+            *reinterpret_cast<float4 *>(hs + i) = v;
+            acc2_fma(sq, v.x, v.x); acc2_fma(sq, v.y, v.y); acc2_fma(sq, v.z, v.z); acc2_fma(sq, v.w, v.w);
+        }
+    }
+    __syncwarp();
+    sq = acc2_warp_sum(sq);
+    if (lane == 0) part[warp][MIX] = acc2_f64(sq);
+    __syncthreads();
+
+    // mixer rows (compensated FP32 sums; the reference's are FP64)
+    const int pieces = ME / 8;
+#pragma unroll 1
+    for (int k0 = 0; k0 < MIX; k0 += HCR_ROWS) {
+        Acc2 acc[HCR_ROWS];
+        uint4 wn[HCR_ROWS];
+        const uint16_t *rows = a.fn + (size_t)k0 * ME;
+        auto load = [&](int piece) {
+#pragma unroll
+            for (int r = 0; r < HCR_ROWS; r++) wn[r] = __ldg(reinterpret_cast<const uint4 *>(rows + (size_t)r * ME + (size_t)piece * 8));
+        };
+        if (tid < pieces) load(tid);
+#pragma unroll 1
+        for (int piece = tid; piece < pieces; piece += HCR_THREADS) {
+            uint4 wv[HCR_ROWS];
+#pragma unroll
+            for (int r = 0; r < HCR_ROWS; r++) wv[r] = wn[r];
+            if (piece + HCR_THREADS < pieces) load(piece + HCR_THREADS);
+            const float4 h0 = *reinterpret_cast<const float4 *>(hs + piece * 8), h1 = *reinterpret_cast<const float4 *>(hs + piece * 8 + 4);
+            const float hd[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int r = 0; r < HCR_ROWS; r++) {
+                    const uint32_t w = j == 0 ? wv[r].x : j == 1 ? wv[r].y : j == 2 ? wv[r].z : wv[r].w;
+                    acc2_fma(acc[r], __uint_as_float(w << 16), hd[2 * j]);
+                    acc2_fma(acc[r], __uint_as_float(w & 0xffff0000u), hd[2 * j + 1]);
+                }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < HCR_ROWS; r++) {
+            const Acc2 v = acc2_warp_sum(acc[r]);
+            if (lane == 0) part[warp][k0 + r] = acc2_f64(v);
+        }
+    }
+    __syncthreads();
+    if (tid <= MIX) {
+        double v = 0.0;
+        for (int w = 0; w < NWARPS; w++) v += part[w][tid];
+        dots[tid] = v;
+    }
+    __syncthreads();
+    if (tid < MIX) {
+        const float inv = (float)(1.0 / sqrt(dots[MIX] / (double)ME + (double)a.rms_eps));
+        mx[tid] = (float)(dots[tid] * (double)inv);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // row softmax + eps, then column / row normalisations (src/core/glm53f_ops.c:577-598)
+        const int el = lane < MM ? lane : 0, i = el / M, j = el % M, k = 2 * M + el;
+        const double l = (double)mul_add_unfused(mx[k], a.scale[2], a.base[k]);
+        double top = -INFINITY;
+#pragma unroll
+        for (int jj = 0; jj < M; jj++) top = fmax(top, __shfl_sync(0xffffffffu, l, i * M + jj));
+        const double ex = exp(l - top);
+        double z = 0.0;
+#pragma unroll
+        for (int jj = 0; jj < M; jj++) z += __shfl_sync(0xffffffffu, ex, i * M + jj);
+        const double v = sinkhorn_passes<M>(ex / z + eps, M, i, j, 2 * a.iters - 1, eps);
+        if (lane < MM) a.comb[(size_t)t * MM + lane] = (float)v;
+    } else {
+        constexpr int NT = HCR_THREADS - 32;
+        const int wt = tid - 32;
+        if (wt < M) {
+            pre[wt] = (double)sigmoid_host(mul_add_unfused(mx[wt], a.scale[0], a.base[wt])) + eps;
+            a.post[(size_t)t * M + wt] = __fmul_rn(2.0f, sigmoid_host(mul_add_unfused(mx[M + wt], a.scale[1], a.base[M + wt])));
+        }
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+        // x[d] = sum_i pre[i] * h[i][d] in FP64 (src/core/glm53f_ops.c:603-607), then RMSNorm(x) * w (:473-480)
+        double s2 = 0.0;
+        for (int d = wt; d < E; d += NT) {
+            double v = 0.0;
+#pragma unroll
+            for (int i = 0; i < M; i++) v += pre[i] * (double)hs[i * E + d];
+            const float xv = (float)v;
+            hs[d] = xv;                                          // (this thread alone reads column d)
+            s2 += (double)xv * (double)xv;
+        }
+        __syncwarp();
+        s2 = warp_sum(s2);
+        if (lane == 0) red[warp] = s2;
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+        double tot = 0.0;
+#pragma unroll
+        for (int w = 1; w < NWARPS; w++) tot += red[w];
+        const float f = (float)(1.0 / sqrt(tot / (double)E + (double)a.rms_eps));
+        for (int d = wt; d < E; d += NT) a.xn[(size_t)t * E + d] = __fmul_rn(a.norm_w[d], __fmul_rn(hs[d], f));
+    }
+}
+
+// Two rounds of the clusters that fit the GPU at once (37): from there on the kernel above is the faster one.
+constexpr int HCR_MIN_T = 75;
+
 static bool hc_pre_cluster_takes(int M, int E)
 {
     const int W = E / HCC_CTAS;
@@ -579,6 +750,12 @@ void hc_pre_fused(cudaStream_t st, float *xn, float *post, float *comb, float *h
 {
     HcFused a{xn, post, comb, h, y_pending, static_cast<const uint16_t *>(w.fn.w), w.base, w.scale, norm_w, part,
               counters, M, E, iters, hc_eps, rms_eps};
+    const size_t rows_smem = (size_t)M * E * sizeof(float);
+    static SmemGrant grant;
+    if (T >= HCR_MIN_T && M == HCR_M && E % 8 == 0 && rows_smem <= HCR_MAX_SMEM && dev_opt_in_smem((const void *)hc_pre_rows_kernel, rows_smem + (8 << 10), grant)) {
+        G5B_LAUNCH_PDL(hc_pre_rows_kernel, dim3(T), dim3(HCR_THREADS), rows_smem, st, a);
+        return;
+    }
     if (hc_pre_cluster_takes(M, E)) G5B_LAUNCH_PDL(hc_pre_cluster_kernel, dim3(HCC_CTAS, T), dim3(HCC_THREADS), 0, st, a);
     else                            G5B_LAUNCH(hc_pre_fused_kernel, dim3(HCF_SLICES, T), HC_THREADS, 0, st, a);
 }

@@ -60,3 +60,20 @@ def test_prompt_of_several_attention_chunks(gpu_lib, binding):
         assert common.rel_err(g, w) < 1e-3 and int(g.argmax()) == int(w.argmax())
         g, w = eng.forward([tok])[0], orc.forward([tok])[0]
     eng.close(); orc.close()
+
+
+@pytest.mark.parametrize("hidden", [512, 4096])
+def test_stream_mixing_of_many_positions(gpu_lib, binding, hidden):
+    """More positions than clusters that fit the GPU at once: one CTA per position; the second layer also applies what the
+    first one owes to the streams. Few pieces per thread and many."""
+    c = pkg.Config(hidden=hidden, n_layers=2, vocab=64, rms_eps=1e-5, hc_mult=4, hc_iters=20, hc_eps=1e-6,
+                   kda_heads=4, kda_head_dim=64, conv_k=4, gate_lb=-5.0, mla_heads=4, q_lora=192, kv_lora=128,
+                   qk_nope=64, v_head=64, index_topk=16, index_kpool=4, index_heads=4, index_dim=32,
+                   n_experts=40, topk=2, n_shared=1, moe_inter=128, dense_inter=256, routed_scale=2.5,
+                   norm_topk=1, swiglu_limit=10.0, fp8_block_r=128, fp8_block_c=128)
+    spec = synth.Spec(c, [0, 1], [1, 0], with_head=True)
+    tensors = synth.make_model(spec, seed=23, recipe="spread")
+    eng, orc = common.build_models(spec, tensors, 128, binding)
+    ids = np.random.default_rng(6).integers(0, c.vocab, 85).astype(np.int32)
+    assert common.rel_err(eng.forward(ids)[0], orc.forward(ids)[0]) < 1e-4
+    eng.close(); orc.close()
