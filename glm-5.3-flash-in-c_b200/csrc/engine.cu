@@ -157,6 +157,7 @@ struct g5b_engine {
     double *hc_part = nullptr; int *hc_count = nullptr;  // fused mHC site: partial sums and per-token counters
     void *xterms = nullptr; float *xinv = nullptr;      // batched expert kernels: F16 terms of the activations
     int   *msel, *mnsel;
+    double *rdots;                               // dot products of the router for many tokens
     float *rscore, *rw, *act, *contrib, *gu, *dact;
     int   *ridx;
     MoePlan plan;
@@ -750,7 +751,7 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         walloc(e, &e->mpart, (size_t)MLA_PART_TOKENS * H * ((stride + 31) / 32) * KL)) return -1;
     e->mpart_bytes = (size_t)MLA_PART_TOKENS * H * ((stride + 31) / 32) * KL * sizeof(double);
     const size_t pairs = N * K + N;
-    if (walloc(e, &e->rscore, N * c.n_experts) || walloc(e, &e->rw, N * K) || walloc(e, &e->ridx, N * K) ||
+    if (walloc(e, &e->rdots, (N > RT_TILE_ROWS ? N : (size_t)RT_TILE_ROWS) * c.n_experts) || walloc(e, &e->rscore, N * c.n_experts) || walloc(e, &e->rw, N * K) || walloc(e, &e->ridx, N * K) ||
         walloc(e, &e->act, pairs * (I > SI ? I : SI)) || walloc(e, &e->contrib, pairs * E) ||
         walloc(e, &e->gu, N * 2 * DI) || walloc(e, &e->dact, N * DI) || walloc(e, &e->xinv, pairs) ||
         walloc(e, &e->hc_part, N * 32 * (MIX + 1)) || walloc(e, &e->hc_count, N) ||
@@ -902,7 +903,7 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
         }
     }
     router_plan(e->st, e->ridx, e->rw, e->rscore, x, c.hidden, w.router.w, w.router.dt, w.bias, n, s, e->plan,
-                shared_in_plan ? 1 : 0, e->counter);
+                shared_in_plan ? 1 : 0, e->counter, 0, -1, e->rdots);
     prof_mark(e, 1);
     auto exchange_and_combine = [&]() {
         // every rank computed the rows of the picks it owns: gather all rows everywhere and combine

@@ -13,6 +13,7 @@
 // Sums that decide indices (pool scores) repeat the reference's order in FP64, so equal inputs
 // give bit-equal scores and therefore the same selection, ties included (lower pool wins).
 #include "dot_rows.cuh"
+#include "f64_tile.cuh"
 #include "kernels.h"
 
 namespace g5b {
@@ -362,8 +363,19 @@ __global__ void __launch_bounds__(AB_COLS * AB_GROUPS) mla_absorb_split_kernel(d
     }
 }
 
+constexpr int F64_MIN_T = 13;
 void mla_absorb(cudaStream_t st, double *qa, const float *q, const DMat &kv_b, int T, const MlaShape &s)
 {
+    // From F64_MIN_T positions on in tiles of 32 (64 positions of 64 heads: 230 -> 109 us, the FP64 pipe's own time);
+    // below, a tile would mostly multiply padding.
+    if (T >= F64_MIN_T && kv_b.dt == DT_BF16 && s.KL % 8 == 0 && s.qn % F64_K == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
+        (reinterpret_cast<uintptr_t>(kv_b.w) & 15) == 0) {
+        const size_t kvd = (size_t)(s.qn + s.vh);
+        const F64Tile f{q, static_cast<const uint16_t *>(kv_b.w), qa, (size_t)s.H * s.qn, (size_t)s.KL, (size_t)s.H * s.KL,
+                        (size_t)s.qn, kvd * s.KL, (size_t)s.KL, T, s.KL, s.qn};
+        G5B_LAUNCH(f64_tile_kernel<true>, dim3((s.KL + F64_N - 1) / F64_N, (T + F64_T - 1) / F64_T, s.H), F64_THREADS, 0, st, f);
+        return;
+    }
     if (kv_b.dt == DT_BF16 && s.KL % AB_COLS == 0 && s.qn % (AB_GROUPS * 8) == 0) {
         if (T >= 4) G5B_LAUNCH(mla_absorb_split_kernel<4>, dim3(s.H, (T + 3) / 4, s.KL / AB_COLS), AB_COLS * AB_GROUPS, 0, st, qa, q, kv_b, s, T);
         else        G5B_LAUNCH(mla_absorb_split_kernel<1>, dim3(s.H, T, s.KL / AB_COLS), AB_COLS * AB_GROUPS, 0, st, qa, q, kv_b, s, T);

@@ -12,6 +12,7 @@
 // (token, slot) pairs that chose it, every pair keeps its own output row, and the rows are
 // summed per token in top-k order in FP64 (:1329-1337), the shared expert added last in FP32.
 #include "dot_rows.cuh"
+#include "f64_tile.cuh"
 #include "kernels.h"
 
 namespace g5b {
@@ -42,6 +43,9 @@ struct RouterArgs {
     int n_local0, n_local, with_shared;
     int *counter;
     int sh_t0, sh_n;                 // the shared expert's slot takes tokens [sh_t0, sh_t0 + sh_n)
+    const double *parts;             // optional: the dot products are there already, in n_parts stretches of the columns
+    int n_parts;                     // ([stretch][token][expert], part_stride between stretches); one CTA per token then
+    size_t part_stride;
 };
 
 // Order-preserving key of a selection score; 0 = not selectable (NaN, -inf, already taken).
@@ -111,7 +115,14 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     __shared__ int is_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int e = blockIdx.x * RT_WARPS + warp, t = blockIdx.y;
-    if (e < a.NE) {
+    if (a.parts) {
+        const double *pt = a.parts + (size_t)t * a.NE;
+        for (int i = tid; i < a.NE; i += RT_WARPS * 32) {
+            double acc = __ldcg(pt + i);
+            for (int k = 1; k < a.n_parts; k++) acc += __ldcg(pt + (size_t)k * a.part_stride + i);
+            a.score[(size_t)t * a.NE + i] = sigmoid_host((float)acc);
+        }
+    } else if (e < a.NE) {
         const float *xt = a.x + (size_t)t * a.ldx;
         double acc = 0.0;
         if (a.gate_dt == DT_BF16 && (a.E & 7) == 0 && (a.ldx & 3) == 0) {
@@ -283,17 +294,33 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, 
     }
 }
 
+constexpr int RT_TILE_MIN_T = 13, RT_TILE_CTAS = 600;
 // p may be null-planned (p.n_slots == nullptr) when only the routing is wanted.
 void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float *x, int ldx, const void *gate,
                  int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &p, int with_shared,
-                 int *counter, int shared_t0, int shared_n)
+                 int *counter, int shared_t0, int shared_n, double *dots)
 {
     const bool one = T <= RT_MAX_TOKENS;
+    // From RT_TILE_MIN_T tokens on the dot products go first, in tiles of 32 x 32 and so many stretches of the columns that there
+    // are a few CTAs per SM (64 tokens: 56 us for everything, now 38); below, a tile would mostly multiply padding.
+    int parts = 0, per = s.E;
+    if (T >= RT_TILE_MIN_T && dots && gate_dt == DT_BF16 && s.E % F64_K == 0 && ldx % 4 == 0 &&
+        (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(gate) & 15) == 0) {
+        const int tiles = (T + F64_T - 1) / F64_T * ((s.NE + F64_N - 1) / F64_N), blocks = s.E / F64_K;
+        parts = (RT_TILE_CTAS + tiles - 1) / tiles;
+        if (parts > RT_TILE_ROWS / T) parts = RT_TILE_ROWS / T;
+        if (parts < 1) parts = 1;
+        while (blocks % parts) parts--;                       // equal stretches
+        per = s.E / parts;
+        const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per};
+        G5B_LAUNCH(f64_tile_kernel<false>, dim3((s.NE + F64_N - 1) / F64_N, (T + F64_T - 1) / F64_T, parts), F64_THREADS, 0, st, f);
+    }
     for (int t0 = 0; t0 < T; t0 += RT_MAX_TOKENS) {
         const int n = T - t0 < RT_MAX_TOKENS ? T - t0 : RT_MAX_TOKENS;
         RouterArgs a{idx + (size_t)t0 * s.K, w + (size_t)t0 * s.K, score + (size_t)t0 * s.NE, x + (size_t)t0 * ldx, ldx, gate, gate_dt, bias, s.NE, s.E, s.K, n,
-                     s.norm_topk, s.routed_scale, one ? p : MoePlan{}, s.n_local0, s.n_local, with_shared, counter, shared_t0, shared_n < 0 ? n : shared_n};
-        G5B_LAUNCH(router_kernel, dim3((s.NE + RT_WARPS - 1) / RT_WARPS, n), RT_WARPS * 32, 0, st, a);
+                     s.norm_topk, s.routed_scale, one ? p : MoePlan{}, s.n_local0, s.n_local, with_shared, counter, shared_t0, shared_n < 0 ? n : shared_n,
+                     parts ? dots + (size_t)t0 * s.NE : nullptr, parts, (size_t)T * s.NE};
+        G5B_LAUNCH(router_kernel, dim3(parts ? 1 : (s.NE + RT_WARPS - 1) / RT_WARPS, n), RT_WARPS * 32, 0, st, a);
     }
     if (!one && p.n_slots) G5B_LAUNCH(moe_plan_kernel, 1, PLAN_THREADS, 0, st, idx, T, s.K, s.n_local0, s.n_local, with_shared, p);
 }

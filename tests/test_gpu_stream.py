@@ -77,3 +77,19 @@ def test_stream_mixing_of_many_positions(gpu_lib, binding, hidden):
     ids = np.random.default_rng(6).integers(0, c.vocab, 85).astype(np.int32)
     assert common.rel_err(eng.forward(ids)[0], orc.forward(ids)[0]) < 1e-4
     eng.close(); orc.close()
+
+
+@pytest.mark.parametrize("T", [13, 32, 33, 64, 65, 150])
+def test_router_of_many_tokens(gpu_lib, binding, T):
+    """Tiles of 32 tokens x 32 experts with ragged edges of both, columns in one and in several stretches."""
+    c = synth.tiny_spec().cfg.copy()
+    c.n_layers, c.n_experts, c.topk, c.hidden = 1, 45, 4, 384
+    spec = synth.Spec(c, [0], [0], with_head=False)
+    tensors = synth.make_model(spec, seed=9, recipe="spread")
+    eng, orc = common.build_models(spec, tensors, 64, binding, options={"allow_partial": 1})
+    x = np.random.default_rng(T).standard_normal((T, c.hidden)).astype(np.float32)
+    assert common.rel_err(eng.op_moe(0, x), orc.op_moe(0, x)) < 1e-5
+    gi, gw = eng.last_picks((T - 1) % 64 + 1)
+    wi, ww = orc.op_router(0, x)
+    assert np.array_equal(gi, wi[-len(gi):]) and common.rel_err(gw, ww[-len(gi):]) < 1e-6
+    eng.close(); orc.close()
