@@ -743,7 +743,7 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
     if (walloc(e, &e->mq_raw, N * c.q_lora) || walloc(e, &e->mct, N * KL) || walloc(e, &e->mwk, N * c.index_dim) ||
         walloc(e, &e->mgate, N * c.index_dim) || walloc(e, &e->mwp, N * c.index_heads) ||
         walloc(e, &e->mq, N * H * c.qk_nope) || walloc(e, &e->mqidx, N * (size_t)c.index_heads * c.index_dim) ||
-        walloc(e, &e->mcb, NA * H * KL) || walloc(e, &e->macc, N * H * c.v_head) ||
+        walloc(e, &e->mcb, N * H * KL) || walloc(e, &e->macc, N * H * c.v_head) ||
         walloc(e, &e->mscore, NA * ((size_t)e->cap / c.index_kpool + 1)) || walloc(e, &e->minvq, N) ||
         walloc(e, &e->mqa, NA * H * KL) || walloc(e, &e->mdsc, NA * H * stride) ||
         walloc(e, &e->msel, NA * stride) || walloc(e, &e->mnsel, NA) ||
@@ -1116,6 +1116,10 @@ static bool mla_heads_split(const g5b_engine *e, const Layer &w, const MlaShape 
     return true;
 }
 
+// From this many positions on W_v multiplies all of a call's positions on the tensor cores, eight heads to a launch; its
+// eight launches cost more than mla_vout's one for fewer (64 positions: 145 us there; 2048: 4.6 ms there, 0.5 here).
+constexpr int VOUT_TC_MIN_T = 75;
+
 static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, float *out, bool batch = false)
 {
     const g5b_config &c = e->c;
@@ -1155,7 +1159,12 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
     // The indexer (pool scores, top-k, expansion: two latency-bound kernels) and the absorption of
     // W_k into the query need nothing from each other: the absorption runs on the side stream
     // meanwhile and the main stream takes it back before the scores.
+    const int VR = s.qn + s.vh;                    // rows of kv_b per head: W_k, then W_v
+    bool wide = n >= VOUT_TC_MIN_T && e->tc && e->tensor_gemm != 0 && e->mla_tensor;
+    for (int h = 0; h < Hl && wide; h++)
+        wide = tc_gemm_takes(e->tc, make_seg(row_slice(kvb, h * VR + s.qn, s.vh), e->mcb + (size_t)h * s.KL, Hl * s.KL, e->macc + (size_t)h * s.vh, Hl * s.vh), n);
     for (int t0 = 0; t0 < n; t0 += CHUNK) {
+        float *cb = e->mcb + (wide ? (size_t)t0 * Hl * s.KL : 0);
         const int nt = n - t0 < CHUNK ? n - t0 : CHUNK, at = batch ? cached : cached + t0;
         const float *mq = e->mq + (size_t)t0 * Hl * c.qk_nope;
         bool forked = false, join = false;
@@ -1170,10 +1179,17 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
         if (!forked) mla_absorb(e->st, e->mqa, mq, kvb, nt, sl);
         else if (join && cudaStreamWaitEvent(e->st, e->side_done, 0) != cudaSuccess) cudaStreamSynchronize(e->side);
         if (flash)
-            mla_attend_flash(e->st, e->mcb, e->mqa, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf);
+            mla_attend_flash(e->st, cb, e->mqa, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf);
         else
-            mla_attend(e->st, e->mcb, e->mqa, lat, e->msel, e->mnsel, e->mdsc, e->mpart, e->mstats, e->mcount, MLA_PART_TOKENS, nt, at, sl);
-        mla_vout(e->st, e->macc + (size_t)t0 * Hl * c.v_head, e->mcb, kvb, nt, sl);
+            mla_attend(e->st, cb, e->mqa, lat, e->msel, e->mnsel, e->mdsc, e->mpart, e->mstats, e->mcount, MLA_PART_TOKENS, nt, at, sl);
+        if (!wide) mla_vout(e->st, e->macc + (size_t)t0 * Hl * c.v_head, cb, kvb, nt, sl);
+    }
+    for (int h = 0; h < Hl && wide; h += GEMV_MAX_SEG) {
+        GemvSeg v[GEMV_MAX_SEG];
+        int nv = 0;
+        for (; nv < GEMV_MAX_SEG && h + nv < Hl; nv++)
+            v[nv] = make_seg(row_slice(kvb, (h + nv) * VR + s.qn, s.vh), e->mcb + (size_t)(h + nv) * s.KL, Hl * s.KL, e->macc + (size_t)(h + nv) * s.vh, Hl * s.vh);
+        if (tc_gemm_run(e->tc, e->st, v, nv, n)) return fail("the value projection could not be launched");
     }
     if (ms) {
         GemvSeg o = make_seg(col_slice(w.mo, h0 * s.vh, Hl * s.vh), e->macc, Hl * c.v_head, e->ts_part, E);

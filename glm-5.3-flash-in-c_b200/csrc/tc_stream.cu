@@ -44,7 +44,7 @@
 
 namespace g5b {
 
-constexpr int TS_MAX_SEG = 6;              // matrices of one launch
+constexpr int TS_MAX_SEG = 8;              // matrices of one launch
 constexpr int TS_N = 64;                   // activation rows per tile at most (TC_TILE_ROWS of an expert)
 constexpr int TS_EN = TS_N / 2;            // rows an epilogue thread holds
 constexpr int TS_MAX_STAGES = 6, TS_XS = 2;    // FP8: activation stages, one per converted unit in tensor memory
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(TS_BF16_THREADS, 1) tc_stream_bf16_kernel(cons
 // mid + lo exactly (24 bits), no scaling (BF16 has FP32's exponent range).
 struct TsSplitIn { const float *x, *xinv, *xw; int ldx; };
 struct TsSplit {
-    TsSplitIn in[2];
+    TsSplitIn in[TS_MAX_SEG];
     const int *rows;            // optional: activation row of each output row
     const int *n_rows;          // optional: how many there are (device)
     void *terms;                // [in][term][plane][C]
@@ -695,10 +695,10 @@ __global__ void __launch_bounds__(512) tc_split_kernel(const TsSplit s)
     __shared__ float wmax[16];
     const int b = blockIdx.x, C = s.C;
     if (s.n_rows && b >= *s.n_rows) return;
-    const bool second = blockIdx.y != 0;
-    const float *xinv = second ? s.in[1].xinv : s.in[0].xinv, *xw = second ? s.in[1].xw : s.in[0].xw;
+    const TsSplitIn &in = s.in[blockIdx.y];
+    const float *xinv = in.xinv, *xw = in.xw;
     const int t = s.rows ? s.rows[b] : b;
-    const float *xt = (second ? s.in[1].x : s.in[0].x) + (size_t)t * (second ? s.in[1].ldx : s.in[0].ldx);
+    const float *xt = in.x + (size_t)t * in.ldx;
     const float rinv = xinv ? xinv[t] : 1.0f;
     auto value = [&](int c) {
         float4 v = *reinterpret_cast<const float4 *>(xt + c);
@@ -796,7 +796,7 @@ bool tc_encode(CUtensorMap *m, const void *base, CUtensorMapDataType dt, int elt
 struct TcGemm {
     void *terms = nullptr;          // 16-bit values: [inputs][terms][plane][columns]
     size_t terms_n = 0;             // how many fit
-    float *inv = nullptr;           // [2][plane]
+    float *inv = nullptr;           // [inputs][plane]
     float *part = nullptr;          // partial results of the CTAs
     int *cnt = nullptr;             // units done per tile
     int max_c = 0, max_t = 0, ctas = 0;
@@ -814,7 +814,7 @@ TcGemm *tc_gemm_create(int max_c, int max_t, int *err)
     g->max_c = max_c; g->err = err; g->ctas = dev_sms();
     g->max_t = max_t > TS_N ? max_t : TS_N;
     g->terms_n = (size_t)3 * (g->max_t > 2 * TS_N ? g->max_t : 2 * TS_N) * max_c;
-    if (cudaMalloc(&g->terms, g->terms_n * 2) != cudaSuccess || cudaMalloc((void **)&g->inv, (size_t)2 * g->max_t * 4) != cudaSuccess ||
+    if (cudaMalloc(&g->terms, g->terms_n * 2) != cudaSuccess || cudaMalloc((void **)&g->inv, (size_t)TS_MAX_SEG * g->max_t * 4) != cudaSuccess ||
         cudaMalloc((void **)&g->part, (size_t)g->ctas * 2 * TS_N * 128 * 4) != cudaSuccess ||
         cudaMalloc((void **)&g->cnt, TS_CNT * 4) != cudaSuccess) {
         cudaGetLastError();
@@ -921,7 +921,7 @@ int tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg *segs, int n, int T)
     bool done[GEMV_MAX_SEG] = {};
     for (int first = 0; first < n; first++) {
         if (done[first]) continue;
-        // matrices of one format and width go out together, with at most two different inputs
+        // matrices of one format and width go out together, with as many different inputs as the terms buffer takes
         const bool fp8 = segs[first].dt == DT_FP8;
         const int C = segs[first].C, terms = fp8 ? 2 : 3;
         TsMaps m;
@@ -936,7 +936,7 @@ int tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg *segs, int n, int T)
             if (done[i] || (s.dt == DT_FP8) != fp8 || s.C != C) continue;
             int k = 0;
             while (k < ins && !(sp.in[k].x == s.x && sp.in[k].xinv == s.xinv && sp.in[k].xw == s.xw && sp.in[k].ldx == s.ldx)) k++;
-            if (k == 2 || (size_t)(k + 1) * terms * plane * C > g->terms_n) continue;
+            if ((size_t)(k + 1) * terms * plane * C > g->terms_n) continue;
             if (k == ins) sp.in[ins++] = TsSplitIn{s.x, s.xinv, s.xw, s.ldx};
             const CUtensorMap *w = w_map(g, s.W, fp8, (size_t)s.R, (size_t)C, (size_t)s.ldw);
             if (!w) return -1;
