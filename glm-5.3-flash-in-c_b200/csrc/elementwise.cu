@@ -13,6 +13,8 @@ unsigned long long g_launches = 0;
 // products with inv and the weight are applied by the consumer (gemv prologue or rms_apply).
 __global__ void rms_factor_kernel(const float *x, int n, int ld, float eps, float *inv)
 {
+    pdl_trigger();
+    pdl_wait();
     __shared__ double red[32];
     const float *row = x + (size_t)blockIdx.x * ld;
     double ss = 0.0;
@@ -24,7 +26,7 @@ __global__ void rms_factor_kernel(const float *x, int n, int ld, float eps, floa
 void rms_factor(cudaStream_t st, const float *x, int n, int ld, int rows, float eps, float *inv)
 {
     const int threads = n >= 4096 ? 512 : n >= 512 ? 256 : 64;
-    G5B_LAUNCH(rms_factor_kernel, rows, threads, 0, st, x, n, ld, eps, inv);
+    G5B_LAUNCH_PDL(rms_factor_kernel, dim3(rows), dim3(threads), 0, st, x, n, ld, eps, inv);
 }
 
 __global__ void rms_apply_kernel(float *y, const float *x, const float *w, const float *inv, int n, int ld)
@@ -66,6 +68,8 @@ __device__ __forceinline__ float swiglu_one(float g, float u, float lim)
 
 __global__ void swiglu_kernel(float *y, const float *gu, int n, float lim)
 {
+    pdl_trigger();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float *row = gu + (size_t)blockIdx.y * 2 * n;
@@ -74,7 +78,7 @@ __global__ void swiglu_kernel(float *y, const float *gu, int n, float lim)
 
 void swiglu(cudaStream_t st, float *y, const float *gu, int n, int rows, float limit)
 {
-    G5B_LAUNCH(swiglu_kernel, dim3((n + 255) / 256, rows), 256, 0, st, y, gu, n, limit);
+    G5B_LAUNCH_PDL(swiglu_kernel, dim3((n + 255) / 256, rows), dim3(256), 0, st, y, gu, n, limit);
 }
 
 // -------------------------------------------------------------- ShortConv ----
@@ -127,6 +131,8 @@ void embed_rows(cudaStream_t st, float *h, const DMat &table, const int *ids, in
 // Mean of the residual streams in FP64 (src/model/glm53f_model.c:463-467).
 __global__ void head_mean_kernel(float *xm, const float *h, int M, int E)
 {
+    pdl_trigger();
+    pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= E) return;
     const float *ht = h + (size_t)blockIdx.y * M * E;
@@ -137,7 +143,7 @@ __global__ void head_mean_kernel(float *xm, const float *h, int M, int E)
 
 void head_mean(cudaStream_t st, float *xm, const float *h, int T, int M, int E)
 {
-    G5B_LAUNCH(head_mean_kernel, dim3((E + 255) / 256, T), 256, 0, st, xm, h, M, E);
+    G5B_LAUNCH_PDL(head_mean_kernel, dim3((E + 255) / 256, T), dim3(256), 0, st, xm, h, M, E);
 }
 
 // ----------------------------------------------------------------- argmax ----
@@ -152,6 +158,8 @@ __device__ __forceinline__ void am_better(float &bv, int &bi, float v, int i)
 
 __global__ void argmax_part_kernel(const float *logits, int n, float *pv, int *pi)
 {
+    pdl_trigger();
+    pdl_wait();
     __shared__ float sv[256];
     __shared__ int   si[256];
     const float *row = logits + (size_t)blockIdx.y * n;
@@ -178,6 +186,8 @@ __global__ void argmax_part_kernel(const float *logits, int n, float *pv, int *p
 
 __global__ void argmax_final_kernel(int *out, const float *pv, const int *pi)
 {
+    pdl_trigger();
+    pdl_wait();
     float bv = -INFINITY;
     int bi = 0x7fffffff;
     if (threadIdx.x == 0) {
@@ -189,8 +199,8 @@ __global__ void argmax_final_kernel(int *out, const float *pv, const int *pi)
 void argmax_rows(cudaStream_t st, int *out, const float *logits, int n, int rows, float *scratch_v,
                  int *scratch_i)
 {
-    G5B_LAUNCH(argmax_part_kernel, dim3(AM_PARTS, rows), 256, 0, st, logits, n, scratch_v, scratch_i);
-    G5B_LAUNCH(argmax_final_kernel, rows, 32, 0, st, out, scratch_v, scratch_i);
+    G5B_LAUNCH_PDL(argmax_part_kernel, dim3(AM_PARTS, rows), dim3(256), 0, st, logits, n, scratch_v, scratch_i);
+    G5B_LAUNCH_PDL(argmax_final_kernel, dim3(rows), dim3(32), 0, st, out, scratch_v, scratch_i);
 }
 
 // -------------------------------------------------------- synthetic experts ----

@@ -4,7 +4,8 @@
 // The FP64 pipe (16 FMA per clock and SM) bounds both. A float becomes a double at half that rate, so a loop that
 // converts its factors for every product, or for four, mostly converts; here a CTA converts a 32 x 32 block of each
 // factor once (BF16 by shifting bits, which needs no FP64 instruction) and uses it for 32 products, and a thread holds
-// 4 x 4 sums. Two warps to a CTA, eight CTAs to an SM: products of some CTAs beside the conversions of others.
+// 4 x 4 sums. Two warps to a CTA, eight CTAs to an SM: products of some CTAs beside the conversions of others. Few rows of A:
+// tiles of eight, 1 x 4 sums to a thread, since a tile of 32 would multiply padding for most of its time.
 #pragma once
 
 #include "common.cuh"
@@ -17,7 +18,7 @@ struct F64Tile {
     size_t za, zb, zo;            // elements between the problems of blockIdx.z (heads, or stretches of k)
     int T, N, K;                  // K: a multiple of 32, rows of A and B 16-byte aligned
 };
-constexpr int F64_T = 32, F64_N = 32, F64_K = 32, F64_THREADS = 64, F64_PITCH = 34;
+constexpr int F64_N = 32, F64_K = 32, F64_THREADS = 64, F64_PITCH = 34;
 
 __device__ __forceinline__ double bf16_to_f64(uint32_t h)
 {
@@ -27,23 +28,26 @@ __device__ __forceinline__ double bf16_to_f64(uint32_t h)
 }
 
 // K_ROWS: B's rows run along n (element (k, n) at B[k * ldb + n], N a multiple of 8); otherwise along k (B[n * ldb + k]).
-template <bool K_ROWS>
+template <bool K_ROWS, int TR>
 __global__ void __launch_bounds__(F64_THREADS, 8) f64_tile_kernel(const F64Tile p)
 {
-    __shared__ __align__(16) double sa[F64_K][F64_PITCH], sb[F64_K][F64_PITCH];
+    pdl_trigger();
+    constexpr int F64_T = 8 * TR;                                 // rows of A in a tile
+    __shared__ __align__(16) double sa[F64_K][F64_T + 2], sb[F64_K][F64_PITCH];
     const int tid = threadIdx.x, t0 = blockIdx.y * F64_T, n0 = blockIdx.x * F64_N;
     const float *A = p.A + (size_t)blockIdx.z * p.za;
     const uint16_t *Bm = p.B + (size_t)blockIdx.z * p.zb;
     double *out = p.out + (size_t)blockIdx.z * p.zo;
-    const int row = tid & 31, half = tid >> 5;                    // a thread loads 16 consecutive k of one row
-    const bool arow = t0 + row < p.T;
-    const int tt = (tid >> 3) * 4, nn = (tid & 7) * 4;
-    float4 ra[4];
+    const int row = tid & 31, half = tid >> 5;                    // a thread loads 16 consecutive k of one row of B
+    const int arow = tid % F64_T, ak = tid / F64_T * (4 * TR);    // and 4 TR of one of A
+    const bool alive = t0 + arow < p.T;
+    const int tt = (tid >> 3) * TR, nn = (tid & 7) * 4;
+    float4 ra[TR];
     uint4 rb[2];
     auto load = [&](int k0) {
 #pragma unroll
-        for (int i = 0; i < 4; i++)
-            ra[i] = arow ? *reinterpret_cast<const float4 *>(A + (size_t)(t0 + row) * p.lda + k0 + half * 16 + i * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < TR; i++)
+            ra[i] = alive ? *reinterpret_cast<const float4 *>(A + (size_t)(t0 + arow) * p.lda + k0 + ak + i * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < 2; i++) {
             if (K_ROWS) {
@@ -53,18 +57,18 @@ __global__ void __launch_bounds__(F64_THREADS, 8) f64_tile_kernel(const F64Tile 
                 rb[i] = n0 + row < p.N ? *reinterpret_cast<const uint4 *>(Bm + (size_t)(n0 + row) * p.ldb + k0 + half * 16 + i * 8) : make_uint4(0u, 0u, 0u, 0u);
         }
     };
-    double acc[4][4];
+    double acc[TR][4];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < TR; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) acc[i][j] = 0.0;
     load(0);
     for (int k0 = 0; k0 < p.K; k0 += F64_K) {
         __syncthreads();
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int k = half * 16 + i * 4;
-            sa[k][row] = (double)ra[i].x; sa[k + 1][row] = (double)ra[i].y; sa[k + 2][row] = (double)ra[i].z; sa[k + 3][row] = (double)ra[i].w;
+        for (int i = 0; i < TR; i++) {
+            const int k = ak + i * 4;
+            sa[k][arow] = (double)ra[i].x; sa[k + 1][arow] = (double)ra[i].y; sa[k + 2][arow] = (double)ra[i].z; sa[k + 3][arow] = (double)ra[i].w;
         }
 #pragma unroll
         for (int i = 0; i < 2; i++) {
@@ -85,21 +89,37 @@ __global__ void __launch_bounds__(F64_THREADS, 8) f64_tile_kernel(const F64Tile 
         if (k0 + F64_K < p.K) load(k0 + F64_K);
 #pragma unroll 4
         for (int k = 0; k < F64_K; k++) {
-            const double2 a0 = *reinterpret_cast<const double2 *>(&sa[k][tt]), a1 = *reinterpret_cast<const double2 *>(&sa[k][tt + 2]);
+            double av[TR];
+            if constexpr (TR == 4) {
+                const double2 a0 = *reinterpret_cast<const double2 *>(&sa[k][tt]), a1 = *reinterpret_cast<const double2 *>(&sa[k][tt + 2]);
+                av[0] = a0.x; av[1] = a0.y; av[2] = a1.x; av[3] = a1.y;
+            } else av[0] = sa[k][tt];
             const double2 b0 = *reinterpret_cast<const double2 *>(&sb[k][nn]), b1 = *reinterpret_cast<const double2 *>(&sb[k][nn + 2]);
-            const double av[4] = {a0.x, a0.y, a1.x, a1.y}, bv[4] = {b0.x, b0.y, b1.x, b1.y};
+            const double bv[4] = {b0.x, b0.y, b1.x, b1.y};
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < TR; i++)
 #pragma unroll
                 for (int j = 0; j < 4; j++) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < TR; i++)
         if (t0 + tt + i < p.T)
 #pragma unroll
             for (int j = 0; j < 4; j++)
                 if (n0 + nn + j < p.N) out[(size_t)(t0 + tt + i) * p.ldo + n0 + nn + j] = acc[i][j];
+}
+
+inline int f64_tile_rows(int T) { return T > 16 ? 32 : 8; }      // (two tiles of eight are as fast as one of 32)
+template <bool K_ROWS>
+void f64_tile(cudaStream_t st, const F64Tile &p, int z)
+{
+    const int rows = f64_tile_rows(p.T);
+    const dim3 grid((p.N + F64_N - 1) / F64_N, (p.T + rows - 1) / rows, z);
+    // (launched the ordinary way: launched early, the CTAs crowd the SMs that the kernel in front has left, eight to an SM, and
+    // the FP64 pipes of the others idle - 486 us became 963)
+    if (rows == 32) G5B_LAUNCH((f64_tile_kernel<K_ROWS, 4>), grid, F64_THREADS, 0, st, p);
+    else            G5B_LAUNCH((f64_tile_kernel<K_ROWS, 1>), grid, F64_THREADS, 0, st, p);
 }
 
 }  // namespace g5b

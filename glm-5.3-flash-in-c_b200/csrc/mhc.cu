@@ -764,6 +764,8 @@ void hc_pre_fused(cudaStream_t st, float *xn, float *post, float *comb, float *h
 // every stream (src/core/glm53f_ops.c:612-625; note comb is used transposed).
 __global__ void hc_post_kernel(float *h, const float *y, const float *post, const float *comb, int M, int E)
 {
+    pdl_trigger();
+    pdl_wait();
     const int t = blockIdx.y;
     const int d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= E) return;
@@ -782,7 +784,7 @@ __global__ void hc_post_kernel(float *h, const float *y, const float *post, cons
 void hc_post(cudaStream_t st, float *h, const float *y, const float *post, const float *comb, int T,
              int M, int E)
 {
-    G5B_LAUNCH(hc_post_kernel, dim3((E + 127) / 128, T), 128, 0, st, h, y, post, comb, M, E);
+    G5B_LAUNCH_PDL(hc_post_kernel, dim3((E + 127) / 128, T), dim3(128), 0, st, h, y, post, comb, M, E);
 }
 
 }  // namespace g5b

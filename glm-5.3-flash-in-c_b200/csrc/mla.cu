@@ -140,45 +140,59 @@ void mla_store(cudaStream_t st, void *latent, float *idx_state, const float *ct_
 // ------------------------------------------------------------------- select ----
 // score[pool] = (float) sum_h w[h]/sqrt(heads) * relu((q_h . P_pool)/sqrt(dim)), FP64, heads and
 // dimensions in ascending order as the reference sums them (glm53f_dsa.c:141-157). A lane owns a
-// head's dot product; lane 0 then adds the heads in order.
-constexpr int DSA_WARPS = 8;
+// head's dot products with DSA_POOLS pools; a lane per pool then adds the heads in order.
+// Bound by the FP64 pipe, and with few pools per warp by the latency of its chains: both factors therefore become
+// doubles once, not for every product, four pools share a chain, and what is not a sum (the weights' products) is
+// taken out of the serial part. 8192 pools, 32 heads of 128: 35 us before, 13 now.
+constexpr int DSA_WARPS = 8, DSA_POOLS = 4;
 __global__ void __launch_bounds__(DSA_WARPS * 32) dsa_score_kernel(
     float *score, const float *idx_state, const float *qidx, const float *wproj, int cached, MlaShape s)
 {
-    extern __shared__ float dsa_smem[];
-    float  *qT = dsa_smem;                                   // [ID][IH]
-    double *dh = reinterpret_cast<double *>(dsa_smem + (size_t)s.ID * s.IH);   // [warps][IH]
+    pdl_trigger();
+    extern __shared__ __align__(16) double dsa_smem[];
+    double *qT = dsa_smem;                                                                   // [ID][IH]
     const int t = blockIdx.y, p = pos_of(s, cached, t);
     idx_state = seq_idx(const_cast<float *>(idx_state), s, t);
     const int np = (p + 1) / s.KP;
-    if (np <= s.topk / s.KP) return;
+    if (np <= s.topk / s.KP || (int)blockIdx.x * DSA_WARPS * DSA_POOLS >= np) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double *mine = qT + (((size_t)s.ID * s.IH + 1) & ~(size_t)1) + (size_t)warp * DSA_POOLS * (s.IH + s.ID);   // [pools][IH]: the heads' terms
+    double *pks = mine + (size_t)DSA_POOLS * s.IH;                                           // [ID][pools]: this warp's pooled keys
     const float *q = qidx + (size_t)t * s.IH * s.ID, *wt = wproj + (size_t)t * s.IH;
-    for (int e = threadIdx.x; e < s.IH * s.ID; e += blockDim.x) qT[(e % s.ID) * s.IH + e / s.ID] = q[e];
+    for (int e = threadIdx.x; e < s.IH * s.ID; e += blockDim.x) {
+        const int h = e % s.IH, i = e / s.IH;
+        qT[e] = (double)q[(size_t)h * s.ID + i];
+    }
     __syncthreads();
     const float hscale = 1.0f / sqrtf((float)s.IH), dscale = 1.0f / sqrtf((float)s.ID);
-    double *mine = dh + (size_t)warp * s.IH;
-    float *pks = reinterpret_cast<float *>(dh + (size_t)DSA_WARPS * s.IH) + (size_t)warp * s.ID;   // this warp's pooled key
-    for (int pp = blockIdx.x * DSA_WARPS + warp; pp < np; pp += gridDim.x * DSA_WARPS) {
-        const float *pk = idx_state + ((size_t)2 * s.cap + pp) * s.ID;
-        // the key goes to shared memory in one coalesced load: read from global inside the dot
-        // product, every one of its ID dependent steps waited for a load
-        for (int i = lane; i < s.ID; i += 32) pks[i] = pk[i];
+    for (int p0 = (blockIdx.x * DSA_WARPS + warp) * DSA_POOLS; p0 < np; p0 += gridDim.x * DSA_WARPS * DSA_POOLS) {
+        const int n = min(DSA_POOLS, np - p0);
+        const float *pk = idx_state + ((size_t)2 * s.cap + p0) * s.ID;
+        for (int i = lane; i < s.ID; i += 32)
+#pragma unroll
+            for (int j = 0; j < DSA_POOLS; j++) pks[i * DSA_POOLS + j] = j < n ? (double)pk[(size_t)j * s.ID + i] : 0.0;
         __syncwarp();
         for (int h = lane; h < s.IH; h += 32) {
-            double d = 0.0;
+            double d[DSA_POOLS] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 8
-            for (int i = 0; i < s.ID; i++) d = fma((double)qT[i * s.IH + h], (double)pks[i], d);
-            mine[h] = __dmul_rn(d, (double)dscale);
+            for (int i = 0; i < s.ID; i++) {
+                const double qv = qT[i * s.IH + h];
+                const double2 k0 = *reinterpret_cast<const double2 *>(pks + i * DSA_POOLS), k1 = *reinterpret_cast<const double2 *>(pks + i * DSA_POOLS + 2);
+                d[0] = fma(qv, k0.x, d[0]); d[1] = fma(qv, k0.y, d[1]); d[2] = fma(qv, k1.x, d[2]); d[3] = fma(qv, k1.y, d[3]);
+            }
+            const double wh = __dmul_rn((double)wt[h], (double)hscale);
+#pragma unroll
+            for (int j = 0; j < DSA_POOLS; j++) {
+                const double v = __dmul_rn(d[j], (double)dscale);
+                mine[j * s.IH + h] = v > 0.0 ? __dmul_rn(wh, v) : 0.0;          // (a head that does not count adds nothing)
+            }
         }
         __syncwarp();
-        if (lane == 0) {
+        if (lane < n) {
             double acc = 0.0;
-            for (int h = 0; h < s.IH; h++) {
-                const double d = mine[h];
-                if (d > 0.0) acc = __dadd_rn(acc, __dmul_rn(__dmul_rn((double)wt[h], (double)hscale), d));
-            }
-            score[(size_t)t * (s.cap / s.KP + 1) + pp] = (float)acc;
+#pragma unroll 8
+            for (int h = 0; h < s.IH; h++) acc = __dadd_rn(acc, mine[lane * s.IH + h]);
+            score[(size_t)t * (s.cap / s.KP + 1) + p0 + lane] = (float)acc;
         }
         __syncwarp();
     }
@@ -188,7 +202,7 @@ __global__ void __launch_bounds__(DSA_WARPS * 32) dsa_score_kernel(
 // the reference's qsort comparator, glm53f_dsa.c:111-116), by radix selection on a 64-bit key,
 // then an order-preserving compaction: kept pools ascending, each expanded to its positions, then
 // the incomplete tail pool.
-constexpr int TOPK_THREADS = 1024;
+constexpr int TOPK_THREADS = 1024, TOPK_KEEP = 8;      // scores a thread keeps in registers: 8192 pools, the rest is read again
 __device__ __forceinline__ unsigned long long rank_key(float sc, int pool)
 {
     if (sc == 0.0f) sc = 0.0f;                                    // -0 and +0 compare equal
@@ -204,26 +218,40 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(int *sel, int *n
     pdl_wait();
     __shared__ int hist[256];
     __shared__ unsigned long long prefix_s;
-    __shared__ int want_s;
-    __shared__ int scan[TOPK_THREADS];
+    __shared__ int want_s, exact_s;
+    __shared__ int scan[TOPK_KEEP * (TOPK_THREADS / 32)];
     const int t = blockIdx.x, p = pos_of(s, cached, t), tid = threadIdx.x;
     const int np = (p + 1) / s.KP, keep = s.topk / s.KP;
     int *out = sel + (size_t)t * (s.topk + s.KP);
     if (np <= keep) { if (tid == 0) nsel[t] = -1; return; }
     const float *sc = score + (size_t)t * (s.cap / s.KP + 1);
 
+    float own[TOPK_KEEP];                                          // pool tid + 1024 k in place k
+#pragma unroll
+    for (int k = 0; k < TOPK_KEEP; k++) own[k] = tid + k * TOPK_THREADS < np ? sc[tid + k * TOPK_THREADS] : 0.f;
+
     // the keep-th largest key, one byte at a time from the top
-    if (tid == 0) { prefix_s = 0ull; want_s = keep; }
+    // (most scores share their upper bits: a warp counts equal digits before it touches the histogram. The search ends as
+    // soon as the digit's pools are just those still wanted, usually after the score's own four bytes: the other four
+    // only tell equal scores apart)
+    if (tid == 0) { prefix_s = 0ull; want_s = keep; exact_s = 0; }
     __syncthreads();
-    for (int shift = 56; shift >= 0; shift -= 8) {
+    for (int shift = 56; shift >= 0 && !exact_s; shift -= 8) {
         if (tid < 256) hist[tid] = 0;
         __syncthreads();
         const unsigned long long prefix = prefix_s;
         const unsigned long long mask = shift == 56 ? 0ull : (~0ull << (shift + 8));
-        for (int i = tid; i < np; i += TOPK_THREADS) {
-            const unsigned long long k = rank_key(sc[i], i);
-            if ((k & mask) == prefix) atomicAdd(&hist[(int)((k >> shift) & 0xff)], 1);
-        }
+        auto count = [&](int i, float v) {
+            const unsigned long long k = rank_key(v, i);
+            const int digit = i < np && (k & mask) == prefix ? (int)((k >> shift) & 0xff) : -1;
+            const unsigned same = __match_any_sync(0xffffffffu, digit);
+            if (digit >= 0 && (tid & 31) == __ffs(same) - 1) atomicAdd(&hist[digit], __popc(same));
+            __syncwarp();
+        };
+#pragma unroll
+        for (int k = 0; k < TOPK_KEEP; k++)
+            if (k * TOPK_THREADS < np) count(tid + k * TOPK_THREADS, own[k]);
+        for (int i0 = TOPK_KEEP * TOPK_THREADS; i0 < np; i0 += TOPK_THREADS) count(i0 + tid, i0 + tid < np ? sc[i0 + tid] : 0.f);
         __syncthreads();
         if (tid < 32) {
             // the digit holding the want-th largest key: lane l owns digits 255 - 8l .. 248 - 8l; a warp
@@ -250,31 +278,52 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(int *sel, int *n
                 if (dgt < 0) dgt = 0;
                 prefix_s = prefix | ((unsigned long long)dgt << shift);
                 want_s = w;
+                exact_s = hist[dgt] == w;
             }
         }
         __syncthreads();
     }
-    const unsigned long long threshold = prefix_s;     // keys are distinct: exactly `keep` are >= it
+    const unsigned long long threshold = prefix_s;     // exactly `keep` keys are >= it (keys are distinct)
 
-    // order-preserving compaction over pool index
-    const int per = (np + TOPK_THREADS - 1) / TOPK_THREADS;
-    const int lo = min(np, tid * per), hi = min(np, lo + per);
-    int mine = 0;
-    for (int i = lo; i < hi; i++) mine += rank_key(sc[i], i) >= threshold;
-    scan[tid] = mine;
-    __syncthreads();
-    for (int o = 1; o < TOPK_THREADS; o <<= 1) {
-        const int v = tid >= o ? scan[tid - o] : 0;
+    // order-preserving compaction over pool index, 8192 pools at a time: pool tid + 1024 k of them is the lane's in place
+    // (k, warp); the places' counts are scanned
+    constexpr int NW = TOPK_THREADS / 32, PLACES = TOPK_KEEP * NW;
+    const int warp = tid >> 5, lane = tid & 31;
+    int before = 0;                                                // kept so far
+    for (int p0 = 0; p0 < np; p0 += TOPK_KEEP * TOPK_THREADS) {
+        unsigned kept[TOPK_KEEP];
+#pragma unroll
+        for (int k = 0; k < TOPK_KEEP; k++) {
+            const int i = p0 + tid + k * TOPK_THREADS;
+            if (p0) own[k] = i < np ? sc[i] : 0.f;
+            kept[k] = __ballot_sync(0xffffffffu, i < np && rank_key(own[k], i) >= threshold);
+            if (lane == 0) scan[k * NW + warp] = __popc(kept[k]);
+        }
         __syncthreads();
-        scan[tid] += v;
+        if (warp == 0) {
+            int c[PLACES / 32], tot = 0;
+#pragma unroll
+            for (int j = 0; j < PLACES / 32; j++) { c[j] = tot; tot += scan[lane * (PLACES / 32) + j]; }
+            int incl = tot;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+#pragma unroll
+            for (int j = 0; j < PLACES / 32; j++) scan[lane * (PLACES / 32) + j] = incl - tot + c[j];
+            if (lane == 31) want_s = incl;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < TOPK_KEEP; k++) {
+            const int i = p0 + tid + k * TOPK_THREADS, at = before + scan[k * NW + warp] + __popc(kept[k] & ((1u << lane) - 1u));
+            if (kept[k] >> lane & 1u)
+                for (int j = 0; j < s.KP; j++) out[at * s.KP + j] = i * s.KP + j;
+        }
+        before += want_s;
         __syncthreads();
     }
-    int at = scan[tid] - mine;
-    for (int i = lo; i < hi; i++)
-        if (rank_key(sc[i], i) >= threshold) {
-            for (int j = 0; j < s.KP; j++) out[at * s.KP + j] = i * s.KP + j;
-            at++;
-        }
     const int base = keep * s.KP;
     for (int j = np * s.KP + tid; j <= p; j += TOPK_THREADS) out[base + (j - np * s.KP)] = j;
     if (tid == 0) nsel[t] = base + (p - np * s.KP + 1);
@@ -285,10 +334,12 @@ void dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, co
 {
     const int np_max = (cached + (s.batch ? 1 : T)) / s.KP;
     if (np_max > s.topk / s.KP) {
-        const size_t smem = (size_t)s.ID * s.IH * sizeof(float) + (size_t)DSA_WARPS * s.IH * sizeof(double) +
-                            (size_t)DSA_WARPS * s.ID * sizeof(float);
-        int blocks = (np_max + DSA_WARPS - 1) / DSA_WARPS;
-        if (blocks > 296) blocks = 296;
+        const size_t smem = ((((size_t)s.ID * s.IH + 1) & ~(size_t)1) + (size_t)DSA_WARPS * DSA_POOLS * (s.IH + s.ID)) * sizeof(double);
+        static SmemGrant grant;
+        if (!dev_opt_in_smem((const void *)dsa_score_kernel, smem, grant)) return;
+        const int want = (np_max + DSA_WARPS * DSA_POOLS - 1) / (DSA_WARPS * DSA_POOLS);
+        int blocks = (444 + T - 1) / T > 32 ? (444 + T - 1) / T : 32;                        // (three fit an SM; each converts the query's heads first)
+        if (blocks > want) blocks = want;
         G5B_LAUNCH(dsa_score_kernel, dim3(blocks, T), DSA_WARPS * 32, smem, st, score, idx_state, qidx, wproj, cached, s);
     }
     G5B_LAUNCH_PDL(dsa_topk_kernel, T, TOPK_THREADS, 0, st, sel, nsel, score, cached, s);
@@ -327,58 +378,42 @@ __global__ void mla_absorb_kernel(double *qa, const float *q, const DMat kv_b, M
 // The same sums with the GPU filled: a CTA takes 128 latent columns of one head, its eight row
 // groups (32 rows each at qk_nope = 256) accumulate in FP64 and are added in ascending order.
 constexpr int AB_COLS = 128, AB_GROUPS = 8;
-// TT queries per block (blockIdx.y = group of TT): a weight is read once for all of them; every query's
-// sum is taken in the same order as alone.
-template <int TT>
-__global__ void __launch_bounds__(AB_COLS * AB_GROUPS) mla_absorb_split_kernel(double *qa, const float *q, const DMat kv_b,
-                                                                              MlaShape s, int T)
+__global__ void __launch_bounds__(AB_COLS * AB_GROUPS) mla_absorb_split_kernel(double *qa, const float *q, const DMat kv_b, MlaShape s)
 {
-    __shared__ double part[TT][AB_GROUPS][AB_COLS];
-    const int h = blockIdx.x, t0 = blockIdx.y * TT, c = blockIdx.z * AB_COLS + (threadIdx.x % AB_COLS), grp = threadIdx.x / AB_COLS;
+    __shared__ double part[AB_GROUPS][AB_COLS];
+    extern __shared__ double ab_q[];                     // the head's query: converted once, not for every column
+    const int h = blockIdx.x, t = blockIdx.y, c = blockIdx.z * AB_COLS + (threadIdx.x % AB_COLS), grp = threadIdx.x / AB_COLS;
     const int kvd = s.qn + s.vh, per = s.qn / AB_GROUPS;
-    const float *qt[TT];
-#pragma unroll
-    for (int k = 0; k < TT; k++) qt[k] = q + ((size_t)min(t0 + k, T - 1) * s.H + h) * s.qn + grp * per;   // past the last query: repeated, unused
+    const float *qt = q + ((size_t)t * s.H + h) * s.qn;
     const uint16_t *w = static_cast<const uint16_t *>(kv_b.w) + ((size_t)h * kvd + (size_t)grp * per) * s.KL + c;
-    double acc[TT];
-#pragma unroll
-    for (int k = 0; k < TT; k++) acc[k] = 0.0;
+    for (int i = threadIdx.x; i < s.qn; i += AB_COLS * AB_GROUPS) ab_q[i] = (double)qt[i];
+    __syncthreads();
+    double acc = 0.0;
 #pragma unroll 8
-    for (int i = 0; i < per; i++) {
-        const double wv = (double)bf16_to_f32(w[(size_t)i * s.KL]);
-#pragma unroll
-        for (int k = 0; k < TT; k++) acc[k] = fma((double)qt[k][i], wv, acc[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < TT; k++) part[k][grp][threadIdx.x % AB_COLS] = acc[k];
+    for (int i = 0; i < per; i++) acc = fma(ab_q[grp * per + i], bf16_to_f64(w[(size_t)i * s.KL]), acc);
+    part[grp][threadIdx.x % AB_COLS] = acc;
     __syncthreads();
     if (grp == 0) {
+        double sum = part[0][threadIdx.x];
 #pragma unroll
-        for (int k = 0; k < TT; k++) {
-            double sum = part[k][0][threadIdx.x];
-#pragma unroll
-            for (int g = 1; g < AB_GROUPS; g++) sum += part[k][g][threadIdx.x];
-            if (t0 + k < T) qa[((size_t)(t0 + k) * s.H + h) * s.KL + c] = sum;
-        }
+        for (int g = 1; g < AB_GROUPS; g++) sum += part[g][threadIdx.x];
+        qa[((size_t)t * s.H + h) * s.KL + c] = sum;
     }
 }
 
-constexpr int F64_MIN_T = 13;
 void mla_absorb(cudaStream_t st, double *qa, const float *q, const DMat &kv_b, int T, const MlaShape &s)
 {
-    // From F64_MIN_T positions on in tiles of 32 (64 positions of 64 heads: 230 -> 109 us, the FP64 pipe's own time);
-    // below, a tile would mostly multiply padding.
-    if (T >= F64_MIN_T && kv_b.dt == DT_BF16 && s.KL % 8 == 0 && s.qn % F64_K == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
+    // Several positions in tiles (64 positions of 64 heads: 230 -> 109 us, the FP64 pipe's own time; 7: 49 -> 42 us).
+    if (T > 1 && kv_b.dt == DT_BF16 && s.KL % 8 == 0 && s.qn % F64_K == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(kv_b.w) & 15) == 0) {
         const size_t kvd = (size_t)(s.qn + s.vh);
         const F64Tile f{q, static_cast<const uint16_t *>(kv_b.w), qa, (size_t)s.H * s.qn, (size_t)s.KL, (size_t)s.H * s.KL,
                         (size_t)s.qn, kvd * s.KL, (size_t)s.KL, T, s.KL, s.qn};
-        G5B_LAUNCH(f64_tile_kernel<true>, dim3((s.KL + F64_N - 1) / F64_N, (T + F64_T - 1) / F64_T, s.H), F64_THREADS, 0, st, f);
+        f64_tile<true>(st, f, s.H);
         return;
     }
-    if (kv_b.dt == DT_BF16 && s.KL % AB_COLS == 0 && s.qn % (AB_GROUPS * 8) == 0) {
-        if (T >= 4) G5B_LAUNCH(mla_absorb_split_kernel<4>, dim3(s.H, (T + 3) / 4, s.KL / AB_COLS), AB_COLS * AB_GROUPS, 0, st, qa, q, kv_b, s, T);
-        else        G5B_LAUNCH(mla_absorb_split_kernel<1>, dim3(s.H, T, s.KL / AB_COLS), AB_COLS * AB_GROUPS, 0, st, qa, q, kv_b, s, T);
+    if (kv_b.dt == DT_BF16 && s.KL % AB_COLS == 0 && s.qn % (AB_GROUPS * 8) == 0 && s.qn <= 4096) {
+        G5B_LAUNCH(mla_absorb_split_kernel, dim3(s.H, T, s.KL / AB_COLS), AB_COLS * AB_GROUPS, (size_t)s.qn * sizeof(double), st, qa, q, kv_b, s);
         return;
     }
     G5B_LAUNCH(mla_absorb_kernel, dim3(s.H, T), s.KL >= 512 ? 512 : 128, 0, st, qa, q, kv_b, s);

@@ -109,6 +109,8 @@ __device__ void topk_one_token(const RouterArgs &a, int t, int lane)
 
 __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs a)
 {
+    pdl_trigger();
+    pdl_wait();
     __shared__ int sidx_buf[RT_MAX_TOKENS * G5B_MAX_TOPK];
     __shared__ int cnt[G5B_MAX_EXPERTS], off[G5B_MAX_EXPERTS];
     __shared__ int psum[RT_WARPS * 32], ssum[RT_WARPS * 32], tsum[RT_WARPS * 32];
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
         const double *pt = a.parts + (size_t)t * a.NE;
         for (int i = tid; i < a.NE; i += RT_WARPS * 32) {
             double acc = __ldcg(pt + i);
+#pragma unroll 8
             for (int k = 1; k < a.n_parts; k++) acc += __ldcg(pt + (size_t)k * a.part_stride + i);
             a.score[(size_t)t * a.NE + i] = sigmoid_host((float)acc);
         }
@@ -244,6 +247,8 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
 constexpr int PLAN_THREADS = 1024;
 __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, int T, int K, int n_local0, int n_local, int with_shared, MoePlan p)
 {
+    pdl_trigger();
+    pdl_wait();
     __shared__ int cnt[G5B_MAX_EXPERTS], off[G5B_MAX_EXPERTS];
     __shared__ int wsum[3][PLAN_THREADS / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = T * K;
@@ -294,35 +299,37 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, 
     }
 }
 
-constexpr int RT_TILE_MIN_T = 13, RT_TILE_CTAS = 600;
+constexpr int RT_TILE_MIN_T = 17, RT_TILE_CTAS = 600, RT_MAX_PARTS = 32;
 // p may be null-planned (p.n_slots == nullptr) when only the routing is wanted.
 void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float *x, int ldx, const void *gate,
                  int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &p, int with_shared,
                  int *counter, int shared_t0, int shared_n, double *dots)
 {
     const bool one = T <= RT_MAX_TOKENS;
-    // From RT_TILE_MIN_T tokens on the dot products go first, in tiles of 32 x 32 and so many stretches of the columns that there
-    // are a few CTAs per SM (64 tokens: 56 us for everything, now 38); below, a tile would mostly multiply padding.
+    // From RT_TILE_MIN_T tokens on the dot products go first, in tiles and so many stretches of the columns that there are a few
+    // CTAs per SM (64 tokens: 56 us for everything, now 38); below, adding up the stretches costs more than they save (7 tokens:
+    // 21 us in one kernel, 36 in two).
     int parts = 0, per = s.E;
     if (T >= RT_TILE_MIN_T && dots && gate_dt == DT_BF16 && s.E % F64_K == 0 && ldx % 4 == 0 &&
         (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(gate) & 15) == 0) {
-        const int tiles = (T + F64_T - 1) / F64_T * ((s.NE + F64_N - 1) / F64_N), blocks = s.E / F64_K;
+        const int rows = f64_tile_rows(T), tiles = (T + rows - 1) / rows * ((s.NE + F64_N - 1) / F64_N), blocks = s.E / F64_K;
         parts = (RT_TILE_CTAS + tiles - 1) / tiles;
         if (parts > RT_TILE_ROWS / T) parts = RT_TILE_ROWS / T;
+        if (parts > RT_MAX_PARTS) parts = RT_MAX_PARTS;
         if (parts < 1) parts = 1;
         while (blocks % parts) parts--;                       // equal stretches
         per = s.E / parts;
         const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per};
-        G5B_LAUNCH(f64_tile_kernel<false>, dim3((s.NE + F64_N - 1) / F64_N, (T + F64_T - 1) / F64_T, parts), F64_THREADS, 0, st, f);
+        f64_tile<false>(st, f, parts);
     }
     for (int t0 = 0; t0 < T; t0 += RT_MAX_TOKENS) {
         const int n = T - t0 < RT_MAX_TOKENS ? T - t0 : RT_MAX_TOKENS;
         RouterArgs a{idx + (size_t)t0 * s.K, w + (size_t)t0 * s.K, score + (size_t)t0 * s.NE, x + (size_t)t0 * ldx, ldx, gate, gate_dt, bias, s.NE, s.E, s.K, n,
                      s.norm_topk, s.routed_scale, one ? p : MoePlan{}, s.n_local0, s.n_local, with_shared, counter, shared_t0, shared_n < 0 ? n : shared_n,
                      parts ? dots + (size_t)t0 * s.NE : nullptr, parts, (size_t)T * s.NE};
-        G5B_LAUNCH(router_kernel, dim3(parts ? 1 : (s.NE + RT_WARPS - 1) / RT_WARPS, n), RT_WARPS * 32, 0, st, a);
+        G5B_LAUNCH_PDL(router_kernel, dim3(parts ? 1 : (s.NE + RT_WARPS - 1) / RT_WARPS, n), dim3(RT_WARPS * 32), 0, st, a);
     }
-    if (!one && p.n_slots) G5B_LAUNCH(moe_plan_kernel, 1, PLAN_THREADS, 0, st, idx, T, s.K, s.n_local0, s.n_local, with_shared, p);
+    if (!one && p.n_slots) G5B_LAUNCH_PDL(moe_plan_kernel, dim3(1), dim3(PLAN_THREADS), 0, st, idx, T, s.K, s.n_local0, s.n_local, with_shared, p);
 }
 
 // ----------------------------------------------------------------- experts ----
@@ -513,6 +520,8 @@ void moe_down(cudaStream_t st, float *contrib, const float *act, const ExpertW *
 __global__ void moe_combine_kernel(float *out, int ldo, const float *contrib, const float *w, int T, int K,
                                    int E, int with_shared)
 {
+    pdl_trigger();
+    pdl_wait();
     const int t = blockIdx.y;
     const int d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= E) return;
@@ -527,7 +536,7 @@ __global__ void moe_combine_kernel(float *out, int ldo, const float *contrib, co
 void moe_combine(cudaStream_t st, float *out, int ldo, const float *contrib, const float *w, int T,
                  const MoeShape &s, int with_shared)
 {
-    G5B_LAUNCH(moe_combine_kernel, dim3((s.E + 255) / 256, T), 256, 0, st, out, ldo, contrib, w, T, s.K, s.E,
+    G5B_LAUNCH_PDL(moe_combine_kernel, dim3((s.E + 255) / 256, T), dim3(256), 0, st, out, ldo, contrib, w, T, s.K, s.E,
                with_shared);
 }
 

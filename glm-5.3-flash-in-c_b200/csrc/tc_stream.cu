@@ -335,7 +335,9 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
     }
     if (warp == 18) tmem_alloc(&s_tmem, 512);
     tc_fence_before();
-    pdl_wait();
+    // A projection's weights and their shares depend on nothing in front: they are under way while the kernel before this one
+    // runs, and only the warps that read its results (the terms) or write (sums) wait. What an expert's tile is, the router says.
+    if (MODE != TS_DENSE) pdl_wait();
     int n_tiles = a.tiles;
     TsPlan plan{s_plan, s_plan + a.slots + 1, s_plan + 2 * a.slots + 1, s_plan + 3 * a.slots + 1, 0};
     if (MODE != TS_DENSE) {
@@ -378,6 +380,7 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
         __syncwarp();
     } else if (warp == 17) {
         // ---------------------------------------------------------- activation terms ----
+        if (MODE == TS_DENSE) pdl_wait();
         if (elect_one()) {
             int s = 0, ph = 1, issued = 0;
             TS_WALK(t, {
@@ -469,6 +472,7 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
         }
     } else {
         // ------------------------------------------------- epilogue: scale, sum, finish, store ----
+        if (MODE == TS_DENSE) pdl_wait();
         const int quarter = warp & 3, eg = warp >> 2;
         const int row = quarter * 32 + lane;                         // lane of tensor memory = weight row of the tile
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
@@ -581,7 +585,6 @@ __global__ void __launch_bounds__(TS_BF16_THREADS, 1) tc_stream_bf16_kernel(cons
     }
     if (warp == 9) tmem_alloc(&s_tmem, 512);
     tc_fence_before();
-    pdl_wait();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
@@ -593,12 +596,25 @@ __global__ void __launch_bounds__(TS_BF16_THREADS, 1) tc_stream_bf16_kernel(cons
 
     if (warp == 8) {
         if (elect_one()) {
+            // the first stages' weights while the kernel in front runs, their terms after it
+            int early = 0;
+            TS_WALK(t, {
+                for (int kb = kb0; kb < kb1 && early < WS; kb++, early++) {
+                    mbar_expect_tx(&full[early], (uint32_t)(TS_UNIT_BYTES + 6 * t.n * 128));
+                    tma_load_3d(smem + (size_t)early * SB, &maps.w[t.which], 0, t.rt * 128, kb * 2, &full[early]);
+                }
+                ok = early < WS;
+            });
+            ok = true;
+            pdl_wait();
             int s = 0, ph = 1, issued = 0;
             TS_WALK(t, {
                 for (int kb = kb0; kb < kb1; kb++) {
                     if (issued >= WS && !(ok = mbar_wait(&empty[s], (uint32_t)ph, a.err, 41))) break;
-                    mbar_expect_tx(&full[s], (uint32_t)(TS_UNIT_BYTES + 6 * t.n * 128));
-                    tma_load_3d(smem + (size_t)s * SB, &maps.w[t.which], 0, t.rt * 128, kb * 2, &full[s]);
+                    if (issued >= early) {
+                        mbar_expect_tx(&full[s], (uint32_t)(TS_UNIT_BYTES + 6 * t.n * 128));
+                        tma_load_3d(smem + (size_t)s * SB, &maps.w[t.which], 0, t.rt * 128, kb * 2, &full[s]);
+                    }
                     tma_load_4d(smem + (size_t)s * SB + TS_UNIT_BYTES, &maps.x[t.n / 8 - 1], 0, t.row0, 0, kb * 2, &full[s]);
                     issued++;
                     if (++s == WS) { s = 0; ph ^= 1; }
@@ -633,6 +649,7 @@ __global__ void __launch_bounds__(TS_BF16_THREADS, 1) tc_stream_bf16_kernel(cons
         }
         __syncwarp();
     } else {
+        pdl_wait();
         const int quarter = warp & 3, eg = warp >> 2, e0 = eg * TS_EN, row = quarter * 32 + lane;
         const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
         const TsEpi<false, MODE> ep{};

@@ -79,7 +79,7 @@ def test_stream_mixing_of_many_positions(gpu_lib, binding, hidden):
     eng.close(); orc.close()
 
 
-@pytest.mark.parametrize("T", [13, 32, 33, 64, 65, 150])
+@pytest.mark.parametrize("T", [16, 17, 32, 33, 64, 65, 150])
 def test_router_of_many_tokens(gpu_lib, binding, T):
     """Tiles of 32 tokens x 32 experts with ragged edges of both, columns in one and in several stretches."""
     c = synth.tiny_spec().cfg.copy()
