@@ -222,13 +222,13 @@ __global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaAr
 // alone walks the positions (kda_scan_kernel); the output's norm and gate follow for all positions at once
 // (kda_out_kernel).
 //
-// The scan: the columns of the state are independent of each other, so a head's 128 are dealt to four CTAs, and a
-// column to PARTS lanes of 128 / PARTS rows each, in registers. Both products of a position are taken with the
-// decayed state, o = q.(aS) + (q.k) u, so that one round of shuffles serves them and the next position waits for u
-// alone; the positions' vectors arrive by asynchronous copies, 8 positions ahead. What bounds it over many positions
-// is that chain (shared loads, sums, three shuffles): eight lanes to a column then. Over one position of many
-// sequences it is the state's memory traffic, and four lanes to a column read it in whole 32-byte sectors.
-// (One CTA per head and one thread per column, sums in one chain of 128: 2.6 us per position, 5.2 ms for 2048.)
+// The scan: the columns of the state are independent of each other, so a head's 128 are dealt to CTAs, and a column's
+// rows to PARTS lanes, in registers. Both products of a position are taken with the decayed state, o = q.(aS) + (q.k) u,
+// so that one round of shuffles serves them and the next position waits for u alone; the positions' vectors arrive by
+// asynchronous copies, 8 positions ahead. Many positions are bound by that chain and by shared-memory wavefronts (vector
+// loads and shuffles): two columns to a lane, which halves the loads per product, and one transposed sum for the four
+// values. 2048 positions of 64 heads: 5.2 ms with a thread per column, 1.7 with eight lanes to each, now 1.07. One position of
+// many sequences is bound by the state's memory traffic: four lanes to a column read it in whole 32-byte sectors.
 // The sums of a column are taken in parts with four accumulators each, products fused.
 struct KdaPrep {
     KdaArgs a;
@@ -325,18 +325,19 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2
 __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
 __device__ __forceinline__ float f2_sum(F2 a) { float x, y; asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); return __fadd_rn(x, y); }
 
-constexpr int KDA_TB = 8, KDA_COLS = 32;
-template <int DS, int PARTS>
-__global__ void __launch_bounds__(32 * PARTS) kda_scan_kernel(const KdaPrep p)
+constexpr int KDA_TB = 8;
+template <int DS, int PARTS, int CPL, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) kda_scan_kernel(const KdaPrep p)
 {
     pdl_trigger();
-    constexpr int D = DS, R = DS / PARTS, PART = R + 4, NT = KDA_COLS * PARTS;   // rows per lane; their stride in shared memory (other banks)
-    __shared__ __align__(16) float vec[2][KDA_TB][3][PARTS * PART];      // decay, k, q
-    __shared__ __align__(16) float sv[2][KDA_TB][KDA_COLS];
+    constexpr int D = DS, R = DS / PARTS, PART = R + 4, LC = 32 / PARTS;    // rows per lane; their stride in shared memory (other banks); lanes side by side
+    constexpr int COLS = LC * CPL * WARPS, NT = 32 * WARPS;                // columns of the CTA
+    __shared__ __align__(16) float vec[2][KDA_TB][3][PARTS * PART];        // decay, k, q
+    __shared__ __align__(16) float sv[2][KDA_TB][COLS];
     __shared__ float2 sb[2][KDA_TB];
     const KdaArgs &a = p.a;
-    const int groups = D / KDA_COLS, hl = blockIdx.x / groups, h = a.head0 + hl, col0 = (blockIdx.x % groups) * KDA_COLS, seq = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane / (32 / PARTS), col = col0 + warp * (32 / PARTS) + lane % (32 / PARTS);
+    const int groups = D / COLS, hl = blockIdx.x / groups, h = a.head0 + hl, col0 = (blockIdx.x % groups) * COLS, seq = blockIdx.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane / LC, cc = warp * LC * CPL + (lane % LC) * CPL, col = col0 + cc;
     const int P = a.H * D, hist = a.K - 1, row0 = seq * a.T;
     float *state = a.state + (size_t)seq * a.seq_stride;
     float *S = state + (size_t)h * D * D + (size_t)part * R * D + col;
@@ -350,8 +351,8 @@ __global__ void __launch_bounds__(32 * PARTS) kda_scan_kernel(const KdaPrep p)
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&vec[buf][j][w][(c * 4 / R) * PART + (c * 4) % R]);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
         }
-        for (int i = threadIdx.x; i < nt * (KDA_COLS / 4); i += NT) {
-            const int j = i / (KDA_COLS / 4), c = i % (KDA_COLS / 4);
+        for (int i = threadIdx.x; i < nt * (COLS / 4); i += NT) {
+            const int j = i / (COLS / 4), c = i % (COLS / 4);
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sv[buf][j][c * 4]);
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(p.vn + (size_t)(row0 + t0 + j) * P + h * D + col0 + c * 4) : "memory");
         }
@@ -359,9 +360,21 @@ __global__ void __launch_bounds__(32 * PARTS) kda_scan_kernel(const KdaPrep p)
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     fetch(0, 0);
-    F2 s[R / 2];
+    F2 s[CPL][R / 2];
 #pragma unroll
-    for (int i = 0; i < R / 2; i++) s[i] = f2(S[(size_t)(2 * i) * D], S[(size_t)(2 * i + 1) * D]);
+    for (int c = 0; c < CPL; c++)
+#pragma unroll
+        for (int i = 0; i < R / 2; i++) s[c][i] = f2(S[(size_t)(2 * i) * D + c], S[(size_t)(2 * i + 1) * D + c]);
+    auto put_state = [&](float *dst) {
+#pragma unroll
+        for (int c = 0; c < CPL; c++)
+#pragma unroll
+            for (int i = 0; i < R / 2; i++) {
+                float x, y;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s[c][i].v));
+                dst[(size_t)(2 * i) * D + c] = x; dst[(size_t)(2 * i + 1) * D + c] = y;
+            }
+    };
     int buf = 0;
     for (int t0 = 0; t0 < a.T; t0 += KDA_TB, buf ^= 1) {
         const int nt = a.T - t0 < KDA_TB ? a.T - t0 : KDA_TB;
@@ -372,54 +385,68 @@ __global__ void __launch_bounds__(32 * PARTS) kda_scan_kernel(const KdaPrep p)
         for (int j = 0; j < nt; j++) {
             const float4 *al4 = reinterpret_cast<const float4 *>(&vec[buf][j][0][part * PART]), *k4 = reinterpret_cast<const float4 *>(&vec[buf][j][1][part * PART]),
                          *q4 = reinterpret_cast<const float4 *>(&vec[buf][j][2][part * PART]);
-            F2 u0 = f2(0.f, 0.f), u1 = u0, o0 = u0, o1 = u0, k[R / 2];
+            const F2 zero = f2(0.f, 0.f);
+            F2 u0[CPL], u1[CPL], o0[CPL], o1[CPL], k[R / 2];
+#pragma unroll
+            for (int c = 0; c < CPL; c++) u0[c] = u1[c] = o0[c] = o1[c] = zero;
 #pragma unroll
             for (int i = 0; i < R / 4; i++) {
                 const float4 al = al4[i], kk = k4[i], q = q4[i];
                 k[2 * i] = f2(kk.x, kk.y); k[2 * i + 1] = f2(kk.z, kk.w);
-                s[2 * i] = f2_mul(s[2 * i], f2(al.x, al.y));
-                s[2 * i + 1] = f2_mul(s[2 * i + 1], f2(al.z, al.w));
-                u0 = f2_fma(s[2 * i], k[2 * i], u0);
-                u1 = f2_fma(s[2 * i + 1], k[2 * i + 1], u1);
-                o0 = f2_fma(s[2 * i], f2(q.x, q.y), o0);
-                o1 = f2_fma(s[2 * i + 1], f2(q.z, q.w), o1);
-            }
-            float u = __fadd_rn(f2_sum(u0), f2_sum(u1)), o = __fadd_rn(f2_sum(o0), f2_sum(o1));
 #pragma unroll
-            for (int m = 32 / PARTS; m < 32; m <<= 1) {
-                u = __fadd_rn(u, __shfl_xor_sync(0xffffffffu, u, m));
-                o = __fadd_rn(o, __shfl_xor_sync(0xffffffffu, o, m));
-            }
-            const float2 b = sb[buf][j];
-            u = __fmul_rn(__fsub_rn(sv[buf][j][col - col0], u), b.x);
-            const F2 uu = f2(u, u);
-#pragma unroll
-            for (int i = 0; i < R / 2; i++) s[i] = f2_fma(k[i], uu, s[i]);
-            if (part == 0) a.o[(size_t)(row0 + t0 + j) * P + h * D + col] = __fmaf_rn(b.y, u, o);
-            if (a.snap && t0 + j == a.snap_after) {
-                float *Sn = a.snap + (size_t)h * D * D + (size_t)part * R * D + col;
-#pragma unroll
-                for (int i = 0; i < R / 2; i++) {
-                    float x, y;
-                    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s[i].v));
-                    Sn[(size_t)(2 * i) * D] = x; Sn[(size_t)(2 * i + 1) * D] = y;
+                for (int c = 0; c < CPL; c++) {
+                    s[c][2 * i] = f2_mul(s[c][2 * i], f2(al.x, al.y));
+                    s[c][2 * i + 1] = f2_mul(s[c][2 * i + 1], f2(al.z, al.w));
+                    u0[c] = f2_fma(s[c][2 * i], k[2 * i], u0[c]);
+                    u1[c] = f2_fma(s[c][2 * i + 1], k[2 * i + 1], u1[c]);
+                    o0[c] = f2_fma(s[c][2 * i], f2(q.x, q.y), o0[c]);
+                    o1[c] = f2_fma(s[c][2 * i + 1], f2(q.z, q.w), o1[c]);
                 }
             }
+            const float2 b = sb[buf][j];
+            float *out = a.o + (size_t)(row0 + t0 + j) * P + h * D + col;
+            float u[CPL];
+            if constexpr (CPL == 2) {
+                // four sums over the eight lanes of a pair of columns: half of them go on with u, half with o, then a quarter each
+                static_assert(PARTS == 8, "three halvings");
+                const float x0 = __fadd_rn(f2_sum(u0[0]), f2_sum(u1[0])), x1 = __fadd_rn(f2_sum(u0[1]), f2_sum(u1[1]));
+                const float y0 = __fadd_rn(f2_sum(o0[0]), f2_sum(o1[0])), y1 = __fadd_rn(f2_sum(o0[1]), f2_sum(o1[1]));
+                const bool is_o = lane & 16, second = lane & 8;
+                const float a0 = __fadd_rn(is_o ? y0 : x0, __shfl_xor_sync(0xffffffffu, is_o ? x0 : y0, 16));
+                const float a1 = __fadd_rn(is_o ? y1 : x1, __shfl_xor_sync(0xffffffffu, is_o ? x1 : y1, 16));
+                float v = __fadd_rn(second ? a1 : a0, __shfl_xor_sync(0xffffffffu, second ? a0 : a1, 8));
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
+                u[0] = __fmul_rn(__fsub_rn(sv[buf][j][cc], __shfl_sync(0xffffffffu, v, lane & 3)), b.x);
+                u[1] = __fmul_rn(__fsub_rn(sv[buf][j][cc + 1], __shfl_sync(0xffffffffu, v, (lane & 3) | 8)), b.x);
+                if ((lane & 20) == 16) out[second] = __fmaf_rn(b.y, second ? u[1] : u[0], v);
+            } else {
+                float o = __fadd_rn(f2_sum(o0[0]), f2_sum(o1[0]));
+                u[0] = __fadd_rn(f2_sum(u0[0]), f2_sum(u1[0]));
+#pragma unroll
+                for (int m = LC; m < 32; m <<= 1) {
+                    u[0] = __fadd_rn(u[0], __shfl_xor_sync(0xffffffffu, u[0], m));
+                    o = __fadd_rn(o, __shfl_xor_sync(0xffffffffu, o, m));
+                }
+                u[0] = __fmul_rn(__fsub_rn(sv[buf][j][cc], u[0]), b.x);
+                if (part == 0) *out = __fmaf_rn(b.y, u[0], o);
+            }
+#pragma unroll
+            for (int c = 0; c < CPL; c++) {
+                const F2 uu = f2(u[c], u[c]);
+#pragma unroll
+                for (int i = 0; i < R / 2; i++) s[c][i] = f2_fma(k[i], uu, s[c][i]);
+            }
+            if (a.snap && t0 + j == a.snap_after) put_state(a.snap + (size_t)h * D * D + (size_t)part * R * D + col);
         }
     }
-#pragma unroll
-    for (int i = 0; i < R / 2; i++) {
-        float x, y;
-        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(s[i].v));
-        S[(size_t)(2 * i) * D] = x; S[(size_t)(2 * i + 1) * D] = y;
-    }
+    put_state(S);
     // the convolution histories of this CTA's channels: the K - 1 inputs before position `upto` (the call's rows, older
     // ones from the old history, which the preparation has read)
     float *cs = state + (size_t)a.H * D * D;
     auto histories = [&](float *dst, int upto) {
         const float *src[3] = {a.q, a.k, a.v};
-        for (int i = threadIdx.x; i < 3 * KDA_COLS; i += NT) {
-            const int w = i / KDA_COLS, ch = h * D + col0 + i % KDA_COLS;
+        for (int i = threadIdx.x; i < 3 * COLS; i += NT) {
+            const int w = i / COLS, ch = h * D + col0 + i % COLS;
             float nv[16];
             for (int j = 0; j < hist; j++) {
                 const int tt = upto - hist + j;
@@ -454,15 +481,19 @@ __global__ void __launch_bounds__(256) kda_out_kernel(const KdaArgs a, int heads
         a.o[off + i] = __fmul_rn(__fmul_rn(a.o_norm[lane * C + i], __fmul_rn(o[i], inv)), sigmoid_near(a.gb[off + i]));
 }
 
+constexpr int KDA_EARLY_T = 8;        // positions whose scan is shorter than a launch
 template <int DS>
 static void kda_rows(cudaStream_t st, const KdaArgs &a, const KdaScratch &x, int heads, int n_seq)
 {
     KdaPrep p{a, x.qn, x.kn, x.vn, x.al, x.beta, heads};
-    const dim3 pg((heads + 7) / 8, (a.T + KDA_RUN - 1) / KDA_RUN * n_seq), sg(heads * (DS / KDA_COLS), n_seq);
+    const dim3 pg((heads + 7) / 8, (a.T + KDA_RUN - 1) / KDA_RUN * n_seq);
     if (a.K == 4) G5B_LAUNCH_PDL((kda_prep_kernel<DS, 4>), pg, dim3(256), 0, st, p);
     else          G5B_LAUNCH_PDL((kda_prep_kernel<DS, 0>), pg, dim3(256), 0, st, p);
-    if (a.T > 1) G5B_LAUNCH_PDL((kda_scan_kernel<DS, 8>), sg, dim3(256), 0, st, p);
-    else         G5B_LAUNCH_PDL((kda_scan_kernel<DS, 4>), sg, dim3(128), 0, st, p);
+    // (many positions: launched the ordinary way - launched early, its few long-running CTAs crowd the SMs that the preparation
+    // leaves first, seven to an SM, and the others idle)
+    if (a.T > KDA_EARLY_T) G5B_LAUNCH((kda_scan_kernel<DS, 8, 2, 2>), dim3(heads * (DS / 16), n_seq), dim3(64), 0, st, p);
+    else if (a.T > 1)      G5B_LAUNCH_PDL((kda_scan_kernel<DS, 8, 2, 2>), dim3(heads * (DS / 16), n_seq), dim3(64), 0, st, p);
+    else                   G5B_LAUNCH_PDL((kda_scan_kernel<DS, 4, 1, 4>), dim3(heads * (DS / 32), n_seq), dim3(128), 0, st, p);
     G5B_LAUNCH_PDL(kda_out_kernel<DS>, dim3((heads + 7) / 8, a.T * n_seq), dim3(256), 0, st, a, heads);
 }
 

@@ -753,7 +753,8 @@ void hc_pre_fused(cudaStream_t st, float *xn, float *post, float *comb, float *h
     const size_t rows_smem = (size_t)M * E * sizeof(float);
     static SmemGrant grant;
     if (T >= HCR_MIN_T && M == HCR_M && E % 8 == 0 && rows_smem <= HCR_MAX_SMEM && dev_opt_in_smem((const void *)hc_pre_rows_kernel, rows_smem + (8 << 10), grant)) {
-        G5B_LAUNCH_PDL(hc_pre_rows_kernel, dim3(T), dim3(HCR_THREADS), rows_smem, st, a);
+        // (launched the ordinary way: launched early, its CTAs crowd the SMs that the kernel in front leaves first)
+        G5B_LAUNCH(hc_pre_rows_kernel, T, HCR_THREADS, rows_smem, st, a);
         return;
     }
     if (hc_pre_cluster_takes(M, E)) G5B_LAUNCH_PDL(hc_pre_cluster_kernel, dim3(HCC_CTAS, T), dim3(HCC_THREADS), 0, st, a);
