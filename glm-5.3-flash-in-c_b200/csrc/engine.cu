@@ -147,6 +147,7 @@ struct g5b_engine {
     float *kq, *kk, *kv, *kz, *kgb, *ko, *kbraw, *klr;
     KdaScratch kscr{};                           // rows of the position-parallel part of the KDA layer for calls with several positions
     float *mq_raw, *mct, *mwk, *mgate, *mwp, *mq, *mqidx, *mcb, *macc, *mscore, *minvq;
+    void *mqt;                                   // absorbed queries as BF16 terms
     double *mqa, *mdsc, *mpart = nullptr, *mstats = nullptr;
     int *mcount = nullptr;
     TcGemm *tc = nullptr;                                // FP8 / BF16 projections of 8+ positions on tcgen05
@@ -745,7 +746,7 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         walloc(e, &e->mq, N * H * c.qk_nope) || walloc(e, &e->mqidx, N * (size_t)c.index_heads * c.index_dim) ||
         walloc(e, &e->mcb, N * H * KL) || walloc(e, &e->macc, N * H * c.v_head) ||
         walloc(e, &e->mscore, NA * ((size_t)e->cap / c.index_kpool + 1)) || walloc(e, &e->minvq, N) ||
-        walloc(e, &e->mqa, NA * H * KL) || walloc(e, &e->mdsc, NA * H * stride) ||
+        walloc(e, &e->mqa, NA * H * KL) || e->dalloc(&e->mqt, NA * H * 3 * KL * 2) || walloc(e, &e->mdsc, NA * H * stride) ||
         walloc(e, &e->msel, NA * stride) || walloc(e, &e->mnsel, NA) ||
         walloc(e, &e->mstats, NA * H * 2) || walloc(e, &e->mcount, NA * H) ||
         walloc(e, &e->mpart, (size_t)MLA_PART_TOKENS * H * ((stride + 31) / 32) * KL)) return -1;
@@ -1141,7 +1142,7 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
     if (!flash && ms && e->mla_tensor && n == 1 && !batch) {
         sf.H = (Hl + 15) / 16 * 16;
         flash = sf.H <= s.H && mla_flash_takes(sf);
-        if (flash) CU(cudaMemsetAsync(e->mqa + (size_t)Hl * s.KL, 0, (size_t)(sf.H - Hl) * s.KL * sizeof(double), e->st));
+        if (flash) CU(cudaMemsetAsync(static_cast<uint16_t *>(e->mqt) + (size_t)Hl * 3 * s.KL, 0, (size_t)(sf.H - Hl) * 3 * s.KL * 2, e->st));
     }
     const DMat qb = ms ? row_slice(w.q_b, h0 * s.qn, Hl * s.qn) : w.q_b;
     const DMat kvb = ms ? row_slice(w.kv_b, h0 * (s.qn + s.vh), Hl * (s.qn + s.vh)) : w.kv_b;
@@ -1170,16 +1171,16 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
         bool forked = false, join = false;
         if (e->side && e->side_ev && e->side_done && cudaEventRecord(e->side_ev, e->st) == cudaSuccess &&
             cudaStreamWaitEvent(e->side, e->side_ev, 0) == cudaSuccess) {
-            mla_absorb(e->side, e->mqa, mq, kvb, nt, sl);
+            mla_absorb(e->side, e->mqa, flash ? e->mqt : nullptr, mq, kvb, nt, sl);
             forked = true;
             join = cudaEventRecord(e->side_done, e->side) == cudaSuccess;
             if (!join) cudaStreamSynchronize(e->side);
         }
         dsa_select(e->st, e->msel, e->mnsel, ist, e->mqidx + (size_t)t0 * c.index_heads * c.index_dim, e->mwp + (size_t)t0 * c.index_heads, e->mscore, nt, at, s);
-        if (!forked) mla_absorb(e->st, e->mqa, mq, kvb, nt, sl);
+        if (!forked) mla_absorb(e->st, e->mqa, flash ? e->mqt : nullptr, mq, kvb, nt, sl);
         else if (join && cudaStreamWaitEvent(e->st, e->side_done, 0) != cudaSuccess) cudaStreamSynchronize(e->side);
         if (flash)
-            mla_attend_flash(e->st, cb, e->mqa, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf);
+            mla_attend_flash(e->st, cb, e->mqt, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf);
         else
             mla_attend(e->st, cb, e->mqa, lat, e->msel, e->mnsel, e->mdsc, e->mpart, e->mstats, e->mcount, MLA_PART_TOKENS, nt, at, sl);
         if (!wide) mla_vout(e->st, e->macc + (size_t)t0 * Hl * c.v_head, cb, kvb, nt, sl);

@@ -8,15 +8,40 @@
 // tiles of eight, 1 x 4 sums to a thread, since a tile of 32 would multiply padding for most of its time.
 #pragma once
 
+#include <cuda_bf16.h>
+
 #include "common.cuh"
 
 namespace g5b {
+
+// v = hi + mid + lo exactly enough (24 bits), each a BF16
+__device__ __forceinline__ void split3_bf16(float v, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo)
+{
+    hi = __float2bfloat16_rn(v);
+    const float e1 = v - __bfloat162float(hi);
+    mid = __float2bfloat16_rn(e1);
+    lo = __float2bfloat16_rn(e1 - __bfloat162float(mid));
+}
+
+// Where an absorbed query goes: doubles [query][head][KL], or, for the tensor-core attention core, the float of v * scale
+// as three BF16 terms [query][head][term][KL] (split here once, not by every CTA that multiplies the query).
+struct QueryOut {
+    double *qa; __nv_bfloat16 *terms; double scale; int H, KL;
+    __device__ __forceinline__ void put(int t, int h, int c, double v) const
+    {
+        if (terms) {
+            __nv_bfloat16 *d = terms + ((size_t)t * H + h) * 3 * KL + c;
+            split3_bf16((float)(v * scale), d[0], d[KL], d[2 * KL]);
+        } else qa[((size_t)t * H + h) * KL + c] = v;
+    }
+};
 
 struct F64Tile {
     const float *A; const uint16_t *B; double *out;
     size_t lda, ldb, ldo;         // elements between rows
     size_t za, zb, zo;            // elements between the problems of blockIdx.z (heads, or stretches of k)
     int T, N, K;                  // K: a multiple of 32, rows of A and B 16-byte aligned
+    QueryOut q;                   // K_ROWS: the results are absorbed queries of head blockIdx.z
 };
 constexpr int F64_N = 32, F64_K = 32, F64_THREADS = 64, F64_PITCH = 34;
 
@@ -37,7 +62,7 @@ __global__ void __launch_bounds__(F64_THREADS, 8) f64_tile_kernel(const F64Tile 
     const int tid = threadIdx.x, t0 = blockIdx.y * F64_T, n0 = blockIdx.x * F64_N;
     const float *A = p.A + (size_t)blockIdx.z * p.za;
     const uint16_t *Bm = p.B + (size_t)blockIdx.z * p.zb;
-    double *out = p.out + (size_t)blockIdx.z * p.zo;
+    double *out = K_ROWS ? nullptr : p.out + (size_t)blockIdx.z * p.zo;
     const int row = tid & 31, half = tid >> 5;                    // a thread loads 16 consecutive k of one row of B
     const int arow = tid % F64_T, ak = tid / F64_T * (4 * TR);    // and 4 TR of one of A
     const bool alive = t0 + arow < p.T;
@@ -107,7 +132,10 @@ __global__ void __launch_bounds__(F64_THREADS, 8) f64_tile_kernel(const F64Tile 
         if (t0 + tt + i < p.T)
 #pragma unroll
             for (int j = 0; j < 4; j++)
-                if (n0 + nn + j < p.N) out[(size_t)(t0 + tt + i) * p.ldo + n0 + nn + j] = acc[i][j];
+                if (n0 + nn + j < p.N) {
+                    if (K_ROWS) p.q.put(t0 + tt + i, blockIdx.z, n0 + nn + j, acc[i][j]);
+                    else        out[(size_t)(t0 + tt + i) * p.ldo + n0 + nn + j] = acc[i][j];
+                }
 }
 
 inline int f64_tile_rows(int T) { return T > 16 ? 32 : 8; }      // (two tiles of eight are as fast as one of 32)

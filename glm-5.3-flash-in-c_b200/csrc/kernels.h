@@ -319,7 +319,8 @@ void mla_store(cudaStream_t st, void *latent, float *idx_state, const float *ct_
                int T, int cached, const MlaShape &s);
 void dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
                 const float *wproj, float *score, int T, int cached, const MlaShape &s);
-void mla_absorb(cudaStream_t st, double *qa, const float *q, const DMat &kv_b, int T, const MlaShape &s);
+// The absorbed queries as doubles [T][H][KL] in qa or, when terms is given, scaled and split for the tensor-core core: [T][H][3][KL] BF16.
+void mla_absorb(cudaStream_t st, double *qa, void *terms, const float *q, const DMat &kv_b, int T, const MlaShape &s);
 // part: FP64 partial sums [part_tokens][H][ceil((topk+KP)/32)][KL], stats [T][H][2]; part == nullptr
 // falls back to one CTA per head.
 // counters: [T][H / 4] zeroed ints (the score kernel's per head-group arrival counts).
@@ -331,7 +332,7 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
 // rescaling reduction. part / part_bytes: scratch for the chunks' partial rows; cstat: room for
 // [T][H][ceil((topk + KP) / 64)][2] doubles.
 bool mla_flash_takes(const MlaShape &s);
-void mla_attend_flash(cudaStream_t st, float *cb, const double *qa, const void *latent, const int *sel, const int *nsel,
+void mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
                       void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s);
 void mla_vout(cudaStream_t st, float *acc_out, const float *cb, const DMat &kv_b, int T, const MlaShape &s);
 

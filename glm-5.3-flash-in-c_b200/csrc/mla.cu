@@ -357,7 +357,7 @@ __device__ __forceinline__ double mat_elem(const DMat &m, int r, int c)
 
 // qa[t][h][c] = sum_i q[t][h][i] * W_k[h][i][c] in FP64, ascending i (matmul_transposed,
 // glm53f_ops.c:793-814). A thread owns a latent column.
-__global__ void mla_absorb_kernel(double *qa, const float *q, const DMat kv_b, MlaShape s)
+__global__ void mla_absorb_kernel(const QueryOut out, const float *q, const DMat kv_b, MlaShape s)
 {
     const int h = blockIdx.x, t = blockIdx.y;
     const int kvd = s.qn + s.vh;
@@ -371,14 +371,14 @@ __global__ void mla_absorb_kernel(double *qa, const float *q, const DMat kv_b, M
         } else {
             for (int i = 0; i < s.qn; i++) acc = __dadd_rn(acc, __dmul_rn((double)qt[i], mat_elem(kv_b, h * kvd + i, c)));
         }
-        qa[((size_t)t * s.H + h) * s.KL + c] = acc;
+        out.put(t, h, c, acc);
     }
 }
 
 // The same sums with the GPU filled: a CTA takes 128 latent columns of one head, its eight row
 // groups (32 rows each at qk_nope = 256) accumulate in FP64 and are added in ascending order.
 constexpr int AB_COLS = 128, AB_GROUPS = 8;
-__global__ void __launch_bounds__(AB_COLS * AB_GROUPS) mla_absorb_split_kernel(double *qa, const float *q, const DMat kv_b, MlaShape s)
+__global__ void __launch_bounds__(AB_COLS * AB_GROUPS) mla_absorb_split_kernel(const QueryOut out, const float *q, const DMat kv_b, MlaShape s)
 {
     __shared__ double part[AB_GROUPS][AB_COLS];
     extern __shared__ double ab_q[];                     // the head's query: converted once, not for every column
@@ -397,26 +397,26 @@ __global__ void __launch_bounds__(AB_COLS * AB_GROUPS) mla_absorb_split_kernel(d
         double sum = part[0][threadIdx.x];
 #pragma unroll
         for (int g = 1; g < AB_GROUPS; g++) sum += part[g][threadIdx.x];
-        qa[((size_t)t * s.H + h) * s.KL + c] = sum;
+        out.put(t, h, c, sum);
     }
 }
 
-void mla_absorb(cudaStream_t st, double *qa, const float *q, const DMat &kv_b, int T, const MlaShape &s)
+void mla_absorb(cudaStream_t st, double *qa, void *terms, const float *q, const DMat &kv_b, int T, const MlaShape &s)
 {
+    const QueryOut out{qa, static_cast<__nv_bfloat16 *>(terms), (double)(1.0f / sqrtf((float)s.qn)), s.H, s.KL};
     // Several positions in tiles (64 positions of 64 heads: 230 -> 109 us, the FP64 pipe's own time; 7: 49 -> 42 us).
     if (T > 1 && kv_b.dt == DT_BF16 && s.KL % 8 == 0 && s.qn % F64_K == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
         (reinterpret_cast<uintptr_t>(kv_b.w) & 15) == 0) {
         const size_t kvd = (size_t)(s.qn + s.vh);
-        const F64Tile f{q, static_cast<const uint16_t *>(kv_b.w), qa, (size_t)s.H * s.qn, (size_t)s.KL, (size_t)s.H * s.KL,
-                        (size_t)s.qn, kvd * s.KL, (size_t)s.KL, T, s.KL, s.qn};
+        const F64Tile f{q, static_cast<const uint16_t *>(kv_b.w), nullptr, (size_t)s.H * s.qn, (size_t)s.KL, 0, (size_t)s.qn, kvd * s.KL, 0, T, s.KL, s.qn, out};
         f64_tile<true>(st, f, s.H);
         return;
     }
     if (kv_b.dt == DT_BF16 && s.KL % AB_COLS == 0 && s.qn % (AB_GROUPS * 8) == 0 && s.qn <= 4096) {
-        G5B_LAUNCH(mla_absorb_split_kernel, dim3(s.H, T, s.KL / AB_COLS), AB_COLS * AB_GROUPS, (size_t)s.qn * sizeof(double), st, qa, q, kv_b, s);
+        G5B_LAUNCH(mla_absorb_split_kernel, dim3(s.H, T, s.KL / AB_COLS), AB_COLS * AB_GROUPS, (size_t)s.qn * sizeof(double), st, out, q, kv_b, s);
         return;
     }
-    G5B_LAUNCH(mla_absorb_kernel, dim3(s.H, T), s.KL >= 512 ? 512 : 128, 0, st, qa, q, kv_b, s);
+    G5B_LAUNCH(mla_absorb_kernel, dim3(s.H, T), s.KL >= 512 ? 512 : 128, 0, st, out, q, kv_b, s);
 }
 
 // d[t][h][jj] = (qa . c_j) * scale in FP64 for the visible positions (all, or the selection).
@@ -772,10 +772,16 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
 // chunk's own maximum and exponentials, multiplies the weighted sum and leaves (max, sum, partial
 // rows) for the reduction kernel, which rescales the chunks to the common maximum the way a
 // two-pass softmax would have (the reference's max over all scores first, then the exponentials).
-constexpr int FL_POS = 64, FL_HEADS = 16, FL_KL = 512, FL_PITCH = FL_KL + 8, FL_PPITCH = FL_POS + 8;
+// A CTA is a chain of phases - gather, scores, exponentials, weighted sum - so two of them share an SM: rows are kept
+// without padding (16-byte pieces of row r at place piece ^ (r & 7), which ldmatrix reads without conflicts) and scores
+// and probabilities take the place of the queries, 114,688 bytes in all. The queries arrive as terms. 64 sequences at 4096
+// positions: 116 us per launch before, 64 now.
+constexpr int FL_POS = 64, FL_HEADS = 16, FL_KL = 512, FL_PPITCH = FL_POS + 8;
 constexpr int FL_THREADS = 256;
-constexpr size_t FL_SMEM = (size_t)3 * FL_HEADS * FL_PITCH * 2 + (size_t)FL_POS * FL_PITCH * 2 +
-                           (size_t)FL_HEADS * FL_POS * 4 + (size_t)3 * FL_HEADS * FL_PPITCH * 2;
+constexpr size_t FL_SMEM = (size_t)3 * FL_HEADS * FL_KL * 2 + (size_t)FL_POS * FL_KL * 2;
+static_assert((size_t)FL_HEADS * FL_POS * 4 + (size_t)3 * FL_HEADS * FL_PPITCH * 2 <= (size_t)3 * FL_HEADS * FL_KL * 2, "scores and probabilities fit where the queries were");
+// element (row, 8 * piece) of rows of FL_KL 16-bit values
+__device__ __forceinline__ int fl_at(int row, int piece) { return row * FL_KL + ((piece ^ (row & 7)) << 3); }
 
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], const void *p)
 {
@@ -798,27 +804,18 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
-// v = hi + mid + lo exactly enough (24 bits), each a BF16
-__device__ __forceinline__ void split3_bf16(float v, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo)
-{
-    hi = __float2bfloat16_rn(v);
-    const float e1 = v - __bfloat162float(hi);
-    mid = __float2bfloat16_rn(e1);
-    lo = __float2bfloat16_rn(e1 - __bfloat162float(mid));
-}
-
 // part: [T][H][nchunks][KL] floats (unnormalised partial rows); cstat: [T][H][nchunks][2] doubles
 // (chunk maximum, sum of exponentials).
-__global__ void __launch_bounds__(FL_THREADS) mla_flash_kernel(float *part, double *cstat, const double *qa, const void *latent,
+__global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *part, double *cstat, const __nv_bfloat16 *qterms, const void *latent,
                                                                const int *sel, const int *nsel, int cached, int nchunks, MlaShape s)
 {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) uint8_t fl_smem[];
-    __nv_bfloat16 *qs = reinterpret_cast<__nv_bfloat16 *>(fl_smem);                          // [3][16][FL_PITCH]
-    __nv_bfloat16 *cs = qs + 3 * FL_HEADS * FL_PITCH;                                       // [64][FL_PITCH]
-    float *ss = reinterpret_cast<float *>(cs + FL_POS * FL_PITCH);                          // [16][64]
-    __nv_bfloat16 *ps = reinterpret_cast<__nv_bfloat16 *>(ss + FL_HEADS * FL_POS);          // [3][16][FL_PPITCH]
+    __nv_bfloat16 *qs = reinterpret_cast<__nv_bfloat16 *>(fl_smem);                          // [3][16][512]
+    __nv_bfloat16 *cs = qs + 3 * FL_HEADS * FL_KL;                                          // [64][512]
+    float *ss = reinterpret_cast<float *>(fl_smem);                                         // [16][64], then
+    __nv_bfloat16 *ps = reinterpret_cast<__nv_bfloat16 *>(ss + FL_HEADS * FL_POS);          // [3][16][FL_PPITCH], over the queries
     const int chunk = blockIdx.x, h0 = blockIdx.y * FL_HEADS, t = blockIdx.z, p = pos_of(s, cached, t);
     const uint16_t *lat = static_cast<const uint16_t *>(seq_latent(latent, s, t));
     const int ns = nsel ? nsel[t] : -1;
@@ -828,61 +825,53 @@ __global__ void __launch_bounds__(FL_THREADS) mla_flash_kernel(float *part, doub
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int *sl = sel ? sel + (size_t)t * (s.topk + s.KP) : nullptr;
 
-    // ---- the chunk's latent rows (16-byte pieces, four threads per row); rows past the last visible
-    // position are zero so that nothing undefined enters a product
-    // (all of a thread's row numbers are requested first, then all of its pieces: one round trip for the
-    // selection list and one for the rows, instead of a dependent pair per piece)
+    // ---- the queries' terms of the 16 heads, and the chunk's latent rows; rows past the last visible position are zero so
+    // that nothing undefined enters a product (all of a thread's row numbers are requested first, then all of its pieces:
+    // one round trip for the selection list and one for everything else)
     {
-        constexpr int PER = FL_POS * (FL_KL / 8) / FL_THREADS;
-        static_assert(FL_POS * (FL_KL / 8) % FL_THREADS == 0, "pieces per thread");
+        constexpr int PIECES = FL_KL / 8, PER = FL_POS * PIECES / FL_THREADS, QPER = 3 * FL_HEADS * PIECES / FL_THREADS;
+        static_assert(FL_POS * PIECES % FL_THREADS == 0 && 3 * FL_HEADS * PIECES % FL_THREADS == 0, "pieces per thread");
+        auto copy = [](const void *dst, const void *src) {
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+        };
         int jrow[PER];
 #pragma unroll
         for (int k = 0; k < PER; k++) {
-            const int jj = j0 + (tid + k * FL_THREADS) / (FL_KL / 8);
+            const int jj = j0 + (tid + k * FL_THREADS) / PIECES;
             jrow[k] = jj < nvis ? (ns < 0 ? jj : sl[jj]) : -1;
         }
-        uint4 v[PER];
+        const __nv_bfloat16 *qt = qterms + ((size_t)t * s.H + h0) * 3 * FL_KL;               // [head][term][512]
 #pragma unroll
-        for (int k = 0; k < PER; k++) {
-            const int c8 = (tid + k * FL_THREADS) % (FL_KL / 8);
-            v[k] = jrow[k] >= 0 ? *reinterpret_cast<const uint4 *>(lat + (size_t)jrow[k] * FL_KL + c8 * 8) : make_uint4(0u, 0u, 0u, 0u);
+        for (int k = 0; k < QPER; k++) {
+            const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES;
+            copy(qs + fl_at((row % 3) * FL_HEADS + row / 3, piece), qt + (size_t)row * FL_KL + piece * 8);
         }
 #pragma unroll
         for (int k = 0; k < PER; k++) {
-            const int i = tid + k * FL_THREADS;
-            *reinterpret_cast<uint4 *>(cs + (size_t)(i / (FL_KL / 8)) * FL_PITCH + (i % (FL_KL / 8)) * 8) = v[k];
+            const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES;
+            if (jrow[k] >= 0) copy(cs + fl_at(row, piece), lat + (size_t)jrow[k] * FL_KL + piece * 8);
+            else              *reinterpret_cast<uint4 *>(cs + fl_at(row, piece)) = make_uint4(0u, 0u, 0u, 0u);
         }
-    }
-    // ---- the absorbed queries of the 16 heads, scaled, as three BF16 terms
-    const double scale = (double)(1.0f / sqrtf((float)s.qn));
-#pragma unroll 8
-    for (int i = tid; i < FL_HEADS * FL_KL; i += FL_THREADS) {
-        const int hh = i / FL_KL, c = i % FL_KL;
-        const float v = (float)(qa[((size_t)t * s.H + h0 + hh) * FL_KL + c] * scale);
-        __nv_bfloat16 a, b, d;
-        split3_bf16(v, a, b, d);
-        qs[(0 * FL_HEADS + hh) * FL_PITCH + c] = a;
-        qs[(1 * FL_HEADS + hh) * FL_PITCH + c] = b;
-        qs[(2 * FL_HEADS + hh) * FL_PITCH + c] = d;
+        asm volatile("cp.async.wait_all;" ::: "memory");
     }
     __syncthreads();
 
     // ---- scores: warp w takes positions 8w..8w+7 of the chunk, all 16 heads, all 512 columns
     {
         float c[4] = {0.f, 0.f, 0.f, 0.f};
-        const __nv_bfloat16 *brow = cs + (size_t)(warp * 8 + (lane & 7)) * FL_PITCH + 8 * ((lane >> 3) & 1);
-        const __nv_bfloat16 *arow = qs + (size_t)((lane & 7) + 8 * ((lane >> 3) & 1)) * FL_PITCH + 8 * (lane >> 4);
+        const int brow = warp * 8 + (lane & 7), arow = (lane & 7) + 8 * ((lane >> 3) & 1);
 #pragma unroll 4
         for (int k0 = 0; k0 < FL_KL; k0 += 16) {
             uint32_t b[2];
-            ldsm_x2(b, brow + k0);
+            ldsm_x2(b, cs + fl_at(brow, k0 / 8 + ((lane >> 3) & 1)));
 #pragma unroll
             for (int term = 0; term < 3; term++) {
                 uint32_t a[4];
-                ldsm_x4(a, arow + (size_t)term * FL_HEADS * FL_PITCH + k0);
+                ldsm_x4(a, qs + fl_at(term * FL_HEADS + arow, k0 / 8 + (lane >> 4)));
                 mma_bf16(c, a, b);
             }
         }
+        __syncthreads();                                     // the queries have been read: the scores go there
         const int r = lane >> 2, col = warp * 8 + 2 * (lane & 3);
         ss[r * FL_POS + col] = c[0]; ss[r * FL_POS + col + 1] = c[1];
         ss[(r + 8) * FL_POS + col] = c[2]; ss[(r + 8) * FL_POS + col + 1] = c[3];
@@ -924,11 +913,10 @@ __global__ void __launch_bounds__(FL_THREADS) mla_flash_kernel(float *part, doub
             uint32_t a[3][4];
 #pragma unroll
             for (int term = 0; term < 3; term++) ldsm_x4(a[term], arow + (size_t)term * FL_HEADS * FL_PPITCH + k0);
-            const __nv_bfloat16 *brow = cs + (size_t)(k0 + (lane & 15)) * FL_PITCH + warp * 64;
 #pragma unroll
             for (int n = 0; n < 8; n++) {
                 uint32_t b[2];
-                ldsm_x2_trans(b, brow + n * 8);
+                ldsm_x2_trans(b, cs + fl_at(k0 + (lane & 15), warp * 8 + n));
 #pragma unroll
                 for (int term = 0; term < 3; term++) mma_bf16(acc[n], a[term], b);
             }
@@ -996,7 +984,7 @@ bool mla_flash_takes(const MlaShape &s)
 }
 
 // scratch: `part_bytes` bytes for the partial rows; `cstat` room for [T][H][nchunks][2] doubles.
-void mla_attend_flash(cudaStream_t st, float *cb, const double *qa, const void *latent, const int *sel, const int *nsel,
+void mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
                       void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s)
 {
     static SmemGrant grant;
@@ -1013,7 +1001,7 @@ void mla_attend_flash(cudaStream_t st, float *cb, const double *qa, const void *
         const void *lat0 = latent;                                 // the kernel's token 0 is sequence t0 of a batch
         if (s.batch) lat0 = static_cast<const void *>(static_cast<const uint16_t *>(latent) + (size_t)t0 * s.lat_seq);
         G5B_LAUNCH_PDL(mla_flash_kernel, dim3(used, s.H / FL_HEADS, n), FL_THREADS, FL_SMEM, st, static_cast<float *>(part), cstat,
-                       qa + (size_t)t0 * s.H * s.KL, lat0, sel ? sel + (size_t)t0 * stride : nullptr, nsel ? nsel + t0 : nullptr,
+                       static_cast<const __nv_bfloat16 *>(qterms) + (size_t)t0 * s.H * 3 * s.KL, lat0, sel ? sel + (size_t)t0 * stride : nullptr, nsel ? nsel + t0 : nullptr,
                        s.batch ? cached : cached + t0, nchunks, s);
         G5B_LAUNCH_PDL(mla_flash_reduce_kernel, dim3(s.H, n), FL_KL, 0, st, cb + (size_t)t0 * s.H * s.KL, static_cast<const float *>(part),
                        cstat, nsel ? nsel + t0 : nullptr, s.batch ? cached : cached + t0, nchunks, s);

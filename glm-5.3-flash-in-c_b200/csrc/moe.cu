@@ -319,7 +319,7 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
         if (parts < 1) parts = 1;
         while (blocks % parts) parts--;                       // equal stretches
         per = s.E / parts;
-        const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per};
+        const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per, {}};
         f64_tile<false>(st, f, parts);
     }
     for (int t0 = 0; t0 < T; t0 += RT_MAX_TOKENS) {
