@@ -47,7 +47,7 @@ namespace g5b {
 constexpr int TS_MAX_SEG = 8;              // matrices of one launch
 constexpr int TS_N = 64;                   // activation rows per tile at most (TC_TILE_ROWS of an expert)
 constexpr int TS_EN = TS_N / 2;            // rows an epilogue thread holds
-constexpr int TS_MAX_STAGES = 6, TS_XS = 2;    // FP8: activation stages, one per converted unit in tensor memory
+constexpr int TS_MAX_STAGES = 6, TS_MAX_XS = 3;    // FP8: activation stages at most
 constexpr int TS_UNIT_BYTES = 32768, TS_EXCH = TS_EN * 128 * 4;
 constexpr int TS_SEG_UNITS = 4;            // BF16: units summed inside the tensor cores before the registers take over
 enum { TS_DENSE = 0, TS_GATEUP = 1, TS_DOWN = 2 };
@@ -75,6 +75,7 @@ struct TsArgs {
     void *out;                 // gate/up: F16 terms, planes of [plane][I]; down: contribution rows [.][E]
     float limit, act_scale, act_inv;   // the scale of the SwiGLU output's terms, a power of two, and its reciprocal
     float *part; int *cnt;     // partial results [CTA][2][row][128], units done per tile (zero between launches)
+    int xs;                    // FP8: activation stages
     int stages, x_stage;       // weight stages (BF16: of weights and terms); bytes of one stage's terms
     int *err;
 };
@@ -314,14 +315,14 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int WS = a.stages, KB = a.KB, XB = a.x_stage;
+    const int WS = a.stages, KB = a.KB, XB = a.x_stage, XS = a.xs;
     uint8_t *wst = smem;                                                   // [WS][32 KB]
-    uint8_t *xst = wst + (size_t)WS * TS_UNIT_BYTES;                       // [TS_XS][XB]
-    float *exch = reinterpret_cast<float *>(xst + (size_t)TS_XS * XB);     // 16 KB
+    uint8_t *xst = wst + (size_t)WS * TS_UNIT_BYTES;                       // [XS][XB]
+    float *exch = reinterpret_cast<float *>(xst + (size_t)XS * XB);        // 16 KB
     uint64_t *bars = reinterpret_cast<uint64_t *>(reinterpret_cast<uint8_t *>(exch) + TS_EXCH);
-    // x_full: the activation terms are there and the unit's codes are converted (four warps)
-    uint64_t *w_full = bars, *w_empty = w_full + TS_MAX_STAGES, *x_full = w_empty + TS_MAX_STAGES, *x_empty = x_full + TS_XS;
-    uint64_t *acc_full = x_empty + TS_XS, *acc_empty = acc_full + 2, *drained = acc_empty + 2;
+    // c_full: a unit's codes are converted (four warps), in one of two places of tensor memory
+    uint64_t *w_full = bars, *w_empty = w_full + TS_MAX_STAGES, *x_full = w_empty + TS_MAX_STAGES, *x_empty = x_full + TS_MAX_XS;
+    uint64_t *c_full = x_empty + TS_MAX_XS, *c_empty = c_full + 2, *acc_full = c_empty + 2, *acc_empty = acc_full + 2, *drained = acc_empty + 2;
     int *s_plan = reinterpret_cast<int *>(drained + 2);                    // experts: per slot first token tile [slots + 1], first pair, pairs, expert
     __shared__ uint32_t s_tmem;
     __shared__ int s_last;
@@ -329,8 +330,11 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
     pdl_trigger();
     if (threadIdx.x == 0) {
         for (int i = 0; i < TS_MAX_STAGES; i++) { mbar_init(&w_full[i], 1); mbar_init(&w_empty[i], 4); }
-        for (int i = 0; i < TS_XS; i++) { mbar_init(&x_full[i], 5); mbar_init(&x_empty[i], 2); }
-        for (int i = 0; i < 2; i++) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); mbar_init(&drained[i], 1); }
+        for (int i = 0; i < TS_MAX_XS; i++) { mbar_init(&x_full[i], 1); mbar_init(&x_empty[i], 2); }
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&c_full[i], 4); mbar_init(&c_empty[i], 2);
+            mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 8); mbar_init(&drained[i], 1);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 18) tmem_alloc(&s_tmem, 512);
@@ -385,15 +389,15 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
             int s = 0, ph = 1, issued = 0;
             TS_WALK(t, {
                 for (int kb = kb0; kb < kb1; kb++) {
-                    if (issued >= TS_XS && !(ok = mbar_wait(&x_empty[s], (uint32_t)ph, a.err, 32))) break;
+                    if (issued >= XS && !(ok = mbar_wait(&x_empty[s], (uint32_t)ph, a.err, 32))) break;
                     mbar_expect_tx(&x_full[s], (uint32_t)(8 * t.n * 128));
                     tma_load_4d(xst + (size_t)s * XB, &maps.x[t.n / 8 - 1], 0, t.row0, 0, kb * 4, &x_full[s]);
                     issued++;
-                    if (++s == TS_XS) { s = 0; ph ^= 1; }
+                    if (++s == XS) { s = 0; ph ^= 1; }
                 }
             });
-            if (!ok)                                          // (the conversion's arrivals may never come: wait as long as a wait is bounded)
-                for (int j = issued - 1; j >= 0 && j >= issued - TS_XS; j--) mbar_wait(&x_full[j % TS_XS], (uint32_t)(j / TS_XS) & 1, a.err, 33);
+            if (!ok)
+                for (int j = issued - 1; j >= 0 && j >= issued - XS; j--) mbar_wait(&x_full[j % XS], (uint32_t)(j / XS) & 1, a.err, 33);
         }
         __syncwarp();
     } else if (warp >= 18) {
@@ -403,18 +407,18 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
             // warps take units in turn; beyond, a unit's first block is the one warp's, the second the other's. Both wait for
             // every unit, so that neither loses count of the barrier's phases.
             const int mine = warp - 18;
-            int it = 0, xp = 0, c = 0;                        // c: uses of the own accumulator so far
+            int it = 0, cp = 0, xs = 0, xp = 0, c = 0;        // c: uses of the own accumulator so far
             TS_WALK(t, {
                 const uint32_t idesc = tc_idesc(0, 2 * t.n);
                 const bool small = t.n <= TS_EN;
                 for (int kb = kb0; kb < kb1; kb++, it++) {
                     const int s = it & 1;
-                    if (!(ok = mbar_wait(&x_full[s], (uint32_t)xp, a.err, 36))) break;
+                    if (!(ok = mbar_wait(&x_full[xs], (uint32_t)xp, a.err, 36) && mbar_wait(&c_full[s], (uint32_t)cp, a.err, 35))) break;
                     if (!small || s == mine) {
                         if (c && !(ok = mbar_wait(&acc_empty[mine], (uint32_t)(c - 1) & 1, a.err, 34))) break;
                         c++;
                         tc_fence_after();
-                        const uint32_t xb = smem_u32(xst) + (uint32_t)(s * XB), ab = tmem + 256u + (uint32_t)s * 128u, d = tmem + (uint32_t)mine * 128u;
+                        const uint32_t xb = smem_u32(xst) + (uint32_t)(xs * XB), ab = tmem + 256u + (uint32_t)s * 128u, d = tmem + (uint32_t)mine * 128u;
                         const int b0 = small ? 0 : mine, b1 = small ? 2 : mine + 1;
                         for (int b = b0; b < b1; b++)
 #pragma unroll
@@ -423,9 +427,11 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
                                 tc_mma_f16_ts(d + (small ? (uint32_t)b * 64u : 0u), ab + (uint32_t)(b * 64 + k * 8), bd, idesc, k ? 1u : 0u);
                             }
                         tc_commit(&acc_full[mine]);
-                        tc_commit(&x_empty[s]);
-                    } else mbar_arrive(&x_empty[s]);
-                    if (s) xp ^= 1;
+                        tc_commit(&x_empty[xs]);
+                        tc_commit(&c_empty[s]);
+                    } else { mbar_arrive(&x_empty[xs]); mbar_arrive(&c_empty[s]); }
+                    if (s) cp ^= 1;
+                    if (++xs == XS) { xs = 0; xp ^= 1; }
                 }
             });
             // nothing of this thread is in flight, and no arrival still to come, when the CTA ends
@@ -441,8 +447,10 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
         const int units = (int)(u1 - u0), x = r & 7;
         int ws = group % WS, wp = 0, xp = 1;
         for (int it = group; it < units; it += 2) {
+            // In this order: with an odd number of stages the groups take turns at one, and only the unit two before having been
+            // multiplied says that the stage's use in between is over (the old phase could be taken for this one).
+            if (it >= 2 && !(ok = mbar_wait_all(&c_empty[group], (uint32_t)xp, a.err, 38))) break;
             if (!(ok = mbar_wait_all(&w_full[ws], (uint32_t)wp, a.err, 37))) break;
-            if (it >= TS_XS && !(ok = mbar_wait_all(&x_empty[group], (uint32_t)xp, a.err, 38))) break;
             tc_fence_after();
             const uint8_t *src = wst + (size_t)ws * TS_UNIT_BYTES + (size_t)r * 128;
 #pragma unroll
@@ -465,7 +473,7 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&x_full[group]);
+            if (lane == 0) mbar_arrive(&c_full[group]);
             xp ^= 1;
             ws += 2;
             if (ws >= WS) { ws -= WS; wp ^= 1; }
@@ -899,7 +907,11 @@ static bool x_maps(TcGemm *g, TsMaps &m, const void *base, bool fp8, size_t plan
 static size_t stage_plan(TsArgs &a, bool fp8, size_t extra)
 {
     a.x_stage = (fp8 ? 8 : 6) * a.n * 128;                           // (a multiple of 1024 per 64-column atom)
-    const size_t fixed = 1024 + 1024 + TS_EXCH + extra + (fp8 ? (size_t)TS_XS * a.x_stage : 0);
+    // A third activation stage where a unit's terms are as large as its weights (tiles of 17 to 32 rows): a stage is only
+    // refilled when its products are done, and with two the way to L2 and back was part of every unit. Smaller terms are
+    // there in time with two, and larger ones leave the weights too few stages.
+    a.xs = a.n > 16 && a.n <= TS_EN ? TS_MAX_XS : 2;
+    const size_t fixed = 1024 + 1024 + TS_EXCH + extra + (fp8 ? (size_t)a.xs * a.x_stage : 0);
     const size_t stage = TS_UNIT_BYTES + (fp8 ? 0 : (size_t)a.x_stage);
     const size_t fit = (227 * 1024 - 512 - fixed) / stage;
     a.stages = (int)(fit < (size_t)TS_MAX_STAGES ? fit : (size_t)TS_MAX_STAGES);
