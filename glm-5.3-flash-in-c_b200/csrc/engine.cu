@@ -150,10 +150,10 @@ struct g5b_engine {
     void *mqt;                                   // absorbed queries as BF16 terms
     double *mqa, *mdsc, *mpart = nullptr, *mstats = nullptr;
     int *mcount = nullptr;
-    TcGemm *tc = nullptr;                                // FP8 / BF16 projections of 8+ positions on tcgen05
+    TcGemm *tc = nullptr;                                // FP8 / BF16 projections of several positions on tcgen05
     int mla_tensor = 1;                                  // option "mla_tensor": 0 keeps the attention core on the FP64 kernels
     size_t mpart_bytes = 0;
-    int tensor_gemm = 1;                                 // option "tensor_gemm": 0 keeps 8+ positions on the one-token kernels
+    int tensor_gemm = 1;                                 // option "tensor_gemm": 0 keeps several positions on the one-token kernels
     float *post_h = nullptr; int post_n = 0;             // positions whose hc_post is still owed (run_layer)
     double *hc_part = nullptr; int *hc_count = nullptr;  // fused mHC site: partial sums and per-token counters
     void *xterms = nullptr; float *xinv = nullptr;      // batched expert kernels: F16 terms of the activations
@@ -974,9 +974,10 @@ static int run_mlp(g5b_engine *e, Layer &w, const float *x, int n, float *out)
     const int DI = c.dense_inter;
     if (!w.d_gate.loaded() || !w.d_up.loaded() || !w.d_down.loaded()) return fail("this layer's dense MLP was not loaded");
     GemvSeg g[2] = {make_seg(w.d_gate, x, c.hidden, e->gu, 2 * DI), make_seg(w.d_up, x, c.hidden, e->gu + DI, 2 * DI)};
-    if (proj_batch(e, g, 2, n)) return -1;
+    if (proj_batch(e, g, 2, n, true)) return -1;
     swiglu(e->st, e->dact, e->gu, DI, n, c.swiglu_limit);
-    return proj(e, w.d_down, e->dact, DI, out, c.hidden, n);
+    GemvSeg d = make_seg(w.d_down, e->dact, DI, out, c.hidden);
+    return proj_batch(e, &d, 1, n, true);
 }
 
 // From this point of the main stream on, fetch a matrix into L2 on the side stream: the kernels
@@ -990,7 +991,7 @@ static void prefetch_beside(g5b_engine *e, const DMat &m)
     l2_prefetch(e->side, m.w, m.bytes());
 }
 
-// Several products sharing (some of) their inputs: with 8 or more positions, FP8 (128 x 128 blocks)
+// Several products sharing (some of) their inputs: with two or more positions, FP8 (128 x 128 blocks)
 // and BF16 matrices whose rows fill 128-row tiles go to the tcgen05 kernel, which reads the weights
 // once; the rest (few rows, odd shapes) to the one-token kernel in one launch.
 static int proj_batch(g5b_engine *e, const GemvSeg *segs, int n, int T, bool early)
@@ -1340,7 +1341,8 @@ static int forward_device(g5b_engine *e, const int *ids_dev, int T, bool all_pos
             head_pick_exchange(e->st, hp);
             continue;
         }
-        if (proj(e, e->lm_head, e->xm, E, e->logits, c.vocab, n, e->inv_head, e->norm)) return -1;
+        GemvSeg head = make_seg(e->lm_head, e->xm, E, e->logits, c.vocab, e->inv_head, e->norm);
+        if (proj_batch(e, &head, 1, n, true)) return -1;
         argmax_rows(e->st, e->am_out + t0, e->logits, c.vocab, n, e->am_v, e->am_i);
         if (logits_host && batch)
             CU(cudaMemcpyAsync(logits_host, e->logits, (size_t)n * c.vocab * 4, cudaMemcpyDeviceToHost, e->st));
