@@ -159,6 +159,36 @@ __device__ __forceinline__ double block_sum(double v, double *red)
     return t;
 }
 
+// 1 / sqrt(x) to a few units of FP64: the single-precision estimate and two Newton steps (the exact sequence of square root
+// and division is a chain of forty FP64 instructions, 0.7 us; what takes this rounds it to float).
+__device__ __forceinline__ double rsqrt_newton(double x)
+{
+    if (!(x > 1e-30 && x < 1e38)) return 1.0 / sqrt(x);              // outside the estimate's range
+    double r = (double)rsqrtf((float)x);
+    r = fma(r, fma(-0.5 * x * r, r, 0.5), r);
+    return fma(r, fma(-0.5 * x * r, r, 0.5), r);
+}
+
+// ---- thread-block clusters
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_cta_rank()
+{
+    uint32_t r;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// the shared variable `p` of CTA `rank` of this cluster
+__device__ __forceinline__ double ld_cluster_f64(const double *p, uint32_t rank)
+{
+    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(p);
+    uint32_t theirs;
+    double v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(rank));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(theirs) : "memory");
+    return v;
+}
+
 // System-scope acquire / release on 64-bit words that another GPU writes or reads.
 __device__ __forceinline__ unsigned long long ld_acquire_sys(const unsigned long long *p)
 {

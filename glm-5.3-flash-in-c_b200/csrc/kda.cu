@@ -44,38 +44,19 @@ __device__ __forceinline__ float conv_step(float cur, const float *w, float *pas
     return __fmul_rn(acc, sigmoid_host(acc));
 }
 
-// DS > 0: head_dim known at compile time, the state column lives in registers.
-// DS == 0: any head_dim up to 512, the state column is re-read from memory.
-template <int DS>
-__global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaArgs a)
+// Any head_dim up to 512: one CTA per head, a thread per column, the state column re-read from memory.
+__global__ void __launch_bounds__(512) kda_core_kernel(const KdaArgs a)
 {
     __shared__ float sq[512], sk[512], sal[512];
     __shared__ double red[32];
     const int h = a.head0 + blockIdx.x, d = threadIdx.x;
-    const int D = DS > 0 ? DS : a.D, P = a.H * D, K = a.K, hist = K - 1;
+    const int D = a.D, P = a.H * D, K = a.K, hist = K - 1;
     const bool live = d < D;
     const int ch = h * D + (live ? d : 0);
     float *state = a.state + (size_t)blockIdx.y * a.seq_stride;
     float *S = state + (size_t)h * D * D;
     float *cs = state + (size_t)a.H * D * D;
     const int row0 = blockIdx.y * a.T;                       // first activation row of this sequence
-
-    // One new token: the two low-rank up-projections z = f_b lrf, gb = g_b lrg of this head's channels
-    // are taken here. Their 2 x D rows of D BF16 are copied to shared memory asynchronously first
-    // thing (16-byte pieces, a warp reads consecutive pieces of consecutive rows), so they travel
-    // beside the state; each thread later multiplies the two rows of its own channel.
-    extern __shared__ __align__(16) uint8_t lrw[];               // [2 D][pitch]: f_b rows, then g_b rows
-    const int pitch = 2 * D + 16;                                // 16 bytes of padding: rows fall on different banks
-    if (a.f_b) {
-        const int per_row = D / 8;
-        for (int i = d; i < 2 * D * per_row; i += (int)blockDim.x) {
-            const int row = i / per_row, piece = i % per_row;
-            const uint16_t *src = (row < D ? a.f_b : a.g_b) + ((size_t)h * D + (row < D ? row : row - D)) * D + piece * 8;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(lrw + (size_t)row * pitch + piece * 16);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
 
     float pq[16], pk[16], pv[16], wq[17], wk[17], wv[17];
     for (int j = 0; j < hist; j++) {
@@ -87,41 +68,6 @@ __global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaAr
         wq[j] = a.q_conv[(size_t)ch * K + j];
         wk[j] = a.k_conv[(size_t)ch * K + j];
         wv[j] = a.v_conv[(size_t)ch * K + j];
-    }
-    float sreg[DS > 0 ? DS : 1];
-    if (DS > 0) {
-#pragma unroll
-        for (int i = 0; i < DS; i++) sreg[i] = S[(size_t)i * DS + d];
-    }
-    // Everything above reads weights and this layer's own state. From here on the projections of the
-    // kernel before this one are read: when this grid was launched early (programmatic stream
-    // serialization), wait until that grid has completed and its results are visible.
-    pdl_wait();
-    // (the low-rank rows requested above have landed by now, under the state's and the histories' loads)
-    float z_own = 0.f, gb_own = 0.f;
-    if (a.f_b) {
-        if (live) { sq[d] = a.lrf[d]; sk[d] = a.lrg[d]; }
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        if (live) {
-            const uint8_t *fr = lrw + (size_t)d * pitch, *gr = lrw + (size_t)(D + d) * pitch;
-            float z0 = 0.f, z1 = 0.f, g0 = 0.f, g1 = 0.f;
-#pragma unroll 4
-            for (int c = 0; c < D; c += 8) {
-                const uint4 fw = *reinterpret_cast<const uint4 *>(fr + 2 * c), gw = *reinterpret_cast<const uint4 *>(gr + 2 * c);
-                const uint32_t fu[4] = {fw.x, fw.y, fw.z, fw.w}, gu[4] = {gw.x, gw.y, gw.z, gw.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    float lo, hi;
-                    bf16x2_to_f32(fu[j], lo, hi);
-                    z0 = fmaf(lo, sq[c + 2 * j], z0); z1 = fmaf(hi, sq[c + 2 * j + 1], z1);
-                    bf16x2_to_f32(gu[j], lo, hi);
-                    g0 = fmaf(lo, sk[c + 2 * j], g0); g1 = fmaf(hi, sk[c + 2 * j + 1], g1);
-                }
-            }
-            z_own = z0 + z1; gb_own = g0 + g1;
-        }
-        __syncthreads();
     }
     const float ea = expf_host(a.A_log[h]);
     const float dtb = a.dt_bias[ch], onw = a.o_norm[live ? d : 0];
@@ -145,7 +91,7 @@ __global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaAr
         if (live) {
             sq[d] = __fmul_rn(__fmul_rn(qv, qinv), qscale);
             sk[d] = __fmul_rn(kv, kinv);
-            const float g = __fmul_rn(a.gate_lb, sigmoid_host(__fmul_rn(ea, __fadd_rn(a.f_b ? z_own : a.z[off], dtb))));
+            const float g = __fmul_rn(a.gate_lb, sigmoid_host(__fmul_rn(ea, __fadd_rn(a.z[off], dtb))));
             sal[d] = expf_host(g);
         }
         __syncthreads();
@@ -153,30 +99,16 @@ __global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaAr
         float ov = 0.f;
         if (live) {
             float u = 0.f;
-            if (DS > 0) {
-#pragma unroll
-                for (int i = 0; i < DS; i++) {
-                    sreg[i] = __fmul_rn(sreg[i], sal[i]);
-                    u = __fadd_rn(u, __fmul_rn(sreg[i], sk[i]));
-                }
-                u = __fmul_rn(__fsub_rn(vv, u), beta);
-#pragma unroll
-                for (int i = 0; i < DS; i++) {
-                    sreg[i] = __fadd_rn(sreg[i], __fmul_rn(sk[i], u));
-                    ov = __fadd_rn(ov, __fmul_rn(sreg[i], sq[i]));
-                }
-            } else {
-                for (int i = 0; i < D; i++) {
-                    const float s = __fmul_rn(S[(size_t)i * D + d], sal[i]);
-                    S[(size_t)i * D + d] = s;
-                    u = __fadd_rn(u, __fmul_rn(s, sk[i]));
-                }
-                u = __fmul_rn(__fsub_rn(vv, u), beta);
-                for (int i = 0; i < D; i++) {
-                    const float s = __fadd_rn(S[(size_t)i * D + d], __fmul_rn(sk[i], u));
-                    S[(size_t)i * D + d] = s;
-                    ov = __fadd_rn(ov, __fmul_rn(s, sq[i]));
-                }
+            for (int i = 0; i < D; i++) {
+                const float s = __fmul_rn(S[(size_t)i * D + d], sal[i]);
+                S[(size_t)i * D + d] = s;
+                u = __fadd_rn(u, __fmul_rn(s, sk[i]));
+            }
+            u = __fmul_rn(__fsub_rn(vv, u), beta);
+            for (int i = 0; i < D; i++) {
+                const float s = __fadd_rn(S[(size_t)i * D + d], __fmul_rn(sk[i], u));
+                S[(size_t)i * D + d] = s;
+                ov = __fadd_rn(ov, __fmul_rn(s, sq[i]));
             }
         }
         // per-head RMSNorm with weight, then the sigmoid output gate (glm53f_ops.c:748-752)
@@ -184,17 +116,12 @@ __global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaAr
         if (live) {
             const float inv = (float)(1.0 / sqrt(oo / (double)D + (double)a.rms_eps));
             const float n = __fmul_rn(onw, __fmul_rn(ov, inv));
-            a.o[off] = __fmul_rn(n, sigmoid_host(a.f_b ? gb_own : a.gb[off]));
+            a.o[off] = __fmul_rn(n, sigmoid_host(a.gb[off]));
         }
         if (a.snap && t == a.snap_after && live) {
             float *sn = a.snap + (size_t)blockIdx.y * a.seq_stride;
             float *Sn = sn + (size_t)h * D * D, *cn = sn + (size_t)a.H * D * D;
-            if (DS > 0) {
-#pragma unroll
-                for (int i = 0; i < DS; i++) Sn[(size_t)i * DS + d] = sreg[i];
-            } else {
-                for (int i = 0; i < D; i++) Sn[(size_t)i * D + d] = S[(size_t)i * D + d];
-            }
+            for (int i = 0; i < D; i++) Sn[(size_t)i * D + d] = S[(size_t)i * D + d];
             for (int j = 0; j < hist; j++) {
                 cn[(size_t)ch * hist + j] = pq[j];
                 cn[(size_t)P * hist + (size_t)ch * hist + j] = pk[j];
@@ -204,10 +131,6 @@ __global__ void __launch_bounds__(DS > 0 ? DS : 512) kda_core_kernel(const KdaAr
     }
 
     if (live) {
-        if (DS > 0) {
-#pragma unroll
-            for (int i = 0; i < DS; i++) S[(size_t)i * DS + d] = sreg[i];
-        }
         for (int j = 0; j < hist; j++) {
             cs[(size_t)ch * hist + j] = pq[j];
             cs[(size_t)P * hist + (size_t)ch * hist + j] = pk[j];
@@ -481,6 +404,193 @@ __global__ void __launch_bounds__(256) kda_out_kernel(const KdaArgs a, int heads
         a.o[off + i] = __fmul_rn(__fmul_rn(a.o_norm[lane * C + i], __fmul_rn(o[i], inv)), sigmoid_near(a.gb[off + i]));
 }
 
+// One position of one sequence. The chain of a single step is all latency: convolutions, norms, gates, two sums over the
+// state, the output's norm. A cluster takes a head, 32 columns of the state to a CTA of 256 threads; what all columns need
+// (q, k, the decays with their low-rank up-projection) every CTA computes for itself, and only the sum of squares of the
+// output crosses the cluster. Weights and state travel before the wait for the kernel in front. Every value is that of
+// the sequential recurrence, bit for bit: i ascending, rounded term by term, 256 dependent additions of one warp with a
+// lane per column. (One CTA per head with its 64 KB of state and 255 registers a thread: 17.8 us cold, now 10.6, 8.7 of them behind the products.)
+constexpr int KDA_STEP_PITCH(int D) { return 2 * D + 16; }               // bytes: consecutive rows begin on different banks
+constexpr int KDA_STEP_SMEM(int D, bool low_rank) { return D * 32 * 4 + (low_rank ? (D + 32) * KDA_STEP_PITCH(D) : 0); }
+template <int DS, int KW>
+__global__ void __cluster_dims__(DS / 32, 1, 1) __launch_bounds__(256) kda_step_kernel(const KdaArgs a)
+{
+    pdl_trigger();
+    constexpr int D = DS, CL = DS / 32, PITCH = KDA_STEP_PITCH(DS), TASKS = 2 * D + 32;
+    extern __shared__ __align__(16) uint8_t smem[];
+    float *st = reinterpret_cast<float *>(smem);                         // [D][32]: this CTA's columns of the state
+    uint8_t *lrw = smem + D * 32 * 4;                                    // D rows of f_b, then 32 rows of g_b
+    __shared__ __align__(16) float vec[3][D];                            // decay, k, q
+    __shared__ __align__(16) float lr[2][D];
+    __shared__ float raw[TASKS], sgb[32];
+    __shared__ double mine;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int rank = blockIdx.x % CL, h = a.head0 + blockIdx.x / CL, col0 = rank * 32, P = a.H * D, K = KW ? KW : a.K, hist = K - 1;
+    float *S = a.state + (size_t)h * D * D + col0, *cs = a.state + (size_t)a.H * D * D;
+    for (int i = tid; i < D * 8; i += 256)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(st + i * 4)), "l"(S + (size_t)(i >> 3) * D + (i & 7) * 4) : "memory");
+    if (a.f_b) {
+        constexpr int PER = D / 8;
+        for (int i = tid; i < (D + 32) * PER; i += 256) {
+            const int row = i / PER, piece = i % PER;
+            const uint16_t *src = (row < D ? a.f_b + ((size_t)h * D + row) * D : a.g_b + ((size_t)h * D + col0 + row - D) * D) + piece * 8;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(lrw + (size_t)row * PITCH + piece * 16)), "l"(src) : "memory");
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // convolution channels: q, then k, of the whole head, then v of this CTA's columns; two per thread at most
+    const float *const xs[3] = {a.q, a.k, a.v}, *const ws[3] = {a.q_conv, a.k_conv, a.v_conv};
+    int which[2], ch[2];
+    bool has[2], own[2];
+    float w[2][KW ? KW : 1], past[2][KW ? KW : 1];
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+        const int task = tid + n * 256;
+        has[n] = task < TASKS;
+        which[n] = task < D ? 0 : task < 2 * D ? 1 : 2;
+        const int c = which[n] < 2 ? task % D : col0 + task - 2 * D;
+        own[n] = has[n] && c >= col0 && c < col0 + 32;
+        ch[n] = h * D + c;
+        if (has[n]) {
+#pragma unroll
+            for (int j = 0; j < KW; j++) w[n][j] = ws[which[n]][(size_t)ch[n] * KW + j];
+#pragma unroll
+            for (int j = 0; j + 1 < KW; j++) past[n][j] = cs[(size_t)which[n] * P * hist + (size_t)ch[n] * hist + j];
+        }
+    }
+    const float ea = expf_host(a.A_log[h]), qscale = 1.0f / sqrtf((float)D);
+    const float dtb = a.dt_bias[h * D + tid % D], onw = a.o_norm[col0 + lane];
+    // everything above is weights and this layer's own state; from here on the kernel in front is read
+    pdl_wait();
+    float now[2];
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+        if (has[n]) now[n] = xs[which[n]][ch[n]];
+    const float beta_raw = a.braw[h];
+    if (a.f_b)
+        for (int i = tid; i < 2 * D; i += 256) lr[i / D][i % D] = (i < D ? a.lrf : a.lrg)[i % D];
+    // ---- convolutions and SiLU
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+        if (has[n]) {
+            float y;
+            if (KW) {
+                y = __fmul_rn(w[n][KW ? KW - 1 : 0], now[n]);
+#pragma unroll
+                for (int j = 0; j + 1 < KW; j++) y = mul_add_unfused(w[n][j], past[n][j], y);
+            } else {
+                const float *wp = ws[which[n]] + (size_t)ch[n] * K, *pp = cs + (size_t)which[n] * P * hist + (size_t)ch[n] * hist;
+                y = __fmul_rn(wp[hist], now[n]);
+                for (int j = 0; j < hist; j++) y = mul_add_unfused(wp[j], pp[j], y);
+            }
+            raw[tid + n * 256] = __fmul_rn(y, sigmoid_host(y));
+        }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    // ---- decays, this CTA's output gates (z = f_b lrf, gb = g_b lrg: even and odd columns apart, ascending) and the l2norm
+    // (divide by sqrt(sum of squares + 1e-6), sums in FP64, glm53f_ops.c:661-667): each to warps of its own
+    if (tid < D + 32) {
+        const bool gate = tid >= D;
+        float z;
+        if (a.f_b) {
+            const uint8_t *row = lrw + (size_t)tid * PITCH;
+            const float *x = lr[gate ? 1 : 0];
+            F2 t = f2(0.f, 0.f);
+#pragma unroll 4
+            for (int c = 0; c < D; c += 8) {
+                const uint4 v = *reinterpret_cast<const uint4 *>(row + 2 * c);
+                const float4 x0 = *reinterpret_cast<const float4 *>(x + c), x1 = *reinterpret_cast<const float4 *>(x + c + 4);
+                float lo, hi;
+                bf16x2_to_f32(v.x, lo, hi); t = f2_fma(f2(lo, hi), f2(x0.x, x0.y), t);
+                bf16x2_to_f32(v.y, lo, hi); t = f2_fma(f2(lo, hi), f2(x0.z, x0.w), t);
+                bf16x2_to_f32(v.z, lo, hi); t = f2_fma(f2(lo, hi), f2(x1.x, x1.y), t);
+                bf16x2_to_f32(v.w, lo, hi); t = f2_fma(f2(lo, hi), f2(x1.z, x1.w), t);
+            }
+            z = f2_sum(t);
+        } else z = gate ? a.gb[h * D + col0 + tid - D] : a.z[h * D + tid];
+        if (gate) sgb[tid - D] = sigmoid_host(z);
+        else      vec[0][tid] = expf_host(__fmul_rn(a.gate_lb, sigmoid_host(__fmul_rn(ea, __fadd_rn(z, dtb)))));
+    } else if (warp >= 6) {
+        double t = 0.0;
+#pragma unroll
+        for (int i = 0; i < D / 32; i++) { const double v = (double)raw[(warp - 6) * D + lane + 32 * i]; t = fma(v, v, t); }
+        t = warp_sum(t);
+        const float inv = (float)rsqrt_newton(t + (double)1e-6f);
+#pragma unroll
+        for (int i = 0; i < D / 32; i++) {
+            const float v = __fmul_rn(raw[(warp - 6) * D + lane + 32 * i], inv);
+            vec[warp == 6 ? 2 : 1][lane + 32 * i] = warp == 6 ? __fmul_rn(v, qscale) : v;
+        }
+    }
+    __syncthreads();
+    // ---- the state's columns: decay, u = k.S, S += k (v - u) beta, o = q.S
+    float o = 0.f;
+    if (warp == 0) {
+        float u = 0.f;
+        const float4 *al4 = reinterpret_cast<const float4 *>(vec[0]), *k4 = reinterpret_cast<const float4 *>(vec[1]), *q4 = reinterpret_cast<const float4 *>(vec[2]);
+        float *sc = st + lane;
+        const float beta = sigmoid_host(beta_raw);
+#pragma unroll 8
+        for (int i = 0; i < D / 4; i++) {
+            const float4 al = al4[i], kk = k4[i];
+            const float s0 = __fmul_rn(sc[(4 * i) * 32], al.x), s1 = __fmul_rn(sc[(4 * i + 1) * 32], al.y), s2 = __fmul_rn(sc[(4 * i + 2) * 32], al.z),
+                        s3 = __fmul_rn(sc[(4 * i + 3) * 32], al.w);
+            u = __fadd_rn(u, __fmul_rn(s0, kk.x)); u = __fadd_rn(u, __fmul_rn(s1, kk.y));
+            u = __fadd_rn(u, __fmul_rn(s2, kk.z)); u = __fadd_rn(u, __fmul_rn(s3, kk.w));
+        }
+        u = __fmul_rn(__fsub_rn(raw[2 * D + lane], u), beta);
+#pragma unroll 8
+        for (int i = 0; i < D / 4; i++) {
+            const float4 al = al4[i], kk = k4[i], q = q4[i];
+            const float s0 = __fadd_rn(__fmul_rn(sc[(4 * i) * 32], al.x), __fmul_rn(kk.x, u)), s1 = __fadd_rn(__fmul_rn(sc[(4 * i + 1) * 32], al.y), __fmul_rn(kk.y, u)),
+                        s2 = __fadd_rn(__fmul_rn(sc[(4 * i + 2) * 32], al.z), __fmul_rn(kk.z, u)), s3 = __fadd_rn(__fmul_rn(sc[(4 * i + 3) * 32], al.w), __fmul_rn(kk.w, u));
+            float *Sp = S + (size_t)(4 * i) * D + lane;
+            Sp[0] = s0; Sp[D] = s1; Sp[2 * D] = s2; Sp[3 * D] = s3;
+            o = __fadd_rn(o, __fmul_rn(s0, q.x)); o = __fadd_rn(o, __fmul_rn(s1, q.y));
+            o = __fadd_rn(o, __fmul_rn(s2, q.z)); o = __fadd_rn(o, __fmul_rn(s3, q.w));
+        }
+        const double oo = warp_sum((double)o * (double)o);
+        if (lane == 0) mine = oo;
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    // ---- per-head RMSNorm with weight, then the sigmoid output gate (glm53f_ops.c:748-752)
+    if (warp == 0) {
+        double tot = 0.0;
+#pragma unroll
+        for (int r = 0; r < CL; r++) tot += ld_cluster_f64(&mine, r);
+        const float inv = (float)rsqrt_newton(tot / (double)D + (double)a.rms_eps);
+        a.o[h * D + col0 + lane] = __fmul_rn(__fmul_rn(onw, __fmul_rn(o, inv)), sgb[lane]);
+    }
+    // the histories move on by one (every CTA of the head has read them: the barrier above); each channel by one thread
+#pragma unroll
+    for (int n = 0; n < 2; n++)
+        if (own[n] && hist > 0) {
+            float *hp = cs + (size_t)which[n] * P * hist + (size_t)ch[n] * hist;
+            if (KW) {
+#pragma unroll
+                for (int j = 0; j + 2 < KW; j++) hp[j] = past[n][j + 1];
+            } else
+                for (int j = 0; j + 1 < hist; j++) hp[j] = hp[j + 1];
+            hp[hist - 1] = now[n];
+        }
+    __syncwarp();
+    cluster_arrive();                                    // no CTA leaves while another may still read its sum
+    cluster_wait();
+}
+
+template <int DS, int KW>
+static bool kda_step(cudaStream_t st, const KdaArgs &a, int heads)
+{
+    static SmemGrant grant;
+    const size_t smem = KDA_STEP_SMEM(DS, a.f_b != nullptr);
+    // (with the static arrays it is above the 48 KB that need no consent before the dynamic part alone is)
+    if (!dev_opt_in_smem((const void *)kda_step_kernel<DS, KW>, smem + (8 << 10), grant)) return false;
+    G5B_LAUNCH_PDL((kda_step_kernel<DS, KW>), dim3(heads * (DS / 32)), dim3(256), smem, st, a);
+    return true;
+}
+
 constexpr int KDA_EARLY_T = 8;        // positions whose scan is shorter than a launch
 template <int DS>
 static void kda_rows(cudaStream_t st, const KdaArgs &a, const KdaScratch &x, int heads, int n_seq)
@@ -509,21 +619,17 @@ void kda_core(cudaStream_t st, float *o, const float *q, const float *k, const f
               fused ? static_cast<const uint16_t *>(lr->f_b) : nullptr, fused ? static_cast<const uint16_t *>(lr->g_b) : nullptr,
               fused ? lr->lrf : nullptr, fused ? lr->lrg : nullptr, snap, snap_after};
     const dim3 grid(heads > 0 ? heads : s.H, n_seq < 1 ? 1 : n_seq);
-    const size_t smem = fused ? (size_t)2 * s.D * (2 * s.D + 16) : 0;
-    if (T * grid.y > 1 && scratch && s.K <= 17 && (s.D == 128 || s.D == 64)) {
+    const bool known = s.K >= 1 && s.K <= 17 && (s.D == 128 || s.D == 64);
+    if (known && T * grid.y == 1) {
+        const bool ok = s.D == 128 ? (s.K == 4 ? kda_step<128, 4>(st, a, (int)grid.x) : kda_step<128, 0>(st, a, (int)grid.x))
+                                   : (s.K == 4 ? kda_step<64, 4>(st, a, (int)grid.x) : kda_step<64, 0>(st, a, (int)grid.x));
+        if (ok || fused) return;             // (a refusal is kept for g5b_last_error)
+    } else if (known && scratch) {
         if (s.D == 128) kda_rows<128>(st, a, *scratch, (int)grid.x, (int)grid.y);
         else            kda_rows<64>(st, a, *scratch, (int)grid.x, (int)grid.y);
         return;
     }
-    if (s.D == 128) {
-        static SmemGrant grant;
-        if (!dev_opt_in_smem((const void *)kda_core_kernel<128>, 2 * 128 * (2 * 128 + 16), grant)) return;
-        // launched early: its CTAs load the 64 KB state and the histories while the projection kernel
-        // before it drains, and wait for that kernel inside (griddepcontrol.wait above)
-        G5B_LAUNCH_PDL(kda_core_kernel<128>, grid, dim3(128), smem, st, a);
-    }
-    else if (s.D == 64) G5B_LAUNCH(kda_core_kernel<64>, grid, 64, smem, st, a);
-    else                G5B_LAUNCH(kda_core_kernel<0>, grid, ((s.D + 31) / 32) * 32, 0, st, a);
+    G5B_LAUNCH(kda_core_kernel, grid, ((s.D + 31) / 32) * 32, 0, st, a);
 }
 
 }  // namespace g5b

@@ -319,25 +319,6 @@ __global__ void __launch_bounds__(HC_THREADS) hc_pre_fused_kernel(const HcFused 
 constexpr int HCC_CTAS = 8, HCC_THREADS = 512, HCC_WARPS = HCC_THREADS / 32, HCC_MAX_W = 1024, HCC_MAX_HS = 4096;
 constexpr int HCC_ROWS = 3, HCC_ROW_WARPS = 8, HCC_SPLITS = HCC_WARPS / HCC_ROW_WARPS;
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_cta_rank()
-{
-    uint32_t r;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-// the shared variable `p` of CTA `rank` of this cluster
-__device__ __forceinline__ double ld_cluster_f64(const double *p, uint32_t rank)
-{
-    const uint32_t mine = (uint32_t)__cvta_generic_to_shared(p);
-    uint32_t theirs;
-    double v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(theirs) : "r"(mine), "r"(rank));
-    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(theirs) : "memory");
-    return v;
-}
-
 // v / d for d > 0 to a relative 2^-40: the hardware's reciprocal estimate r (20 bits), its error
 // e = 1 - d r, and v r (1 + e). An FP64 instruction occupies its pipe for 32 cycles per warp here
 // and a Sinkhorn pass is a chain of nothing else, so every instruction less is 0.6 us per site; the
