@@ -857,6 +857,7 @@ static int run_moe_seq_split(g5b_engine *e, Layer &w, const float *x, int n, flo
         const int m = (r1 - r0) * n, g0 = r0 * n;
         const bool last = gi == mine;
         const float *xg = all + (size_t)g0 * c.hidden;
+        e->plan.tile_shift = tc_tile_shift((long)m * s.K, s.n_local);
         router_plan(e->st, e->ridx, e->rw, e->rscore, xg, c.hidden, w.router.w, w.router.dt, w.bias, m, s, e->plan,
                     with_shared ? 1 : 0, e->counter, last ? me * n - g0 : 0, last ? n : 0);
         if (e->expert_path >= 1 && tc_moe_takes(e->tc, s, m)) {
@@ -903,6 +904,7 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
             return 0;
         }
     }
+    e->plan.tile_shift = tc_tile_shift((long)n * s.K, s.n_local);
     router_plan(e->st, e->ridx, e->rw, e->rscore, x, c.hidden, w.router.w, w.router.dt, w.bias, n, s, e->plan,
                 shared_in_plan ? 1 : 0, e->counter, 0, -1, e->rdots);
     prof_mark(e, 1);

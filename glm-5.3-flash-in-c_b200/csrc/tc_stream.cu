@@ -45,7 +45,7 @@
 namespace g5b {
 
 constexpr int TS_MAX_SEG = 8;              // matrices of one launch
-constexpr int TS_N = 64;                   // activation rows per tile at most (TC_TILE_ROWS of an expert)
+constexpr int TS_N = 64;                   // activation rows per tile at most (of an expert: tc_tile_shift)
 constexpr int TS_EN = TS_N / 2;            // rows an epilogue thread holds
 constexpr int TS_PARTS = 4;                 // partial results of a tile that are read at once
 constexpr int TS_MAX_STAGES = 6, TS_MAX_XS = 3;    // FP8: activation stages at most
@@ -81,18 +81,18 @@ struct TsArgs {
     int *err;
 };
 
-// How a slot's cnt rows are cut into tiles: equal shares of at most TC_TILE_ROWS rows, rounded up to 8.
-__device__ __forceinline__ int ts_tile_rows(int cnt)
+// How a slot's cnt rows are cut into tiles: equal shares of at most 1 << shift rows, rounded up to 8.
+__device__ __forceinline__ int ts_tile_rows(int cnt, int shift)
 {
-    if (cnt <= TC_TILE_ROWS) return (cnt + 7) & ~7;
-    const int k = (cnt + TC_TILE_ROWS - 1) / TC_TILE_ROWS;
+    if (cnt <= 1 << shift) return (cnt + 7) & ~7;
+    const int k = (cnt + (1 << shift) - 1) >> shift;
     return ((cnt + k - 1) / k + 7) & ~7;
 }
 
 // Walks the tiles of a CTA's share in order: matrix (or expert) `which`, its row tile rt, the np activation rows from
 // row0 on, n = np rounded up to 8. An expert's row tile goes past its token tiles one after the other: its weights
 // come from L2 then.
-struct TsPlan { const int *tile0, *off, *cnt, *exp; int slots; };
+struct TsPlan { const int *tile0, *off, *cnt, *exp; int slots, shift; };
 template <int MODE>
 struct TsCursor {
     int which, rt, row0, np, n;
@@ -113,7 +113,7 @@ struct TsCursor {
     }
     __device__ __forceinline__ void enter(const TsPlan &p)
     {
-        which = p.exp[slot]; cnt = p.cnt[slot]; rows = ts_tile_rows(cnt); nt = p.tile0[slot + 1] - p.tile0[slot];
+        which = p.exp[slot]; cnt = p.cnt[slot]; rows = ts_tile_rows(cnt, p.shift); nt = p.tile0[slot + 1] - p.tile0[slot];
     }
     __device__ __forceinline__ void start(const TsArgs &a, const TsPlan &p, int tile)
     {
@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
     // runs, and only the warps that read its results (the terms) or write (sums) wait. What an expert's tile is, the router says.
     if (MODE != TS_DENSE) pdl_wait();
     int n_tiles = a.tiles;
-    TsPlan plan{s_plan, s_plan + a.slots + 1, s_plan + 2 * a.slots + 1, s_plan + 3 * a.slots + 1, 0};
+    TsPlan plan{s_plan, s_plan + a.slots + 1, s_plan + 2 * a.slots + 1, s_plan + 3 * a.slots + 1, 0, a.p.tile_shift};
     if (MODE != TS_DENSE) {
         plan.slots = min(*a.p.n_slots, a.slots);
         for (int i = threadIdx.x; i < plan.slots; i += blockDim.x) {
@@ -926,10 +926,10 @@ static bool x_maps(TcGemm *g, TsMaps &m, const void *base, bool fp8, size_t plan
 static size_t stage_plan(TsArgs &a, bool fp8, size_t extra)
 {
     a.x_stage = (fp8 ? 8 : 6) * a.n * 128;                           // (a multiple of 1024 per 64-column atom)
-    // A third activation stage where a unit's terms are as large as its weights (tiles of 17 to 32 rows): a stage is only
-    // refilled when its products are done, and with two the way to L2 and back was part of every unit. Smaller terms are
-    // there in time with two, and larger ones leave the weights too few stages.
-    a.xs = a.n > 16 && a.n <= TS_EN ? TS_MAX_XS : 2;
+    // A third activation stage in tiles of up to 32 rows: a stage is only refilled when its products are done, and with two the
+    // way to L2 and back was part of every unit. The terms of larger tiles would leave
+    // the weights too few stages.
+    a.xs = a.n <= TS_EN ? TS_MAX_XS : 2;
     const size_t fixed = 1024 + 1024 + TS_EXCH + extra + (fp8 ? (size_t)a.xs * a.x_stage : 0);
     const size_t stage = TS_UNIT_BYTES + (fp8 ? 0 : (size_t)a.x_stage);
     const size_t fit = (227 * 1024 - 512 - fixed) / stage;
@@ -1014,7 +1014,7 @@ bool tc_moe_takes(const TcGemm *g, const MoeShape &s, int T)
     if (!g || T < 1 || T > g->max_t || s.dt != DT_FP8 || s.br != 128 || s.bc != 128 || s.E % 128 || s.I % 128) return false;
     if (!(s.limit > 0.f) || s.limit * s.limit > 60000.f) return false;                  // activations must fit F16
     const int slots = (T * s.K < s.n_local ? T * s.K : s.n_local) + 1;
-    return (long)(slots + (T * s.K + T) / TC_TILE_ROWS) * (s.I / 64 > s.E / 128 ? s.I / 64 : s.E / 128) <= TS_CNT;
+    return (long)(slots + ((T * s.K + T) >> tc_tile_shift((long)T * s.K, s.n_local))) * (s.I / 64 > s.E / 128 ? s.I / 64 : s.E / 128) <= TS_CNT;
 }
 
 static const std::pair<CUtensorMap, CUtensorMap> *expert_maps(TcGemm *g, const ExpertSlab &w, const MoeShape &s)
@@ -1046,7 +1046,7 @@ int tc_moe_run(TcGemm *g, cudaStream_t st, float *contrib, void *act, void *xter
     G5B_LAUNCH_PDL(tc_split_kernel<true>, dim3(pairs), dim3(512), 0, st, sp);
     TsMaps m;
     TsArgs a{};
-    a.T = T; a.n = T < TC_TILE_ROWS ? (T + 7) & ~7 : TC_TILE_ROWS; a.plane = P; a.p = p; a.E = s.E; a.I = s.I; a.xinv = xinv; a.limit = s.limit; a.act_scale = act_term_scale(s.limit); a.act_inv = 1.0f / a.act_scale;
+    a.T = T; a.n = T < 1 << p.tile_shift ? (T + 7) & ~7 : 1 << p.tile_shift; a.plane = P; a.p = p; a.E = s.E; a.I = s.I; a.xinv = xinv; a.limit = s.limit; a.act_scale = act_term_scale(s.limit); a.act_inv = 1.0f / a.act_scale;
     a.slots = (T * s.K < s.n_local ? T * s.K : s.n_local) + 1;
     a.part = g->part; a.cnt = g->cnt; a.err = g->err;
     const size_t plan_bytes = (size_t)(4 * a.slots + 4) * sizeof(int);
