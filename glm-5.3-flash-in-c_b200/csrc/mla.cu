@@ -990,7 +990,9 @@ void mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void
     static SmemGrant grant;
     if (!dev_opt_in_smem((const void *)mla_flash_kernel, FL_SMEM, grant)) return;
     const int stride = s.topk + s.KP;
-    const int nchunks = (stride + FL_POS - 1) / FL_POS;
+    // partial rows are laid out for the chunks that the call's last position can see: an early stretch of a prompt goes in
+    // few launches of many queries
+    const int last = s.batch ? cached + 1 : cached + T, nchunks = ((last < stride ? last : stride) + FL_POS - 1) / FL_POS;
     const size_t per_token = (size_t)s.H * nchunks * FL_KL * sizeof(float);
     int group = (int)(part_bytes / per_token);
     if (group < 1) group = 1;
