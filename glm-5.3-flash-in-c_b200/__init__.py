@@ -98,6 +98,7 @@ def lib() -> C.CDLL:
     L.g5b_engine_load_checkpoint.argtypes = [C.c_void_p, C.c_char_p, C.c_int]
     L.g5b_engine_synth_session.argtypes = [C.c_void_p, C.c_uint64, C.c_int]
     L.g5b_engine_last_picks.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
+    L.g5b_debug_moe_rows.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p]
     L.g5b_engine_decode_greedy.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_void_p]
     L.g5b_engine_ep_handle_bytes.restype = C.c_size_t
     L.g5b_engine_ep_export.argtypes = [C.c_void_p, C.c_void_p]
@@ -383,6 +384,16 @@ class Engine(FlatModel):
         if self.L.g5b_engine_last_picks(self.handle, T, idx.ctypes.data, w.ctypes.data) != 0:
             self._err("last_picks")
         return idx, w
+
+    def debug_moe_rows(self, layer: int, x):
+        """Contribution rows of a MoE layer before exchange and combine: (picks' rows [T][topk][hidden], zero where another
+        rank owns the pick, and the shared expert's [T][hidden]) (g5b_debug_moe_rows)."""
+        x = _f32(x)
+        T, K, E = x.shape[0], self.cfg.topk, self.cfg.hidden
+        rows = np.zeros((T * K + T, E), np.float32)
+        if self.L.g5b_debug_moe_rows(self.handle, layer, x.ctypes.data, T, rows.ctypes.data) != 0:
+            self._err("debug_moe_rows")
+        return rows[:T * K].reshape(T, K, E), rows[T * K:]
 
     def use_sequence(self, seq: int):
         if self.L.g5b_engine_use_sequence(self.handle, seq) != 0:

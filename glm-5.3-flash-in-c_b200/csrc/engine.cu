@@ -782,7 +782,7 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         int max_c = e->mtp ? 2 * c.hidden : c.hidden;
         for (int v : {P, c.q_lora, c.kv_lora, c.kda_head_dim, c.mla_heads * c.v_head}) max_c = v > max_c ? v : max_c;
         for (int v : {c.dense_inter, c.moe_inter * c.n_shared}) max_c = v > max_c ? v : max_c;
-        e->tc = tc_gemm_create(max_c, e->pass, e->err_dev);
+        e->tc = tc_gemm_create(max_c, c.hidden > c.moe_inter ? c.hidden : c.moe_inter, e->pass, e->err_dev);
         if (!e->tc) return fail("the tensor-core projection path could not be set up (tensor-map encoder or scratch)");
     }
     e->cached_seq.assign((size_t)e->n_seq, 0);
@@ -1923,6 +1923,37 @@ extern "C" int g5b_op_router(g5b_engine *e, int layer, const float *x, int T, in
     }
     CU(cudaGetLastError());
     return 0;
+}
+
+// A MoE layer's contribution rows as they are before the exchange and the combine (test aid): the rows of the picks that this
+// engine owns, and the shared expert's; the others are zero. Needs no connected peers.
+extern "C" int g5b_debug_moe_rows(g5b_engine *e, int layer, const float *x, int T, float *rows)
+{
+    if (check_op(e, layer, T)) return -1;
+    Layer &w = e->L[layer];
+    const g5b_config &c = e->c;
+    if (w.is_dense || !w.table_dev || !w.router.loaded() || !w.bias) return fail("layer %d has no routed experts", layer);
+    if (T > e->pass) return fail("at most %d rows", e->pass);
+    const MoeShape s = moe_shape(e, w);
+    const int shared = c.n_shared == 1 && w.sh_gate.dt == s.dt && w.sh_down.loaded() ? 1 : 0;
+    const size_t n = ((size_t)T * c.topk + T) * c.hidden;
+    Staged st{e};
+    float *xd = st.in(x, (size_t)T * c.hidden);
+    if (!xd) return fail("out of device memory");
+    CU(cudaMemsetAsync(e->contrib, 0, n * 4, e->st));
+    e->plan.tile_shift = tc_tile_shift((long)T * s.K, s.n_local);
+    router_plan(e->st, e->ridx, e->rw, e->rscore, xd, c.hidden, w.router.w, w.router.dt, w.bias, T, s, e->plan, shared, e->counter, 0, -1, e->rdots);
+    if (e->expert_path >= 1 && tc_moe_takes(e->tc, s, T)) {
+        if (tc_moe_run(e->tc, e->st, e->contrib, e->act, e->xterms, e->xinv, xd, c.hidden, expert_slab(e, w), e->plan, T, s))
+            return fail("the expert kernels could not be launched");
+    } else {
+        moe_gateup(e->st, e->act, xd, c.hidden, w.table_dev, e->plan, T, s);
+        moe_down(e->st, e->contrib, e->act, w.table_dev, e->plan, T, s);
+    }
+    CU(cudaMemcpyAsync(rows, e->contrib, n * 4, cudaMemcpyDeviceToHost, e->st));
+    CU(cudaStreamSynchronize(e->st));
+    CU(cudaGetLastError());
+    return check_device_error(e);
 }
 
 // The expert picks and weights of the most recent MoE pass (its last chunk of T <= 64 positions),

@@ -11,8 +11,9 @@
 //   3. waits - bounded - until every rank's word for this step has arrived here, and
 //   4. combines: out[t][d] = (float) sum_j w[t][j] * row[t*K+j][d] in FP64 in top-k order, plus the
 //      shared expert's row (computed on every rank) in FP32: the arithmetic of the one-GPU combine
-//      and of the reference (src/core/glm53f_ops.c:1329-1340), so the result does not depend on
-//      the number of ranks.
+//      and of the reference (src/core/glm53f_ops.c:1329-1340). The expert kernels sum every row in an order
+//      that depends on neither the rank nor the other rows of the launch, so all ranks hold the same
+//      shared rows, bit for bit, and the result does not depend on the number of ranks.
 //
 // Two exchange buffers alternate by step parity: a rank can be at most one step ahead of a peer
 // (its next combine needs that peer's next word), so rows of step s+1 never land in a buffer

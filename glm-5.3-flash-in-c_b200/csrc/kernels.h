@@ -75,7 +75,7 @@ inline void gemv(cudaStream_t st, const DMat &m, const float *x, int ldx, float 
 // second pass over the weights of those that do costs more (1355 -> 1420 us).
 inline int tc_tile_shift(long pairs, int experts) { return pairs <= 3l * experts ? 4 : 5; }   // log2: tiles are counted by every role
 struct TcGemm;
-TcGemm *tc_gemm_create(int max_c, int max_t, int *err);      // widest input, most positions
+TcGemm *tc_gemm_create(int max_c, int max_ec, int max_t, int *err);      // widest input, that of an expert, most positions
 void tc_gemm_free(TcGemm *g);
 void tc_gemm_recover(TcGemm *g, cudaStream_t st);
 bool tc_gemm_takes(const TcGemm *g, const GemvSeg &s, int T);

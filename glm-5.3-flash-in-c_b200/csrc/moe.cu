@@ -9,7 +9,8 @@
 // weight table with them.
 //
 // Expert-major like the reference: each distinct expert's weights are streamed once for all
-// (token, slot) pairs that chose it, every pair keeps its own output row, and the rows are
+// (token, slot) pairs that chose it, every pair keeps its own output row, whose bits depend on the pair
+// alone (not on the other pairs of the call), and the rows are
 // summed per token in top-k order in FP64 (:1329-1337), the shared expert added last in FP32.
 #include "dot_rows.cuh"
 #include "f64_tile.cuh"
@@ -183,7 +184,8 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
 
     // Group the (token, slot) pairs by expert. Slots are numbered in expert order; the shared
     // expert, when asked for, is the last slot and takes every token. Which pair of an expert
-    // lands where inside its slot does not matter: every pair has its own output row.
+    // lands where inside its slot does not matter (the atomics below leave it open): every pair has its own
+    // output row, and no expert kernel sums a row in an order that depends on its place or on the rows beside it.
     const int n = a.T * a.K, nth = RT_WARPS * 32;
     int *sidx = sidx_buf;                                     // [T*K] ids
     for (int i = tid; i < n; i += nth) sidx[i] = __ldcg(a.idx + i);

@@ -9,7 +9,10 @@
 // weights (256 FP8 codes or 128 BF16 values per row). All units of the launch are numbered in a row and
 // every CTA takes an equal, contiguous share, whatever the shapes: no last wave of tiles, no choice of a split.
 // A tile that two or more CTAs worked on is put together by the one that finishes last (partial sums in
-// an L2-resident buffer, added in the order of the columns, so the result does not depend on who that is).
+// an L2-resident buffer, added in the order of the columns, so the result does not depend on who that is). Where a
+// projection's tile is cut depends on the launch, so the last bits of a row do too (its matrices, the number of positions, which
+// tile of rows it is in): the ranks of a group agree because they run the same launch. An expert's tile is summed in
+// one order wherever it is cut (ts_finish_expert): the ranks of a group launch different experts.
 //
 //   A operand  = 128 rows of W. BF16: the TMA tile in shared memory as stored. FP8: eight converter
 //                warps turn the TMA tile's codes into F16 (exact) and put them into tensor memory, from
@@ -51,6 +54,7 @@ constexpr int TS_PARTS = 4;                 // partial results of a tile that ar
 constexpr int TS_MAX_STAGES = 6, TS_MAX_XS = 3;    // FP8: activation stages at most
 constexpr int TS_UNIT_BYTES = 32768, TS_EXCH = TS_EN * 128 * 4;
 constexpr int TS_SEG_UNITS = 4;            // BF16: units summed inside the tensor cores before the registers take over
+constexpr int TS_SLAB = TS_EN * 128;        // values of one partial result of an expert's tile
 enum { TS_DENSE = 0, TS_GATEUP = 1, TS_DOWN = 2 };
 constexpr int TS_FP8_THREADS = 20 * 32, TS_BF16_THREADS = 10 * 32;
 
@@ -64,6 +68,7 @@ struct TsArgs {
     TsSeg seg[TS_MAX_SEG];
     int n_seg, tiles;          // projections: tiles of all matrices
     int KB;                    // units per tile
+    int part_slabs;            // experts: unit sums that fit one CTA's partial results
     int blocks;                // FP8: 128-column blocks per row (2 KB, or one less)
     int T, n, plane;           // rows, rows of the largest tile (a multiple of 8); rows between the terms' planes
     int nt;                    // projections: tiles of n rows that T rows make
@@ -75,7 +80,7 @@ struct TsArgs {
     const float *xinv;         // 2^-e of each pair's activation
     void *out;                 // gate/up: F16 terms, planes of [plane][I]; down: contribution rows [.][E]
     float limit, act_scale, act_inv;   // the scale of the SwiGLU output's terms, a power of two, and its reciprocal
-    float *part; int *cnt;     // partial results [CTA][2][row][128], units done per tile (zero between launches)
+    float *part; int *cnt;     // partial results [CTA][2][row][128] (experts: ts_slab), units done per tile (zero between launches)
     int xs;                    // FP8: activation stages
     int stages, x_stage;       // weight stages (BF16: of weights and terms); bytes of one stage's terms
     int *err;
@@ -226,11 +231,26 @@ __device__ __forceinline__ void ts_store(const TsArgs &a, const TsCursor<MODE> &
     __syncwarp();
 }
 
-// The 256 epilogue threads after a CTA's share kb0 .. kb1 of a tile. acc[i]: this thread's sums of weight row `row`. A
+// Projections: the 256 epilogue threads after a CTA's share kb0 .. kb1 of a tile. acc[i]: this thread's sums of weight row `row`. A
 // tile of at most 32 rows (`small`): both groups of warps hold rows 0 .. 31, each the sums of its own units;
 // otherwise group eg holds rows 32 eg .. The sums go through shared memory (exch: [32][128]), 32 rows at a time; a
 // tile shared with other CTAs is put together by the one that finishes last.
 __device__ __forceinline__ void ts_bar() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// A CTA's partial results of a tile, `units` of it, are written: true (for all 256 threads) if they were the tile's last.
+__device__ __forceinline__ bool ts_last(const TsArgs &a, int tile, int units, int *s_last)
+{
+    __threadfence();
+    ts_bar();
+    if (threadIdx.x == 0) {
+        const int done = atomicAdd(a.cnt + tile, units) + units;
+        *s_last = done == a.KB;
+        if (done == a.KB) a.cnt[tile] = 0;
+    }
+    ts_bar();
+    if (!*s_last) return false;
+    __threadfence();
+    return true;
+}
 template <bool FP8, int MODE>
 __device__ __forceinline__ void ts_finish(const TsArgs &a, const TsCursor<MODE> &t, const TsEpi<FP8, MODE> &ep, float (&acc)[TS_EN], int tile, bool first,
                                           int kb0, int kb1, long long U, bool small, int eg, int row, float *exch, int *s_last)
@@ -261,16 +281,7 @@ __device__ __forceinline__ void ts_finish(const TsArgs &a, const TsCursor<MODE> 
                 __stcg(reinterpret_cast<float4 *>(pr + r0 * 128 + i), *reinterpret_cast<const float4 *>(exch + i));
     }
     if (whole) return;
-    __threadfence();
-    ts_bar();
-    if (threadIdx.x == 0) {
-        const int done = atomicAdd(a.cnt + tile, kb1 - kb0) + (kb1 - kb0);
-        *s_last = done == a.KB;
-        if (done == a.KB) a.cnt[tile] = 0;
-    }
-    ts_bar();
-    if (!*s_last) return;
-    __threadfence();
+    if (!ts_last(a, tile, kb1 - kb0, s_last)) return;
     const long long G = gridDim.x, ub = (long long)tile * a.KB;
     const int c0 = (int)(((ub + 1) * G - 1) / U), c1 = (int)(((ub + a.KB) * G - 1) / U);     // CTAs holding the first / last unit
     const int slot0 = (int)(U * c0 / G / a.KB) == tile ? 0 : 1;     // only the first of them began in an earlier tile
@@ -298,6 +309,75 @@ __device__ __forceinline__ void ts_finish(const TsArgs &a, const TsCursor<MODE> 
         ts_store<FP8, MODE>(a, t, ep, r0, nr, [&](int r, int c) { return exch[(r - r0) * 128 + c]; });
         ts_bar();                                             // (the buffer is free again)
     }
+}
+
+// Experts. A tile's sum has one order of additions, whatever the launch holds beside it: the even units in order, the odd
+// ones in order, then the two sums (the groups of epilogue warps take units in turn, so each has one of them). A share
+// that begins its tile leaves its two sums where the tile is cut, one that does not the sum of every unit, and the
+// last CTA adds them on (a share is cut inside one tile at most at either end, so few tiles pay for the unit sums: 8 tokens
+// of 288 experts 283 us, 293 with sums grouped by the cuts; with shares of whole quarters of a tile and every warp
+// at every unit 316). So a row of an expert has the same bits wherever its tile lies, which CTAs work on it and
+// what other rows are beside it: on every rank of an expert-parallel group (each computes the shared expert's rows
+// itself, in a launch with other experts than its peers') and on one GPU, in every batch and in every run.
+constexpr int TS_ADD = 8;                                     // unit sums that are read at once
+__device__ __forceinline__ float *ts_slab(const TsArgs &a, long long cta, int k) { return a.part + ((size_t)cta * a.part_slabs + k) * TS_SLAB; }
+// The 256 epilogue threads after a CTA's share kb0 .. kb1 of an expert's tile. acc: this thread's sums of weight row `row` over
+// its group's units, if the share begins the tile; what a part leaves is written already.
+template <int MODE>
+__device__ __forceinline__ void ts_finish_expert(const TsArgs &a, const TsCursor<MODE> &t, const TsEpi<true, MODE> &ep, const float (&acc)[TS_EN], int tile,
+                                                 int kb0, int kb1, long long U, int eg, int row, float *exch, int *s_last)
+{
+    if (kb0 == 0 && kb1 == a.KB) {
+#pragma unroll
+        for (int turn = 1; turn >= 0; turn--) {
+            if (eg == turn) {
+#pragma unroll
+                for (int g = 0; g < TS_EN; g += 8)
+                    if (g < t.np) {
+#pragma unroll
+                        for (int i = g; i < g + 8; i++) exch[i * 128 + row] = turn ? acc[i] : __fadd_rn(acc[i], exch[i * 128 + row]);
+                    }
+                __syncwarp();
+            }
+            if (turn) ts_bar();
+        }
+    } else {
+        if (!ts_last(a, tile, kb1 - kb0, s_last)) return;
+        const long long G = gridDim.x, ub = (long long)tile * a.KB;
+        const long long c0 = ((ub + 1) * G - 1) / U, b0 = U * c0 / G;                       // the CTA that had the first unit
+        const float *lead = ts_slab(a, c0, b0 >= ub ? 0 : a.part_slabs - 2);                  // (of a tile that it did not begin with: at the end)
+        const int k0 = (int)(U * (c0 + 1) / G - ub);
+        for (int i = threadIdx.x * 4; i < t.np * 128; i += 1024) {
+            float4 v[2];                                      // the sum that unit k0 goes to, and the other
+            v[0] = __ldcg(reinterpret_cast<const float4 *>(lead + (k0 & 1 ? TS_SLAB : 0) + i));
+            v[1] = __ldcg(reinterpret_cast<const float4 *>(lead + (k0 & 1 ? 0 : TS_SLAB) + i));
+            long long c = c0;
+            const float *p = nullptr;                         // CTA c's sum of unit kb
+            for (int kb = k0, end = k0; kb < a.KB;) {
+                float4 w[TS_ADD];
+#pragma unroll
+                for (int k = 0; k < TS_ADD; k++) {
+                    while (kb + k >= end && kb + k < a.KB) {      // (a CTA without units is passed over)
+                        c++;
+                        end = (int)(U * (c + 1) / G - ub);
+                        p = ts_slab(a, c, 0) + i;
+                    }
+                    w[k] = kb + k < a.KB ? __ldcg(reinterpret_cast<const float4 *>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    p += TS_SLAB;
+                }
+#pragma unroll
+                for (int k = 0; k < TS_ADD; k++)
+                    if (kb + k < a.KB) {
+                        float4 &u = v[k & 1];
+                        u.x = __fadd_rn(u.x, w[k].x); u.y = __fadd_rn(u.y, w[k].y); u.z = __fadd_rn(u.z, w[k].z); u.w = __fadd_rn(u.w, w[k].w);
+                    }
+                kb += TS_ADD;
+            }
+            *reinterpret_cast<float4 *>(exch + i) = make_float4(__fadd_rn(v[0].x, v[1].x), __fadd_rn(v[0].y, v[1].y), __fadd_rn(v[0].z, v[1].z), __fadd_rn(v[0].w, v[1].w));
+        }
+    }
+    ts_bar();
+    ts_store<true, MODE>(a, t, ep, 0, t.np, [&](int r, int c) { return exch[r * 128 + c]; });
 }
 
 // True when it is true for all 256 epilogue threads: they go on together or not at all (barriers follow).
@@ -521,70 +601,125 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
                 nx.next(a, plan);
                 ep_next.fetch(a, nx, 0, lane, quarter);
             }
-            const bool small = t.n <= TS_EN;
-            const int e0 = small ? 0 : eg * TS_EN;                   // this thread's rows: e0 .. e0 + 31 of the tile
-            const int np = t.np - e0 < 0 ? 0 : t.np - e0 < TS_EN ? t.np - e0 : TS_EN;
-            float acc[TS_EN];
+            if constexpr (MODE != TS_DENSE) {
+                // units of the other group's parity are its own; a unit's sum is rounded by itself before it is added (or left)
+                float acc[TS_EN];
 #pragma unroll
-            for (int i = 0; i < TS_EN; i++) acc[i] = 0.f;
-            // scale and add one block's products (columns past the rows hold nothing that is stored)
-            auto take = [&](uint32_t base, float sc) {
-#pragma unroll
-                for (int g = 0; g < TS_EN; g += 16) {
-                    if (g < np) {
-                        uint32_t h[16], m[16];
-                        tmem_ld16(base + e0 + g, h);
-                        tmem_ld16(base + t.n + e0 + g, m);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 16; i++)
-                            acc[g + i] = fmaf(fmaf(__uint_as_float(m[i]), 1.0f / 2048.0f, __uint_as_float(h[i])), sc, acc[g + i]);
-                    }
-                }
-            };
-            float2 sc = ep.s0;
-            if (small) {
-                // (units of the other group's parity are its own)
+                for (int i = 0; i < TS_EN; i++) acc[i] = 0.f;
                 const int skip = (it & 1) != eg;
-                if (skip && kb0 + 1 < kb1) sc = ep.pair(a, kb0 + 1);
+                float2 sc = skip && kb0 + 1 < kb1 ? ep.pair(a, kb0 + 1) : ep.s0;
+                float *slab = ts_slab(a, blockIdx.x, kb0 ? skip : tile == tile_first ? skip : a.part_slabs - 2 + skip) + row;
                 for (int kb = kb0 + skip; kb < kb1; kb += 2) {
                     const float2 sn = kb + 2 < kb1 ? ep.pair(a, kb + 2) : sc;
                     if (!(ok = mbar_wait_all(&acc_full[eg], (uint32_t)(eg ? c1 : c0) & 1, a.err, 39))) break;
                     tc_fence_after();
-                    take(lane_addr + (uint32_t)(eg * 128), sc.x);
-                    take(lane_addr + (uint32_t)(eg * 128 + 64), sc.y);
+                    const uint32_t d = lane_addr + (uint32_t)(eg * 128);
+#pragma unroll
+                    for (int g = 0; g < TS_EN; g += 8) {
+                        if (g < t.np) {
+                            uint32_t h0[8], m0[8], h1[8], m1[8];
+                            tmem_ld8(d + g, h0);
+                            tmem_ld8(d + t.n + g, m0);
+                            tmem_ld8(d + 64 + g, h1);
+                            tmem_ld8(d + 64 + t.n + g, m1);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                const float v0 = fmaf(__uint_as_float(m0[i]), 1.0f / 2048.0f, __uint_as_float(h0[i]));
+                                const float v1 = fmaf(__uint_as_float(m1[i]), 1.0f / 2048.0f, __uint_as_float(h1[i]));
+                                const float x = fmaf(v1, sc.y, __fmul_rn(v0, sc.x));
+                                if (kb0) __stcg(slab + (g + i) * 128, x);
+                                else     acc[g + i] = __fadd_rn(acc[g + i], x);
+                            }
+                        }
+                    }
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive_n(&acc_empty[eg], 2);
                     if (eg) c1++; else c0++;
+                    slab += 2 * TS_SLAB;
                     sc = sn;
+                }
+                if (kb0 == 0 && kb1 < KB) {
+#pragma unroll
+                    for (int g = 0; g < TS_EN; g += 8)
+                        if (g < t.np) {
+#pragma unroll
+                            for (int i = g; i < g + 8; i++) __stcg(ts_slab(a, blockIdx.x, tile == tile_first ? skip : a.part_slabs - 2 + skip) + i * 128 + row, acc[i]);
+                        }
                 }
                 // the uses of the other accumulator in this tile
                 const int n_units = kb1 - kb0, own = (n_units + ((it & 1) == eg)) >> 1;
                 if (eg) c0 += n_units - own; else c1 += n_units - own;
                 it += n_units;
+                if (!(ok = ts_all(ok))) break;
+                ts_finish_expert<MODE>(a, t, ep, acc, tile, kb0, kb1, U, eg, row, exch, &s_last);
             } else {
-                for (int kb = kb0; kb < kb1; kb++) {
-                    const float2 sn = kb + 1 < kb1 ? ep.pair(a, kb + 1) : sc;
-                    if (!(ok = mbar_wait_all(&acc_full[0], (uint32_t)c0 & 1, a.err, 39))) break;
-                    tc_fence_after();
-                    take(lane_addr, sc.x);
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[0]);
-                    if (!(ok = mbar_wait_all(&acc_full[1], (uint32_t)c1 & 1, a.err, 39))) break;
-                    tc_fence_after();
-                    take(lane_addr + 128u, sc.y);
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&acc_empty[1]);
-                    c0++; c1++;
-                    sc = sn;
+                const bool small = t.n <= TS_EN;
+                const int e0 = small ? 0 : eg * TS_EN;                   // this thread's rows: e0 .. e0 + 31 of the tile
+                const int np = t.np - e0 < 0 ? 0 : t.np - e0 < TS_EN ? t.np - e0 : TS_EN;
+                float acc[TS_EN];
+#pragma unroll
+                for (int i = 0; i < TS_EN; i++) acc[i] = 0.f;
+                // scale and add one block's products (columns past the rows hold nothing that is stored)
+                auto take = [&](uint32_t base, float sc) {
+#pragma unroll
+                    for (int g = 0; g < TS_EN; g += 16) {
+                        if (g < np) {
+                            uint32_t h[16], m[16];
+                            tmem_ld16(base + e0 + g, h);
+                            tmem_ld16(base + t.n + e0 + g, m);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 16; i++)
+                                acc[g + i] = fmaf(fmaf(__uint_as_float(m[i]), 1.0f / 2048.0f, __uint_as_float(h[i])), sc, acc[g + i]);
+                        }
+                    }
+                };
+                float2 sc = ep.s0;
+                if (small) {
+                    // (units of the other group's parity are its own)
+                    const int skip = (it & 1) != eg;
+                    if (skip && kb0 + 1 < kb1) sc = ep.pair(a, kb0 + 1);
+                    for (int kb = kb0 + skip; kb < kb1; kb += 2) {
+                        const float2 sn = kb + 2 < kb1 ? ep.pair(a, kb + 2) : sc;
+                        if (!(ok = mbar_wait_all(&acc_full[eg], (uint32_t)(eg ? c1 : c0) & 1, a.err, 39))) break;
+                        tc_fence_after();
+                        take(lane_addr + (uint32_t)(eg * 128), sc.x);
+                        take(lane_addr + (uint32_t)(eg * 128 + 64), sc.y);
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_n(&acc_empty[eg], 2);
+                        if (eg) c1++; else c0++;
+                        sc = sn;
+                    }
+                    // the uses of the other accumulator in this tile
+                    const int n_units = kb1 - kb0, own = (n_units + ((it & 1) == eg)) >> 1;
+                    if (eg) c0 += n_units - own; else c1 += n_units - own;
+                    it += n_units;
+                } else {
+                    for (int kb = kb0; kb < kb1; kb++) {
+                        const float2 sn = kb + 1 < kb1 ? ep.pair(a, kb + 1) : sc;
+                        if (!(ok = mbar_wait_all(&acc_full[0], (uint32_t)c0 & 1, a.err, 39))) break;
+                        tc_fence_after();
+                        take(lane_addr, sc.x);
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&acc_empty[0]);
+                        if (!(ok = mbar_wait_all(&acc_full[1], (uint32_t)c1 & 1, a.err, 39))) break;
+                        tc_fence_after();
+                        take(lane_addr + 128u, sc.y);
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&acc_empty[1]);
+                        c0++; c1++;
+                        sc = sn;
+                    }
+                    it += kb1 - kb0;
                 }
-                it += kb1 - kb0;
+                if (!(ok = ts_all(ok))) break;
+                ts_finish<true, MODE>(a, t, ep, acc, tile, tile == tile_first, kb0, kb1, U, small, eg, row, exch, &s_last);
             }
-            if (!(ok = ts_all(ok))) break;
-            ts_finish<true, MODE>(a, t, ep, acc, tile, tile == tile_first, kb0, kb1, U, small, eg, row, exch, &s_last);
         }
     }
     tc_fence_before();
@@ -843,7 +978,7 @@ struct TcGemm {
     float *inv = nullptr;           // [inputs][plane]
     float *part = nullptr;          // partial results of the CTAs
     int *cnt = nullptr;             // units done per tile
-    int max_c = 0, max_t = 0, ctas = 0;
+    int max_c = 0, max_ec = 0, max_t = 0, ctas = 0, part_slabs = 0;
     int *err = nullptr;
     // maps by (pointer, kind, rows, columns, pitch or inputs, box)
     std::map<std::tuple<const void *, int, size_t, size_t, size_t, int>, CUtensorMap> maps;
@@ -851,15 +986,18 @@ struct TcGemm {
 };
 constexpr int TS_CNT = 1 << 16;     // tiles of one launch at most
 
-TcGemm *tc_gemm_create(int max_c, int max_t, int *err)
+TcGemm *tc_gemm_create(int max_c, int max_ec, int max_t, int *err)
 {
     if (!encode_fn()) return nullptr;
     TcGemm *g = new TcGemm;
     g->max_c = max_c; g->err = err; g->ctas = dev_sms();
     g->max_t = max_t > TS_N ? max_t : TS_N;
+    // per CTA two partial results of a projection (two slabs each), or of experts the sums of a first tile's units and those of a last one
+    g->max_ec = max_ec;
+    g->part_slabs = (max_ec + 255) / 256 + 2 > 4 ? (max_ec + 255) / 256 + 2 : 4;
     g->terms_n = (size_t)3 * (g->max_t > 2 * TS_N ? g->max_t : 2 * TS_N) * max_c;
     if (cudaMalloc(&g->terms, g->terms_n * 2) != cudaSuccess || cudaMalloc((void **)&g->inv, (size_t)TS_MAX_SEG * g->max_t * 4) != cudaSuccess ||
-        cudaMalloc((void **)&g->part, (size_t)g->ctas * 2 * TS_N * 128 * 4) != cudaSuccess ||
+        cudaMalloc((void **)&g->part, (size_t)g->ctas * g->part_slabs * TS_SLAB * 4) != cudaSuccess ||
         cudaMalloc((void **)&g->cnt, TS_CNT * 4) != cudaSuccess) {
         cudaGetLastError();
         tc_gemm_free(g);
@@ -1011,7 +1149,7 @@ int tc_gemm_run(TcGemm *g, cudaStream_t st, const GemvSeg *segs, int n, int T)
 // ------------------------------------------------------------------ routed experts ----
 bool tc_moe_takes(const TcGemm *g, const MoeShape &s, int T)
 {
-    if (!g || T < 1 || T > g->max_t || s.dt != DT_FP8 || s.br != 128 || s.bc != 128 || s.E % 128 || s.I % 128) return false;
+    if (!g || T < 1 || T > g->max_t || s.E > g->max_ec || s.I > g->max_ec || s.dt != DT_FP8 || s.br != 128 || s.bc != 128 || s.E % 128 || s.I % 128) return false;
     if (!(s.limit > 0.f) || s.limit * s.limit > 60000.f) return false;                  // activations must fit F16
     const int slots = (T * s.K < s.n_local ? T * s.K : s.n_local) + 1;
     return (long)(slots + ((T * s.K + T) >> tc_tile_shift((long)T * s.K, s.n_local))) * (s.I / 64 > s.E / 128 ? s.I / 64 : s.E / 128) <= TS_CNT;
@@ -1049,6 +1187,7 @@ int tc_moe_run(TcGemm *g, cudaStream_t st, float *contrib, void *act, void *xter
     a.T = T; a.n = T < 1 << p.tile_shift ? (T + 7) & ~7 : 1 << p.tile_shift; a.plane = P; a.p = p; a.E = s.E; a.I = s.I; a.xinv = xinv; a.limit = s.limit; a.act_scale = act_term_scale(s.limit); a.act_inv = 1.0f / a.act_scale;
     a.slots = (T * s.K < s.n_local ? T * s.K : s.n_local) + 1;
     a.part = g->part; a.cnt = g->cnt; a.err = g->err;
+    a.part_slabs = g->part_slabs;
     const size_t plan_bytes = (size_t)(4 * a.slots + 4) * sizeof(int);
     // gate/up with the clamped SwiGLU
     a.KB = (s.E + 255) / 256; a.blocks = s.E / 128; a.RT = s.I / 64; a.out = act;

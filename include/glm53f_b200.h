@@ -332,6 +332,11 @@ int g5b_engine_decode_speculative(g5b_engine *e, int first, int n, int *out, lon
  * change, rotating over `accs` accumulators. cycles[0]: until issued, cycles[1]: until complete. */
 int g5b_debug_mma_rate(int n, int fp8, int accs, int ctas, int reps, double *cycles);
 
+/* Test aid, no counterpart in the reference: a MoE layer's contribution rows before the exchange and the combine,
+ * [T * topk + T][hidden] (pick j of token t in row t * topk + j, then the shared expert's row of each token). Picks that
+ * another rank of an expert-parallel group owns are zero; the ranks need not be connected. */
+int g5b_debug_moe_rows(g5b_engine *e, int layer, const float *x, int T, float *rows);
+
 /* RMSNorm of `rows` rows of n floats on DEVICE buffers of the current CUDA device, enqueued on
  * `stream` (a cudaStream_t, NULL for the default stream) without waiting: y = w * x / sqrt(mean(x^2)
  * + eps), w may be NULL. This entry point has no counterpart in the reference. It exists for

@@ -93,3 +93,41 @@ def test_router_of_many_tokens(gpu_lib, binding, T):
     wi, ww = orc.op_router(0, x)
     assert np.array_equal(gi, wi[-len(gi):]) and common.rel_err(gw, ww[-len(gi):]) < 1e-6
     eng.close(); orc.close()
+
+
+def _moe_engine(hidden, inter, cap, rank=0, ranks=1):
+    c = synth.layer_spec("moe", n_experts=24).cfg.copy()
+    c.hidden, c.moe_inter, c.topk = hidden, inter, 4
+    spec = synth.Spec(c, [0], [0], with_head=False)
+    eng = pkg.Engine(c, spec.is_mla, spec.is_dense, cap, 0, rank, ranks)
+    eng.set_option("allow_partial", 1)
+    eng.load_all(synth.moe_layer_trunk(spec, 5))
+    for x in range(rank * c.n_experts // ranks, (rank + 1) * c.n_experts // ranks):
+        eng.fill_expert(0, x, 5, *synth.expert_scales(c, 0, x, 5))
+    eng.finalize()
+    return spec, eng
+
+
+@pytest.mark.parametrize("hidden,inter", [(4096, 2048), (2304, 1152)])
+def test_expert_rows_do_not_depend_on_what_is_beside_them(gpu_lib, hidden, inter):
+    """Sixteen, eight, nine and five units to a tile, cut between the CTAs at other places in every launch below: a row of an
+    expert has the same bits in any batch, on every rank of a group and on one GPU, and in every run."""
+    spec, one = _moe_engine(hidden, inter, 512)
+    ranks = [_moe_engine(hidden, inter, 64, r, 2)[1] for r in (0, 1)]
+    x = np.random.default_rng(7).standard_normal((300, hidden)).astype(np.float32)
+    picks, shared = one.debug_moe_rows(0, x)
+    for first, n in ((0, 2), (3, 7), (20, 31), (200, 64)):
+        rows = slice(first, first + n)
+        p, s = one.debug_moe_rows(0, x[rows])
+        assert np.array_equal(p, picks[rows]) and np.array_equal(s, shared[rows]), n
+        parts = [e.debug_moe_rows(0, x[rows]) for e in ranks]
+        for r, (p, s) in enumerate(parts):
+            assert np.array_equal(s, shared[rows]), (n, r)
+        assert not np.any((parts[0][0] != 0) & (parts[1][0] != 0))
+        assert np.array_equal(parts[0][0] + parts[1][0], picks[rows]), n
+    for n in (64, 300):
+        first = one.op_moe(0, x[:n])
+        for _ in range(3):
+            assert np.array_equal(one.op_moe(0, x[:n]), first), n
+    for e in (one, *ranks):
+        e.close()
