@@ -919,9 +919,9 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
     };
     if (e->ep_size > 1 && e->expert_path >= 1 && (shared_in_plan || !with_shared) && moe_mma_supported(s, n)) {
         // batch 1 across ranks: the tensor-core kernels on this rank's picks, contributions only
-        moe_mma_gateup(e->st, e->act, x, w.table_dev, e->plan, s, e->err_dev);
+        if (moe_mma_gateup(e->st, e->act, x, w.table_dev, e->plan, s, e->err_dev)) return -1;
         prof_mark(e, 2);
-        moe_mma_down(e->st, nullptr, e->contrib, e->act, e->rw, w.table_dev, e->plan, s, with_shared, e->tile_done, e->err_dev);
+        if (moe_mma_down(e->st, nullptr, e->contrib, e->act, e->rw, w.table_dev, e->plan, s, with_shared, e->tile_done, e->err_dev)) return -1;
         prof_mark(e, 3);
         exchange_and_combine();
         prof_mark(e, 4);
@@ -929,9 +929,9 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
         return 0;
     }
     if (e->expert_path == 1 && one_gpu_decode && moe_mma_supported(s, n)) {
-        moe_mma_gateup(e->st, e->act, x, w.table_dev, e->plan, s, e->err_dev);
+        if (moe_mma_gateup(e->st, e->act, x, w.table_dev, e->plan, s, e->err_dev)) return -1;
         prof_mark(e, 2);
-        moe_mma_down(e->st, out, e->contrib, e->act, e->rw, w.table_dev, e->plan, s, with_shared, e->tile_done, e->err_dev);
+        if (moe_mma_down(e->st, out, e->contrib, e->act, e->rw, w.table_dev, e->plan, s, with_shared, e->tile_done, e->err_dev)) return -1;
         prof_mark(e, 3);
         prof_mark(e, 4);
         prof_collect(e, 4);
@@ -1065,14 +1065,14 @@ static int run_kda(g5b_engine *e, Layer &w, const float *x, int n, float *out, b
     }
     KdaShape ks{H, D, c.conv_k, c.gate_lb, c.rms_eps};
     if (n == 1 && !ts) prefetch_beside(e, w.ko);        // the recurrence below leaves half the SMs and all of HBM idle
-    if (batch)
-        kda_core(e->st, e->ko, e->kq, e->kk, e->kv, e->kz, e->kbraw, e->kgb, w.q_conv, w.k_conv, w.v_conv,
-                 w.A_log, w.dt_bias, w.o_norm, w.kda_state, 1, ks, n, e->kda_seq, nullptr, h0, Hl, nullptr, 0, &e->kscr);
-    else
-        kda_core(e->st, e->ko, e->kq, e->kk, e->kv, e->kz, e->kbraw, e->kgb, w.q_conv, w.k_conv, w.v_conv,
-                 w.A_log, w.dt_bias, w.o_norm, w.kda_state + (size_t)e->cur_seq * e->kda_seq, n, ks, 1, 0,
-                 lr_inside ? &lr : nullptr, h0, Hl,
-                 e->snap_first && n > 1 ? e->kda_snap[(size_t)(&w - e->L.data())] : nullptr, 0, &e->kscr);
+    const int rc = batch
+        ? kda_core(e->st, e->ko, e->kq, e->kk, e->kv, e->kz, e->kbraw, e->kgb, w.q_conv, w.k_conv, w.v_conv,
+                   w.A_log, w.dt_bias, w.o_norm, w.kda_state, 1, ks, n, e->kda_seq, nullptr, h0, Hl, nullptr, 0, &e->kscr)
+        : kda_core(e->st, e->ko, e->kq, e->kk, e->kv, e->kz, e->kbraw, e->kgb, w.q_conv, w.k_conv, w.v_conv,
+                   w.A_log, w.dt_bias, w.o_norm, w.kda_state + (size_t)e->cur_seq * e->kda_seq, n, ks, 1, 0,
+                   lr_inside ? &lr : nullptr, h0, Hl,
+                   e->snap_first && n > 1 ? e->kda_snap[(size_t)(&w - e->L.data())] : nullptr, 0, &e->kscr);
+    if (rc) return -1;                           // (the reason is in g5b_last_error)
     if (!ts) return proj(e, w.ko, e->ko, P, out, E, n);
     {
         GemvSeg o = make_seg(col_slice(w.ko, p0, Pl), e->ko + p0, P, e->ts_part, E);
@@ -1179,12 +1179,13 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
             join = cudaEventRecord(e->side_done, e->side) == cudaSuccess;
             if (!join) cudaStreamSynchronize(e->side);
         }
-        dsa_select(e->st, e->msel, e->mnsel, ist, e->mqidx + (size_t)t0 * c.index_heads * c.index_dim, e->mwp + (size_t)t0 * c.index_heads, e->mscore, nt, at, s);
+        const int rc = dsa_select(e->st, e->msel, e->mnsel, ist, e->mqidx + (size_t)t0 * c.index_heads * c.index_dim, e->mwp + (size_t)t0 * c.index_heads, e->mscore, nt, at, s);
         if (!forked) mla_absorb(e->st, e->mqa, flash ? e->mqt : nullptr, mq, kvb, nt, sl);
         else if (join && cudaStreamWaitEvent(e->st, e->side_done, 0) != cudaSuccess) cudaStreamSynchronize(e->side);
-        if (flash)
-            mla_attend_flash(e->st, cb, e->mqt, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf);
-        else
+        if (rc) return -1;                         // (after the join: the side stream writes buffers of the next call; the reason is in g5b_last_error)
+        if (flash) {
+            if (mla_attend_flash(e->st, cb, e->mqt, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf)) return -1;
+        } else
             mla_attend(e->st, cb, e->mqa, lat, e->msel, e->mnsel, e->mdsc, e->mpart, e->mstats, e->mcount, MLA_PART_TOKENS, nt, at, sl);
         if (!wide) mla_vout(e->st, e->macc + (size_t)t0 * Hl * c.v_head, cb, kvb, nt, sl);
     }

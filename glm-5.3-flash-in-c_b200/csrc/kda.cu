@@ -607,7 +607,7 @@ static void kda_rows(cudaStream_t st, const KdaArgs &a, const KdaScratch &x, int
     G5B_LAUNCH_PDL(kda_out_kernel<DS>, dim3((heads + 7) / 8, a.T * n_seq), dim3(256), 0, st, a, heads);
 }
 
-void kda_core(cudaStream_t st, float *o, const float *q, const float *k, const float *v, const float *z,
+int kda_core(cudaStream_t st, float *o, const float *q, const float *k, const float *v, const float *z,
               const float *braw, const float *gb, const float *q_conv, const float *k_conv,
               const float *v_conv, const float *A_log, const float *dt_bias, const float *o_norm,
               float *state, int T, const KdaShape &s, int n_seq, size_t seq_stride, const KdaLowRank *lr, int head0, int heads,
@@ -623,13 +623,15 @@ void kda_core(cudaStream_t st, float *o, const float *q, const float *k, const f
     if (known && T * grid.y == 1) {
         const bool ok = s.D == 128 ? (s.K == 4 ? kda_step<128, 4>(st, a, (int)grid.x) : kda_step<128, 0>(st, a, (int)grid.x))
                                    : (s.K == 4 ? kda_step<64, 4>(st, a, (int)grid.x) : kda_step<64, 0>(st, a, (int)grid.x));
-        if (ok || fused) return;             // (a refusal is kept for g5b_last_error)
+        if (ok) return 0;
+        if (fused) return -1;                // the kernel below does not take the up-projections itself
     } else if (known && scratch) {
         if (s.D == 128) kda_rows<128>(st, a, *scratch, (int)grid.x, (int)grid.y);
         else            kda_rows<64>(st, a, *scratch, (int)grid.x, (int)grid.y);
-        return;
+        return 0;
     }
     G5B_LAUNCH(kda_core_kernel, grid, ((s.D + 31) / 32) * 32, 0, st, a);
+    return 0;
 }
 
 }  // namespace g5b

@@ -162,13 +162,13 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
 // dots: room for RT_TILE_ROWS (or T, if that is more) rows of n_experts dot products, which many tokens take apart
 constexpr int RT_TILE_ROWS = 2048;
 // Batch-1 experts multiplied by the tensor cores from their FP8 codes (moe_mma.cu); act_terms holds
-// the SwiGLU output split into two F16 terms per element, [pairs][2][I].
+// the SwiGLU output split into two F16 terms per element, [pairs][2][I]. 0, or -1 where the device refuses the shared memory.
 bool moe_mma_supported(const MoeShape &s, int T);
-void moe_mma_gateup(cudaStream_t st, void *act_terms, const float *x, const ExpertW *experts, const MoePlan &p,
-                    const MoeShape &s, int *err);
-void moe_mma_down(cudaStream_t st, float *out, float *contrib, const void *act_terms, const float *w,
-                  const ExpertW *experts, const MoePlan &p, const MoeShape &s, int with_shared, int *tile_done,
-                  int *err);
+int moe_mma_gateup(cudaStream_t st, void *act_terms, const float *x, const ExpertW *experts, const MoePlan &p,
+                   const MoeShape &s, int *err);
+int moe_mma_down(cudaStream_t st, float *out, float *contrib, const void *act_terms, const float *w,
+                 const ExpertW *experts, const MoePlan &p, const MoeShape &s, int with_shared, int *tile_done,
+                 int *err);
 // Batches: the experts' matrices streamed past the rows that chose them (tc_stream.cu), gate/up with the
 // clamped SwiGLU, then down. act, xterms: scratch for F16 terms [2][max_pairs][I] and [2][max_pairs][E], xinv:
 // [max_pairs]. Contributions only; the caller combines.
@@ -298,7 +298,8 @@ struct KdaLowRank {
 // the reference lays it out (S [H][D][D] then conv histories q|k|v, glm53f.h:363-367).
 // Rows for calls with several positions: [T][H * D] normalised q, normalised k, v, exp(gate) and [T][H] beta.
 struct KdaScratch { float *qn, *kn, *vn, *al, *beta; };
-void kda_core(cudaStream_t st, float *o, const float *q, const float *k, const float *v, const float *z,
+// 0, or -1 where the device refuses the one-token kernel its shared memory.
+int kda_core(cudaStream_t st, float *o, const float *q, const float *k, const float *v, const float *z,
               const float *braw, const float *gb, const float *q_conv, const float *k_conv,
               const float *v_conv, const float *A_log, const float *dt_bias, const float *o_norm,
               float *state, int T, const KdaShape &s, int n_seq = 1, size_t seq_stride = 0,
@@ -322,8 +323,9 @@ void mla_store(cudaStream_t st, void *latent, float *idx_state, const float *ct_
                const float *kv_norm_w, const float *wk_raw, const float *gate_raw,
                const float *k_norm_w, const float *k_norm_b, const float *ape, const float *q_raw, float *q_inv,
                int T, int cached, const MlaShape &s);
-void dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
-                const float *wproj, float *score, int T, int cached, const MlaShape &s);
+// (0, or -1 with the reason in g5b_last_error where the device refuses a kernel its shared memory; nothing was selected then)
+int dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
+               const float *wproj, float *score, int T, int cached, const MlaShape &s);
 // The absorbed queries as doubles [T][H][KL] in qa or, when terms is given, scaled and split for the tensor-core core: [T][H][3][KL] BF16.
 void mla_absorb(cudaStream_t st, double *qa, void *terms, const float *q, const DMat &kv_b, int T, const MlaShape &s);
 // part: FP64 partial sums [part_tokens][H][ceil((topk+KP)/32)][KL], stats [T][H][2]; part == nullptr
@@ -335,10 +337,10 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
 // The same attention core on the tensor cores (BF16 latent cache, kv_lora 512): scores and weighted
 // sums as mma.sync products on exact BF16 term splits, softmax per chunk of 64 positions and a
 // rescaling reduction. part / part_bytes: scratch for the chunks' partial rows; cstat: room for
-// [T][H][ceil((topk + KP) / 64)][2] doubles.
+// [T][H][ceil((topk + KP) / 64)][2] doubles. 0, or -1 where the device refuses the kernel its shared memory.
 bool mla_flash_takes(const MlaShape &s);
-void mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
-                      void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s);
+int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
+                     void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s);
 void mla_vout(cudaStream_t st, float *acc_out, const float *cb, const DMat &kv_b, int T, const MlaShape &s);
 
 }  // namespace g5b

@@ -329,20 +329,21 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(int *sel, int *n
     if (tid == 0) nsel[t] = base + (p - np * s.KP + 1);
 }
 
-void dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
-                const float *wproj, float *score, int T, int cached, const MlaShape &s)
+int dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
+               const float *wproj, float *score, int T, int cached, const MlaShape &s)
 {
     const int np_max = (cached + (s.batch ? 1 : T)) / s.KP;
     if (np_max > s.topk / s.KP) {
         const size_t smem = ((((size_t)s.ID * s.IH + 1) & ~(size_t)1) + (size_t)DSA_WARPS * DSA_POOLS * (s.IH + s.ID)) * sizeof(double);
         static SmemGrant grant;
-        if (!dev_opt_in_smem((const void *)dsa_score_kernel, smem, grant)) return;
+        if (!dev_opt_in_smem((const void *)dsa_score_kernel, smem, grant)) return -1;     // (many heads of many dimensions)
         const int want = (np_max + DSA_WARPS * DSA_POOLS - 1) / (DSA_WARPS * DSA_POOLS);
         int blocks = (444 + T - 1) / T > 32 ? (444 + T - 1) / T : 32;                        // (three fit an SM; each converts the query's heads first)
         if (blocks > want) blocks = want;
         G5B_LAUNCH(dsa_score_kernel, dim3(blocks, T), DSA_WARPS * 32, smem, st, score, idx_state, qidx, wproj, cached, s);
     }
     G5B_LAUNCH_PDL(dsa_topk_kernel, T, TOPK_THREADS, 0, st, sel, nsel, score, cached, s);
+    return 0;
 }
 
 // ---------------------------------------------------------------- attention ----
@@ -984,11 +985,11 @@ bool mla_flash_takes(const MlaShape &s)
 }
 
 // scratch: `part_bytes` bytes for the partial rows; `cstat` room for [T][H][nchunks][2] doubles.
-void mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
-                      void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s)
+int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
+                     void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s)
 {
     static SmemGrant grant;
-    if (!dev_opt_in_smem((const void *)mla_flash_kernel, FL_SMEM, grant)) return;
+    if (!dev_opt_in_smem((const void *)mla_flash_kernel, FL_SMEM, grant)) return -1;
     const int stride = s.topk + s.KP;
     // partial rows are laid out for the chunks that the call's last position can see: an early stretch of a prompt goes in
     // few launches of many queries
@@ -1008,6 +1009,7 @@ void mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void
         G5B_LAUNCH_PDL(mla_flash_reduce_kernel, dim3(s.H, n), FL_KL, 0, st, cb + (size_t)t0 * s.H * s.KL, static_cast<const float *>(part),
                        cstat, nsel ? nsel + t0 : nullptr, s.batch ? cached : cached + t0, nchunks, s);
     }
+    return 0;
 }
 
 

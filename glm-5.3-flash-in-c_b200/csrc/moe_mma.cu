@@ -255,26 +255,27 @@ bool moe_mma_supported(const MoeShape &s, int T)
 }
 
 template <bool GATEUP>
-static void launch_mma(cudaStream_t st, const MmaArgs &a, size_t smem)
+static int launch_mma(cudaStream_t st, const MmaArgs &a, size_t smem)
 {
     static SmemGrant grant;
-    if (!dev_opt_in_smem((const void *)moe_mma_kernel<GATEUP>, smem, grant)) return;
+    if (!dev_opt_in_smem((const void *)moe_mma_kernel<GATEUP>, smem, grant)) return -1;
     G5B_LAUNCH(moe_mma_kernel<GATEUP>, dev_sms(), MM_THREADS, smem, st, a);
+    return 0;
 }
 
-void moe_mma_gateup(cudaStream_t st, void *act_terms, const float *x, const ExpertW *experts, const MoePlan &p,
-                    const MoeShape &s, int *err)
+int moe_mma_gateup(cudaStream_t st, void *act_terms, const float *x, const ExpertW *experts, const MoePlan &p,
+                   const MoeShape &s, int *err)
 {
     MmaArgs a{experts, p, x, act_terms, s.E, s.I, s.br, s.bc, s.limit, nullptr, nullptr, s.K, 0, nullptr, err};
-    launch_mma<true>(st, a, mma_smem_bytes(true, s.E, s.I));
+    return launch_mma<true>(st, a, mma_smem_bytes(true, s.E, s.I));
 }
 
-void moe_mma_down(cudaStream_t st, float *out, float *contrib, const void *act_terms, const float *w,
-                  const ExpertW *experts, const MoePlan &p, const MoeShape &s, int with_shared, int *tile_done,
-                  int *err)
+int moe_mma_down(cudaStream_t st, float *out, float *contrib, const void *act_terms, const float *w,
+                 const ExpertW *experts, const MoePlan &p, const MoeShape &s, int with_shared, int *tile_done,
+                 int *err)
 {
     MmaArgs a{experts, p, act_terms, contrib, s.E, s.I, s.br, s.bc, s.limit, out, w, s.K, with_shared, tile_done, err};
-    launch_mma<false>(st, a, mma_smem_bytes(false, s.E, s.I));
+    return launch_mma<false>(st, a, mma_smem_bytes(false, s.E, s.I));
 }
 
 }  // namespace g5b

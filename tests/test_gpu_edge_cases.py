@@ -210,3 +210,22 @@ def test_expert_parallel_group_inside_one_process(gpu_lib, binding):
     for e in engines:
         e.close()
     orc.close()
+
+
+def test_indexer_that_does_not_fit_shared_memory_is_refused(gpu_lib, binding):
+    """128 heads of 192 dimensions need more shared memory than the device grants the score kernel: a call whose positions
+    need a selection ends in an error, one that sees few enough to take all still gives the CPU path's output."""
+    c = synth.tiny_spec().cfg.copy()
+    c.n_layers, c.index_heads, c.index_dim = 1, 128, 192
+    spec = synth.Spec(c, [1], [0], with_head=False)
+    tensors = synth.make_model(spec, seed=2, recipe="spread")
+    eng, orc = common.build_models(spec, tensors, 64, binding, options={"allow_partial": 1})
+    x = np.random.default_rng(1).standard_normal((40, c.hidden)).astype(np.float32)
+    few = c.index_topk + c.index_kpool - 1
+    assert common.rel_err(eng.op_mla(0, x[:few], 0)[0], orc.op_mla(0, x[:few], 0)[0]) < 1e-5
+    for first, n in ((few, 1), (few, 9), (0, 40)):
+        with pytest.raises(RuntimeError, match="shared memory"):
+            eng.op_mla(0, x[first:first + n], first)
+    again = eng.op_mla(0, x[:few], 0)[0]
+    assert common.rel_err(again, orc.op_mla(0, x[:few], 0)[0]) < 1e-5
+    eng.close(); orc.close()
