@@ -938,9 +938,8 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
         return 0;
     }
     if (e->expert_path >= 1 && (shared_in_plan || !with_shared) && tc_moe_takes(e->tc, s, n)) {
-        if (tc_moe_run(e->tc, e->st, e->contrib, e->act, e->xterms, e->xinv, x, c.hidden, expert_slab(e, w), e->plan, n, s))
+        if (tc_moe_run(e->tc, e->st, e->contrib, e->act, e->xterms, e->xinv, x, c.hidden, expert_slab(e, w), e->plan, n, s, e->profile ? e->prof_ev[2] : nullptr))
             return fail("the expert kernels could not be launched");
-        prof_mark(e, 2);                          // (gate/up and down are not told apart here)
         prof_mark(e, 3);
     } else {
         moe_gateup(e->st, e->act, x, c.hidden, w.table_dev, e->plan, n, s);

@@ -171,7 +171,7 @@ int moe_mma_down(cudaStream_t st, float *out, float *contrib, const void *act_te
                  int *err);
 // Batches: the experts' matrices streamed past the rows that chose them (tc_stream.cu), gate/up with the
 // clamped SwiGLU, then down. act, xterms: scratch for F16 terms [2][max_pairs][I] and [2][max_pairs][E], xinv:
-// [max_pairs]. Contributions only; the caller combines.
+// [max_pairs]. Contributions only; the caller combines. between: optional event, recorded after gate/up.
 struct ExpertSlab {       // a layer's experts in one allocation: expert i's gate | up | down codes at base + i * stride, `mat` bytes apart
     const uint8_t *base;   // (then the scales: gate | up | down, scale_gate bytes each for the first two)
     size_t mat, stride, scale_gate;
@@ -179,7 +179,7 @@ struct ExpertSlab {       // a layer's experts in one allocation: expert i's gat
 };
 bool tc_moe_takes(const TcGemm *g, const MoeShape &s, int T);
 int  tc_moe_run(TcGemm *g, cudaStream_t st, float *contrib, void *act, void *xterms, float *xinv, const float *x, int ldx,
-                const ExpertSlab &w, const MoePlan &p, int T, const MoeShape &s);
+                const ExpertSlab &w, const MoePlan &p, int T, const MoeShape &s, cudaEvent_t between = nullptr);
 // The whole batch-1 layer (router, top-k, experts, combine) as one cooperative kernel
 // (moe_decode.cu). `sync` holds two device counters that only grow; `launches` is the host's count of
 // launches so far on them. Returns -1 when the cooperative launch is refused.

@@ -1173,7 +1173,7 @@ static const std::pair<CUtensorMap, CUtensorMap> *expert_maps(TcGemm *g, const E
 }
 
 int tc_moe_run(TcGemm *g, cudaStream_t st, float *contrib, void *act, void *xterms, float *xinv, const float *x, int ldx,
-               const ExpertSlab &w, const MoePlan &p, int T, const MoeShape &s)
+               const ExpertSlab &w, const MoePlan &p, int T, const MoeShape &s, cudaEvent_t between)
 {
     const std::pair<CUtensorMap, CUtensorMap> *em = expert_maps(g, w, s);
     if (!em) return -1;
@@ -1196,6 +1196,7 @@ int tc_moe_run(TcGemm *g, cudaStream_t st, float *contrib, void *act, void *xter
     if (!x_maps(g, m, xterms, true, (size_t)P, (size_t)s.E, 1)) return -1;
     size_t smem = stage_plan(a, true, plan_bytes);
     if (launch_stream(tc_stream_fp8_kernel<TS_GATEUP>, grant_gateup, st, m, a, smem, g->ctas, TS_FP8_THREADS)) return -1;
+    if (between) cudaEventRecord(between, st);
     // down
     a.KB = (s.I + 255) / 256; a.blocks = s.I / 128; a.RT = s.E / 128; a.out = contrib;
     a.scales = w.base + 3 * w.mat + 2 * w.scale_gate;

@@ -131,3 +131,23 @@ def test_expert_rows_do_not_depend_on_what_is_beside_them(gpu_lib, hidden, inter
             assert np.array_equal(one.op_moe(0, x[:n]), first), n
     for e in (one, *ranks):
         e.close()
+
+
+def test_profile_tells_the_expert_phases_of_a_batch_apart(gpu_lib):
+    """Option "profile": router and plan, gate/up, down and combine each take measurable time; gate/up is two of the three matrices."""
+    import ctypes as C
+    spec, eng = _moe_engine(2048, 1024, 64)
+    x = np.random.default_rng(3).standard_normal((48, 2048)).astype(np.float32)
+    eng.op_moe(0, x)
+    ms, count = (C.c_float * 8)(), C.c_long(0)
+    read = eng.L.g5b_engine_profile_read
+    read.argtypes = [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int]
+    eng.set_option("profile", 1)
+    for _ in range(20):
+        eng.op_moe(0, x)
+    assert read(eng.handle, C.addressof(ms), 8, C.addressof(count), 1) == 0 and count.value == 20
+    router, gateup, down, combine = (v / 20 for v in list(ms)[:4])
+    # an empty phase is the 1 to 2 us between two events; these are launches of tens of microseconds
+    assert min(router, gateup, down) > 5e-3 and combine > 1e-3, list(ms)
+    assert down < gateup, list(ms)
+    eng.close()
