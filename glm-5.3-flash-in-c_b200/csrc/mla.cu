@@ -1006,7 +1006,9 @@ int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void 
         G5B_LAUNCH_PDL(mla_flash_kernel, dim3(used, s.H / FL_HEADS, n), FL_THREADS, FL_SMEM, st, static_cast<float *>(part), cstat,
                        static_cast<const __nv_bfloat16 *>(qterms) + (size_t)t0 * s.H * 3 * s.KL, lat0, sel ? sel + (size_t)t0 * stride : nullptr, nsel ? nsel + t0 : nullptr,
                        s.batch ? cached : cached + t0, nchunks, s);
-        G5B_LAUNCH_PDL(mla_flash_reduce_kernel, dim3(s.H, n), FL_KL, 0, st, cb + (size_t)t0 * s.H * s.KL, static_cast<const float *>(part),
+        // (launched the ordinary way: launched early, its CTAs crowd the SMs beside the core's, of which two fit an SM - one
+        // token at 2048 / 8192 / 32768 positions: MLA layer 102.4 / 112.6 / 120.9 us, 96.3 / 106.6 / 114.8 so)
+        G5B_LAUNCH(mla_flash_reduce_kernel, dim3(s.H, n), FL_KL, 0, st, cb + (size_t)t0 * s.H * s.KL, static_cast<const float *>(part),
                        cstat, nsel ? nsel + t0 : nullptr, s.batch ? cached : cached + t0, nchunks, s);
     }
     return 0;
