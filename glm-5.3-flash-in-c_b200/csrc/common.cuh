@@ -101,7 +101,9 @@ __device__ __forceinline__ float sigmoid_host(float x)
 // instructions: Cody and Waite's reduction x = n ln 2 + r with ln 2 cut after 14 bits (n times that is exact),
 // Taylor's series of e^r to r^9 with its terms up to r^2 / 2 as pairs of floats, one rounding at the end. For
 // places that take millions: FP64 instructions issue at an eighth of the FP32 rate here, and an exponential is
-// about thirty of either. Equal to the correctly rounded result for 99.8 % of all arguments.
+// about thirty of either. Equal to the correctly rounded result for 99.75 % of the arguments when they are spread evenly over
+// -87 .. 88, for 99.98 % when they are spread evenly over the floats there (the test of both is a sweep of either kind);
+// subnormal results are off by less than one of their units.
 __device__ __forceinline__ float expf_near(float x)
 {
     const float n = rintf(x * 1.44269504f);
@@ -123,7 +125,8 @@ __device__ __forceinline__ float expf_near(float x)
     return x > 89.0f ? INFINITY : x < -104.0f ? 0.0f : v;
 }
 
-// The sigmoid of the function above, with this exponential.
+// The sigmoid of the function above, with this exponential: three roundings, 1.53 units of 2^-23 at most relative to the exact
+// value (0.53 of the exponential, a half each of the sum and the quotient).
 __device__ __forceinline__ float sigmoid_near(float x) { return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf_near(-x))); }
 
 // a*b + c with two float roundings, as C compiled without FMA contraction evaluates it.

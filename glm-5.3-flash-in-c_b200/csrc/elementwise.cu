@@ -81,6 +81,20 @@ void swiglu(cudaStream_t st, float *y, const float *gu, int n, int rows, float l
     G5B_LAUNCH_PDL(swiglu_kernel, dim3((n + 255) / 256, rows), dim3(256), 0, st, y, gu, n, limit);
 }
 
+// The exponential and the sigmoid of the kernels that take millions of them (common.cuh), element by element (test aid).
+__global__ void exp_near_kernel(float *e, float *sig, const float *x, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    e[i] = expf_near(x[i]);
+    sig[i] = sigmoid_near(x[i]);
+}
+
+void exp_near(cudaStream_t st, float *e, float *sig, const float *x, int n)
+{
+    G5B_LAUNCH(exp_near_kernel, (n + 255) / 256, 256, 0, st, e, sig, x, n);
+}
+
 // -------------------------------------------------------------- ShortConv ----
 // glm53f_shortconv, src/core/glm53f_ops.c:517-542: one thread per channel walks the T positions;
 // current-input term first, then history terms oldest first, each product and sum rounded.

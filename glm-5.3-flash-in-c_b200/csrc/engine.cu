@@ -2242,6 +2242,21 @@ extern "C" int g5b_swiglu_host(float *y, const float *gu, int n, int rows, float
     return 0;
 }
 
+extern "C" int g5b_debug_exp(const float *x, int n, float *e, float *sig, int device)
+{
+    cudaStream_t st;
+    if (with_device(device, &st)) return -1;
+    if (n < 1) return fail("no arguments");
+    Tmp t;
+    float *xd = (float *)t.up(x, (size_t)n * 4), *ed = (float *)t.up(nullptr, (size_t)n * 4), *sd = (float *)t.up(nullptr, (size_t)n * 4);
+    if (!xd || !ed || !sd) return fail("out of device memory");
+    exp_near(st, ed, sd, xd, n);
+    CU(cudaMemcpy(e, ed, (size_t)n * 4, cudaMemcpyDeviceToHost));
+    CU(cudaMemcpy(sig, sd, (size_t)n * 4, cudaMemcpyDeviceToHost));
+    CU(cudaGetLastError());
+    return 0;
+}
+
 extern "C" int g5b_shortconv_host(float *y, const float *x, const float *w, float *state, int channels, int k,
                                   int T, int device)
 {

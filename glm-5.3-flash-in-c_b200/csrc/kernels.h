@@ -88,6 +88,7 @@ void rms_factor(cudaStream_t st, const float *x, int n, int ld, int rows, float 
 void rms_apply(cudaStream_t st, float *y, const float *x, const float *w, const float *inv, int n,
                int ld, int rows);
 void swiglu(cudaStream_t st, float *y, const float *gu, int n, int rows, float limit);
+void exp_near(cudaStream_t st, float *e, float *sig, const float *x, int n);
 void shortconv(cudaStream_t st, float *y, const float *x, const float *w, float *state, int channels,
                int k, int T);
 void embed_rows(cudaStream_t st, float *h, const DMat &table, const int *ids, int T, int M);

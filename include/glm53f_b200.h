@@ -337,6 +337,9 @@ int g5b_debug_mma_rate(int n, int fp8, int accs, int ctas, int reps, double *cyc
  * another rank of an expert-parallel group owns are zero; the ranks need not be connected. */
 int g5b_debug_moe_rows(g5b_engine *e, int layer, const float *x, int T, float *rows);
 
+/* Test aid: the exponential and the sigmoid that the kernels over many positions use, of n host values. */
+int g5b_debug_exp(const float *x, int n, float *e, float *sig, int device);
+
 /* RMSNorm of `rows` rows of n floats on DEVICE buffers of the current CUDA device, enqueued on
  * `stream` (a cudaStream_t, NULL for the default stream) without waiting: y = w * x / sqrt(mean(x^2)
  * + eps), w may be NULL. This entry point has no counterpart in the reference. It exists for

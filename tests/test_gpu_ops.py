@@ -96,6 +96,33 @@ def test_rmsnorm_swiglu_shortconv(gpu_lib, binding):
     assert np.array_equal(s1, s2)
 
 
+@pytest.mark.parametrize("spread", ["values", "floats"])
+def test_exponential_of_the_many_position_kernels(gpu_lib, spread):
+    """The figures that its comment states, against the double-precision exponential: 0.53 units in the last place, how often
+    it is the correctly rounded value, and what leaves the range of the normal floats."""
+    n = 1 << 22
+    if spread == "values":
+        x = np.linspace(-87.3, 88.7, n).astype(np.float32)
+    else:
+        up = [np.linspace(int(np.float32(1e-30).view(np.uint32)), int(np.float32(top).view(np.uint32)), n // 2).astype(np.uint32).view(np.float32)
+              for top in (88.7, 87.3)]
+        x = np.concatenate([up[0], -up[1]])
+    special = np.array([np.inf, -np.inf, np.nan, 0.0, -0.0, 1e-45, 88.72284, 90, 1e30, -106, -1e30], np.float32)
+    below = np.linspace(-103.9, -87.4, 1 << 16).astype(np.float32)
+    a = np.ascontiguousarray(np.concatenate([x, below, special]))
+    e, s = np.empty_like(a), np.empty_like(a)
+    assert gpu_lib.g5b_debug_exp(a.ctypes.data, a.size, e.ctypes.data, s.ctypes.data, 0) == 0
+    want = np.exp(a[:n].astype(np.float64))
+    assert np.max(np.abs(e[:n] - want) / np.exp2(np.floor(np.log2(want)) - 23)) < 0.531
+    assert np.mean(e[:n] == want.astype(np.float32)) > (0.9974 if spread == "values" else 0.9997)
+    exact = 1.0 / (1.0 + np.exp(-a[:n].astype(np.float64)))
+    inner = np.abs(a[:n]) <= 87                              # (beyond, the exponential overflows as the C library's does)
+    assert np.max((np.abs(s[:n] - exact) / exact)[inner]) < 1.53 * 2.0 ** -23
+    assert np.max(np.abs(e[n:n + below.size] - np.exp(below.astype(np.float64)))) < 2.0 ** -149
+    with np.errstate(over="ignore"):
+        assert np.array_equal(e[-special.size:], np.exp(special.astype(np.float64)).astype(np.float32), equal_nan=True)
+
+
 @pytest.fixture(scope="module", params=["tiny", "micro"])
 def pair(request, gpu_lib, binding):
     """(spec, engine, oracle) on the benchmark's tiny configuration (streaming kernels) and on the
