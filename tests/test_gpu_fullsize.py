@@ -1,5 +1,6 @@
 """GPU parity at the benchmark's full sizes: one MoE layer with 288 experts (batch 1, 8, 64), one
-KDA layer (32 and 64 heads), one MLA layer at contexts 2048 / 8192 / 32768."""
+KDA layer (32 and 64 heads), one MLA layer at contexts 2048 / 8192 / 32768, and every kind of
+layer over 150 positions of a prompt."""
 import numpy as np
 import pytest
 
@@ -121,3 +122,73 @@ def test_expert_kernel_variants_agree(moe_layer, binding):
         for _ in range(3):
             assert np.array_equal(outs[2], eng.op_moe(0, xin))      # deterministic, counters carry over
         orc.close()
+
+
+# The prompt path at the released widths: more than 64 positions in one pass, so tiles of 32 rows of a 2048-row plane of terms,
+# the last one ragged, several chunks of the attention core and the router, the value projection on the tensor cores.
+ROWS, PLANE = 150, 2048
+
+
+def _pair(spec, tensors, binding, cap, options=None):
+    return common.build_models(spec, tensors, cap, binding, options={"allow_partial": 1, **(options or {})})
+
+
+def test_full_size_moe_layer_over_a_prompt(gpu_lib, binding):
+    """24 experts, so that most of them have more than one tile of rows."""
+    spec = synth.layer_spec("moe", n_experts=24)
+    trunk = synth.moe_layer_trunk(spec, SEED)
+    eng = pkg.Engine(spec.cfg, spec.is_mla, spec.is_dense, PLANE)
+    eng.set_option("allow_partial", 1)
+    eng.load_all(trunk)
+    for ex in range(spec.cfg.n_experts):
+        eng.fill_expert(0, ex, SEED, *synth.expert_scales(spec.cfg, 0, ex, SEED))
+    eng.finalize()
+    orc = synth.oracle_moe_layer(binding, spec, trunk, SEED, range(spec.cfg.n_experts))
+    x = synth.moe_inputs(spec.cfg, ROWS, SEED)
+    assert common.rel_err(eng.op_moe(0, x), orc.op_moe(0, x)) < 1e-5
+    gi, wi = eng.last_picks((ROWS - 1) % 64 + 1)[0], orc.op_router(0, x)[0]
+    assert np.array_equal(gi, wi[-len(gi):])
+    eng.close(); orc.close()
+
+
+@pytest.mark.parametrize("kind", ["kda", "mlp"])
+def test_full_size_layers_over_a_prompt(gpu_lib, binding, kind):
+    if kind == "kda":
+        spec = synth.layer_spec("kda")
+    else:
+        c = pkg.full_size_config()
+        c.n_layers = 1
+        spec = synth.Spec(c, [0], [1], with_head=False, only="moe")
+    eng, orc = _pair(spec, synth.make_model(spec, seed=4, recipe="baseline"), binding, PLANE)
+    rng = np.random.default_rng(4)
+    x = synth.bf16_round(rng.standard_normal((ROWS, spec.cfg.hidden)).astype(np.float32))
+    if kind == "mlp":
+        assert common.rel_err(eng.op_mlp(0, x), orc.op_mlp(0, x)) < 1e-5
+    else:
+        H, D, K = spec.cfg.kda_heads, spec.cfg.kda_head_dim, spec.cfg.conv_k
+        n = H * D * D + 3 * H * D * (K - 1)
+        state = (rng.standard_normal(n) * 0.1).astype(np.float32)
+        eng.state_write(0, 0, 0, state); orc.state_write(0, 0, 0, state)
+        assert common.rel_err(eng.op_kda(0, x), orc.op_kda(0, x)) < 2e-5
+        assert common.rel_err(eng.state_read(0, 0, 0, n), orc.state_read(0, 0, 0, n)) < 2e-5
+    eng.close(); orc.close()
+
+
+@pytest.mark.parametrize("latent_bf16", [0, 1])
+def test_full_size_mla_layer_over_a_prompt(gpu_lib, binding, latent_bf16):
+    """From position 1990: the first 61 of the call's positions see everything, the others a selection."""
+    spec = synth.layer_spec("mla")
+    c, cap, cached = spec.cfg, 2304, 1990
+    eng, orc = _pair(spec, synth.make_model(spec, seed=5, recipe="spread"), binding, cap, {"latent_bf16": latent_bf16})
+    rng = np.random.default_rng(5)
+    lat = synth.bf16_round(rng.standard_normal((cap, c.kv_lora)).astype(np.float32))
+    idx = rng.standard_normal(2 * cap * c.index_dim + (cap // c.index_kpool) * c.index_dim).astype(np.float32)
+    for m in (eng, orc):
+        m.state_write(0, 1, 0, lat)
+        m.state_write(0, 2, 0, idx)
+    x = synth.bf16_round(rng.standard_normal((ROWS, c.hidden)).astype(np.float32))
+    (g, gs), (w, ws) = eng.op_mla(0, x, cached), orc.op_mla(0, x, cached)
+    assert ws is not None and np.array_equal(gs, ws)
+    # (a BF16 cache rounds the call's own latent rows; the CPU path's cache holds FP32)
+    assert common.rel_err(g, w) < (3e-3 if latent_bf16 else 2e-5)
+    eng.close(); orc.close()

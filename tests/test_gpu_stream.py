@@ -151,3 +151,26 @@ def test_profile_tells_the_expert_phases_of_a_batch_apart(gpu_lib):
     assert min(router, gateup, down) > 5e-3 and combine > 1e-3, list(ms)
     assert down < gateup, list(ms)
     eng.close()
+
+
+def test_prompts_and_batches_repeat_bit_for_bit(gpu_lib):
+    """The same prompt and the same step of a batch of sequences again, from the same state: the same logits."""
+    spec = synth.tiny_spec()
+    tensors = synth.make_model(spec, seed=33, recipe="spread")
+    eng, _ = common.build_models(spec, tensors, 300, oracle=False, options={"sequences": 9})
+    rng = np.random.default_rng(8)
+    ids, step = rng.integers(0, spec.cfg.vocab, 270).astype(np.int32), rng.integers(0, spec.cfg.vocab, 9).astype(np.int32)
+
+    def both():
+        eng.use_sequence(0)
+        eng.reset()
+        prompt = eng.forward(ids)[0]
+        eng.reset()
+        eng.synth_session(4, 100)
+        return prompt, eng.decode_batch(step)[0]
+
+    first = both()
+    for _ in range(3):
+        again = both()
+        assert np.array_equal(again[0], first[0]) and np.array_equal(again[1], first[1])
+    eng.close()
