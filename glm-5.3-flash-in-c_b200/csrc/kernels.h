@@ -70,10 +70,11 @@ inline void gemv(cudaStream_t st, const DMat &m, const float *x, int ldx, float 
 // cores, weights streamed once by TMA; activations as exact 16-bit term sums. Matrices of one format and
 // width go out in one launch. err: where a bounded wait that ran out is recorded (tc_gemm_recover after it).
 // Rows of one expert that a weight tile is multiplied with at once, at most, for `pairs` rows over `experts` experts. A tile's
-// terms take shared memory from the weights in flight: stages for 16 rows leave four of weights, for 32 three. With up to
-// three rows per expert on average hardly any expert has more than 16 (64 tokens: 945 -> 850 us); with four (150 tokens) the
-// second pass over the weights of those that do costs more (1355 -> 1420 us).
-inline int tc_tile_shift(long pairs, int experts) { return pairs <= 3l * experts ? 4 : 5; }   // log2: tiles are counted by every role
+// terms take shared memory from the weights in flight: stages for 16 rows leave four of weights, for 32 three. With few rows per
+// expert hardly any expert has more than 16 (gate/up and down of 288 experts top-8, tiles of 32 and of 16 rows: 64 tokens
+// 689 and 590 us, 120 tokens 800 and 753); then the second pass over the weights of those that do costs more (150 tokens, 4.2
+// rows per expert on average: 843 and 831; 200 tokens: 966 and 998).
+inline int tc_tile_shift(long pairs, int experts) { return pairs <= 4l * experts ? 4 : 5; }   // log2: tiles are counted by every role
 struct TcGemm;
 TcGemm *tc_gemm_create(int max_c, int max_ec, int max_t, int *err);      // widest input, that of an expert, most positions
 void tc_gemm_free(TcGemm *g);
