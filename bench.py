@@ -41,7 +41,6 @@ EXPERT_BYTES = 3 * 2048 * 4096 + 3 * 16 * 32 * 4            # codes + block scal
 GATEUP_BYTES = 2 * 2048 * 4096 + 2 * 16 * 32 * 4            # what the gate/up kernel reads per expert
 ROUTER_BYTES = 288 * 4096 * 2                               # BF16 router matrix
 FLUSH_BYTES = 512 << 20                                     # two halves, each > 126 MB of L2: write one, read the other
-# dram__bytes_read.sum + dram__bytes_write.sum of one gate/up launch at batch 1 (profiles/), or None
 # DRAM bytes (read + write) per launch from the ncu captures summarised under profiles/
 GATEUP_TRAFFIC_NCU = None
 DECODE_TRAFFIC_NCU = 233.9e6      # moe_decode_kernel: 231.8 MB captured with 32 resident experts + 2.1 MB for 256 more router rows
@@ -578,7 +577,8 @@ def run_batch_decode(pkg, torch, ranks, local: int, rank: int, world: int, layer
     runs attention and all other per-token work for sequences / N of them, MoE layers gather the
     ranks' tokens and send contribution rows to the rank a token lives on. Both arms start from the
     same synthetic state, so the split arm must reproduce the first arm's tokens. Then one
-    `prefill_tokens`-token prompt through the prefill path of sequence 0 (chunks of 64 positions).
+    `prefill_tokens`-token prompt through the prefill path of sequence 0 (passes of 2048 positions on one
+    GPU, of 64 where the ranks exchange rows).
     As many layers as the GPUs hold."""
     import fullmodel
     import synth
@@ -647,7 +647,7 @@ def run_batch_decode(pkg, torch, ranks, local: int, rank: int, world: int, layer
                 eng.reset()
                 prompt = np.random.default_rng(SEED + 1).integers(0, c.vocab, prefill_tokens).astype(np.int32)
                 eng.use_sequence(0)
-                eng.forward(prompt[:128], want_logits=False)           # warm-up chunk pair
+                eng.forward(prompt[:128], want_logits=False)           # warm-up
                 eng.reset()
                 eng.use_sequence(0)
                 ranks.barrier()
@@ -667,7 +667,8 @@ def run_batch_decode(pkg, torch, ranks, local: int, rank: int, world: int, layer
         res = {"sequences_per_rank": own, "timed_steps": steps, "ms_per_step": 1e3 * decode_s / steps,
                "tokens_per_s": sequences * steps / decode_s, "tokens_per_s_per_sequence": steps / decode_s}
         if with_prefill:
-            res["prefill"] = {"tokens": prefill_tokens, "ms": 1e3 * prefill_s, "tokens_per_s": prefill_tokens / prefill_s, "chunk": 64}
+            res["prefill"] = {"tokens": prefill_tokens, "ms": 1e3 * prefill_s, "tokens_per_s": prefill_tokens / prefill_s,
+                              "chunk": 64 if world > 1 else min(2048, -(-cap // 64) * 64)}
         return res, all_toks, all_early
 
     out = {"layers": n_layers, "of_layers": 45, "n_gpus": world, "sequences": sequences, "context": context,

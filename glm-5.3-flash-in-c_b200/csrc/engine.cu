@@ -46,7 +46,8 @@ constexpr int CHUNK = 64;       // positions of a batch step, of a device op, of
                                 // (the reference's MoE chunk, glm53f_ops.c:988)
 // Positions one pass of a layer works on: a prompt goes through a layer in passes this long, so that the weights are
 // read once per pass. 2048 positions fill the tensor cores (a routed expert then has about 60 of them) and take 2.3 GB
-// of work buffers at full size; engines with short sessions keep fewer (host ops may still bring that many rows).
+// of work buffers at full size; engines with short sessions keep fewer (host ops may still bring that many rows), and the ranks
+// of an expert-parallel group CHUNK: their exchange regions hold that many positions' rows.
 constexpr int PASS_MAX = 2048, PASS_MIN = 256;
 constexpr int TC_MIN_T = 2;     // positions from which the projections go to the tensor cores
 constexpr int PROF_SLOTS = 8;
@@ -150,7 +151,7 @@ struct g5b_engine {
     void *mqt;                                   // absorbed queries as BF16 terms
     double *mqa, *mdsc, *mpart = nullptr, *mstats = nullptr;
     int *mcount = nullptr;
-    TcGemm *tc = nullptr;                                // FP8 / BF16 projections of several positions on tcgen05
+    TcGemm *tc = nullptr;                                // projections and experts of two or more positions on tcgen05
     int mla_tensor = 1;                                  // option "mla_tensor": 0 keeps the attention core on the FP64 kernels
     size_t mpart_bytes = 0;
     int tensor_gemm = 1;                                 // option "tensor_gemm": 0 keeps several positions on the one-token kernels

@@ -1,17 +1,21 @@
 // kda.cu - the gated delta-rule linear attention step (KDA), everything between the input
-// projections and the output projection in one kernel.
+// projections and the output projection.
 //
 // Reference: glm53f_kda_layer and kda_step (src/core/glm53f_ops.c:630-755). Its device form was
 // nine launches per layer and token (three k_shortconv, k_kda_prep, k_kda_decay, k_kda_read,
 // k_kda_write, k_kda_out, k_onorm_gate; src/gpu/glm53f_gpu_kernels.cu:243-450) that passed over
-// the 64 KB per-head state four times. Here one CTA per head does: short convolution + SiLU of
-// q/k/v with the carried history, L2 norm of q and k, beta and the per-channel decay, the
-// recurrence, and the gated per-head RMSNorm of the output. A thread owns one value column of
-// the state and keeps it in registers, so the state is read once and written once per call
-// however many tokens the call carries.
+// the 64 KB per-head state four times. Here it is short convolution + SiLU of q/k/v with the
+// carried history, L2 norm of q and k, beta and the per-channel decay, the recurrence, and the
+// gated per-head RMSNorm of the output, with the state in registers, read once and written once
+// per call however many tokens the call carries:
+//   one position of one sequence, head_dim 64 or 128   kda_step_kernel, a cluster of CTAs per head
+//   several positions, or one of several sequences     kda_prep_kernel, kda_scan_kernel, kda_out_kernel
+//   other head sizes                                   kda_core_kernel, a CTA per head, the state in memory
 //
-// The recurrence keeps the reference's order of FP32 operations (decay row i, u_j += S_ij k_i,
-// S_ij += k_i u_j, o_j += S_ij q_i, ascending i, products and sums rounded separately).
+// The one-position and the any-size kernel keep the reference's order of FP32 operations (decay row
+// i, u_j += S_ij k_i, S_ij += k_i u_j, o_j += S_ij q_i, ascending i, products and sums rounded
+// separately) and its exactly rounded exponential. The kernels over many rows do not: products are
+// fused, sums taken in parts, o from the decayed state, exponentials within 0.53 units (expf_near).
 #include "common.cuh"
 #include "kernels.h"
 

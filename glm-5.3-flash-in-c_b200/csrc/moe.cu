@@ -31,7 +31,7 @@ constexpr int MOE_WARPS = MOE_THREADS / 32;
 // index wins ties; weights from the unbiased scores, normalised in FP64, times the routed scale
 // (reference glm53f_router, src/core/glm53f_ops.c:945-976).
 constexpr int RT_WARPS = 4;
-constexpr int RT_MAX_TOKENS = 64;            // tokens per launch (the engine's pass size)
+constexpr int RT_MAX_TOKENS = 64;            // tokens per launch; a pass of more is routed in several and grouped by moe_plan_kernel
 
 struct RouterArgs {
     int *idx; float *w; float *score;

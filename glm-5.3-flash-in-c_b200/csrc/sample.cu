@@ -13,8 +13,9 @@
 // FP64 sums are taken in a different association on the two sides, so a draw can differ only when
 // a running sum falls within rounding (1e-16 relative) of a threshold.
 //
-// Four small launches over the whole GPU (as one CTA walking the vocabulary seven times a draw from 154880
-// logits took 1.9 ms, as much as the eight decoder layers before it; now 15 us):
+// Four small launches over the whole GPU (as one CTA walking the vocabulary seven times a draw from 154880 logits
+// took 1.9 ms, as much as the eight decoder layers before it; now a sampled token takes 41 us more than a greedy
+// one with a nucleus of 0.95, 9 us more with top_p = 1):
 //   max    each CTA's largest logit
 //   prob   p_i, each CTA's mass, and the mass per bin of the upper 12 bits of p (p >= 0: bits order like values)
 //   cut    every CTA finds the bin in which the nucleus mass is reached (top_p < 1), adds the mass of its

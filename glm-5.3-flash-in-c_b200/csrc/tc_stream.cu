@@ -1,6 +1,9 @@
-// tc_stream.cu - weights streamed once from HBM past up to 64 activation rows on the 5th-generation
-// tensor cores: the projections of 2..64 positions, and the routed experts of any batch (at most 64 rows
-// of one expert per tile).
+// tc_stream.cu - weights streamed once from HBM past the activation rows of a call on the 5th-generation
+// tensor cores: the projections of two and more positions (up to the engine's pass of 2048), and the experts
+// of two and more tokens.
+//
+// Rows go past a weight tile at most 64 at a time (BF16; FP8 calls of up to 64 positions), 32 (FP8 beyond) or, of one
+// expert, 16 or 32 (tc_tile_shift); the further tiles of rows find the weights in L2.
 //
 // Reference: glm53f_mm_batch / matmul_f8_batch / matmul_bf16 (src/core/glm53f_ops.c:101-154,
 // 378-444) and moe_chunk (:1144-1342), which decode each block of codes once for up to 64 inputs.
@@ -33,7 +36,8 @@
 // only 22 - and HBM delivers 32 KB to an SM in about 1400 cycles. So: units of 32 KB, not 16; one load
 // instruction per unit for the weights and one for all terms; one barrier for both operands of an MMA; two warps that
 // issue the MMAs of units in turn; and two groups of epilogue warps, which take units in turn while a tile has at
-// most 32 rows and half of the rows each beyond.
+// most 32 rows and half of the rows each beyond. A unit of an expert then takes 1750 cycles (8 tokens), 1880 (64), 2390 (333)
+// and 2800 (2048 tokens, weights from L2) for gate/up; its products 22 cycles x 16 with 8 rows, 37 x 16 with 32.
 //
 // Warps (FP8): 0-7 epilogue (tcgen05.ld: warp w reaches lanes 32 (w % 4) ..), 8-15 conversion, 16 weights, 17 terms,
 // 18 and 19 MMA. BF16: 0-7 epilogue, 8 weights and terms, 9 MMA. Every wait is bounded; one that runs out records a
