@@ -162,7 +162,7 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
                  int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &p, int with_shared,
                  int *counter, int shared_t0 = 0, int shared_n = -1, double *dots = nullptr);
 // dots: room for RT_TILE_ROWS (or T, if that is more) rows of n_experts dot products, which many tokens take apart
-constexpr int RT_TILE_ROWS = 2048;
+constexpr int RT_TILE_ROWS = 16384;
 // Batch-1 experts multiplied by the tensor cores from their FP8 codes (moe_mma.cu); act_terms holds
 // the SwiGLU output split into two F16 terms per element, [pairs][2][I]. 0, or -1 where the device refuses the shared memory.
 bool moe_mma_supported(const MoeShape &s, int T);

@@ -158,18 +158,21 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     // the last selection then groups the pairs.
     __threadfence();
     __syncthreads();
-    if (tid == 0) {
-        const int prev = atomicAdd(a.counter + 1 + t, 1);
-        is_last = prev == (int)gridDim.x - 1;
-        if (is_last) a.counter[1 + t] = 0;
+    if (gridDim.x > 1) {
+        if (tid == 0) {
+            const int prev = atomicAdd(a.counter + 1 + t, 1);
+            is_last = prev == (int)gridDim.x - 1;
+            if (is_last) a.counter[1 + t] = 0;
+        }
+        __syncthreads();
+        if (!is_last) return;
+        __threadfence();
     }
-    __syncthreads();
-    if (!is_last) return;
-    __threadfence();
     if (warp == 0) {
         if (a.NE <= 512) topk_one_token<16>(a, t, lane);
         else             topk_one_token<32>(a, t, lane);
     }
+    if (!a.p.n_slots) return;
     __threadfence();
     __syncthreads();
     if (tid == 0) {
@@ -180,7 +183,6 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    if (!a.p.n_slots) return;
 
     // Group the (token, slot) pairs by expert. Slots are numbered in expert order; the shared
     // expert, when asked for, is the last slot and takes every token. Which pair of an expert
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, 
     }
 }
 
-constexpr int RT_TILE_MIN_T = 17, RT_TILE_CTAS = 600, RT_MAX_PARTS = 32;
+constexpr int RT_TILE_MIN_T = 17, RT_TILE_CTAS = 1200, RT_MAX_PARTS = 32;
 // p may be null-planned (p.n_slots == nullptr) when only the routing is wanted.
 void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float *x, int ldx, const void *gate,
                  int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &p, int with_shared,
@@ -312,7 +314,7 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
     // CTAs per SM (64 tokens: 56 us for everything, now 38); below, adding up the stretches costs more than they save (7 tokens:
     // 21 us in one kernel, 36 in two).
     int parts = 0, per = s.E;
-    if (T >= RT_TILE_MIN_T && dots && gate_dt == DT_BF16 && s.E % F64_K == 0 && ldx % 4 == 0 &&
+    if (T >= RT_TILE_MIN_T && dots && gate_dt == DT_BF16 && s.E % F64_K == 0 && s.NE % 2 == 0 && ldx % 4 == 0 &&
         (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(gate) & 15) == 0) {
         const int rows = f64_tile_rows(T), tiles = (T + rows - 1) / rows * ((s.NE + F64_N - 1) / F64_N), blocks = s.E / F64_K;
         parts = (RT_TILE_CTAS + tiles - 1) / tiles;
@@ -324,8 +326,11 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
         const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per, {}};
         f64_tile<false>(st, f, parts);
     }
-    for (int t0 = 0; t0 < T; t0 += RT_MAX_TOKENS) {
-        const int n = T - t0 < RT_MAX_TOKENS ? T - t0 : RT_MAX_TOKENS;
+    // (with the dot products there a token is one CTA's, which needs no counter: one launch selects for all of them. 2048 tokens:
+    // 403 us in 32 launches)
+    const int most = parts ? T : RT_MAX_TOKENS;
+    for (int t0 = 0; t0 < T; t0 += most) {
+        const int n = T - t0 < most ? T - t0 : most;
         RouterArgs a{idx + (size_t)t0 * s.K, w + (size_t)t0 * s.K, score + (size_t)t0 * s.NE, x + (size_t)t0 * ldx, ldx, gate, gate_dt, bias, s.NE, s.E, s.K, n,
                      s.norm_topk, s.routed_scale, one ? p : MoePlan{}, s.n_local0, s.n_local, with_shared, counter, shared_t0, shared_n < 0 ? n : shared_n,
                      parts ? dots + (size_t)t0 * s.NE : nullptr, parts, (size_t)T * s.NE};
