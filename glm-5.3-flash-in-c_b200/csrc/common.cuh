@@ -100,8 +100,8 @@ __device__ __forceinline__ float sigmoid_host(float x)
 // exp(x) to 0.53 units in the last place (the double-precision route above: 0.5), in thirty FP32
 // instructions: Cody and Waite's reduction x = n ln 2 + r with ln 2 cut after 14 bits (n times that is exact),
 // Taylor's series of e^r to r^9 with its terms up to r^2 / 2 as pairs of floats, one rounding at the end. For
-// places that take millions: FP64 instructions issue at an eighth of the FP32 rate here, and an exponential is
-// about thirty of either. Equal to the correctly rounded result for 99.75 % of the arguments when they are spread evenly over
+// places that take millions: FP64 instructions issue at half of the FP32 rate here, conversions to and from doubles at an eighth, and an
+// exponential is about thirty instructions of either. Equal to the correctly rounded result for 99.75 % of the arguments when they are spread evenly over
 // -87 .. 88, for 99.98 % when they are spread evenly over the floats there (the test of both is a sweep of either kind);
 // subnormal results are off by less than one of their units.
 __device__ __forceinline__ float expf_near(float x)
@@ -171,6 +171,13 @@ __device__ __forceinline__ double rsqrt_newton(double x)
     r = fma(r, fma(-0.5 * x * r, r, 0.5), r);
     return fma(r, fma(-0.5 * x * r, r, 0.5), r);
 }
+
+// 16 bytes from global to shared memory, without a register on the way; both addresses 16-byte aligned
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // ---- thread-block clusters
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }

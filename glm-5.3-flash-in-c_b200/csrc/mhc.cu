@@ -7,6 +7,7 @@
 // normalises the mixer while the other warps collapse the streams, which only need `pre`.
 #include "acc2.cuh"
 #include "common.cuh"
+#include "f64_tile.cuh"
 #include "kernels.h"
 
 namespace g5b {
@@ -540,176 +541,305 @@ __global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCC_THREADS) 
     cluster_wait();
 }
 
-// ---- the same site for many positions (four streams): one CTA per position, three at a time on an SM.
-// A cluster finishes one position sooner, but only 37 fit the GPU at once and each is a chain of latencies: 45 us for 64
-// positions, 1197 us for 2048. What bounds many positions is arithmetic - (2 + M) M products per stream element, ten
-// FP32 instructions each to carry the sums like FP64: 31,000 cycles per position and SM, 223 us for 2048 - so the chains of one
-// position (exponentials, Sinkhorn, norms) run beside the products of the others. Measured: 453 us for 2048 positions.
-// The streams stay in shared memory; a thread takes every 256th piece of eight elements and six mixer rows at a time.
-constexpr int HCR_THREADS = 256, HCR_ROWS = 6, HCR_M = 4, HCR_MIX = (2 + HCR_M) * HCR_M;
-constexpr size_t HCR_MAX_SMEM = (size_t)200 << 10;
+// ---- the same site for several positions (four streams): a cluster takes eight positions at once.
+// A cluster per position multiplies the mixer rows, which every position shares, position by position, with sums like
+// FP64's made of ten FP32 instructions per term (acc2.cuh): 45 us for 64 positions, and one CTA per position 442 us for 2048. With
+// eight positions the mixer product is a contraction, [24 rows] x [8 positions] over the CTA's columns, and the FP64 matrix
+// instruction does it: 64 FMA per clock and SM, while a mixer element becomes a double once per eight products and a
+// stream element once per 24. The columns' order in the sum is the lanes' own: lane q of four takes eight consecutive columns, one
+// 16-byte piece of a mixer row and two of a stream, for eight steps of the instruction. Everything else is in FP64
+// too, with a column's streams converted once. A CTA keeps its columns of the eight positions in shared memory from the first
+// load to the last store; gates, Sinkhorn and norms run as in the cluster kernel above, the Sinkhorn chain of position r in
+// warp 0 of CTA r. 64 positions: 26 us, 45 with a cluster
+// per position; 2048: 222, 442 with a CTA per position (the FP64 products alone 45, HBM 56: a cluster is a chain of phases, and two CTAs
+// of 100 KB fit an SM).
+constexpr int HCG_POS = 8, HCG_WARPS = 8, HCG_THREADS = HCG_WARPS * 32, HCG_M = 4, HCG_MIX = (2 + HCG_M) * HCG_M;
+static_assert(HCG_POS == HCC_CTAS && HCG_POS == HCG_WARPS && HCG_MIX == 24, "a CTA of the cluster and a warp per position; three tiles of rows");
+// streams of a position in shared memory: 4 more than a multiple of 32 words, so that two positions' pieces share a wavefront
+__host__ __device__ constexpr int hcg_pitch(int W) { return (HCG_M * W + 31) / 32 * 32 + 4; }
 
-__device__ __forceinline__ void acc2_merge(Acc2 &a, float s, float c)
+__global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCG_THREADS, 2) hc_pre_group_kernel(const HcFused a, int T)
 {
-    acc2_add(a, s);
-    a.c = __fadd_rn(a.c, c);
-}
-__device__ __forceinline__ Acc2 acc2_warp_sum(Acc2 a)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float s = __shfl_xor_sync(0xffffffffu, a.s, o), c = __shfl_xor_sync(0xffffffffu, a.c, o);
-        acc2_merge(a, s, c);
-    }
-    return a;
-}
-
-__global__ void __launch_bounds__(HCR_THREADS, 3) hc_pre_rows_kernel(const HcFused a)
-{
-    extern __shared__ __align__(16) float hs[];                  // [4][E]; the collapsed vector later takes the first E
-    __shared__ double part[HCR_THREADS / 32][HCR_MIX + 1], dots[HCR_MIX + 1], pre[HCR_M], red[HCR_THREADS / 32];
-    __shared__ float mx[HCR_MIX];
-    constexpr int M = HCR_M, MM = M * M, MIX = HCR_MIX, NWARPS = HCR_THREADS / 32;
+    extern __shared__ __align__(16) float hs[];                  // [8][pitch]: this CTA's columns of the positions' streams
+    __shared__ double part[HCG_WARPS][HCG_MIX + 1][HCG_POS];     // the warps' parts of the dots, and of sum h^2
+    __shared__ double mine[HCG_MIX + 1][HCG_POS], dots[HCG_MIX + 1][HCG_POS], mine_s2[HCG_POS];
+    __shared__ double cbs[HCG_POS][HCG_M * HCG_M + HCG_M], pre[HCG_POS][HCG_M];
+    __shared__ float mx[HCG_POS][HCG_MIX], factor[HCG_POS];
+    constexpr int M = HCG_M, MM = M * M, MIX = HCG_MIX;
     pdl_trigger();
-    const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, E = a.E, ME = M * E;
-    float *ht = a.h + (size_t)t * ME;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    const uint32_t rank = cluster_cta_rank();
+    const int E = a.E, ME = M * E, W = E / HCC_CTAS, d0 = (int)rank * W, P = hcg_pitch(W);
+    const int t0 = blockIdx.y * HCG_POS, np = T - t0 < HCG_POS ? T - t0 : HCG_POS;
     const double eps = (double)a.hc_eps;
+
+    float *ys = hs + HCG_POS * P;                                // [8][W]: the pending output
+    float *norm = ys + HCG_POS * W;                              // [W]
+    const int groups = (W + 127) / 128;                          // of 128 columns of a position: at most 8
+    // The warp's blocks of 32 columns of a stream; the first two blocks' mixer rows are asked for before anything else.
+    const int per = (W + 31) / 32, blocks = M * per;
+    uint4 wn[2][3];
+    auto load_rows = [&](uint4 (&w)[3], int blk) {
+        const int c = (blk % per) * 32 + q * 8;
+#pragma unroll
+        for (int m = 0; m < 3; m++)
+            w[m] = blk < blocks && c < W ? __ldg(reinterpret_cast<const uint4 *>(a.fn + (size_t)(m * 8 + g) * ME + (size_t)(blk / per) * E + d0 + c)) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    load_rows(wn[0], warp);
+    load_rows(wn[1], warp + HCG_WARPS);
+    for (int i = tid * 4; i < W; i += HCG_THREADS * 4) cp_async16(norm + i, a.norm_w + d0 + i);
     pdl_wait();
 
-    Acc2 sq;
+    // ---- the streams, all of them on their way at once: 80 KB per SM and CTA, one round trip
+    for (int i = tid; i < HCG_POS * M * (W / 4); i += HCG_THREADS) {
+        const int p = i / (M * (W / 4)), r = i % (M * (W / 4)), k = r / (W / 4), c = (r % (W / 4)) * 4;
+        float *dst = hs + p * P + k * W + c;
+        if (p < np) cp_async16(dst, a.h + (size_t)(t0 + p) * ME + (size_t)k * E + d0 + c);
+        else        *reinterpret_cast<float4 *>(dst) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
     if (a.y) {
-        // the pending hc_post of the previous site, as in the kernel above
-        float cb[MM], po[M];
+        for (int i = tid; i < np * (W / 4); i += HCG_THREADS) {
+            const int p = i / (W / 4), c = (i % (W / 4)) * 4;
+            cp_async16(ys + p * W + c, a.y + (size_t)(t0 + p) * E + d0 + c);
+        }
+        for (int i = tid; i < np * (MM + M); i += HCG_THREADS) {
+            const int p = i / (MM + M), k = i % (MM + M);
+            cbs[p][k] = (double)(k < MM ? __ldcg(a.comb + (size_t)(t0 + p) * MM + k) : __ldcg(a.post + (size_t)(t0 + p) * M + k - MM));
+        }
+    }
+    cp_async_wait();
+    __syncthreads();
+    // ---- the pending hc_post of the previous site (src/core/glm53f_ops.c:612-625): warp p has position p
+    if (a.y && warp < np) {
+        const int p = warp;
+        float *hp = hs + p * P, *ht = a.h + (size_t)(t0 + p) * ME + d0;
+#pragma unroll 1
+        for (int c = lane * 4; c < W; c += 128) {
+            double hx[M], hy[M], hz[M], hw[M];
 #pragma unroll
-        for (int i = 0; i < MM; i++) cb[i] = __ldcg(a.comb + (size_t)t * MM + i);
+            for (int i = 0; i < M; i++) {
+                const float4 v = *reinterpret_cast<const float4 *>(hp + i * W + c);
+                hx[i] = (double)v.x; hy[i] = (double)v.y; hz[i] = (double)v.z; hw[i] = (double)v.w;
+            }
+            const float4 yv = *reinterpret_cast<const float4 *>(ys + p * W + c);
+            const double yx = (double)yv.x, yy = (double)yv.y, yz = (double)yv.z, yw = (double)yv.w;
+#pragma unroll 1
+            for (int j = 0; j < M; j++) {                        // rolled: a launch runs this code once or twice, from a cold cache
+                const double po = cbs[p][MM + j];
+                double sx = po * yx, sy = po * yy, sz = po * yz, sw = po * yw;
 #pragma unroll
-        for (int i = 0; i < M; i++) po[i] = __ldcg(a.post + (size_t)t * M + i);
-        for (int d = tid * 2; d < E; d += HCR_THREADS * 2) {
-            const float2 yv = *reinterpret_cast<const float2 *>(a.y + (size_t)t * E + d);
-            float2 hv[M];
-#pragma unroll
-            for (int i = 0; i < M; i++) hv[i] = *reinterpret_cast<const float2 *>(ht + (size_t)i * E + d);
-#pragma unroll
-            for (int j = 0; j < M; j++) {
-                Acc2 s0, s1;
-                acc2_fma(s0, po[j], yv.x);
-                acc2_fma(s1, po[j], yv.y);
-#pragma unroll
-                for (int i = 0; i < M; i++) { acc2_fma(s0, cb[i * M + j], hv[i].x); acc2_fma(s1, cb[i * M + j], hv[i].y); }
-                const float2 nv = make_float2(acc2_f32(s0), acc2_f32(s1));
-                *reinterpret_cast<float2 *>(hs + j * E + d) = nv;
-                *reinterpret_cast<float2 *>(ht + (size_t)j * E + d) = nv;
-                acc2_fma(sq, nv.x, nv.x);
-                acc2_fma(sq, nv.y, nv.y);
+                for (int i = 0; i < M; i++) {
+                    const double cb = cbs[p][i * M + j];
+                    sx = fma(cb, hx[i], sx); sy = fma(cb, hy[i], sy); sz = fma(cb, hz[i], sz); sw = fma(cb, hw[i], sw);
+                }
+                const float4 v = make_float4((float)sx, (float)sy, (float)sz, (float)sw);
+                *reinterpret_cast<float4 *>(hp + j * W + c) = v;
+                *reinterpret_cast<float4 *>(ht + (size_t)j * E + c) = v;
             }
         }
-    } else {
-        for (int i = tid * 4; i < ME; i += HCR_THREADS * 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(ht + i);
-            *reinterpret_cast<float4 *>(hs + i) = v;
-            acc2_fma(sq, v.x, v.x); acc2_fma(sq, v.y, v.y); acc2_fma(sq, v.z, v.z); acc2_fma(sq, v.w, v.w);
-        }
     }
-    __syncwarp();
-    sq = acc2_warp_sum(sq);
-    if (lane == 0) part[warp][MIX] = acc2_f64(sq);
     __syncthreads();
 
-    // mixer rows (compensated FP32 sums; the reference's are FP64)
-    const int pieces = ME / 8;
-#pragma unroll 1
-    for (int k0 = 0; k0 < MIX; k0 += HCR_ROWS) {
-        Acc2 acc[HCR_ROWS];
-        uint4 wn[HCR_ROWS];
-        const uint16_t *rows = a.fn + (size_t)k0 * ME;
-        auto load = [&](int piece) {
+    // ---- mixer rows, and the sums of squares of the values that the lanes have as doubles then anyway
+    {
+        double acc[2][3][2] = {}, sq[4] = {};                    // (several sums each: a product waits for the one before it in its sum)
+        uint32_t special = 0;                                    // an infinity or NaN among this lane's mixer elements
+        // A BF16's bits put where a double has them are its value times 2^-896 (zero and subnormal ones too): two instructions,
+        // where the exponent's own bias takes eight. The sums are scaled back at the end. Sums of such small numbers lose
+        // nothing to underflow before 2^-52 of mixer elements below 2^-110.
+        auto multiply = [&](const uint4 (&wv)[3], int blk, auto widen) {
+            const int c = (blk % per) * 32 + q * 8;
+            float hv[8];
+            if (c < W) {
+                const float *hp = hs + g * P + (blk / per) * W + c;
+                const float4 h0 = *reinterpret_cast<const float4 *>(hp), h1 = *reinterpret_cast<const float4 *>(hp + 4);
+                hv[0] = h0.x; hv[1] = h0.y; hv[2] = h0.z; hv[3] = h0.w; hv[4] = h1.x; hv[5] = h1.y; hv[6] = h1.z; hv[7] = h1.w;
+            } else {
 #pragma unroll
-            for (int r = 0; r < HCR_ROWS; r++) wn[r] = __ldg(reinterpret_cast<const uint4 *>(rows + (size_t)r * ME + (size_t)piece * 8));
-        };
-        if (tid < pieces) load(tid);
-#pragma unroll 1
-        for (int piece = tid; piece < pieces; piece += HCR_THREADS) {
-            uint4 wv[HCR_ROWS];
+                for (int k = 0; k < 8; k++) hv[k] = 0.f;
+            }
+            // Two steps' factors become doubles while the two before them are multiplied, in registers of their own: written as
+            // plain expressions they shared a few registers and every product waited for the one before to have read them.
+            double av[2][2][3], bv[2][2];
+            auto take = [&](int j) {
 #pragma unroll
-            for (int r = 0; r < HCR_ROWS; r++) wv[r] = wn[r];
-            if (piece + HCR_THREADS < pieces) load(piece + HCR_THREADS);
-            const float4 h0 = *reinterpret_cast<const float4 *>(hs + piece * 8), h1 = *reinterpret_cast<const float4 *>(hs + piece * 8 + 4);
-            const float hd[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                for (int k = 0; k < 2; k++) {
 #pragma unroll
-            for (int j = 0; j < 4; j++)
-#pragma unroll
-                for (int r = 0; r < HCR_ROWS; r++) {
-                    const uint32_t w = j == 0 ? wv[r].x : j == 1 ? wv[r].y : j == 2 ? wv[r].z : wv[r].w;
-                    acc2_fma(acc[r], __uint_as_float(w << 16), hd[2 * j]);
-                    acc2_fma(acc[r], __uint_as_float(w & 0xffff0000u), hd[2 * j + 1]);
+                    for (int m = 0; m < 3; m++) {
+                        const uint32_t u = j == 0 ? wv[m].x : j == 1 ? wv[m].y : j == 2 ? wv[m].z : wv[m].w;
+                        widen(av[j & 1][k][m], k ? u : u << 16);
+                    }
+                    asm volatile("cvt.f64.f32 %0, %1;" : "=d"(bv[j & 1][k]) : "f"(hv[2 * j + k]));
                 }
-        }
-        __syncwarp();
+            };
+            take(0);
 #pragma unroll
-        for (int r = 0; r < HCR_ROWS; r++) {
-            const Acc2 v = acc2_warp_sum(acc[r]);
-            if (lane == 0) part[warp][k0 + r] = acc2_f64(v);
+            for (int j = 0; j < 4; j++) {
+                if (j < 3) take(j + 1);
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+#pragma unroll
+                    for (int m = 0; m < 3; m++) mma_f64(acc[k][m], av[j & 1][k][m], bv[j & 1][k]);
+                    sq[2 * (j & 1) + k] = fma(bv[j & 1][k], bv[j & 1][k], sq[2 * (j & 1) + k]);
+                }
+            }
+        };
+        auto step = [&](uint4 (&wv)[3], int blk) {
+#pragma unroll
+            for (int m = 0; m < 3; m++) {
+                const uint32_t u[4] = {wv[m].x, wv[m].y, wv[m].z, wv[m].w};
+#pragma unroll
+                for (int k = 0; k < 4; k++) special |= ((u[k] & 0x7f807f80u) + 0x00800080u) & 0x80008000u;
+            }
+            multiply(wv, blk, [](double &d, uint32_t u) {
+                asm volatile("{\n\t.reg .b32 t;\n\tshr.s32 t, %1, 3;\n\tand.b32 t, t, 0x8fffe000;\n\tmov.b64 %0, {0, t};\n\t}" : "=d"(d) : "r"(u));
+            });
+            load_rows(wv, blk + 2 * HCG_WARPS);
+        };
+#pragma unroll 1
+        for (int blk = warp; blk < blocks; blk += 2 * HCG_WARPS) {
+            step(wn[0], blk);
+            if (blk + HCG_WARPS < blocks) step(wn[1], blk + HCG_WARPS);
         }
+        const double scale = __hiloint2double((896 + 1023) << 20, 0);
+#pragma unroll
+        for (int m = 0; m < 3; m++)
+#pragma unroll
+            for (int i = 0; i < 2; i++) acc[0][m][i] = (acc[0][m][i] + acc[1][m][i]) * scale;
+        if (__any_sync(0xffffffffu, special)) {
+            // those have no place among the scaled ones: the warp's products once more, element by element
+            sq[0] = sq[1] = sq[2] = sq[3] = 0.0;
+#pragma unroll
+            for (int m = 0; m < 3; m++) acc[0][m][0] = acc[0][m][1] = acc[1][m][0] = acc[1][m][1] = 0.0;
+#pragma unroll 1
+            for (int blk = warp; blk < blocks; blk += HCG_WARPS) {
+                uint4 wv[3];
+                load_rows(wv, blk);
+                multiply(wv, blk, [](double &d, uint32_t u) { d = (double)__uint_as_float(u & 0xffff0000u); });
+            }
+#pragma unroll
+            for (int m = 0; m < 3; m++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) acc[0][m][i] += acc[1][m][i];
+        }
+        double ss = (sq[0] + sq[1]) + (sq[2] + sq[3]);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+        ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+        if (q == 0) part[warp][MIX][g] = ss;
+#pragma unroll
+        for (int m = 0; m < 3; m++) { part[warp][m * 8 + g][2 * q] = acc[0][m][0]; part[warp][m * 8 + g][2 * q + 1] = acc[0][m][1]; }
     }
     __syncthreads();
-    if (tid <= MIX) {
-        double v = 0.0;
-        for (int w = 0; w < NWARPS; w++) v += part[w][tid];
-        dots[tid] = v;
+    if (tid < (MIX + 1) * HCG_POS) {
+        const int k = tid / HCG_POS, p = tid % HCG_POS;
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < HCG_WARPS; w++) s += part[w][k][p];
+        mine[k][p] = s;
     }
     __syncthreads();
-    if (tid < MIX) {
-        const float inv = (float)(1.0 / sqrt(dots[MIX] / (double)ME + (double)a.rms_eps));
-        mx[tid] = (float)(dots[tid] * (double)inv);
+    cluster_arrive();
+    cluster_wait();
+
+    // ---- every CTA: the positions' sums in CTA order, the norm factors, the gates
+    if (tid < (MIX + 1) * HCG_POS) {
+        double s = 0.0;
+#pragma unroll
+        for (uint32_t r = 0; r < HCC_CTAS; r++) s += ld_cluster_f64(&mine[0][0] + tid, r);
+        (&dots[0][0])[tid] = s;
     }
+    __syncthreads();
+    if (tid < MIX * HCG_POS) {
+        const int k = tid / HCG_POS, p = tid % HCG_POS;
+        const float inv = (float)rsqrt_newton(dots[MIX][p] / (double)ME + (double)a.rms_eps);
+        mx[p][k] = (float)(dots[k][p] * (double)inv);
+    }
+    __syncthreads();
+    if (tid < HCG_POS * M) pre[tid / M][tid % M] = (double)sigmoid_host(mul_add_unfused(mx[tid / M][tid % M], a.scale[0], a.base[tid % M])) + eps;
     __syncthreads();
     if (warp == 0) {
-        // row softmax + eps, then column / row normalisations (src/core/glm53f_ops.c:577-598)
-        const int el = lane < MM ? lane : 0, i = el / M, j = el % M, k = 2 * M + el;
-        const double l = (double)mul_add_unfused(mx[k], a.scale[2], a.base[k]);
-        double top = -INFINITY;
+        cluster_arrive();                                        // nothing of this warp goes into the sums of x^2
+        if ((int)rank < np) {
+            // position `rank`: row softmax + eps, then column / row normalisations (src/core/glm53f_ops.c:577-598)
+            const float *m = mx[rank];
+            const int t = t0 + (int)rank, el = lane < MM ? lane : 0, i = el / M, j = el % M, k = 2 * M + el;
+            const double l = (double)mul_add_unfused(m[k], a.scale[2], a.base[k]);
+            double top = -INFINITY;
 #pragma unroll
-        for (int jj = 0; jj < M; jj++) top = fmax(top, __shfl_sync(0xffffffffu, l, i * M + jj));
-        const double ex = exp(l - top);
-        double z = 0.0;
+            for (int jj = 0; jj < M; jj++) top = fmax(top, __shfl_sync(0xffffffffu, l, i * M + jj));
+            const double ex = exp(l - top);
+            double z = 0.0;
 #pragma unroll
-        for (int jj = 0; jj < M; jj++) z += __shfl_sync(0xffffffffu, ex, i * M + jj);
-        const double v = sinkhorn_passes<M>(ex / z + eps, M, i, j, 2 * a.iters - 1, eps);
-        if (lane < MM) a.comb[(size_t)t * MM + lane] = (float)v;
+            for (int jj = 0; jj < M; jj++) z += __shfl_sync(0xffffffffu, ex, i * M + jj);
+            const double v = sinkhorn_passes<M>(ex / z + eps, M, i, j, 2 * a.iters - 1, eps);
+            if (lane < MM) a.comb[(size_t)t * MM + lane] = (float)v;
+            if (lane >= MM && lane < MM + M) {
+                const int i2 = lane - MM;
+                a.post[(size_t)t * M + i2] = __fmul_rn(2.0f, sigmoid_host(mul_add_unfused(m[M + i2], a.scale[1], a.base[M + i2])));
+            }
+            __syncwarp();
+        }
+        cluster_wait();
     } else {
-        constexpr int NT = HCR_THREADS - 32;
+        // x[d] = sum_i pre[i] * h[i][d] in FP64 (src/core/glm53f_ops.c:603-607) for this CTA's columns of the eight positions
+        // (a warp takes 128 columns of a position at a time)
+        constexpr int NT = HCG_THREADS - 32;
         const int wt = tid - 32;
-        if (wt < M) {
-            pre[wt] = (double)sigmoid_host(mul_add_unfused(mx[wt], a.scale[0], a.base[wt])) + eps;
-            a.post[(size_t)t * M + wt] = __fmul_rn(2.0f, sigmoid_host(mul_add_unfused(mx[M + wt], a.scale[1], a.base[M + wt])));
+        for (int i = warp - 1; i < HCG_POS * groups; i += HCG_WARPS - 1) {
+            const int p = i / groups, c = i % groups * 128 + lane * 4;
+            float *hp = hs + p * P + c;
+            double s2 = 0.0;
+            if (c < W) {
+                double x = 0.0, y = 0.0, z = 0.0, w = 0.0;
+#pragma unroll
+                for (int k = 0; k < M; k++) {
+                    const float4 v = *reinterpret_cast<const float4 *>(hp + k * W);
+                    const double pr = pre[p][k];
+                    x += pr * (double)v.x; y += pr * (double)v.y; z += pr * (double)v.z; w += pr * (double)v.w;
+                }
+                const float4 xv = make_float4((float)x, (float)y, (float)z, (float)w);
+                *reinterpret_cast<float4 *>(hp) = xv;            // (this thread alone reads these columns)
+                x = (double)xv.x; y = (double)xv.y; z = (double)xv.z; w = (double)xv.w;
+                s2 = fma(x, x, y * y) + fma(z, z, w * w);
+            }
+            s2 = warp_sum(s2);
+            if (lane == 0) (&part[0][0][0])[i] = s2;
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
+        if (wt < HCG_POS) {
+            double s = 0.0;
+            for (int i = 0; i < groups; i++) s += (&part[0][0][0])[wt * groups + i];
+            mine_s2[wt] = s;
         }
         __syncwarp();
-        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
-        // x[d] = sum_i pre[i] * h[i][d] in FP64 (src/core/glm53f_ops.c:603-607), then RMSNorm(x) * w (:473-480)
-        double s2 = 0.0;
-        for (int d = wt; d < E; d += NT) {
-            double v = 0.0;
+        cluster_arrive();
+        cluster_wait();
+        // the sub-blocks' inputs: RMSNorm(x) * w (:473-480)
+        if (wt < HCG_POS) {
+            double tot = 0.0;
 #pragma unroll
-            for (int i = 0; i < M; i++) v += pre[i] * (double)hs[i * E + d];
-            const float xv = (float)v;
-            hs[d] = xv;                                          // (this thread alone reads column d)
-            s2 += (double)xv * (double)xv;
+            for (uint32_t r = 0; r < HCC_CTAS; r++) tot += ld_cluster_f64(&mine_s2[wt], r);
+            factor[wt] = (float)rsqrt_newton(tot / (double)E + (double)a.rms_eps);
         }
-        __syncwarp();
-        s2 = warp_sum(s2);
-        if (lane == 0) red[warp] = s2;
-        __syncwarp();
         asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
-        double tot = 0.0;
-#pragma unroll
-        for (int w = 1; w < NWARPS; w++) tot += red[w];
-        const float f = (float)(1.0 / sqrt(tot / (double)E + (double)a.rms_eps));
-        for (int d = wt; d < E; d += NT) a.xn[(size_t)t * E + d] = __fmul_rn(a.norm_w[d], __fmul_rn(hs[d], f));
+        for (int i = warp - 1; i < np * groups; i += HCG_WARPS - 1) {
+            const int p = i / groups, c = i % groups * 128 + lane * 4;
+            if (c < W) {
+                const float4 v = *reinterpret_cast<const float4 *>(hs + p * P + c), w = *reinterpret_cast<const float4 *>(norm + c);
+                const float f = factor[p];
+                *reinterpret_cast<float4 *>(a.xn + (size_t)(t0 + p) * E + d0 + c) =
+                    make_float4(__fmul_rn(w.x, __fmul_rn(v.x, f)), __fmul_rn(w.y, __fmul_rn(v.y, f)), __fmul_rn(w.z, __fmul_rn(v.z, f)), __fmul_rn(w.w, __fmul_rn(v.w, f)));
+            }
+        }
     }
+    // no CTA leaves while another may still read its shared memory
+    cluster_arrive();
+    cluster_wait();
 }
 
-// Two rounds of the clusters that fit the GPU at once (37): from there on the kernel above is the faster one.
-constexpr int HCR_MIN_T = 75;
+// From here on eight positions to a cluster are faster than one (alone, 5 us of launch included: 12 positions 26.7 against 20.5 us,
+// 16: 26.7 and 27.7, 32: 26.7 and 27.6, 40: 27.6 and 45)
+constexpr int HCG_MIN_T = 16;
 
 static bool hc_pre_cluster_takes(int M, int E)
 {
@@ -731,12 +861,13 @@ void hc_pre_fused(cudaStream_t st, float *xn, float *post, float *comb, float *h
 {
     HcFused a{xn, post, comb, h, y_pending, static_cast<const uint16_t *>(w.fn.w), w.base, w.scale, norm_w, part,
               counters, M, E, iters, hc_eps, rms_eps};
-    const size_t rows_smem = (size_t)M * E * sizeof(float);
-    static SmemGrant grant;
-    if (T >= HCR_MIN_T && M == HCR_M && E % 8 == 0 && rows_smem <= HCR_MAX_SMEM && dev_opt_in_smem((const void *)hc_pre_rows_kernel, rows_smem + (8 << 10), grant)) {
-        // (launched the ordinary way: launched early, its CTAs crowd the SMs that the kernel in front leaves first)
-        G5B_LAUNCH(hc_pre_rows_kernel, T, HCR_THREADS, rows_smem, st, a);
-        return;
+    if (T >= HCG_MIN_T && M == HCG_M && hc_pre_cluster_takes(M, E)) {
+        const size_t smem = ((size_t)HCG_POS * (hcg_pitch(E / HCC_CTAS) + E / HCC_CTAS) + E / HCC_CTAS) * sizeof(float);
+        static SmemGrant grant;
+        if (dev_opt_in_smem((const void *)hc_pre_group_kernel, smem + (20 << 10), grant)) {
+            G5B_LAUNCH(hc_pre_group_kernel, dim3(HCC_CTAS, (T + HCG_POS - 1) / HCG_POS), HCG_THREADS, smem, st, a, T);
+            return;
+        }
     }
     if (hc_pre_cluster_takes(M, E)) G5B_LAUNCH_PDL(hc_pre_cluster_kernel, dim3(HCC_CTAS, T), dim3(HCC_THREADS), 0, st, a);
     else                            G5B_LAUNCH(hc_pre_fused_kernel, dim3(HCF_SLICES, T), HC_THREADS, 0, st, a);
