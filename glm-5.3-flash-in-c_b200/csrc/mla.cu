@@ -198,6 +198,84 @@ __global__ void __launch_bounds__(DSA_WARPS * 32) dsa_score_kernel(
     }
 }
 
+// The same scores, bit for bit, with the FP64 matrix instruction: mma.sync.m8n8k4 on doubles is four fused multiply-adds in ascending
+// k (equal in 12800 random sums of 256 products; a test compares both kernels' scores), so a sum over dimensions in steps of
+// four is the chain above. A CTA takes all heads (a multiple of 8, up to 32) of one query and 64 pools, a warp 16 of the pools;
+// a pooled key becomes a double once, as it is read. 64 queries of 1024 pools: 32 us, 110 before; one query of 8192: the layer
+// takes 8 us less.
+constexpr int DSM_POOLS = 64, DSM_WARPS = 4, DSM_HEADS = 32;
+static size_t dsm_smem(int IH, int ID) 
+{
+    const size_t keys = (size_t)DSM_POOLS * (ID + 4) * 4, terms = (size_t)DSM_POOLS * (IH + 1) * 8;
+    return (size_t)IH * (ID + 4) * 8 + (keys > terms ? keys : terms);
+}
+static bool dsm_takes(const MlaShape &s) { return s.IH % 8 == 0 && s.IH <= DSM_HEADS && s.ID % 16 == 0 && s.ID <= 256; }
+__global__ void __launch_bounds__(DSM_WARPS * 32) dsa_score_tile_kernel(float *score, const float *idx_state, const float *qidx, const float *wproj, int cached, MlaShape s)
+{
+    pdl_trigger();
+    extern __shared__ __align__(16) double dsa_smem[];
+    const int t = blockIdx.y, p = pos_of(s, cached, t), QP = s.ID + 4, KP = s.ID + 4, MP = s.IH + 1;
+    double *qs = dsa_smem;                                       // [IH][QP]
+    float *ks = reinterpret_cast<float *>(qs + (size_t)s.IH * QP);           // [pools][KP]: pooled keys, and in their place
+    double *terms = qs + (size_t)s.IH * QP;                      // [pools][MP]: the heads' terms
+    idx_state = seq_idx(const_cast<float *>(idx_state), s, t);
+    const int np = (p + 1) / s.KP, p0 = blockIdx.x * DSM_POOLS;
+    if (np <= s.topk / s.KP || p0 >= np) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3;
+    const float *pk = idx_state + ((size_t)2 * s.cap + p0) * s.ID;
+    const int n = min(DSM_POOLS, np - p0), pieces = s.ID / 4;
+    for (int i = tid; i < DSM_POOLS * pieces; i += DSM_WARPS * 32) {
+        const int r = i / pieces, c = (i % pieces) * 4;
+        if (r < n) cp_async16(ks + r * KP + c, pk + (size_t)r * s.ID + c);
+        else       *reinterpret_cast<float4 *>(ks + r * KP + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float *qt = qidx + (size_t)t * s.IH * s.ID, *wt = wproj + (size_t)t * s.IH;
+#pragma unroll 8
+    for (int i = tid; i < s.IH * pieces; i += DSM_WARPS * 32) {
+        const int h = i / pieces, c = (i % pieces) * 4;
+        const float4 v = *reinterpret_cast<const float4 *>(qt + (size_t)h * s.ID + c);
+        double2 *d = reinterpret_cast<double2 *>(qs + (size_t)h * QP + c);
+        d[0] = make_double2((double)v.x, (double)v.y); d[1] = make_double2((double)v.z, (double)v.w);
+    }
+    cp_async_wait();
+    __syncthreads();
+    const int MT = s.IH / 8, w0 = warp * 16;
+    double acc[DSM_HEADS / 8][2][2] = {};
+#pragma unroll 4
+    for (int k = 0; k < s.ID; k += 4) {
+        const double b0 = (double)ks[(w0 + g) * KP + k + q], b1 = (double)ks[(w0 + 8 + g) * KP + k + q];
+#pragma unroll
+        for (int m = 0; m < DSM_HEADS / 8; m++)
+            if (m < MT) {
+                const double av = qs[(size_t)(m * 8 + g) * QP + k + q];
+                mma_f64(acc[m][0], av, b0);
+                mma_f64(acc[m][1], av, b1);
+            }
+    }
+    __syncthreads();                                             // the keys have been read
+    const float hscale = 1.0f / sqrtf((float)s.IH), dscale = 1.0f / sqrtf((float)s.ID);
+#pragma unroll
+    for (int m = 0; m < DSM_HEADS / 8; m++)
+        if (m < MT) {
+            const int h = m * 8 + g;
+            const double wh = __dmul_rn((double)wt[h], (double)hscale);
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const double v = __dmul_rn(acc[m][j][i], (double)dscale);
+                    terms[(w0 + j * 8 + 2 * q + i) * MP + h] = v > 0.0 ? __dmul_rn(wh, v) : 0.0;      // (a head that does not count adds nothing)
+                }
+        }
+    __syncwarp();
+    if (lane < 16 && w0 + lane < n) {
+        double sum = 0.0;
+#pragma unroll 8
+        for (int h = 0; h < s.IH; h++) sum = __dadd_rn(sum, terms[(w0 + lane) * MP + h]);
+        score[(size_t)t * (s.cap / s.KP + 1) + p0 + w0 + lane] = (float)sum;
+    }
+}
+
 // Exact top-k of the pool scores (score descending, pool index ascending on ties, the order of
 // the reference's qsort comparator, glm53f_dsa.c:111-116), by radix selection on a 64-bit key,
 // then an order-preserving compaction: kept pools ascending, each expanded to its positions, then
@@ -333,7 +411,12 @@ int dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, con
                const float *wproj, float *score, int T, int cached, const MlaShape &s)
 {
     const int np_max = (cached + (s.batch ? 1 : T)) / s.KP;
-    if (np_max > s.topk / s.KP) {
+    if (np_max > s.topk / s.KP && dsm_takes(s)) {
+        static SmemGrant grant;
+        const size_t smem = dsm_smem(s.IH, s.ID);
+        if (!dev_opt_in_smem((const void *)dsa_score_tile_kernel, smem, grant)) return -1;
+        G5B_LAUNCH(dsa_score_tile_kernel, dim3((np_max + DSM_POOLS - 1) / DSM_POOLS, T), DSM_WARPS * 32, smem, st, score, idx_state, qidx, wproj, cached, s);
+    } else if (np_max > s.topk / s.KP) {
         const size_t smem = ((((size_t)s.ID * s.IH + 1) & ~(size_t)1) + (size_t)DSA_WARPS * DSA_POOLS * (s.IH + s.ID)) * sizeof(double);
         static SmemGrant grant;
         if (!dev_opt_in_smem((const void *)dsa_score_kernel, smem, grant)) return -1;     // (many heads of many dimensions)
@@ -716,6 +799,163 @@ __global__ void __launch_bounds__(256) mla_wsum_reduce_kernel(float *cb, const d
     cb[i] = (float)acc;
 }
 
+// ---- the FP64 core for several queries and the FP32 cache: both contractions with the FP64 matrix instruction (f64_tile.cuh).
+// A thread or a warp per sum, as above, reads a factor from memory or shared memory for every product or four of them and
+// converts it; a tile of 64 heads x 64 positions (or latent columns) converts and reads each once for 64, and the pipe's 64 FMA
+// per clock and SM are what is left. Three launches, sums in FP64 throughout, positions ascending:
+//   score   d[t][h][j] = (q~ . c_j) * scale
+//   prob    p_j = exp((double)(float) d_j - max) / z in place (the reference's softmax, src/core/glm53f_ops.c:890-903)
+//   sum     sum_j p_j c_j in stretches of AT_SPAN positions, added in order by mla_wsum_reduce_kernel if there are several
+// A prompt of 333: 0.6 ms a layer, 2.1 before.
+constexpr int AT_TILE = 64, AT_SPAN = 512, AT_MIN_T = 6;
+
+// visible position jj of the query: a row of the cache
+__device__ __forceinline__ int vis_row(const int *sl, int ns, int jj) { return ns < 0 ? jj : sl[jj]; }
+
+__global__ void __launch_bounds__(F64_THREADS, 3) mla_score_tile_kernel(double *dsc, const double *qa, const float *latent, const int *sel, const int *nsel,
+                                                                       int cached, int stride, MlaShape s)
+{
+    __shared__ __align__(16) double sa[AT_TILE][F64_KPITCH], sb[AT_TILE][F64_KPITCH];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int h0 = blockIdx.y * AT_TILE, t = blockIdx.z, pos = pos_of(s, cached, t), j0 = blockIdx.x * AT_TILE;
+    const int ns = nsel ? nsel[t] : -1, nvis = ns < 0 ? pos + 1 : ns;
+    if (j0 >= nvis) return;
+    latent = static_cast<const float *>(seq_latent(latent, s, t));
+    const int *sl = sel ? sel + (size_t)t * (s.topk + s.KP) : nullptr;
+    // eight lanes take 32 columns of a row, 16 rows at a time
+    const int lr = tid >> 3, lk = (tid & 7) * 4;
+    const double *A = qa + ((size_t)t * s.H + h0 + lr) * s.KL + lk;
+    const float *B[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int jj = j0 + lr + 16 * i;
+        B[i] = jj < nvis ? latent + (size_t)vis_row(sl, ns, jj) * s.KL + lk : nullptr;
+    }
+    double2 ra[4][2];
+    float4 rb[4];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            ra[i][0] = *reinterpret_cast<const double2 *>(A + (size_t)(16 * i) * s.KL + k0);
+            ra[i][1] = *reinterpret_cast<const double2 *>(A + (size_t)(16 * i) * s.KL + k0 + 2);
+            rb[i] = B[i] ? *reinterpret_cast<const float4 *>(B[i] + k0) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    double acc[4][4][2] = {};
+    load(0);
+    for (int k0 = 0; k0 < s.KL; k0 += F64_K) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            double2 *da = reinterpret_cast<double2 *>(&sa[lr + 16 * i][lk]), *db = reinterpret_cast<double2 *>(&sb[lr + 16 * i][lk]);
+            da[0] = ra[i][0]; da[1] = ra[i][1];
+            db[0] = make_double2((double)rb[i].x, (double)rb[i].y); db[1] = make_double2((double)rb[i].z, (double)rb[i].w);
+        }
+        __syncthreads();
+        if (k0 + F64_K < s.KL) load(k0 + F64_K);
+#pragma unroll
+        for (int k = 0; k < F64_K; k += 4) {
+            double av[4], bv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) { av[i] = sa[wm + i * 8 + g][k + q]; bv[i] = sb[wn + i * 8 + g][k + q]; }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_f64(acc[i][j], av[i], bv[j]);
+        }
+    }
+    const double scale = (double)(1.0f / sqrtf((float)s.qn));
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int jj = j0 + wn + j * 8 + 2 * q;
+            double *d = dsc + ((size_t)t * s.H + h0 + wm + i * 8 + g) * stride + jj;
+            if (jj < nvis) d[0] = acc[i][j][0] * scale;
+            if (jj + 1 < nvis) d[1] = acc[i][j][1] * scale;
+        }
+}
+
+// A warp per (query, head); `rows` of them.
+__global__ void __launch_bounds__(256) mla_prob_kernel(double *dsc, const int *nsel, int cached, int stride, int rows, MlaShape s)
+{
+    const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= rows) return;
+    const int t = r / s.H, ns = nsel ? nsel[t] : -1, nvis = ns < 0 ? pos_of(s, cached, t) + 1 : ns;
+    double *d = dsc + (size_t)r * stride;
+    double top = -INFINITY, z = 0.0;
+    for (int j = lane; j < nvis; j += 32) top = fmax(top, d[j]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) top = fmax(top, __shfl_xor_sync(0xffffffffu, top, o));
+    for (int j = lane; j < nvis; j += 32) {
+        const double e = exp((double)(float)d[j] - top);
+        d[j] = e;
+        z += e;
+    }
+    z = warp_sum(z);
+    for (int j = lane; j < nvis; j += 32) d[j] = d[j] / z;
+}
+
+// 64 heads x 64 latent columns over the positions [AT_SPAN blockIdx.y % spans ..) of a query; one stretch: the sums go to cb.
+__global__ void __launch_bounds__(F64_THREADS, 3) mla_sum_tile_kernel(float *cb, double *part, const double *dsc, const float *latent, const int *sel, const int *nsel,
+                                                                     int cached, int stride, int spans, MlaShape s)
+{
+    __shared__ __align__(16) double sa[AT_TILE][F64_KPITCH], sb[F64_K][F64_NPITCH];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q = lane & 3, wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
+    const int n0 = blockIdx.x * AT_TILE, h0 = (int)blockIdx.y / spans * AT_TILE, span = (int)blockIdx.y % spans, t = blockIdx.z, pos = pos_of(s, cached, t);
+    const int ns = nsel ? nsel[t] : -1, nvis = ns < 0 ? pos + 1 : ns;
+    const int j0 = span * AT_SPAN, j1 = min(nvis, j0 + AT_SPAN);
+    latent = static_cast<const float *>(seq_latent(latent, s, t));
+    const int *sl = sel ? sel + (size_t)t * (s.topk + s.KP) : nullptr;
+    const int lr = tid >> 3, lk = (tid & 7) * 4;                  // probabilities: eight lanes take 32 positions of a head
+    const int br = tid >> 4, bc = (tid & 15) * 4;                 // latents: 16 lanes take 64 columns of a position
+    const double *A = dsc + ((size_t)t * s.H + h0 + lr) * stride;
+    double ra[4][4];
+    float4 rb[4];
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const int jb = k0 + br + 8 * i;
+#pragma unroll
+            for (int k = 0; k < 4; k++) ra[i][k] = k0 + lk + k < j1 ? A[(size_t)(16 * i) * stride + k0 + lk + k] : 0.0;
+            rb[i] = jb < j1 ? *reinterpret_cast<const float4 *>(latent + (size_t)vis_row(sl, ns, jb) * s.KL + n0 + bc) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    };
+    double acc[4][4][2] = {};
+    if (j0 < j1) load(j0);
+    for (int k0 = j0; k0 < j1; k0 += F64_K) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            double2 *da = reinterpret_cast<double2 *>(&sa[lr + 16 * i][lk]), *db = reinterpret_cast<double2 *>(&sb[br + 8 * i][bc]);
+            da[0] = make_double2(ra[i][0], ra[i][1]); da[1] = make_double2(ra[i][2], ra[i][3]);
+            db[0] = make_double2((double)rb[i].x, (double)rb[i].y); db[1] = make_double2((double)rb[i].z, (double)rb[i].w);
+        }
+        __syncthreads();
+        if (k0 + F64_K < j1) load(k0 + F64_K);
+#pragma unroll
+        for (int k = 0; k < F64_K; k += 4) {
+            double av[4], bv[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) { av[i] = sa[wm + i * 8 + g][k + q]; bv[i] = sb[k + q][wn + i * 8 + g]; }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) mma_f64(acc[i][j], av[i], bv[j]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const size_t th = (size_t)t * s.H + h0 + wm + i * 8 + g;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int n = n0 + wn + j * 8 + 2 * q;
+            if (spans == 1) *reinterpret_cast<float2 *>(cb + th * s.KL + n) = make_float2((float)acc[i][j][0], (float)acc[i][j][1]);
+            else            *reinterpret_cast<double2 *>(part + (th * spans + span) * s.KL + n) = make_double2(acc[i][j][0], acc[i][j][1]);
+        }
+    }
+}
+
 void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent, const int *sel,
                 const int *nsel, double *dsc, double *part, double *stats, int *counters, int part_tokens, int T,
                 int cached, const MlaShape &s)
@@ -723,6 +963,23 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
     const int span = s.batch ? 1 : T;                                      // positions this call adds to a sequence
     const int nvis_max = cached + span < s.topk + s.KP ? cached + span : s.topk + s.KP;
     const int stride = s.topk + s.KP;
+    // few queries do not fill the GPU with tiles (layer, us, one head after the other / in tiles: 4 queries at 300 positions 228 / 240, 6 at
+    // 64 240 / 226, 3 at 1000 252 / 266, 3 at 2000 304 / 272, 12 at 8000 687 / 408)
+    const int spans = (nvis_max + AT_SPAN - 1) / AT_SPAN;
+    if ((T >= AT_MIN_T || (T >= 3 && nvis_max >= 1500)) && !s.latent_bf16 && s.H % AT_TILE == 0 && s.KL % AT_TILE == 0 && part && part_tokens > 0) {
+        const float *lat = static_cast<const float *>(latent);
+        G5B_LAUNCH(mla_score_tile_kernel, dim3((nvis_max + AT_TILE - 1) / AT_TILE, s.H / AT_TILE, T), F64_THREADS, 0, st, dsc, qa, lat, sel, nsel, cached, stride, s);
+        G5B_LAUNCH(mla_prob_kernel, (T * s.H + 7) / 8, 256, 0, st, dsc, nsel, cached, stride, T * s.H, s);
+        const int most = part_tokens * ((stride + WS_CHUNK - 1) / WS_CHUNK) / spans;      // queries whose stretches fit
+        for (int t0 = 0; t0 < T; t0 += spans > 1 ? most : T) {
+            const int n = spans > 1 && T - t0 > most ? most : T - t0;
+            const size_t d0 = (size_t)t0 * s.H;
+            G5B_LAUNCH(mla_sum_tile_kernel, dim3(s.KL / AT_TILE, s.H / AT_TILE * spans, n), F64_THREADS, 0, st, cb + d0 * s.KL, part, dsc + d0 * stride,
+                       s.batch ? lat + (size_t)t0 * s.lat_seq : lat, sel ? sel + (size_t)t0 * stride : nullptr, nsel ? nsel + t0 : nullptr, s.batch ? cached : cached + t0, stride, spans, s);
+            if (spans > 1) G5B_LAUNCH(mla_wsum_reduce_kernel, (n * s.H * s.KL + 255) / 256, 256, 0, st, cb + d0 * s.KL, part, spans, spans, n * s.H * s.KL, s.KL);
+        }
+        return;
+    }
     int blocks = (nvis_max + ATT_WARPS - 1) / ATT_WARPS;
     if (blocks > 32) blocks = 32;
     const bool fast_score = s.KL == 512 && s.H % SC_HEADS == 0 && stats && counters;
@@ -832,9 +1089,6 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *part, d
     {
         constexpr int PIECES = FL_KL / 8, PER = FL_POS * PIECES / FL_THREADS, QPER = 3 * FL_HEADS * PIECES / FL_THREADS;
         static_assert(FL_POS * PIECES % FL_THREADS == 0 && 3 * FL_HEADS * PIECES % FL_THREADS == 0, "pieces per thread");
-        auto copy = [](const void *dst, const void *src) {
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-        };
         int jrow[PER];
 #pragma unroll
         for (int k = 0; k < PER; k++) {
@@ -845,15 +1099,15 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *part, d
 #pragma unroll
         for (int k = 0; k < QPER; k++) {
             const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES;
-            copy(qs + fl_at((row % 3) * FL_HEADS + row / 3, piece), qt + (size_t)row * FL_KL + piece * 8);
+            cp_async16(qs + fl_at((row % 3) * FL_HEADS + row / 3, piece), qt + (size_t)row * FL_KL + piece * 8);
         }
 #pragma unroll
         for (int k = 0; k < PER; k++) {
             const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES;
-            if (jrow[k] >= 0) copy(cs + fl_at(row, piece), lat + (size_t)jrow[k] * FL_KL + piece * 8);
+            if (jrow[k] >= 0) cp_async16(cs + fl_at(row, piece), lat + (size_t)jrow[k] * FL_KL + piece * 8);
             else              *reinterpret_cast<uint4 *>(cs + fl_at(row, piece)) = make_uint4(0u, 0u, 0u, 0u);
         }
-        asm volatile("cp.async.wait_all;" ::: "memory");
+        cp_async_wait();
     }
     __syncthreads();
 
