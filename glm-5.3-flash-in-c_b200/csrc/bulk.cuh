@@ -29,9 +29,19 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
                  : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
     return ok != 0;
 }
+// Whether the phase is over, without waiting for it: several barriers can be looked at together, where waiting for one after the
+// other takes each one's latency even when all are.
+__device__ __forceinline__ bool mbar_test(uint64_t *bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0;
+}
 // Bounded wait: false (and an error code in *err) when the barrier never completes.
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *err, int code)
 {
+#pragma unroll 1
     for (int i = 0; i < ST_WAIT_LIMIT; i++)
         if (mbar_try_wait(bar, parity)) return true;
     atomicExch(err, code);
@@ -46,6 +56,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, i
     bool ok = true;
     if ((threadIdx.x & 31) == 0) {
         ok = false;
+#pragma unroll 1
         for (int i = 0; i < ST_WAIT_LIMIT; i++) {
             if (mbar_try_wait(bar, parity)) { ok = true; break; }
             __nanosleep(20);
@@ -55,6 +66,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, i
     ok = __all_sync(0xffffffffu, ok);
     if (ok) {
         ok = false;
+#pragma unroll 1
         for (int i = 0; i < 1024 && !ok; i++) ok = mbar_try_wait(bar, parity);
         ok = __all_sync(0xffffffffu, ok);
     }

@@ -858,7 +858,6 @@ static int run_moe_seq_split(g5b_engine *e, Layer &w, const float *x, int n, flo
         const int m = (r1 - r0) * n, g0 = r0 * n;
         const bool last = gi == mine;
         const float *xg = all + (size_t)g0 * c.hidden;
-        e->plan.tile_shift = tc_tile_shift((long)m * s.K, s.n_local);
         router_plan(e->st, e->ridx, e->rw, e->rscore, xg, c.hidden, w.router.w, w.router.dt, w.bias, m, s, e->plan,
                     with_shared ? 1 : 0, e->counter, last ? me * n - g0 : 0, last ? n : 0);
         if (e->expert_path >= 1 && tc_moe_takes(e->tc, s, m)) {
@@ -905,7 +904,6 @@ static int run_moe(g5b_engine *e, Layer &w, const float *x, int n, float *out, i
             return 0;
         }
     }
-    e->plan.tile_shift = tc_tile_shift((long)n * s.K, s.n_local);
     router_plan(e->st, e->ridx, e->rw, e->rscore, x, c.hidden, w.router.w, w.router.dt, w.bias, n, s, e->plan,
                 shared_in_plan ? 1 : 0, e->counter, 0, -1, e->rdots);
     prof_mark(e, 1);
@@ -1942,7 +1940,6 @@ extern "C" int g5b_debug_moe_rows(g5b_engine *e, int layer, const float *x, int 
     float *xd = st.in(x, (size_t)T * c.hidden);
     if (!xd) return fail("out of device memory");
     CU(cudaMemsetAsync(e->contrib, 0, n * 4, e->st));
-    e->plan.tile_shift = tc_tile_shift((long)T * s.K, s.n_local);
     router_plan(e->st, e->ridx, e->rw, e->rscore, xd, c.hidden, w.router.w, w.router.dt, w.bias, T, s, e->plan, shared, e->counter, 0, -1, e->rdots);
     if (e->expert_path >= 1 && tc_moe_takes(e->tc, s, T)) {
         if (tc_moe_run(e->tc, e->st, e->contrib, e->act, e->xterms, e->xinv, xd, c.hidden, expert_slab(e, w), e->plan, T, s))

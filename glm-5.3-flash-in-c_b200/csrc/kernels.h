@@ -69,12 +69,7 @@ inline void gemv(cudaStream_t st, const DMat &m, const float *x, int ldx, float 
 // FP8 block-scaled (128 x 128 blocks) and BF16 matrices times 2 positions or more on tcgen05 tensor
 // cores, weights streamed once by TMA; activations as exact 16-bit term sums. Matrices of one format and
 // width go out in one launch. err: where a bounded wait that ran out is recorded (tc_gemm_recover after it).
-// Rows of one expert that a weight tile is multiplied with at once, at most, for `pairs` rows over `experts` experts. A tile's
-// terms take shared memory from the weights in flight: stages for 16 rows leave four of weights, for 32 three. With few rows per
-// expert hardly any expert has more than 16 (gate/up and down of 288 experts top-8, tiles of 32 and of 16 rows: 64 tokens
-// 689 and 590 us, 120 tokens 800 and 753); then the second pass over the weights of those that do costs more (150 tokens, 4.2
-// rows per expert on average: 843 and 831; 200 tokens: 966 and 998).
-inline int tc_tile_shift(long pairs, int experts) { return pairs <= 4l * experts ? 4 : 5; }   // log2: tiles are counted by every role
+constexpr int TC_TILE_SHIFT = 5;     // log2 of the rows of one expert that a weight tile is multiplied with at once, at most (every role counts tiles)
 struct TcGemm;
 TcGemm *tc_gemm_create(int max_c, int max_ec, int max_t, int *err);      // widest input, that of an expert, most positions
 void tc_gemm_free(TcGemm *g);
@@ -146,10 +141,9 @@ struct MoePlan {          // device arrays describing which expert multiplies wh
     int *slot_cnt;        // [max_slots] pairs of the slot
     int *pair_tok;        // [max_pairs] activation row of the pair
     int *pair_dst;        // [max_pairs] row of the contribution buffer the pair writes
-    int *slot_tile0;      // [max_slots + 1] first token tile of the slot (tiles of at most 1 << tile_shift pairs)
+    int *slot_tile0;      // [max_slots + 1] first token tile of the slot (tiles of at most 1 << TC_TILE_SHIFT pairs)
     int *n_pairs;         // [1] pairs of all slots
     int  max_slots, max_pairs;
-    int  tile_shift;      // of the call's tokens (tc_tile_shift)
 };
 struct MoeShape {
     int E, I, NE, K, br, bc, dt;       // dt of expert matrices

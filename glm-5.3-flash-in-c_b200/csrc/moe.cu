@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     int pairs = 0, slots = 0, tiles = 0;
     for (int k = 0; k < per; k++) {
         const int le = tid * per + k;
-        if (le < a.n_local && cnt[le]) { pairs += cnt[le]; slots++; tiles += (cnt[le] + (1 << a.p.tile_shift) - 1) >> a.p.tile_shift; }
+        if (le < a.n_local && cnt[le]) { pairs += cnt[le]; slots++; tiles += (cnt[le] + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT; }
     }
     psum[tid] = pairs; ssum[tid] = slots; tsum[tid] = tiles;
     __syncthreads();
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
         if (cnt[le]) {
             a.p.slot_expert[sbase] = le; a.p.slot_off[sbase] = pbase; a.p.slot_cnt[sbase] = cnt[le];
             a.p.slot_tile0[sbase] = tbase;
-            pbase += cnt[le]; sbase++; tbase += (cnt[le] + (1 << a.p.tile_shift) - 1) >> a.p.tile_shift;
+            pbase += cnt[le]; sbase++; tbase += (cnt[le] + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT;
         }
     }
     __syncthreads();
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     }
     if (tid == 0) {
         a.p.slot_tile0[total_slots] = total_tiles;
-        if (shared) a.p.slot_tile0[total_slots + 1] = total_tiles + ((a.sh_n + (1 << a.p.tile_shift) - 1) >> a.p.tile_shift);
+        if (shared) a.p.slot_tile0[total_slots + 1] = total_tiles + ((a.sh_n + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT);
         *a.p.n_slots = total_slots + (shared ? 1 : 0);
         *a.p.n_pairs = total_pairs + (shared ? a.sh_n : 0);
     }
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, 
     }
     __syncthreads();
     const int mine = tid < n_local ? cnt[tid] : 0;            // one expert per thread (at most G5B_MAX_EXPERTS of them)
-    int v[3] = {mine, mine > 0, (mine + (1 << p.tile_shift) - 1) >> p.tile_shift}, own[3];
+    int v[3] = {mine, mine > 0, (mine + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT}, own[3];
     for (int k = 0; k < 3; k++) {
         own[k] = v[k];
         for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v[k], o); if (lane >= o) v[k] += u; }
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, 
     if (tid == 0) {
         if (with_shared) { p.slot_expert[total[1]] = n_local; p.slot_off[total[1]] = total[0]; p.slot_cnt[total[1]] = T; }
         p.slot_tile0[total[1]] = total[2];
-        if (with_shared) p.slot_tile0[total[1] + 1] = total[2] + ((T + (1 << p.tile_shift) - 1) >> p.tile_shift);
+        if (with_shared) p.slot_tile0[total[1] + 1] = total[2] + ((T + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT);
         *p.n_slots = total[1] + (with_shared ? 1 : 0);
         *p.n_pairs = total[0] + (with_shared ? T : 0);
     }

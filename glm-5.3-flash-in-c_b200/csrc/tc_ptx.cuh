@@ -121,6 +121,7 @@ __device__ __forceinline__ uint32_t tc_idesc(int fmt, int n)
 // vote took 180 cycles more per wait.)
 __device__ __forceinline__ bool mbar_wait_all(uint64_t *bar, uint32_t parity, int *err, int code)
 {
+#pragma unroll 1
     for (int i = 0; i < ST_WAIT_LIMIT; i++)
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     if ((threadIdx.x & 31) == 0) atomicExch(err, code);
