@@ -70,6 +70,18 @@ __device__ __forceinline__ double bf16_to_f64(uint32_t h)
     return (double)bf16_to_f32((uint16_t)h);                      // zero, subnormal, infinite, NaN
 }
 
+// A BF16's bits (the upper half of u) put where a double has them: its value times 2^-896, zero and subnormal ones too. Two instructions,
+// where the exponent's own bias takes eight; a sum of such products is scaled back at the end. Sums lose nothing to underflow
+// before 2^-52 of terms whose BF16 factor is above 2^-110. Infinities and NaN have no place among them (bf16_special).
+constexpr double BF16_BITS_SCALE = 0x1p896;
+__device__ __forceinline__ double bf16_bits_f64(uint32_t u)
+{
+    double d;
+    asm volatile("{\n\t.reg .b32 t;\n\tshr.s32 t, %1, 3;\n\tand.b32 t, t, 0x8fffe000;\n\tmov.b64 %0, {0, t};\n\t}" : "=d"(d) : "r"(u));
+    return d;
+}
+__device__ __forceinline__ uint32_t bf16_special(uint32_t two) { return ((two & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+
 // K_ROWS: B's rows run along n (element (k, n) at B[k * ldb + n], N a multiple of 8); otherwise along k (B[n * ldb + k]).
 // A CTA of four warps takes 8 TM rows of A and 64 columns: TM = 8: two by two warps of 32 x 32 each, otherwise a warp has 16
 // of the columns.

@@ -541,6 +541,218 @@ __global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCC_THREADS) 
     cluster_wait();
 }
 
+// ---- the same site for one position and four streams, what a decode step runs twice per layer: a chain of latencies.
+// In the kernel above (28,600 cycles from its first instruction to its last, cold) the mixer product took 9800 of them - ten FP32
+// instructions a term - and the pending expansion 4400, most of them the way of y, post and comb from L2, one after the other. Here
+// everything that comes from memory is asked for at once: the mixer rows and norm weights before the wait for the kernel in front, the
+// rest after it; streams become doubles once, in shared memory; and the products are FP64 FMA (64 per clock and SM) whose BF16 factor is
+// its bits put where a double has them, two instructions and a value 2^896 times too small (bf16_bits_f64). 20,500 cycles cold; under ncu
+// 16.6 -> 12.5 us, one token of eight layers 1617 -> 1550 us. What is left: one round trip to memory, two cluster barriers, the Sinkhorn chain.
+constexpr int HCO_M = 4, HCO_MIX = (2 + HCO_M) * HCO_M;
+static size_t hco_smem(int W) { return (size_t)HCO_M * 4 * (W / 8 + 1) * sizeof(double2) + (size_t)HCO_MIX * HCO_M * W * 2; }
+
+__global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCC_THREADS, 1) hc_pre_one_kernel(const HcFused a)
+{
+    // piece p's elements 2 e2, 2 e2 + 1 of stream i: double2 at [i][e2][p], so that lanes with consecutive pieces read side by side
+    extern __shared__ __align__(16) double2 hd[];
+    __shared__ float xs[HCC_MAX_W];                     // this CTA's columns of the collapsed vector
+    __shared__ double red[HCC_WARPS], mine[HCC_SPLITS][HCO_MIX + 1], dots[HCO_MIX + 1], pre[HCO_M], mine_s2;
+    __shared__ float mx[HCO_MIX];
+    constexpr int M = HCO_M, MM = M * M, MIX = HCO_MIX;
+    pdl_trigger();
+    const int t = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t rank = cluster_cta_rank();
+    const int E = a.E, ME = M * E, W = E / HCC_CTAS, d0 = (int)rank * W, per = W / 8, pitch = per + 1;
+    float *ht = a.h + (size_t)t * ME + d0;
+    const double eps = (double)a.hc_eps;
+    auto at = [&](int i, int d) -> double & { return reinterpret_cast<double *>(hd + (i * 4 + ((d & 7) >> 1)) * pitch + (d >> 3))[d & 1]; };
+
+    // warp (q, b): mixer rows b, b + 8, b + 16, every HCC_SPLITS-th group of 32 pieces of each
+    const int q = warp / HCC_ROW_WARPS, b = warp % HCC_ROW_WARPS, pieces = M * per;
+    uint4 *wm = reinterpret_cast<uint4 *>(hd + M * 4 * pitch);   // [24][pieces]: on their way past the registers
+#pragma unroll 1
+    for (int p = lane + 32 * q; p < pieces; p += 32 * HCC_SPLITS)
+#pragma unroll
+        for (int r = 0; r < 3; r++) cp_async16(wm + (b + 8 * r) * pieces + p, a.fn + (size_t)(b + 8 * r) * ME + (size_t)(p / per) * E + d0 + (p % per) * 8);
+    pdl_wait();                  // the streams and y come from earlier kernels; the mixer rows do not
+
+    double sq = 0.0;
+    {
+        float cb[MM], po[M];
+        if (a.y) {
+#pragma unroll
+            for (int i = 0; i < MM; i++) cb[i] = __ldcg(a.comb + (size_t)t * MM + i);
+#pragma unroll
+            for (int i = 0; i < M; i++) po[i] = __ldcg(a.post + (size_t)t * M + i);
+        }
+#pragma unroll 1
+        for (int d = tid; d < W; d += HCC_THREADS) {
+            float hv[M];
+#pragma unroll
+            for (int i = 0; i < M; i++) hv[i] = __ldcg(ht + (size_t)i * E + d);
+            if (a.y) {
+                // the pending hc_post of the previous site: h'[j][d] = post[j] y[d] + sum_i comb[i][j] h[i][d] (src/core/glm53f_ops.c:612-625)
+                const double y = (double)__ldcg(a.y + (size_t)t * E + d0 + d);
+                double h[M];
+#pragma unroll
+                for (int i = 0; i < M; i++) h[i] = (double)hv[i];
+#pragma unroll
+                for (int j = 0; j < M; j++) {
+                    double v = (double)po[j] * y;
+#pragma unroll
+                    for (int i = 0; i < M; i++) v = fma((double)cb[i * M + j], h[i], v);
+                    hv[j] = (float)v;
+                    ht[(size_t)j * E + d] = hv[j];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < M; i++) {
+                const double h = (double)hv[i];
+                at(i, d) = h;
+                sq = fma(h, h, sq);
+            }
+        }
+    }
+    sq = warp_sum(sq);
+    if (lane == 0) red[warp] = sq;
+    cp_async_wait();
+    __syncthreads();
+
+    // ---- mixer rows
+    {
+        double acc[3] = {};
+        uint32_t special = 0;                            // an infinity or NaN among this lane's mixer elements: no place among the scaled ones
+        auto products = [&](auto widen) {
+#pragma unroll 1
+            for (int p = lane + 32 * q; p < pieces; p += 32 * HCC_SPLITS) {    // (rolled: this code runs from a cold instruction cache)
+                const double2 *h = hd + (p / per) * 4 * pitch + p % per;
+                uint4 wv[3];
+#pragma unroll
+                for (int r = 0; r < 3; r++) wv[r] = wm[(b + 8 * r) * pieces + p];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const double2 v = h[e * pitch];
+#pragma unroll
+                    for (int r = 0; r < 3; r++) {
+                        const uint32_t u = e == 0 ? wv[r].x : e == 1 ? wv[r].y : e == 2 ? wv[r].z : wv[r].w;
+                        special |= bf16_special(u);
+                        acc[r] = fma(widen(u << 16), v.x, acc[r]);
+                        acc[r] = fma(widen(u), v.y, acc[r]);
+                    }
+                }
+            }
+        };
+        products([](uint32_t u) { return bf16_bits_f64(u); });
+#pragma unroll
+        for (int r = 0; r < 3; r++) acc[r] *= BF16_BITS_SCALE;
+        if (__any_sync(0xffffffffu, special)) {
+            acc[0] = acc[1] = acc[2] = 0.0;
+            products([](uint32_t u) { return (double)__uint_as_float(u & 0xffff0000u); });
+        }
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            acc[r] = warp_sum(acc[r]);
+            if (lane == 0) mine[q][b + 8 * r] = acc[r];
+        }
+        if (tid == 0) {
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < HCC_WARPS; w++) s += red[w];
+            mine[0][MIX] = s;
+        }
+    }
+    __syncthreads();
+    cluster_arrive();
+    cluster_wait();
+
+    // ---- every CTA: the token's sums in CTA order, the norm factor, the gates
+    if (tid <= MIX) {
+        double part[HCC_CTAS][HCC_SPLITS];
+#pragma unroll
+        for (uint32_t r = 0; r < HCC_CTAS; r++)
+#pragma unroll
+            for (int k = 0; k < HCC_SPLITS; k++) part[r][k] = k == 0 || tid < MIX ? ld_cluster_f64(&mine[k][tid], r) : 0.0;
+        double s = 0.0;
+#pragma unroll
+        for (uint32_t r = 0; r < HCC_CTAS; r++) {
+            double v = part[r][0];
+#pragma unroll
+            for (int k = 1; k < HCC_SPLITS; k++) v += part[r][k];
+            s += v;
+        }
+        dots[tid] = s;
+    }
+    __syncthreads();
+    if (tid < MIX) mx[tid] = (float)(dots[tid] * (double)(float)rsqrt_newton(dots[MIX] / (double)ME + (double)a.rms_eps));
+    __syncthreads();
+    if (warp == 0) {
+        cluster_arrive();                                // nothing of this warp goes into sum x^2
+        if (rank == 0) {
+            // row softmax + eps, then column / row normalisations (src/core/glm53f_ops.c:577-598): a
+            // lane per matrix element, the row's / column's members gathered with shuffles
+            const int el = lane < MM ? lane : 0, i = el / M, j = el % M;
+            const int k = 2 * M + el;
+            const double l = (double)mul_add_unfused(mx[k], a.scale[2], a.base[k]);
+            double top = -INFINITY;
+#pragma unroll
+            for (int jj = 0; jj < M; jj++) top = fmax(top, __shfl_sync(0xffffffffu, l, i * M + jj));
+            const double ex = exp(l - top);
+            double z = 0.0;
+#pragma unroll
+            for (int jj = 0; jj < M; jj++) z += __shfl_sync(0xffffffffu, ex, i * M + jj);
+            const double v = sinkhorn_passes<M>(ex / z + eps, M, i, j, 2 * a.iters - 1, eps);
+            if (lane < MM) a.comb[(size_t)t * MM + lane] = (float)v;
+            __syncwarp();
+        }
+        cluster_wait();
+    } else {
+        // x[d] = sum_i pre[i] * h[i][d] in FP64 (src/core/glm53f_ops.c:603-607) for this CTA's columns
+        constexpr int NW = HCC_THREADS - 32;
+        const int wt = tid - 32;
+        if (wt < M) {
+            pre[wt] = (double)sigmoid_host(mul_add_unfused(mx[wt], a.scale[0], a.base[wt])) + eps;
+            if (rank == 0) a.post[(size_t)t * M + wt] = __fmul_rn(2.0f, sigmoid_host(mul_add_unfused(mx[M + wt], a.scale[1], a.base[M + wt])));
+        }
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(NW) : "memory");     // `pre` comes from threads of these warps
+        double s2 = 0.0;
+#pragma unroll 1
+        for (int d = wt; d < W; d += NW) {
+            double v = 0.0;
+#pragma unroll
+            for (int i = 0; i < M; i++) v += pre[i] * at(i, d);
+            const float xv = (float)v;
+            xs[d] = xv;
+            s2 += (double)xv * (double)xv;
+        }
+        s2 = warp_sum(s2);
+        if (lane == 0) red[warp] = s2;
+        asm volatile("bar.sync 1, %0;" ::"n"(NW) : "memory");
+        if (wt == 0) {
+            double v = 0.0;
+#pragma unroll
+            for (int w = 1; w < HCC_WARPS; w++) v += red[w];
+            mine_s2 = v;
+        }
+        __syncwarp();
+        cluster_arrive();
+        const float nw = wt < W ? a.norm_w[d0 + wt] : 0.f;
+        cluster_wait();
+        // ---- the sub-block's input: RMSNorm(x) * w (glm53f_rmsnorm, src/core/glm53f_ops.c:473-480)
+        double part[HCC_CTAS], tot = 0.0;
+#pragma unroll
+        for (uint32_t r = 0; r < HCC_CTAS; r++) part[r] = ld_cluster_f64(&mine_s2, r);
+#pragma unroll
+        for (uint32_t r = 0; r < HCC_CTAS; r++) tot += part[r];
+        const float f = (float)rsqrt_newton(tot / (double)E + (double)a.rms_eps);
+#pragma unroll 1
+        for (int d = wt; d < W; d += NW) a.xn[(size_t)t * E + d0 + d] = __fmul_rn(d == wt ? nw : a.norm_w[d0 + d], __fmul_rn(xs[d], f));
+    }
+    // no CTA leaves while another may still read its shared memory
+    cluster_arrive();
+    cluster_wait();
+}
+
 // ---- the same site for several positions (four streams): a cluster takes eight positions at once.
 // A cluster per position multiplies the mixer rows, which every position shares, position by position, with sums like
 // FP64's made of ten FP32 instructions per term (acc2.cuh): 45 us for 64 positions, and one CTA per position 442 us for 2048. With
@@ -644,9 +856,6 @@ __global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCG_THREADS, 
     {
         double acc[2][3][2] = {}, sq[4] = {};                    // (several sums each: a product waits for the one before it in its sum)
         uint32_t special = 0;                                    // an infinity or NaN among this lane's mixer elements
-        // A BF16's bits put where a double has them are its value times 2^-896 (zero and subnormal ones too): two instructions,
-        // where the exponent's own bias takes eight. The sums are scaled back at the end. Sums of such small numbers lose
-        // nothing to underflow before 2^-52 of mixer elements below 2^-110.
         auto multiply = [&](const uint4 (&wv)[3], int blk, auto widen) {
             const int c = (blk % per) * 32 + q * 8;
             float hv[8];
@@ -689,10 +898,10 @@ __global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCG_THREADS, 
             for (int m = 0; m < 3; m++) {
                 const uint32_t u[4] = {wv[m].x, wv[m].y, wv[m].z, wv[m].w};
 #pragma unroll
-                for (int k = 0; k < 4; k++) special |= ((u[k] & 0x7f807f80u) + 0x00800080u) & 0x80008000u;
+                for (int k = 0; k < 4; k++) special |= bf16_special(u[k]);
             }
             multiply(wv, blk, [](double &d, uint32_t u) {
-                asm volatile("{\n\t.reg .b32 t;\n\tshr.s32 t, %1, 3;\n\tand.b32 t, t, 0x8fffe000;\n\tmov.b64 %0, {0, t};\n\t}" : "=d"(d) : "r"(u));
+                d = bf16_bits_f64(u);
             });
             load_rows(wv, blk + 2 * HCG_WARPS);
         };
@@ -701,11 +910,10 @@ __global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCG_THREADS, 
             step(wn[0], blk);
             if (blk + HCG_WARPS < blocks) step(wn[1], blk + HCG_WARPS);
         }
-        const double scale = __hiloint2double((896 + 1023) << 20, 0);
 #pragma unroll
         for (int m = 0; m < 3; m++)
 #pragma unroll
-            for (int i = 0; i < 2; i++) acc[0][m][i] = (acc[0][m][i] + acc[1][m][i]) * scale;
+            for (int i = 0; i < 2; i++) acc[0][m][i] = (acc[0][m][i] + acc[1][m][i]) * BF16_BITS_SCALE;
         if (__any_sync(0xffffffffu, special)) {
             // those have no place among the scaled ones: the warp's products once more, element by element
             sq[0] = sq[1] = sq[2] = sq[3] = 0.0;
@@ -866,6 +1074,14 @@ void hc_pre_fused(cudaStream_t st, float *xn, float *post, float *comb, float *h
         static SmemGrant grant;
         if (dev_opt_in_smem((const void *)hc_pre_group_kernel, smem + (20 << 10), grant)) {
             G5B_LAUNCH(hc_pre_group_kernel, dim3(HCC_CTAS, (T + HCG_POS - 1) / HCG_POS), HCG_THREADS, smem, st, a, T);
+            return;
+        }
+    }
+    if (M == HCO_M && hc_pre_cluster_takes(M, E)) {
+        const size_t smem = hco_smem(E / HCC_CTAS);
+        static SmemGrant grant;
+        if (dev_opt_in_smem((const void *)hc_pre_one_kernel, smem + (8 << 10), grant)) {
+            G5B_LAUNCH_PDL(hc_pre_one_kernel, dim3(HCC_CTAS, T), dim3(HCC_THREADS), smem, st, a);
             return;
         }
     }

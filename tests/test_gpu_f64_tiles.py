@@ -30,13 +30,14 @@ def test_mixing_sites_in_groups_of_eight(gpu_lib, binding, hidden, T):
     eng.close(); orc.close()
 
 
-def test_mixing_sites_with_extreme_mixer_elements(gpu_lib, binding):
-    """Infinite elements (no place among the scaled ones), the smallest subnormal, zeros and the largest finite one:
-    positions in groups give what the CPU path's FP64 sums give."""
+@pytest.mark.parametrize("T", [1, 16])
+def test_mixing_sites_with_extreme_mixer_elements(gpu_lib, binding, T):
+    """Infinite elements (no place among the scaled ones), the smallest subnormal, zeros and the largest finite one, one position
+    and groups of eight: what the CPU path's FP64 sums give."""
     c = _config()
     spec = synth.Spec(c, [0, 0], [1, 1], with_head=True)
     tensors = synth.make_model(spec, seed=23, recipe="spread")
-    h = np.abs(np.random.default_rng(4).standard_normal((16, 4, c.hidden))).astype(np.float32)
+    h = np.abs(np.random.default_rng(4).standard_normal((T, 4, c.hidden))).astype(np.float32)
     for values in ((0x0001, 0x8001, 0x0000, 0x8000, 0x0080), (0x3000, 0x7f7f, 0x0001, 0xb000, 0x0000), (0x7f80, 0x0001, 0x3f80, 0x0000, 0x3f80)):
         arr, dt, sc = tensors["layers.0.hc_attn_fn"]
         arr = arr.copy()
@@ -56,8 +57,9 @@ def test_router_of_several_tokens(gpu_lib, binding, n_experts):
     rng = np.random.default_rng(n_experts)
     for T in (16, 17, 32, 33, 64, 65, 130):
         x = rng.standard_normal((T, c.hidden)).astype(np.float32)
-        (gi, gw), (wi, ww) = eng.op_router(0, x), orc.op_router(0, x)
-        assert np.array_equal(gi, wi) and common.rel_err(gw, ww) < 1e-6, T
+        eng.op_moe(0, x)                                    # (the router op itself takes the untiled path)
+        (gi, gw), (wi, ww) = eng.last_picks((T - 1) % 64 + 1), orc.op_router(0, x)
+        assert np.array_equal(gi, wi[-len(gi):]) and common.rel_err(gw, ww[-len(gi):]) < 1e-6, T
     eng.close(); orc.close()
 
 
