@@ -13,8 +13,11 @@ include/glm53f/glm53f.h:136-360.
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
+import math
 import os
+import threading
 
 import numpy as np
 
@@ -91,6 +94,8 @@ def lib() -> C.CDLL:
     L = C.CDLL(LIB_PATH, mode=C.RTLD_GLOBAL)
     _declare(L, "g5b", C.c_void_p)
     L.g5b_last_error.restype = C.c_char_p
+    L.g5b_host_alloc.restype, L.g5b_host_alloc.argtypes = C.c_void_p, [C.c_size_t]
+    L.g5b_host_free.restype, L.g5b_host_free.argtypes = None, [C.c_void_p]
     L.g5b_engine_create.restype = C.c_void_p
     L.g5b_engine_create.argtypes = [C.POINTER(Config), C.c_char_p, C.c_char_p, C.c_int, C.c_int, C.c_int, C.c_int]
     L.g5b_engine_fill_expert.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_uint64, C.c_void_p, C.c_void_p, C.c_void_p]
@@ -164,6 +169,77 @@ def _declare(L, prefix: str, handle):
     sig("mtp_hidden", [handle, C.c_int, C.c_int, f32p])
 
 
+class _Block:
+    """A piece of pinned memory that an array lies in (the array keeps it alive and gives it back)."""
+    __slots__ = ("pool", "ptr", "free", "__array_interface__")
+
+    def __init__(self, pool, ptr, free, shape):
+        self.pool, self.ptr, self.free = pool, ptr, free
+        self.__array_interface__ = {"data": (ptr, False), "shape": shape, "typestr": "<f4", "version": 3}
+
+    def __del__(self):
+        self.free.append(self.ptr)
+        if self.pool.closed:
+            self.pool.drain()
+
+
+class _ResultPool:
+    """Large results in pinned host memory: the device writes them in one transfer, 15 us for the 620 KB of a token's logits and
+    90 for seven tokens', where a fresh pageable array takes 150 and 640, most of them page faults. An array that is dropped gives its
+    memory to a later result. At most KEEP pieces of a size and LIMIT bytes in all, whoever holds them; beyond that, and below
+    SMALL, results are ordinary arrays. Threads may share it: a list of free pieces is a deque, whose append and pop are atomic."""
+    SMALL, KEEP, LIMIT = 128 << 10, 4, 256 << 20
+
+    def __init__(self, L):
+        self.L, self.closed, self.bytes = L, False, 0
+        self.free, self.made, self.lock = {}, {}, threading.Lock()
+
+    def _grow(self, size):
+        """One more piece of `size` bytes, if there may be one."""
+        with self.lock:
+            if self.closed or self.made.get(size, 0) >= self.KEEP or self.bytes + size > self.LIMIT:
+                return None
+            self.made[size] = self.made.get(size, 0) + 1
+            self.bytes += size
+        return self.L.g5b_host_alloc(size)
+
+    def array(self, shape):
+        n = 4 * math.prod(shape)
+        if n < self.SMALL:
+            return np.empty(shape, np.float32)
+        size = 1 << (n - 1).bit_length()
+        free = self.free.setdefault(size, collections.deque())
+        try:
+            ptr = free.pop()
+        except IndexError:
+            ptr = self._grow(size)
+        return np.asarray(_Block(self, ptr, free, shape)) if ptr else np.empty(shape, np.float32)
+
+    def reserve(self, n, count):
+        """`count` pieces for results of n bytes, ahead of the first call."""
+        if n >= self.SMALL:
+            size = 1 << (n - 1).bit_length()
+            free = self.free.setdefault(size, collections.deque())
+            for _ in range(count - len(free)):
+                ptr = self._grow(size)
+                if ptr:
+                    free.append(ptr)
+
+    def drain(self):
+        for free in list(self.free.values()):
+            try:
+                while True:
+                    self.L.g5b_host_free(free.pop())
+            except IndexError:
+                pass
+
+    def close(self):
+        """Give back what is free now; pieces that arrays still lie in follow as those are dropped."""
+        with self.lock:
+            self.closed = True
+        self.drain()
+
+
 def _f32(a) -> np.ndarray:
     return np.ascontiguousarray(a, dtype=np.float32)
 
@@ -174,6 +250,10 @@ class FlatModel:
     L = None
     prefix = ""
     model_word = "model"
+
+    def _result(self, *shape) -> np.ndarray:
+        """An uninitialised FP32 array for a call to fill."""
+        return np.empty(shape, np.float32)
 
     def _fn(self, name):
         return getattr(self.L, f"{self.prefix}_{name}")
@@ -203,7 +283,7 @@ class FlatModel:
     def forward(self, ids, want_logits=True, want_argmax=False):
         ids = np.ascontiguousarray(ids, dtype=np.int32)
         T = int(ids.size)
-        logits = np.zeros(self.cfg.vocab, np.float32) if want_logits else None
+        logits = self._result(self.cfg.vocab) if want_logits else None
         am = np.zeros(T, np.int32) if want_argmax else None
         rc = self._fn(f"{self.model_word}_forward")(
             self.handle, ids.ctypes.data, T,
@@ -278,13 +358,13 @@ class FlatModel:
         return h
 
     def op_kda(self, layer, x):
-        x = _f32(x); out = np.empty_like(x)
+        x = _f32(x); out = self._result(*x.shape)
         if self._fn("op_kda")(self.handle, layer, x.ctypes.data, x.shape[0], out.ctypes.data) != 0:
             self._err("op_kda")
         return out
 
     def op_mla(self, layer, x, cached):
-        x = _f32(x); out = np.empty_like(x)
+        x = _f32(x); out = self._result(*x.shape)
         sel = np.zeros(self.cfg.index_topk + self.cfg.index_kpool, np.int32)
         n = C.c_int(0)
         if self._fn("op_mla")(self.handle, layer, x.ctypes.data, x.shape[0], cached, out.ctypes.data,
@@ -300,14 +380,14 @@ class FlatModel:
         return idx, w
 
     def op_moe(self, layer, x, with_shared=True):
-        x = _f32(x); out = np.empty_like(x)
+        x = _f32(x); out = self._result(*x.shape)
         if self._fn("op_moe")(self.handle, layer, x.ctypes.data, x.shape[0], out.ctypes.data,
                               1 if with_shared else 0) != 0:
             self._err("op_moe")
         return out
 
     def op_mlp(self, layer, x):
-        x = _f32(x); out = np.empty_like(x)
+        x = _f32(x); out = self._result(*x.shape)
         if self._fn("op_mlp")(self.handle, layer, x.ctypes.data, x.shape[0], out.ctypes.data) != 0:
             self._err("op_mlp")
         return out
@@ -346,6 +426,20 @@ class Engine(FlatModel):
         if not self.handle:
             self._err("engine_create")
         self._rows = {}
+        self._options = {}
+        self._pool = _ResultPool(self.L)
+
+    def _result(self, *shape):
+        return self._pool.array(shape)
+
+    def finalize(self):
+        super().finalize()
+        # results of the calls that a program makes again and again: logits of one token and (a few sequences) of a batch
+        if not self._options.get("allow_partial"):
+            self._pool.reserve(4 * self.cfg.vocab, 2)
+            rows = 4 * self.cfg.vocab * self._options.get("sequences", 1)
+            if rows <= 16 << 20:
+                self._pool.reserve(rows, 2)
 
     def load(self, name, arr, dtype, scale=None):
         super().load(name, arr, dtype, scale)
@@ -354,6 +448,7 @@ class Engine(FlatModel):
     def set_option(self, name: str, value: int):
         if self.L.g5b_engine_set_option(self.handle, name.encode(), value) != 0:
             self._err(f"set_option({name})")
+        self._options[name] = value
 
     def fill_expert(self, layer, expert, seed, gate_s, up_s, down_s):
         g, u, d = _f32(gate_s), _f32(up_s), _f32(down_s)
@@ -404,7 +499,7 @@ class Engine(FlatModel):
         """One new token per sequence (option "sequences"): returns (logits [S][vocab] or None, argmax [S])."""
         ids = np.ascontiguousarray(ids, dtype=np.int32)
         S = ids.size
-        lg = np.zeros((S, self.cfg.vocab), np.float32) if want_logits else None
+        lg = self._result(S, self.cfg.vocab) if want_logits else None
         am = np.zeros(S, np.int32)
         if self.L.g5b_engine_decode_batch(self.handle, ids.ctypes.data, lg.ctypes.data if want_logits else None,
                                           am.ctypes.data) != 0:
@@ -465,6 +560,8 @@ class Engine(FlatModel):
             self._err("sync")
 
     def close(self):
+        if getattr(self, "_pool", None):
+            self._pool.close()
         if getattr(self, "handle", None):
             self.L.g5b_engine_free(self.handle)
             self.handle = None

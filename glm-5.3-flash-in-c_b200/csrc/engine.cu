@@ -1831,6 +1831,19 @@ static float *mapped_on_device(const void *p)
     return nullptr;
 }
 
+// Pinned, mapped host memory for results: a copy into it is one transfer, where ordinary memory goes through the driver's staging
+// and takes its page faults inside the copy.
+extern "C" void *g5b_host_alloc(size_t bytes)
+{
+    void *p = nullptr;
+    if (bytes == 0 || cudaHostAlloc(&p, bytes, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+    return p;
+}
+extern "C" void g5b_host_free(void *p)
+{
+    if (p && cudaFreeHost(p) != cudaSuccess) cudaGetLastError();
+}
+
 // Pinned, mapped staging rows for calls on ordinary host memory: as many as the largest call so far, at most one pass's.
 static bool ensure_io(g5b_engine *e, size_t rows)
 {

@@ -286,6 +286,10 @@ int g5b_engine_last_picks(g5b_engine *e, int T, int *idx, float *w);
  * memory is accepted; when `out` is pinned and mapped (cudaHostAlloc / cudaHostRegister) the layer's
  * last kernel writes it directly and the device-to-host copy is skipped. */
 int g5b_op_moe(g5b_engine *e, int layer, const float *x, int T, float *out, int with_shared);
+/* Pinned, mapped host memory, for results that are read on the host: the logits of g5b_engine_forward and
+ * g5b_engine_decode_batch and the rows of the layer calls then arrive in one transfer. NULL if there is none. */
+void *g5b_host_alloc(size_t bytes);
+void g5b_host_free(void *p);
 /* glm53f_mlp on a dense layer's gate/up/down (glm53f.h:352). */
 int g5b_op_mlp(g5b_engine *e, int layer, const float *x, int T, float *out);
 /* glm53f_decoder_layer (glm53f.h:358): h [T][M][hidden] in place at position `cached`. */
