@@ -1,5 +1,5 @@
-// f64_tile.cuh - out[z][t][n] = sum_k A[z][t][k] B[z](k, n) with FP64 sums, A in FP32 and B in BF16: the router's scores
-// and the absorption of W_k into the queries for several positions at once.
+// f64_tile.cuh - out[z][t][n] = sum_k A[z][t][k] B[z](k, n) with FP64 sums, A in FP32 and B in BF16: the router's scores,
+// the absorption of W_k into the queries and the value projection for several positions at once.
 //
 // The FP64 pipe bounds both: 64 FMA per clock and SM, as DFMA or as mma.sync.m8n8k4 (measured: 63 and 64), while a float
 // becomes a double at 16 per clock and SM. Threads that hold 4 x 4 sums read 64 bytes of shared memory for 16 products and
@@ -51,6 +51,7 @@ struct F64Tile {
     size_t za, zb, zo;            // elements between the problems of blockIdx.z (heads, or stretches of k)
     int T, N, K;                  // K: a multiple of 32, rows of A and B 16-byte aligned
     QueryOut q;                   // K_ROWS: the results are absorbed queries of head blockIdx.z
+    float *rounded;               // otherwise, instead of out if not null: the sums rounded to floats
 };
 constexpr int F64_N = 64, F64_K = 32, F64_THREADS = 128;
 // Rows of the blocks in shared memory, in doubles: 4 more than a multiple of 16, so that the 4 x 4 or 8 x 4 elements that a
@@ -157,7 +158,6 @@ __global__ void __launch_bounds__(F64_THREADS, 4) f64_tile_kernel(const F64Tile 
                 for (int j = 0; j < NT; j++) mma_f64(acc[i][j], av[i], bv[j]);
         }
     }
-    double *out = K_ROWS ? nullptr : p.out + (size_t)blockIdx.z * p.zo;
 #pragma unroll
     for (int i = 0; i < MT; i++) {
         const int t = t0 + wm + i * 8 + g;
@@ -167,7 +167,11 @@ __global__ void __launch_bounds__(F64_THREADS, 4) f64_tile_kernel(const F64Tile 
                 const int n = n0 + wn + j * 8 + 2 * q;        // (N is even)
                 if (n < p.N) {
                     if (K_ROWS) p.q.put2(t, blockIdx.z, n, acc[i][j][0], acc[i][j][1]);
-                    else        *reinterpret_cast<double2 *>(out + (size_t)t * p.ldo + n) = make_double2(acc[i][j][0], acc[i][j][1]);
+                    else {
+                        const size_t at = (size_t)blockIdx.z * p.zo + (size_t)t * p.ldo + n;
+                        if (p.rounded) *reinterpret_cast<float2 *>(p.rounded + at) = make_float2((float)acc[i][j][0], (float)acc[i][j][1]);
+                        else           *reinterpret_cast<double2 *>(p.out + at) = make_double2(acc[i][j][0], acc[i][j][1]);
+                    }
                 }
             }
     }

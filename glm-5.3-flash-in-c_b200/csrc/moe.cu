@@ -323,7 +323,7 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
         if (parts < 1) parts = 1;
         while (blocks % parts) parts--;                       // equal stretches
         per = s.E / parts;
-        const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per, {}};
+        const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per, {}, nullptr};
         f64_tile<false>(st, f, parts);
     }
     // (with the dot products there a token is one CTA's, which needs no counter: one launch selects for all of them. 2048 tokens:
