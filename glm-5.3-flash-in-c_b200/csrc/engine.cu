@@ -41,6 +41,7 @@ void set_last_error(const char *msg) { snprintf(g_err, sizeof g_err, "%s", msg);
 
 constexpr size_t EP_FLAG_BYTES = 1024;   // exchange region: the ranks' step words, then the row buffers
 constexpr int EP_HEAD_WORD0 = 64;        // words [64, 64 + 5 x 8): the vocabulary-split head's (value, index) slots of two parities and its arrival counters (up to 8 ranks)
+constexpr int MLA_STEP = 512;          // queries of a prompt that go through the tensor-core attention core together
 constexpr int MLA_PART_TOKENS = 4;     // tokens whose attention partial sums are held at once
 constexpr int CHUNK = 64;       // positions of a batch step, of a device op, of one pass of the attention core and the head
                                 // (the reference's MoE chunk, glm53f_ops.c:988)
@@ -122,6 +123,7 @@ struct g5b_engine {
                                                  // gather the ranks' tokens and send contribution rows home
     int *ep_arrive = nullptr;
     int pass = CHUNK;                            // positions one pass of a layer works on
+    int mla_step = 0;              // queries per launch of the tensor-core attention core
     int pick0 = 0;                               // first row of the most recent MoE pass's last CHUNK (g5b_engine_last_picks)
     int ep_wait_ms = 5000;                       // wall-clock limit of a wait for the other ranks (option "ep_wait_ms")
     bool dirty = false;                          // a call failed half-way: session state is undefined until reset
@@ -159,6 +161,7 @@ struct g5b_engine {
     double *hc_part = nullptr; int *hc_count = nullptr;  // fused mHC site: partial sums and per-token counters
     void *xterms = nullptr; float *xinv = nullptr;      // batched expert kernels: F16 terms of the activations
     int   *msel, *mnsel;
+    int   sel_row = 0;                           // the last call's last query in them
     double *rdots;                               // dot products of the router for many tokens
     float *rscore, *rw, *act, *contrib, *gu, *dact;
     int   *ridx;
@@ -729,7 +732,9 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
     }
     // (the ranks of an expert-parallel group exchange buffers of CHUNK positions)
     e->pass = e->ep_size > 1 ? CHUNK : e->cap <= PASS_MIN ? PASS_MIN : e->cap >= PASS_MAX ? PASS_MAX : (e->cap + CHUNK - 1) / CHUNK * CHUNK;
-    const size_t N = (size_t)e->pass, NA = CHUNK, E = c.hidden, M = c.hc_mult, MIX = (2 + M) * M;
+    // queries that the tensor-core attention core takes at a time: a prompt's 64 are 256 of its CTAs, fewer than fit the GPU
+    e->mla_step = e->latent_bf16 && e->cap <= 1 << 18 ? (e->pass < MLA_STEP ? e->pass : MLA_STEP) : CHUNK;
+    const size_t N = (size_t)e->pass, NA = CHUNK, NQ = e->mla_step > CHUNK ? e->mla_step : CHUNK, E = c.hidden, M = c.hc_mult, MIX = (2 + M) * M;
     const size_t P = (size_t)c.kda_heads * c.kda_head_dim, D = c.kda_head_dim;
     const size_t H = c.mla_heads, KL = c.kv_lora, stride = (size_t)c.index_topk + c.index_kpool;
     const size_t K = c.topk, I = c.moe_inter, SI = (size_t)c.moe_inter * c.n_shared;
@@ -746,9 +751,9 @@ extern "C" int g5b_engine_finalize(g5b_engine *e)
         walloc(e, &e->mgate, N * c.index_dim) || walloc(e, &e->mwp, N * c.index_heads) ||
         walloc(e, &e->mq, N * H * c.qk_nope) || walloc(e, &e->mqidx, N * (size_t)c.index_heads * c.index_dim) ||
         walloc(e, &e->mcb, N * H * KL) || walloc(e, &e->macc, N * H * c.v_head) ||
-        walloc(e, &e->mscore, NA * ((size_t)e->cap / c.index_kpool + 1)) || walloc(e, &e->minvq, N) ||
-        walloc(e, &e->mqa, NA * H * KL) || e->dalloc(&e->mqt, NA * H * 3 * KL * 2) || walloc(e, &e->mdsc, NA * H * stride) ||
-        walloc(e, &e->msel, NA * stride) || walloc(e, &e->mnsel, NA) ||
+        walloc(e, &e->mscore, NQ * ((size_t)e->cap / c.index_kpool + 1)) || walloc(e, &e->minvq, N) ||
+        walloc(e, &e->mqa, NA * H * KL) || e->dalloc(&e->mqt, NQ * H * 3 * KL * 2) || walloc(e, &e->mdsc, NA * H * stride) ||
+        walloc(e, &e->msel, NQ * stride) || walloc(e, &e->mnsel, NQ) ||
         walloc(e, &e->mstats, NA * H * 2) || walloc(e, &e->mcount, NA * H) ||
         walloc(e, &e->mpart, (size_t)MLA_PART_TOKENS * H * ((stride + 31) / 32) * KL)) return -1;
     e->mpart_bytes = (size_t)MLA_PART_TOKENS * H * ((stride + 31) / 32) * KL * sizeof(double);
@@ -1157,7 +1162,7 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
     GemvSeg b[2] = {make_seg(qb, e->mq_raw, c.q_lora, e->mq, Hl * c.qk_nope, e->minvq, w.q_a_norm),
                     make_seg(w.wq_b, e->mq_raw, c.q_lora, e->mqidx, c.index_heads * c.index_dim, e->minvq, w.q_a_norm)};
     if (proj_batch(e, b, 2, n, true)) return -1;
-    // The attention core takes CHUNK positions at a time.
+    // The attention core takes CHUNK positions at a time, on the tensor cores MLA_STEP.
     // The indexer (pool scores, top-k, expansion: two latency-bound kernels) and the absorption of
     // W_k into the query need nothing from each other: the absorption runs on the side stream
     // meanwhile and the main stream takes it back before the scores.
@@ -1165,10 +1170,12 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
     bool wide = n >= VOUT_TC_MIN_T && e->tc && e->tensor_gemm != 0 && e->mla_tensor;
     for (int h = 0; h < Hl && wide; h++)
         wide = tc_gemm_takes(e->tc, make_seg(row_slice(kvb, h * VR + s.qn, s.vh), e->mcb + (size_t)h * s.KL, Hl * s.KL, e->macc + (size_t)h * s.vh, Hl * s.vh), n);
-    for (int t0 = 0; t0 < n; t0 += CHUNK) {
+    const int step = flash && wide && e->mla_step > CHUNK ? e->mla_step : CHUNK;
+    for (int t0 = 0; t0 < n; t0 += step) {
         float *cb = e->mcb + (wide ? (size_t)t0 * Hl * s.KL : 0);
-        const int nt = n - t0 < CHUNK ? n - t0 : CHUNK, at = batch ? cached : cached + t0;
+        const int nt = n - t0 < step ? n - t0 : step, at = batch ? cached : cached + t0;
         const float *mq = e->mq + (size_t)t0 * Hl * c.qk_nope;
+        e->sel_row = nt - 1;
         bool forked = false, join = false;
         if (e->side && e->side_ev && e->side_done && cudaEventRecord(e->side_ev, e->st) == cudaSuccess &&
             cudaStreamWaitEvent(e->side, e->side_ev, 0) == cudaSuccess) {
@@ -2016,7 +2023,7 @@ extern "C" int g5b_op_mla(g5b_engine *e, int layer, const float *x, int T, int c
     }
     if (host_op(e, x, T, out, [&](const float *xd, int n, float *od, int t0) {
             if (run_mla(e, e->L[layer], xd, n, cached + t0, od)) return -1;
-            const int at = (n - 1) % CHUNK;
+            const int at = e->sel_row;
             if (n_sel_out && t0 + n == T) selection_out(e->st, e->io_sel_dev, e->mnsel + at, e->msel + (size_t)at * most);
             return 0;
         }, e->ep_size <= 1)) return -1;

@@ -1023,21 +1023,26 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
 // the 512 latent columns, and the weighted sum of the latent rows - are small GEMMs whose one
 // operand (the cache) is already exact in BF16. The other operand is split into three BF16 terms
 // (24 significant bits: the absorbed query after the 1/sqrt(d) scaling, the probabilities), so the
-// products are exact and only the FP32 accumulation of mma.sync rounds (about 1e-6 relative; the
+// products are exact and only the FP32 accumulation of mma.sync rounds (about 4e-7 relative; the
 // reference, src/core/glm53f_ops.c:879-911, accumulates in FP64 and rounds the score to float).
-// A CTA takes FL_POS visible positions and FL_HEADS heads of one query: it gathers the latent rows
-// into shared memory once (the DSA selection is a list of row numbers), multiplies scores, takes the
-// chunk's own maximum and exponentials, multiplies the weighted sum and leaves (max, sum, partial
-// rows) for the reduction kernel, which rescales the chunks to the common maximum the way a
-// two-pass softmax would have (the reference's max over all scores first, then the exponentials).
-// A CTA is a chain of phases - gather, scores, exponentials, weighted sum - so two of them share an SM: rows are kept
-// without padding (16-byte pieces of row r at place piece ^ (r & 7), which ldmatrix reads without conflicts) and scores
-// and probabilities take the place of the queries, 114,688 bytes in all. The queries arrive as terms. 64 sequences at 4096
-// positions: 116 us per launch before, 64 now.
-constexpr int FL_POS = 64, FL_HEADS = 16, FL_KL = 512, FL_PPITCH = FL_POS + 8;
-constexpr int FL_THREADS = 256;
-constexpr size_t FL_SMEM = (size_t)3 * FL_HEADS * FL_KL * 2 + (size_t)FL_POS * FL_KL * 2;
-static_assert((size_t)FL_HEADS * FL_POS * 4 + (size_t)3 * FL_HEADS * FL_PPITCH * 2 <= (size_t)3 * FL_HEADS * FL_KL * 2, "scores and probabilities fit where the queries were");
+// A CTA takes FL_HEADS heads of one query and a stretch of its visible positions, FL_POS of them at a time: it gathers the latent
+// rows into shared memory (the DSA selection is a list of row numbers), multiplies scores, takes exponentials, multiplies the weighted
+// sum and adds it to its own, in registers. A query's reference R for the exponents is its first chunk's maximum, and a later
+// one that exceeds it by 16 (the reference takes the maximum of all scores first; e^16 more is nothing to a float's range): so the sums
+// are hardly ever rescaled. Few queries are split
+// into stretches, which a second kernel puts together.
+// Bound by mma.sync (1024 products per clock and SM, measured: a quarter of the tcgen05 rate) and nearly as much by shared memory: per chunk of
+// 48 positions x 16 heads 2300 cycles of products, 2350 of ldmatrix and the rest. A CTA is a chain of phases, so two of them share an SM: rows are kept
+// without padding (16-byte pieces of row r at place piece ^ (r & 7), which ldmatrix reads without conflicts) and probabilities
+// take the place of the scores' parts, 113 KB in all. Scores are dealt out as two groups of positions x four quarters of the columns: all
+// warps at all 512 columns of eight positions each read the query's 48 KB eight times over.
+// Measured, with the reduction: 64 queries of 2051 positions 437 -> 256 us, a prompt of 2048 6.9 -> 3.2 ms a layer (a chunk of 64 positions per CTA, its
+// sums in memory, before); one query 15.6 -> 19.5. Against the FP64 core on the same cache 1.3e-6 -> 3.5e-7: fewer and better ordered
+// truncations of the tensor cores' sums.
+constexpr int FL_POS = 48, FL_HEADS = 16, FL_KL = 512, FL_PPITCH = FL_POS + 8, FL_SPITCH = FL_POS + 8;
+constexpr int FL_THREADS = 256, FL_KQ = 4;
+constexpr size_t FL_SMEM = (size_t)3 * FL_HEADS * FL_KL * 2 + (size_t)FL_POS * FL_KL * 2 + (size_t)FL_KQ * FL_HEADS * FL_SPITCH * 4;
+static_assert((size_t)3 * FL_HEADS * FL_PPITCH * 2 <= (size_t)FL_KQ * FL_HEADS * FL_SPITCH * 4, "probabilities fit where the scores' parts were");
 // element (row, 8 * piece) of rows of FL_KL 16-bit values
 __device__ __forceinline__ int fl_at(int row, int piece) { return row * FL_KL + ((piece ^ (row & 7)) << 3); }
 
@@ -1051,219 +1056,272 @@ __device__ __forceinline__ void ldsm_x2(uint32_t (&r)[2], const void *p)
     asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0, %1}, [%2];"
                  : "=r"(r[0]), "=r"(r[1]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
-__device__ __forceinline__ void ldsm_x2_trans(uint32_t (&r)[2], const void *p)
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t (&r)[4], const void *p)
 {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];"
-                 : "=r"(r[0]), "=r"(r[1]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
 }
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2])
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// part: [T][H][nchunks][KL] floats (unnormalised partial rows); cstat: [T][H][nchunks][2] doubles
-// (chunk maximum, sum of exponentials).
-__global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *part, double *cstat, const __nv_bfloat16 *qterms, const void *latent,
-                                                               const int *sel, const int *nsel, int cached, int nchunks, MlaShape s)
+// part: [T][H][splits][KL] floats (unnormalised rows of a stretch), cstat: [T][H][splits][2] doubles (its reference, its sum of exponentials);
+// one stretch: the finished rows go to cb. span: chunks per stretch.
+__global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, float *part, double *cstat, const __nv_bfloat16 *qterms, const void *latent,
+                                                               const int *sel, const int *nsel, int cached, int splits, int span, MlaShape s)
 {
     pdl_trigger();
     pdl_wait();
     extern __shared__ __align__(16) uint8_t fl_smem[];
+    __shared__ float s_scale[FL_HEADS];
+    __shared__ double s_z[FL_HEADS];
+    __shared__ int s_rows[FL_POS];                                 // cache rows of the next chunk to fetch
     __nv_bfloat16 *qs = reinterpret_cast<__nv_bfloat16 *>(fl_smem);                          // [3][16][512]
-    __nv_bfloat16 *cs = qs + 3 * FL_HEADS * FL_KL;                                          // [64][512]
-    float *ss = reinterpret_cast<float *>(fl_smem);                                         // [16][64], then
-    __nv_bfloat16 *ps = reinterpret_cast<__nv_bfloat16 *>(ss + FL_HEADS * FL_POS);          // [3][16][FL_PPITCH], over the queries
-    const int chunk = blockIdx.x, h0 = blockIdx.y * FL_HEADS, t = blockIdx.z, p = pos_of(s, cached, t);
+    __nv_bfloat16 *cs = qs + 3 * FL_HEADS * FL_KL;                                          // [48][512]
+    float *ss = reinterpret_cast<float *>(cs + FL_POS * FL_KL);                             // [4][16][FL_SPITCH], then
+    __nv_bfloat16 *ps = reinterpret_cast<__nv_bfloat16 *>(ss);                              // [3][16][FL_PPITCH]
+    const int split = blockIdx.x, h0 = blockIdx.y * FL_HEADS, t = blockIdx.z, p = pos_of(s, cached, t);
     const uint16_t *lat = static_cast<const uint16_t *>(seq_latent(latent, s, t));
     const int ns = nsel ? nsel[t] : -1;
     const int nvis = ns < 0 ? p + 1 : ns;
-    const int j0 = chunk * FL_POS;
-    if (j0 >= nvis) return;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+    const int first = split * span * FL_POS, end = min(nvis, first + span * FL_POS);
+    if (first >= nvis) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int *sl = sel ? sel + (size_t)t * (s.topk + s.KP) : nullptr;
 
-    // ---- the queries' terms of the 16 heads, and the chunk's latent rows; rows past the last visible position are zero so
-    // that nothing undefined enters a product (all of a thread's row numbers are requested first, then all of its pieces:
-    // one round trip for the selection list and one for everything else)
-    {
-        constexpr int PIECES = FL_KL / 8, PER = FL_POS * PIECES / FL_THREADS, QPER = 3 * FL_HEADS * PIECES / FL_THREADS;
-        static_assert(FL_POS * PIECES % FL_THREADS == 0 && 3 * FL_HEADS * PIECES % FL_THREADS == 0, "pieces per thread");
-        int jrow[PER];
+    // a chunk's rows; those past the last visible position are zero so that nothing undefined enters a product
+    constexpr int PIECES = FL_KL / 8, PER = FL_POS * PIECES / FL_THREADS, QPER = 3 * FL_HEADS * PIECES / FL_THREADS;
+    static_assert(FL_POS * PIECES % FL_THREADS == 0 && 3 * FL_HEADS * PIECES % FL_THREADS == 0, "pieces per thread");
+    auto row_of = [&](int jj) { return jj < end ? (ns < 0 ? jj : sl[jj]) : -1; };
+    auto gather = [&]() {
 #pragma unroll
         for (int k = 0; k < PER; k++) {
-            const int jj = j0 + (tid + k * FL_THREADS) / PIECES;
-            jrow[k] = jj < nvis ? (ns < 0 ? jj : sl[jj]) : -1;
+            const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES, j = s_rows[row];
+            if (j >= 0) cp_async16(cs + fl_at(row, piece), lat + (size_t)j * FL_KL + piece * 8);
+            else        *reinterpret_cast<uint4 *>(cs + fl_at(row, piece)) = make_uint4(0u, 0u, 0u, 0u);
         }
+    };
+    if (tid < FL_POS) s_rows[tid] = row_of(first + tid);
+    {
         const __nv_bfloat16 *qt = qterms + ((size_t)t * s.H + h0) * 3 * FL_KL;               // [head][term][512]
 #pragma unroll
         for (int k = 0; k < QPER; k++) {
             const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES;
             cp_async16(qs + fl_at((row % 3) * FL_HEADS + row / 3, piece), qt + (size_t)row * FL_KL + piece * 8);
         }
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-            const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES;
-            if (jrow[k] >= 0) cp_async16(cs + fl_at(row, piece), lat + (size_t)jrow[k] * FL_KL + piece * 8);
-            else              *reinterpret_cast<uint4 *>(cs + fl_at(row, piece)) = make_uint4(0u, 0u, 0u, 0u);
-        }
-        cp_async_wait();
     }
     __syncthreads();
+    gather();
 
-    // ---- scores: warp w takes positions 8w..8w+7 of the chunk, all 16 heads, all 512 columns
-    {
-        float c[4] = {0.f, 0.f, 0.f, 0.f};
-        const int brow = warp * 8 + (lane & 7), arow = (lane & 7) + 8 * ((lane >> 3) & 1);
-#pragma unroll 4
-        for (int k0 = 0; k0 < FL_KL; k0 += 16) {
-            uint32_t b[2];
-            ldsm_x2(b, cs + fl_at(brow, k0 / 8 + ((lane >> 3) & 1)));
+    const int pg = warp >> 2, kq = warp & 3;                        // scores: positions 24 pg .., columns 128 kq ..
+    const int row = 2 * warp + (lane >> 4), l16 = lane & 15;        // exponentials: this lane's head, positions l16, l16 + 16, l16 + 32
+    const int arow = (lane & 7) + 8 * ((lane >> 3) & 1), ahalf = lane >> 4;
+    float ref = -INFINITY;
+    double z = 0.0;
+    float sum[8][4];                                                // weighted sums: columns 64 warp + 8 n + 2 (lane % 4), heads lane / 4 and + 8
 #pragma unroll
-            for (int term = 0; term < 3; term++) {
-                uint32_t a[4];
-                ldsm_x4(a, qs + fl_at(term * FL_HEADS + arow, k0 / 8 + (lane >> 4)));
-                mma_bf16(c, a, b);
+    for (int n = 0; n < 8; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) sum[n][i] = 0.f;
+
+#pragma unroll 1
+    for (int j0 = first; j0 < end; j0 += FL_POS) {
+        cp_async_wait();
+        __syncthreads();
+        const int next = tid < FL_POS ? row_of(j0 + FL_POS + tid) : -1;   // (on its way while the scores are multiplied)
+        // ---- scores
+        {
+            float c[3][4];
+#pragma unroll
+            for (int n = 0; n < 3; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
+            const int b4 = pg * 24 + (lane & 7) + 8 * (lane >> 4), b2 = pg * 24 + 16 + (lane & 7), bhalf = (lane >> 3) & 1;
+#pragma unroll 2
+            for (int k = 0; k < 8; k++) {
+                const int piece = kq * 16 + k * 2;
+                uint32_t b[4], d[2];
+                ldsm_x4(b, cs + fl_at(b4, piece + bhalf));
+                ldsm_x2(d, cs + fl_at(b2, piece + bhalf));
+#pragma unroll
+                for (int term = 2; term >= 0; term--) {
+                    uint32_t a[4];
+                    ldsm_x4(a, qs + fl_at(term * FL_HEADS + arow, piece + ahalf));
+                    mma_bf16(c[0], a, b[0], b[1]);
+                    mma_bf16(c[1], a, b[2], b[3]);
+                    mma_bf16(c[2], a, d[0], d[1]);
+                }
+            }
+            float *o = ss + (kq * FL_HEADS + (lane >> 2)) * FL_SPITCH + pg * 24 + 2 * (lane & 3);
+#pragma unroll
+            for (int n = 0; n < 3; n++) {
+                *reinterpret_cast<float2 *>(o + 8 * n) = make_float2(c[n][0], c[n][1]);
+                *reinterpret_cast<float2 *>(o + 8 * FL_SPITCH + 8 * n) = make_float2(c[n][2], c[n][3]);
             }
         }
-        __syncthreads();                                     // the queries have been read: the scores go there
-        const int r = lane >> 2, col = warp * 8 + 2 * (lane & 3);
-        ss[r * FL_POS + col] = c[0]; ss[r * FL_POS + col + 1] = c[1];
-        ss[(r + 8) * FL_POS + col] = c[2]; ss[(r + 8) * FL_POS + col + 1] = c[3];
-    }
-    __syncthreads();
-
-    // ---- the chunk's maximum and exponentials: a warp takes two heads, a lane two positions
-    for (int hh = warp * 2; hh < warp * 2 + 2; hh++) {
-        const int ja = lane, jb = lane + 32;
-        const float sa = j0 + ja < nvis ? ss[hh * FL_POS + ja] : -INFINITY;
-        const float sb = j0 + jb < nvis ? ss[hh * FL_POS + jb] : -INFINITY;
-        float m = fmaxf(sa, sb);
+        if (tid < FL_POS) s_rows[tid] = next;
+        __syncthreads();
+        // ---- exponentials
+        float e[3], scale = 1.f;
+        {
+            float m = -INFINITY, v[3];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const double ea = j0 + ja < nvis ? exp((double)sa - (double)m) : 0.0;
-        const double eb = j0 + jb < nvis ? exp((double)sb - (double)m) : 0.0;
-        const double z = warp_sum(ea + eb);
-        __nv_bfloat16 a, b, d;
-        split3_bf16((float)ea, a, b, d);
-        ps[(0 * FL_HEADS + hh) * FL_PPITCH + ja] = a; ps[(1 * FL_HEADS + hh) * FL_PPITCH + ja] = b; ps[(2 * FL_HEADS + hh) * FL_PPITCH + ja] = d;
-        split3_bf16((float)eb, a, b, d);
-        ps[(0 * FL_HEADS + hh) * FL_PPITCH + jb] = a; ps[(1 * FL_HEADS + hh) * FL_PPITCH + jb] = b; ps[(2 * FL_HEADS + hh) * FL_PPITCH + jb] = d;
-        if (lane == 0) {
-            double *st = cstat + (((size_t)t * s.H + h0 + hh) * nchunks + chunk) * 2;
-            st[0] = (double)m;
+            for (int k = 0; k < 3; k++) {
+                const float *o = ss + row * FL_SPITCH + l16 + 16 * k;
+                const float x = __fadd_rn(__fadd_rn(o[0], o[FL_HEADS * FL_SPITCH]), __fadd_rn(o[2 * FL_HEADS * FL_SPITCH], o[3 * FL_HEADS * FL_SPITCH]));
+                v[k] = j0 + l16 + 16 * k < end ? x : -INFINITY;
+                m = fmaxf(m, v[k]);
+            }
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            if (!(m <= ref + 16.f)) {                               // (the first chunk, a score much larger, NaN)
+                const double f = exp((double)ref - (double)m);
+                scale = (float)f;
+                z *= f;
+                ref = m;
+            }
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                const double x = j0 + l16 + 16 * k < end ? exp((double)v[k] - (double)ref) : 0.0;
+                z += x;
+                e[k] = (float)x;
+            }
+            if (l16 == 0) s_scale[row] = scale;
+        }
+        __syncthreads();                                            // the scores have been read: probabilities go there
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            __nv_bfloat16 a, b, d;
+            split3_bf16(e[k], a, b, d);
+            __nv_bfloat16 *o = ps + row * FL_PPITCH + l16 + 16 * k;
+            o[0] = a; o[FL_HEADS * FL_PPITCH] = b; o[2 * FL_HEADS * FL_PPITCH] = d;
+        }
+        if (__syncthreads_or(scale != 1.f)) {
+            const float f0 = s_scale[lane >> 2], f1 = s_scale[(lane >> 2) + 8];
+#pragma unroll
+            for (int n = 0; n < 8; n++) { sum[n][0] *= f0; sum[n][1] *= f0; sum[n][2] *= f1; sum[n][3] *= f1; }
+        }
+        // ---- weighted sum of the rows: this warp's 64 columns for the 16 heads
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            float acc[4][4];
+#pragma unroll
+            for (int n = 0; n < 4; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
+            uint32_t b[FL_POS / 16][2][4];
+#pragma unroll
+            for (int k = 0; k < FL_POS / 16; k++)
+#pragma unroll
+                for (int n = 0; n < 2; n++) ldsm_x4_trans(b[k][n], cs + fl_at(k * 16 + (lane & 15), warp * 8 + half * 4 + n * 2 + (lane >> 4)));
+#pragma unroll
+            for (int term = 2; term >= 0; term--)                   // (the small terms first: the tensor cores truncate to the sum's last place)
+#pragma unroll
+                for (int k = 0; k < FL_POS / 16; k++) {
+                    uint32_t a[4];
+                    ldsm_x4(a, ps + (size_t)(term * FL_HEADS + arow) * FL_PPITCH + k * 16 + 8 * ahalf);
+#pragma unroll
+                    for (int n = 0; n < 2; n++) { mma_bf16(acc[2 * n], a, b[k][n][0], b[k][n][1]); mma_bf16(acc[2 * n + 1], a, b[k][n][2], b[k][n][3]); }
+                }
+#pragma unroll
+            for (int n = 0; n < 4; n++)
+#pragma unroll
+                for (int i = 0; i < 4; i++) sum[half * 4 + n][i] = __fadd_rn(sum[half * 4 + n][i], acc[n][i]);
+        }
+        __syncthreads();                                            // the rows have been read
+        if (j0 + FL_POS < end) gather();
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
+    if (l16 == 0) {
+        s_z[row] = z;
+        if (splits > 1) {
+            double *st = cstat + (((size_t)t * s.H + h0 + row) * splits + split) * 2;
+            st[0] = (double)ref;
             st[1] = z;
         }
     }
     __syncthreads();
-
-    // ---- weighted sum of the rows: warp w takes latent columns 64w..64w+63 for the 16 heads
-    {
-        float acc[8][4];
 #pragma unroll
-        for (int n = 0; n < 8; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
-        const __nv_bfloat16 *arow = ps + (size_t)((lane & 7) + 8 * ((lane >> 3) & 1)) * FL_PPITCH + 8 * (lane >> 4);
+    for (int i = 0; i < 4; i += 2) {
+        const int r = (lane >> 2) + 4 * i;
+        const double inv = splits > 1 ? 1.0 : 1.0 / s_z[r];
+        float *o = (splits > 1 ? part + (((size_t)t * s.H + h0 + r) * splits + split) * FL_KL : cb + ((size_t)t * s.H + h0 + r) * FL_KL) + warp * 64 + 2 * (lane & 3);
 #pragma unroll
-        for (int k0 = 0; k0 < FL_POS; k0 += 16) {
-            uint32_t a[3][4];
-#pragma unroll
-            for (int term = 0; term < 3; term++) ldsm_x4(a[term], arow + (size_t)term * FL_HEADS * FL_PPITCH + k0);
-#pragma unroll
-            for (int n = 0; n < 8; n++) {
-                uint32_t b[2];
-                ldsm_x2_trans(b, cs + fl_at(k0 + (lane & 15), warp * 8 + n));
-#pragma unroll
-                for (int term = 0; term < 3; term++) mma_bf16(acc[n], a[term], b);
-            }
-        }
-        const int r = lane >> 2;
-        float *o0 = part + (((size_t)t * s.H + h0 + r) * nchunks + chunk) * FL_KL + warp * 64 + 2 * (lane & 3);
-        float *o1 = part + (((size_t)t * s.H + h0 + r + 8) * nchunks + chunk) * FL_KL + warp * 64 + 2 * (lane & 3);
-#pragma unroll
-        for (int n = 0; n < 8; n++) {
-            *reinterpret_cast<float2 *>(o0 + n * 8) = make_float2(acc[n][0], acc[n][1]);
-            *reinterpret_cast<float2 *>(o1 + n * 8) = make_float2(acc[n][2], acc[n][3]);
-        }
+        for (int n = 0; n < 8; n++)
+            *reinterpret_cast<float2 *>(o + n * 8) = make_float2((float)((double)sum[n][i] * inv), (float)((double)sum[n][i + 1] * inv));
     }
 }
 
-// cb[t][h][c] = sum_chunks e^(m_c - M) part_c[c] / sum_chunks e^(m_c - M) z_c, chunks ascending, FP64.
-// The chunk weights are computed once per (query, head) - one exponential per chunk, by as many
-// threads - and shared; a thread then owns latent columns.
-constexpr int FL_MAX_CHUNKS = 64;
+// cb[t][h][c] = sum_s e^(R_s - M) part_s[c] / sum_s e^(R_s - M) z_s over the stretches s, ascending, FP64.
+// A thread owns a latent column. Everything is asked for before anything is used (the rows do not depend on the weights), the weights are
+// computed by the first two warps, one exponential per stretch. FL_AHEAD: rows asked for, 48 for a query in many stretches (43: 10.7 -> 8.2 us), 8 for many
+// queries in few (64 queries in five: 98 us with the registers of 48, 27 so).
+constexpr int FL_MAX_SPLITS = 64;
+template <int FL_AHEAD>
 __global__ void __launch_bounds__(FL_KL) mla_flash_reduce_kernel(float *cb, const float *part, const double *cstat, const int *nsel,
-                                                               int cached, int nchunks, MlaShape s)
+                                                               int cached, int splits, int span, MlaShape s)
 {
     pdl_trigger();
     pdl_wait();
-    __shared__ double s_m[FL_MAX_CHUNKS], s_w[FL_MAX_CHUNKS];
-    __shared__ double s_z;
-    const int h = blockIdx.x, t = blockIdx.y, p = pos_of(s, cached, t);
+    __shared__ double s_m[FL_MAX_SPLITS], s_w[FL_MAX_SPLITS], s_z[2];
+    const int h = blockIdx.x, t = blockIdx.y, p = pos_of(s, cached, t), tid = threadIdx.x;
+    const float *pr = part + ((size_t)t * s.H + h) * splits * FL_KL + tid;
+    float v[FL_AHEAD];
+#pragma unroll
+    for (int i = 0; i < FL_AHEAD; i++) v[i] = i < splits ? __ldcg(pr + (size_t)i * FL_KL) : 0.f;      // (unused stretches too: they are not multiplied)
     const int ns = nsel ? nsel[t] : -1;
     const int nvis = ns < 0 ? p + 1 : ns;
-    const int used = (nvis + FL_POS - 1) / FL_POS;
-    const double *st = cstat + ((size_t)t * s.H + h) * nchunks * 2;
-    double zc = 0.0;
-    if ((int)threadIdx.x < used) { s_m[threadIdx.x] = st[2 * threadIdx.x]; zc = st[2 * threadIdx.x + 1]; }
-    __syncthreads();
-    double M = -INFINITY;
-    for (int c = 0; c < used; c++) M = fmax(M, s_m[c]);
-    if ((int)threadIdx.x < used) s_w[threadIdx.x] = exp(s_m[threadIdx.x] - M);
-    __syncthreads();
-    if ((int)threadIdx.x < used) s_m[threadIdx.x] = s_w[threadIdx.x] * zc;       // reuse: the chunk's share of the denominator
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double Z = 0.0;
-        for (int c = 0; c < used; c++) Z += s_m[c];
-        s_z = Z;
+    const int used = (nvis + span * FL_POS - 1) / (span * FL_POS);
+    if (tid < FL_MAX_SPLITS) {
+        const double *st = cstat + ((size_t)t * s.H + h) * splits * 2;
+        double m = -INFINITY, zc = 0.0;
+        if (tid < used) { m = st[2 * tid]; zc = st[2 * tid + 1]; }
+        s_m[tid] = m;
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        double M = fmax(s_m[tid & 31], s_m[(tid & 31) + 32]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) M = fmax(M, __shfl_xor_sync(0xffffffffu, M, o));
+        const double w = tid < used ? exp(m - M) : 0.0;
+        s_w[tid] = w;
+        const double z = warp_sum(w * zc);
+        if ((tid & 31) == 0) s_z[tid >> 5] = z;
     }
     __syncthreads();
-    const double Z = s_z;
-    const float *pr = part + ((size_t)t * s.H + h) * nchunks * FL_KL;
-    for (int col = threadIdx.x; col < FL_KL; col += blockDim.x) {
-        double acc = 0.0;
-        for (int c0 = 0; c0 < used; c0 += 8) {                 // eight chunks' rows requested before the first is used
-            float v[8];
+    double acc = 0.0;
 #pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = c0 + i < used ? __ldcg(pr + (size_t)(c0 + i) * FL_KL + col) : 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; i++) if (c0 + i < used) acc = fma(s_w[c0 + i], (double)v[i], acc);
-        }
-        cb[((size_t)t * s.H + h) * FL_KL + col] = (float)(acc / Z);
-    }
+    for (int i = 0; i < FL_AHEAD; i++) if (i < used) acc = fma(s_w[i], (double)v[i], acc);
+    for (int i = FL_AHEAD; i < used; i++) acc = fma(s_w[i], (double)__ldcg(pr + (size_t)i * FL_KL), acc);
+    cb[((size_t)t * s.H + h) * FL_KL + tid] = (float)(acc / (s_z[0] + s_z[1]));
 }
 
 bool mla_flash_takes(const MlaShape &s)
 {
-    return s.latent_bf16 && s.KL == FL_KL && s.H % FL_HEADS == 0 && (s.topk + s.KP + FL_POS - 1) / FL_POS <= FL_MAX_CHUNKS;
+    return s.latent_bf16 && s.KL == FL_KL && s.H % FL_HEADS == 0 && (s.topk + s.KP + FL_POS - 1) / FL_POS <= FL_MAX_SPLITS;
 }
 
-// scratch: `part_bytes` bytes for the partial rows; `cstat` room for [T][H][nchunks][2] doubles.
+// scratch: `part_bytes` bytes for the stretches' rows; `cstat` room for [T][H][splits][2] doubles.
 int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
                      void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s)
 {
     static SmemGrant grant;
     if (!dev_opt_in_smem((const void *)mla_flash_kernel, FL_SMEM, grant)) return -1;
     const int stride = s.topk + s.KP;
-    // partial rows are laid out for the chunks that the call's last position can see: an early stretch of a prompt goes in
-    // few launches of many queries
-    const int last = s.batch ? cached + 1 : cached + T, nchunks = ((last < stride ? last : stride) + FL_POS - 1) / FL_POS;
-    const size_t per_token = (size_t)s.H * nchunks * FL_KL * sizeof(float);
-    int group = (int)(part_bytes / per_token);
-    if (group < 1) group = 1;
-    for (int t0 = 0; t0 < T; t0 += group) {
-        const int n = T - t0 < group ? T - t0 : group;
-        const int reach = s.batch ? cached + 1 : cached + t0 + n;
-        const int used = (((reach < stride) ? reach : stride) + FL_POS - 1) / FL_POS;
-        const void *lat0 = latent;                                 // the kernel's token 0 is sequence t0 of a batch
-        if (s.batch) lat0 = static_cast<const void *>(static_cast<const uint16_t *>(latent) + (size_t)t0 * s.lat_seq);
-        G5B_LAUNCH_PDL(mla_flash_kernel, dim3(used, s.H / FL_HEADS, n), FL_THREADS, FL_SMEM, st, static_cast<float *>(part), cstat,
-                       static_cast<const __nv_bfloat16 *>(qterms) + (size_t)t0 * s.H * 3 * s.KL, lat0, sel ? sel + (size_t)t0 * stride : nullptr, nsel ? nsel + t0 : nullptr,
-                       s.batch ? cached : cached + t0, nchunks, s);
-        // (launched the ordinary way: launched early, its CTAs crowd the SMs beside the core's, of which two fit an SM - one
-        // token at 2048 / 8192 / 32768 positions: MLA layer 102.4 / 112.6 / 120.9 us, 96.3 / 106.6 / 114.8 so)
-        G5B_LAUNCH(mla_flash_reduce_kernel, dim3(s.H, n), FL_KL, 0, st, cb + (size_t)t0 * s.H * s.KL, static_cast<const float *>(part),
-                       cstat, nsel ? nsel + t0 : nullptr, s.batch ? cached : cached + t0, nchunks, s);
+    const int last = s.batch ? cached + 1 : cached + T, chunks = ((last < stride ? last : stride) + FL_POS - 1) / FL_POS;
+    // As many stretches as give every SM two CTAs four times over, so that the last ones to end are a small part: a stretch reads the
+    // query's 48 KB once more. Queries of a long prompt are enough by themselves, and need no second kernel.
+    const int ctas = T * (s.H / FL_HEADS), room = (int)(part_bytes / ((size_t)T * s.H * FL_KL * sizeof(float)));
+    int splits = (8 * dev_sms() + ctas - 1) / ctas;
+    if (ctas >= 4 * dev_sms()) splits = 1;
+    if (splits > chunks) splits = chunks;
+    if (splits > room) splits = room < 1 ? 1 : room;
+    const int span = (chunks + splits - 1) / splits;
+    splits = (chunks + span - 1) / span;
+    G5B_LAUNCH_PDL(mla_flash_kernel, dim3(splits, s.H / FL_HEADS, T), FL_THREADS, FL_SMEM, st, cb, static_cast<float *>(part), cstat,
+                   static_cast<const __nv_bfloat16 *>(qterms), latent, sel, nsel, cached, splits, span, s);
+    // (launched the ordinary way: launched early, its CTAs crowd the SMs beside the core's, of which two fit an SM - one
+    // token at 2048 / 8192 / 32768 positions: MLA layer 102.4 / 112.6 / 120.9 us, 96.3 / 106.6 / 114.8 so)
+    if (splits > 1) {
+        auto reduce = splits > 8 ? mla_flash_reduce_kernel<48> : mla_flash_reduce_kernel<8>;
+        G5B_LAUNCH(reduce, dim3(s.H, T), FL_KL, 0, st, cb, static_cast<const float *>(part), cstat, nsel, cached, splits, span, s);
     }
     return 0;
 }
