@@ -44,8 +44,8 @@ struct RouterArgs {
     int n_local0, n_local, with_shared;
     int *counter;
     int sh_t0, sh_n;                 // the shared expert's slot takes tokens [sh_t0, sh_t0 + sh_n)
-    const double *parts;             // optional: the dot products are there already, in n_parts stretches of the columns
-    int n_parts;                     // ([stretch][token][expert], part_stride between stretches); one CTA per token then
+    const double *parts;             // router_select_kernel: the dot products, in n_parts stretches of the columns
+    int n_parts;                     // ([stretch][token][expert], part_stride between stretches)
     size_t part_stride;
 };
 
@@ -118,15 +118,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     __shared__ int is_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
     const int e = blockIdx.x * RT_WARPS + warp, t = blockIdx.y;
-    if (a.parts) {
-        const double *pt = a.parts + (size_t)t * a.NE;
-        for (int i = tid; i < a.NE; i += RT_WARPS * 32) {
-            double acc = __ldcg(pt + i);
-#pragma unroll 8
-            for (int k = 1; k < a.n_parts; k++) acc += __ldcg(pt + (size_t)k * a.part_stride + i);
-            a.score[(size_t)t * a.NE + i] = sigmoid_host((float)acc);
-        }
-    } else if (e < a.NE) {
+    if (e < a.NE) {
         const float *xt = a.x + (size_t)t * a.ldx;
         double acc = 0.0;
         if (a.gate_dt == DT_BF16 && (a.E & 7) == 0 && (a.ldx & 3) == 0) {
@@ -158,16 +150,14 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     // the last selection then groups the pairs.
     __threadfence();
     __syncthreads();
-    if (gridDim.x > 1) {
-        if (tid == 0) {
-            const int prev = atomicAdd(a.counter + 1 + t, 1);
-            is_last = prev == (int)gridDim.x - 1;
-            if (is_last) a.counter[1 + t] = 0;
-        }
-        __syncthreads();
-        if (!is_last) return;
-        __threadfence();
+    if (tid == 0) {
+        const int prev = atomicAdd(a.counter + 1 + t, 1);
+        is_last = prev == (int)gridDim.x - 1;
+        if (is_last) a.counter[1 + t] = 0;
     }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
     if (warp == 0) {
         if (a.NE <= 512) topk_one_token<16>(a, t, lane);
         else             topk_one_token<32>(a, t, lane);
@@ -247,63 +237,157 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     }
 }
 
-// The same grouping for more tokens than one router launch takes: one CTA, the expert ids read from memory.
-constexpr int PLAN_THREADS = 1024;
-__global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, int T, int K, int n_local0, int n_local, int with_shared, MoePlan p)
+// The same grouping by NT threads of one CTA with an expert each (n_local <= NT), the expert ids read from memory; the shared expert takes
+// tokens [sh_t0, sh_t0 + sh_n).
+template <int NT>
+__device__ __forceinline__ void group_pairs(const int *idx, int T, int K, int n_local0, int n_local, bool with_shared, int sh_t0, int sh_n, const MoePlan &p)
 {
-    pdl_trigger();
-    pdl_wait();
-    __shared__ int cnt[G5B_MAX_EXPERTS], off[G5B_MAX_EXPERTS];
-    __shared__ int wsum[3][PLAN_THREADS / 32];
+    __shared__ int cnt[NT], off[NT], wsum[3][NT / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = T * K;
     cnt[tid] = 0;
     __syncthreads();
-    for (int i = tid; i < n; i += PLAN_THREADS) {
-        const int le = idx[i] - n_local0;
+    for (int i = tid; i < n; i += NT) {
+        const int le = __ldcg(idx + i) - n_local0;
         if (le >= 0 && le < n_local) atomicAdd(&cnt[le], 1);
     }
     __syncthreads();
-    const int mine = tid < n_local ? cnt[tid] : 0;            // one expert per thread (at most G5B_MAX_EXPERTS of them)
+    const int mine = tid < n_local ? cnt[tid] : 0;
     int v[3] = {mine, mine > 0, (mine + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT}, own[3];
+#pragma unroll
     for (int k = 0; k < 3; k++) {
         own[k] = v[k];
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, v[k], o); if (lane >= o) v[k] += u; }
         if (lane == 31) wsum[k][warp] = v[k];
     }
     __syncthreads();
     int total[3];
+#pragma unroll
     for (int k = 0; k < 3; k++) {
-        int before = 0, all = 0;
-        for (int w = 0; w < PLAN_THREADS / 32; w++) { if (w < warp) before += wsum[k][w]; all += wsum[k][w]; }
-        v[k] += before - own[k];                              // exclusive
-        total[k] = all;
+        // the warps' sums, scanned by every warp for itself
+        const int x = lane < NT / 32 ? wsum[k][lane] : 0;
+        int y = x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, y, o); if (lane >= o) y += u; }
+        v[k] += __shfl_sync(0xffffffffu, y - x, warp) - own[k];      // exclusive
+        total[k] = __shfl_sync(0xffffffffu, y, 31);
     }
     if (mine) {
         p.slot_expert[v[1]] = tid; p.slot_off[v[1]] = v[0]; p.slot_cnt[v[1]] = mine; p.slot_tile0[v[1]] = v[2];
     }
     off[tid] = v[0];
-    __syncthreads();
     cnt[tid] = 0;                                             // reused as the write cursor of each expert
     __syncthreads();
-    for (int i = tid; i < n; i += PLAN_THREADS) {
-        const int le = idx[i] - n_local0;
+    for (int i = tid; i < n; i += NT) {
+        const int le = __ldcg(idx + i) - n_local0;
         if (le < 0 || le >= n_local) continue;
         const int pos = off[le] + atomicAdd(&cnt[le], 1);
         p.pair_tok[pos] = i / K;
         p.pair_dst[pos] = i;
     }
-    if (with_shared)
-        for (int t = tid; t < T; t += PLAN_THREADS) { p.pair_tok[total[0] + t] = t; p.pair_dst[total[0] + t] = n + t; }
+    const bool shared = with_shared && sh_n > 0;
+    if (shared)
+        for (int t = tid; t < sh_n; t += NT) { p.pair_tok[total[0] + t] = sh_t0 + t; p.pair_dst[total[0] + t] = n + sh_t0 + t; }
     if (tid == 0) {
-        if (with_shared) { p.slot_expert[total[1]] = n_local; p.slot_off[total[1]] = total[0]; p.slot_cnt[total[1]] = T; }
+        if (shared) { p.slot_expert[total[1]] = n_local; p.slot_off[total[1]] = total[0]; p.slot_cnt[total[1]] = sh_n; }
         p.slot_tile0[total[1]] = total[2];
-        if (with_shared) p.slot_tile0[total[1] + 1] = total[2] + ((T + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT);
-        *p.n_slots = total[1] + (with_shared ? 1 : 0);
-        *p.n_pairs = total[0] + (with_shared ? T : 0);
+        if (shared) p.slot_tile0[total[1] + 1] = total[2] + ((sh_n + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT);
+        *p.n_slots = total[1] + shared;
+        *p.n_pairs = total[0] + (shared ? sh_n : 0);
     }
 }
 
-constexpr int RT_TILE_MIN_T = 17, RT_TILE_CTAS = 1200, RT_MAX_PARTS = 32;
+// for more tokens than one router launch plans
+constexpr int PLAN_THREADS = 1024;
+__global__ void __launch_bounds__(PLAN_THREADS) moe_plan_kernel(const int *idx, int T, int K, int n_local0, int n_local, int with_shared, MoePlan p)
+{
+    pdl_trigger();
+    pdl_wait();
+    group_pairs<PLAN_THREADS>(idx, T, K, n_local0, n_local, with_shared, 0, T, p);
+}
+
+// Selection from dot products that are there already, a CTA per token and a thread per expert: the chain of one token is what it takes (the
+// kernel above, with 128 threads and one warp for eight rounds of arg-max, 27.6 us for 64 tokens with the plan; this one 10.5). A
+// thread adds its expert's stretches, all of them on their way at once; the experts of a warp that are among its K best go on to a list, and
+// an entry's place in the order (larger score first, then the lower expert) is how many entries precede it.
+constexpr int RS_THREADS = 512, RS_MAX_K = 16, RS_AHEAD = 16;
+__global__ void __launch_bounds__(RS_THREADS) router_select_kernel(const RouterArgs a)
+{
+    pdl_trigger();
+    constexpr int NW = RS_THREADS / 32;
+    __shared__ uint32_t s_key[NW * RS_MAX_K];
+    __shared__ int s_exp[NW * RS_MAX_K], s_pick[RS_MAX_K], is_last;
+    __shared__ float s_val[NW * RS_MAX_K], s_w[RS_MAX_K], s_first;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = blockIdx.x, K = a.K, slots = (a.NE + 31) / 32 * K;
+    const float bias = tid < a.NE ? a.bias[tid] : 0.f;
+    pdl_wait();
+    float sc = 0.f;
+    uint32_t key = 0u;
+    if (tid < a.NE) {
+        const double *pt = a.parts + (size_t)t * a.NE + tid;
+        double acc = 0.0;
+#pragma unroll 1
+        for (int k0 = 0; k0 < a.n_parts; k0 += RS_AHEAD) {
+            double v[RS_AHEAD];
+#pragma unroll
+            for (int k = 0; k < RS_AHEAD; k++) v[k] = k0 + k < a.n_parts ? __ldcg(pt + (size_t)(k0 + k) * a.part_stride) : 0.0;
+#pragma unroll
+            for (int k = 0; k < RS_AHEAD; k++) if (k0 + k < a.n_parts) acc = k0 + k ? acc + v[k] : v[k];
+        }
+        sc = sigmoid_host((float)acc);
+        a.score[(size_t)t * a.NE + tid] = sc;
+        key = choice_key(__fadd_rn(sc, bias));
+        if (tid == 0) s_first = sc;
+    }
+    // place among the warp's experts; the K best go on the list (those that cannot be selected as zeros)
+    if (warp * 32 < a.NE) {
+        int before = 0;
+#pragma unroll 8
+        for (int j = 0; j < 32; j++) {
+            const uint32_t other = __shfl_sync(0xffffffffu, key, j);
+            before += other > key || (other == key && j < lane);
+        }
+        if (before < K) { s_key[warp * K + before] = key; s_exp[warp * K + before] = tid; s_val[warp * K + before] = sc; }
+    }
+    if (tid < K) { s_pick[tid] = 0; s_w[tid] = -1.f; }
+    __syncthreads();
+    if (tid < slots) {
+        const uint32_t mine = s_key[tid];
+        if (mine) {
+            int before = 0;
+#pragma unroll 8
+            for (int j = 0; j < slots; j++) { const uint32_t other = s_key[j]; before += other > mine || (other == mine && j < tid); }
+            if (before < K) { s_pick[before] = s_exp[tid]; s_w[before] = s_val[tid]; }
+        }
+    }
+    __syncthreads();
+    if (tid < K) {
+        // (a place that nothing selectable is left for goes to expert 0; the reference aborts there)
+        float w = s_w[tid] < 0.f ? s_first : s_w[tid];
+        if (a.norm_topk) {
+            double tot = 0.0;
+            for (int j = 0; j < K; j++) tot += (double)(s_w[j] < 0.f ? s_first : s_w[j]);
+            w = (float)((double)w / (tot + 1e-20));
+        }
+        a.idx[(size_t)t * K + tid] = s_pick[tid];
+        a.w[(size_t)t * K + tid] = __fmul_rn(w, a.routed_scale);
+    }
+    if (!a.p.n_slots) return;
+    // the CTA that selects last groups the pairs
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+        const int prev = atomicAdd(a.counter, 1);
+        is_last = prev == (int)gridDim.x - 1;
+        if (is_last) *a.counter = 0;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    group_pairs<RS_THREADS>(a.idx, a.T, K, a.n_local0, a.n_local, a.with_shared, a.sh_t0, a.sh_n, a.p);
+}
+
+constexpr int RT_TILE_MIN_T = 2, RT_TILE_CTAS = 1200, RT_MAX_PARTS = 32;
 // p may be null-planned (p.n_slots == nullptr) when only the routing is wanted.
 void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float *x, int ldx, const void *gate,
                  int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &p, int with_shared,
@@ -311,10 +395,9 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
 {
     const bool one = T <= RT_MAX_TOKENS;
     // From RT_TILE_MIN_T tokens on the dot products go first, in tiles and so many stretches of the columns that there are a few
-    // CTAs per SM (64 tokens: 56 us for everything, now 38); below, adding up the stretches costs more than they save (7 tokens:
-    // 21 us in one kernel, 36 in two).
+    // CTAs per SM, then the selection (7 tokens: 5.9 + 9.8 us, in one kernel 20.4; 64: 14.6 + 10.5).
     int parts = 0, per = s.E;
-    if (T >= RT_TILE_MIN_T && dots && gate_dt == DT_BF16 && s.E % F64_K == 0 && s.NE % 2 == 0 && ldx % 4 == 0 &&
+    if (T >= RT_TILE_MIN_T && dots && s.NE <= RS_THREADS && s.K <= RS_MAX_K && s.K <= 32 && (!p.n_slots || s.n_local <= RS_THREADS) && gate_dt == DT_BF16 && s.E % F64_K == 0 && s.NE % 2 == 0 && ldx % 4 == 0 &&
         (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(gate) & 15) == 0) {
         const int rows = f64_tile_rows(T), tiles = (T + rows - 1) / rows * ((s.NE + F64_N - 1) / F64_N), blocks = s.E / F64_K;
         parts = (RT_TILE_CTAS + tiles - 1) / tiles;
@@ -326,15 +409,15 @@ void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float 
         const F64Tile f{x, static_cast<const uint16_t *>(gate), dots, (size_t)ldx, (size_t)s.E, (size_t)s.NE, (size_t)per, (size_t)per, (size_t)T * s.NE, T, s.NE, per, {}, nullptr};
         f64_tile<false>(st, f, parts);
     }
-    // (with the dot products there a token is one CTA's, which needs no counter: one launch selects for all of them. 2048 tokens:
-    // 403 us in 32 launches)
+    // (with the dot products there, one launch selects for all tokens. 2048: 403 us in 32 launches, now 32 us)
     const int most = parts ? T : RT_MAX_TOKENS;
     for (int t0 = 0; t0 < T; t0 += most) {
         const int n = T - t0 < most ? T - t0 : most;
         RouterArgs a{idx + (size_t)t0 * s.K, w + (size_t)t0 * s.K, score + (size_t)t0 * s.NE, x + (size_t)t0 * ldx, ldx, gate, gate_dt, bias, s.NE, s.E, s.K, n,
                      s.norm_topk, s.routed_scale, one ? p : MoePlan{}, s.n_local0, s.n_local, with_shared, counter, shared_t0, shared_n < 0 ? n : shared_n,
-                     parts ? dots + (size_t)t0 * s.NE : nullptr, parts, (size_t)T * s.NE};
-        G5B_LAUNCH_PDL(router_kernel, dim3(parts ? 1 : (s.NE + RT_WARPS - 1) / RT_WARPS, n), dim3(RT_WARPS * 32), 0, st, a);
+                     dots, parts, (size_t)T * s.NE};
+        if (parts) G5B_LAUNCH_PDL(router_select_kernel, dim3(n), dim3(RS_THREADS), 0, st, a);
+        else       G5B_LAUNCH_PDL(router_kernel, dim3((s.NE + RT_WARPS - 1) / RT_WARPS, n), dim3(RT_WARPS * 32), 0, st, a);
     }
     if (!one && p.n_slots) G5B_LAUNCH_PDL(moe_plan_kernel, dim3(1), dim3(PLAN_THREADS), 0, st, idx, T, s.K, s.n_local0, s.n_local, with_shared, p);
 }
