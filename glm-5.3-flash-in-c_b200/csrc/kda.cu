@@ -9,7 +9,8 @@
 // gated per-head RMSNorm of the output, with the state in registers, read once and written once
 // per call however many tokens the call carries:
 //   one position of one sequence, head_dim 64 or 128   kda_step_kernel, a cluster of CTAs per head
-//   several positions, or one of several sequences     kda_prep_kernel, kda_scan_kernel, kda_out_kernel
+//   one position of each of several sequences          kda_each_kernel, a CTA per head and sequence
+//   several positions                                  kda_prep_kernel, kda_scan_kernel, kda_out_kernel
 //   other head sizes                                   kda_core_kernel, a CTA per head, the state in memory
 //
 // The one-position and the any-size kernel keep the reference's order of FP32 operations (decay row
@@ -408,6 +409,124 @@ __global__ void __launch_bounds__(256) kda_out_kernel(const KdaArgs a, int heads
         a.o[off + i] = __fmul_rn(__fmul_rn(a.o_norm[lane * C + i], __fmul_rn(o[i], inv)), sigmoid_near(a.gb[off + i]));
 }
 
+// One position of each of several sequences, convolutions of width 4: a CTA takes a head of a sequence from its inputs to its gated output.
+// Bound by the states' way from HBM and back (64 sequences of 64 heads: 0.54 GB, 82 us). The three kernels above, of which the scan
+// read a state in pieces of 32 bytes, took 171 us a layer (27 + 139 + 5); here a thread holds two columns of 32 rows, asked for
+// before anything else, so that 128 KB are on their way to an SM while the convolutions, norms and gates of the two CTAs on it are
+// computed. Arithmetic as above: products fused, sums in parts. 64 sequences:
+// 111 us, 7: 17.3 (34 before); a step of 64 sequences over eight layers 6.80 -> 6.39 ms.
+template <int DS>
+__global__ void __launch_bounds__(256, 2) kda_each_kernel(const KdaArgs a)
+{
+    pdl_trigger();
+    constexpr int D = DS, KW = 4, HIST = KW - 1, CP = D / 2, RG = 256 / CP, R = D / RG, CH = (3 * D + 255) / 256;
+    __shared__ __align__(16) float sal[D], sk[D], sq[D], raw[3 * D];
+    __shared__ __align__(16) F2 us[RG][CP], os[RG][CP];
+    __shared__ double red[8][3];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, cp = tid % CP, rg = tid / CP, h = a.head0 + blockIdx.x, seq = blockIdx.y, P = a.H * D;
+    float *state = a.state + (size_t)seq * a.seq_stride, *cs = state + (size_t)a.H * D * D;
+    unsigned long long *S = reinterpret_cast<unsigned long long *>(state + (size_t)h * D * D + (size_t)rg * R * D + 2 * cp);
+    F2 s[R];
+#pragma unroll
+    for (int i = 0; i < R; i++) s[i].v = __ldcs(S + (size_t)i * (D / 2));
+    float w[CH][KW], past[CH][HIST];
+#pragma unroll
+    for (int n = 0; n < CH; n++) {
+        const int i = tid + 256 * n, c = i / D, ch = h * D + i % D;
+        if (i < 3 * D) {
+            const float *wp = (c == 0 ? a.q_conv : c == 1 ? a.k_conv : a.v_conv) + (size_t)ch * KW, *hp = cs + (size_t)c * P * HIST + (size_t)ch * HIST;
+#pragma unroll
+            for (int j = 0; j < KW; j++) w[n][j] = wp[j];
+#pragma unroll
+            for (int j = 0; j < HIST; j++) past[n][j] = hp[j];
+        }
+    }
+    const float dt = tid < D ? a.dt_bias[h * D + tid] : 0.f, onw = tid < D ? a.o_norm[tid] : 0.f;
+    const float ea = expf_host(a.A_log[h]), qscale = 1.0f / sqrtf((float)D);
+    pdl_wait();
+    const size_t off = (size_t)seq * P + h * D;
+    const float z = tid < D ? a.z[off + tid] : 0.f, gate = tid < D ? a.gb[off + tid] : 0.f, braw = a.braw[(size_t)seq * a.H + h];
+#pragma unroll
+    for (int n = 0; n < CH; n++) {
+        const int i = tid + 256 * n, c = i / D, d = i % D;
+        if (i < 3 * D) {
+            const float now = (c == 0 ? a.q : c == 1 ? a.k : a.v)[off + d];
+            float y = __fmul_rn(w[n][HIST], now);
+#pragma unroll
+            for (int j = 0; j < HIST; j++) y = mul_add_unfused(w[n][j], past[n][j], y);
+            raw[i] = __fmul_rn(y, sigmoid_near(y));
+            float *hp = cs + (size_t)c * P * HIST + (size_t)(h * D + d) * HIST;      // (each channel by one thread)
+            hp[0] = past[n][1]; hp[1] = past[n][2]; hp[2] = now;
+        }
+    }
+    __syncthreads();
+    // l2norm: divide by sqrt(sum of squares + 1e-6), sums in FP64 (glm53f_ops.c:661-667)
+    const float yq = tid < D ? raw[tid] : 0.f, yk = tid < D ? raw[D + tid] : 0.f;
+    {
+        const double qq = warp_sum((double)yq * (double)yq), kk = warp_sum((double)yk * (double)yk);
+        if (lane == 0) { red[warp][0] = qq; red[warp][1] = kk; }
+    }
+    if (tid < D) sal[tid] = expf_near(__fmul_rn(a.gate_lb, sigmoid_near(__fmul_rn(ea, __fadd_rn(z, dt)))));
+    __syncthreads();
+    double tq = 0.0, tk = 0.0;
+#pragma unroll
+    for (int i = 0; i < D / 32; i++) { tq += red[i][0]; tk += red[i][1]; }
+    const float qinv = (float)rsqrt_newton(tq + (double)1e-6f), kinv = (float)rsqrt_newton(tk + (double)1e-6f);
+    if (tid < D) { sq[tid] = __fmul_rn(__fmul_rn(yq, qinv), qscale); sk[tid] = __fmul_rn(yk, kinv); }
+    __syncthreads();
+    // q.k of the normalised vectors, for o = q.(aS) + (q.k) u
+    {
+        const double qk = tid < D ? warp_sum((double)sq[tid] * (double)sk[tid]) : 0.0;
+        if (tid < D && lane == 0) red[warp][2] = qk;
+    }
+    const float beta = sigmoid_near(braw);
+    F2 u = f2(0.f, 0.f), o = u;
+    const float4 *al4 = reinterpret_cast<const float4 *>(sal + rg * R), *k4 = reinterpret_cast<const float4 *>(sk + rg * R), *q4 = reinterpret_cast<const float4 *>(sq + rg * R);
+#pragma unroll
+    for (int i = 0; i < R / 4; i++) {
+        const float4 al = al4[i], k = k4[i], q = q4[i];
+        s[4 * i] = f2_mul(s[4 * i], f2(al.x, al.x)); s[4 * i + 1] = f2_mul(s[4 * i + 1], f2(al.y, al.y));
+        s[4 * i + 2] = f2_mul(s[4 * i + 2], f2(al.z, al.z)); s[4 * i + 3] = f2_mul(s[4 * i + 3], f2(al.w, al.w));
+        u = f2_fma(s[4 * i], f2(k.x, k.x), u); u = f2_fma(s[4 * i + 1], f2(k.y, k.y), u); u = f2_fma(s[4 * i + 2], f2(k.z, k.z), u); u = f2_fma(s[4 * i + 3], f2(k.w, k.w), u);
+        o = f2_fma(s[4 * i], f2(q.x, q.x), o); o = f2_fma(s[4 * i + 1], f2(q.y, q.y), o); o = f2_fma(s[4 * i + 2], f2(q.z, q.z), o); o = f2_fma(s[4 * i + 3], f2(q.w, q.w), o);
+    }
+    us[rg][cp] = u; os[rg][cp] = o;
+    __syncthreads();
+    float ux = 0.f, uy = 0.f, ox = 0.f, oy = 0.f;
+#pragma unroll
+    for (int i = 0; i < RG; i++) {
+        const float2 p = *reinterpret_cast<const float2 *>(&us[i][cp]), q = *reinterpret_cast<const float2 *>(&os[i][cp]);
+        ux = __fadd_rn(ux, p.x); uy = __fadd_rn(uy, p.y); ox = __fadd_rn(ox, q.x); oy = __fadd_rn(oy, q.y);
+    }
+    double qk = 0.0;
+#pragma unroll
+    for (int i = 0; i < D / 32; i++) qk += red[i][2];
+    ux = __fmul_rn(__fsub_rn(raw[2 * D + 2 * cp], ux), beta); uy = __fmul_rn(__fsub_rn(raw[2 * D + 2 * cp + 1], uy), beta);
+    ox = __fmaf_rn((float)qk, ux, ox); oy = __fmaf_rn((float)qk, uy, oy);
+    const F2 uu = f2(ux, uy);
+#pragma unroll
+    for (int i = 0; i < R / 4; i++) {
+        const float4 k = k4[i];
+        const F2 r0 = f2_fma(f2(k.x, k.x), uu, s[4 * i]), r1 = f2_fma(f2(k.y, k.y), uu, s[4 * i + 1]), r2 = f2_fma(f2(k.z, k.z), uu, s[4 * i + 2]), r3 = f2_fma(f2(k.w, k.w), uu, s[4 * i + 3]);
+        __stcs(S + (size_t)(4 * i) * (D / 2), r0.v); __stcs(S + (size_t)(4 * i + 1) * (D / 2), r1.v);
+        __stcs(S + (size_t)(4 * i + 2) * (D / 2), r2.v); __stcs(S + (size_t)(4 * i + 3) * (D / 2), r3.v);
+    }
+    // per-head RMSNorm with weight, then the sigmoid output gate (glm53f_ops.c:748-752)
+    if (rg == 0) { sal[2 * cp] = ox; sal[2 * cp + 1] = oy; }          // (the decays have been read: the barrier above)
+    __syncthreads();
+    const float ov = tid < D ? sal[tid] : 0.f;
+    const double oo = warp_sum((double)ov * (double)ov);
+    if (lane == 0) red[warp][0] = oo;
+    __syncthreads();
+    if (tid < D) {
+        double tot = 0.0;
+#pragma unroll
+        for (int i = 0; i < D / 32; i++) tot += red[i][0];
+        const float inv = (float)rsqrt_newton(tot / (double)D + (double)a.rms_eps);
+        a.o[off + tid] = __fmul_rn(__fmul_rn(onw, __fmul_rn(ov, inv)), sigmoid_near(gate));
+    }
+}
+
 // One position of one sequence. The chain of a single step is all latency: convolutions, norms, gates, two sums over the
 // state, the output's norm. A cluster takes a head, 32 columns of the state to a CTA of 256 threads; what all columns need
 // (q, k, the decays with their low-rank up-projection) every CTA computes for itself, and only the sum of squares of the
@@ -629,6 +748,10 @@ int kda_core(cudaStream_t st, float *o, const float *q, const float *k, const fl
                                    : (s.K == 4 ? kda_step<64, 4>(st, a, (int)grid.x) : kda_step<64, 0>(st, a, (int)grid.x));
         if (ok) return 0;
         if (fused) return -1;                // the kernel below does not take the up-projections itself
+    } else if (known && T == 1 && s.K == 4) {
+        if (s.D == 128) G5B_LAUNCH_PDL(kda_each_kernel<128>, grid, dim3(256), 0, st, a);
+        else            G5B_LAUNCH_PDL(kda_each_kernel<64>, grid, dim3(256), 0, st, a);
+        return 0;
     } else if (known && scratch) {
         if (s.D == 128) kda_rows<128>(st, a, *scratch, (int)grid.x, (int)grid.y);
         else            kda_rows<64>(st, a, *scratch, (int)grid.x, (int)grid.y);
