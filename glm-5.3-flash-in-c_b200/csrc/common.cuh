@@ -97,6 +97,14 @@ __device__ __forceinline__ float sigmoid_host(float x)
     return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf_host(-x)));
 }
 
+// v 2^k for the exponential of x: k is the low part of t's bits (t = k + 1.5 2^23); in two steps, so that a subnormal result is rounded once
+__device__ __forceinline__ float exp_scaled(float v, float t, float x)
+{
+    const int k = __float_as_int(t) - 0x4b400000, k0 = k >> 1;
+    v = v * __int_as_float((k0 + 127) << 23) * __int_as_float((k - k0 + 127) << 23);
+    return x > 89.0f ? INFINITY : x < -104.0f ? 0.0f : v;
+}
+
 // exp(x) to 0.53 units in the last place (the double-precision route above: 0.5), in thirty FP32
 // instructions: Cody and Waite's reduction x = n ln 2 + r with ln 2 cut after 14 bits (n times that is exact),
 // Taylor's series of e^r to r^9 with its terms up to r^2 / 2 as pairs of floats, one rounding at the end. For
@@ -106,9 +114,9 @@ __device__ __forceinline__ float sigmoid_host(float x)
 // subnormal results are off by less than one of their units.
 __device__ __forceinline__ float expf_near(float x)
 {
-    const float n = rintf(x * 1.44269504f);
-    const float rh = fmaf(n, -0.693115234375f, x), rl = n * -3.19461849453e-05f;
-    const float sh = rh + rl, sl = (rh - sh) + rl;
+    const float t = fmaf(x, 1.44269504f, 0x1.8p23f), n = __fsub_rn(t, 0x1.8p23f);      // rounded to an integer, which also lies in t's low bits
+    const float rh = fmaf(n, -0.693115234375f, x);
+    const float sh = fmaf(n, -3.19461849453e-05f, rh), sl = fmaf(n, -3.19461849453e-05f, __fsub_rn(rh, sh));
     float q = fmaf(sh, 1.0f / 362880.0f, 1.0f / 40320.0f);
     q = fmaf(sh, q, 1.0f / 5040.0f);
     q = fmaf(sh, q, 1.0f / 720.0f);
@@ -120,14 +128,74 @@ __device__ __forceinline__ float expf_near(float x)
     const float a = __fadd_rn(h, c), ae = __fadd_rn(__fsub_rn(h, a), c);
     const float b = __fadd_rn(sh, a), be = __fadd_rn(__fsub_rn(sh, b), a);
     const float d = __fadd_rn(1.0f, b), de = __fadd_rn(__fsub_rn(1.0f, d), b);
-    const int k = (int)fminf(fmaxf(n, -160.0f), 160.0f), k0 = k / 2;
-    const float v = __fadd_rn(d, __fadd_rn(de, __fadd_rn(be, ae))) * __int_as_float((k0 + 127) << 23) * __int_as_float((k - k0 + 127) << 23);
-    return x > 89.0f ? INFINITY : x < -104.0f ? 0.0f : v;
+    return exp_scaled(__fadd_rn(d, __fadd_rn(de, __fadd_rn(be, ae))), t, x);
+}
+
+// 1 / d rounded to nearest, d from 1 on: the estimate and one step of Newton's, whose residual is exact in a fused product, without the
+// branch that a division has for its special cases - a dozen of them in a row waited for each other. Equal to the division for every
+// mantissa (all 2^23 compared); 0 for an infinite d, NaN for NaN; from 2^126 on (subnormal results) off by less than one of their units.
+// (Taken of d / 2^26, so that neither the argument nor the estimate leaves the range of normal numbers.)
+__device__ __forceinline__ float rcp_estimate(float d)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return r;
+}
+__device__ __forceinline__ float recip_from_one(float d)
+{
+    const float ds = d * 0x1p-26f, r = rcp_estimate(ds);
+    return d == INFINITY ? 0.0f : fmaf(r, fmaf(-ds, r, 1.0f), r) * 0x1p-26f;
 }
 
 // The sigmoid of the function above, with this exponential: three roundings, 1.53 units of 2^-23 at most relative to the exact
 // value (0.53 of the exponential, a half each of the sum and the quotient).
-__device__ __forceinline__ float sigmoid_near(float x) { return __fdiv_rn(1.0f, __fadd_rn(1.0f, expf_near(-x))); }
+__device__ __forceinline__ float sigmoid_near(float x) { return recip_from_one(__fadd_rn(1.0f, expf_near(-x))); }
+
+// Two floats side by side: one instruction for both (rounded like two of the scalar ones).
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float x, float y) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y)); return r; }
+__device__ __forceinline__ void f2_get(F2 a, float &x, float &y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); }
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 f2_sub(F2 a, F2 b) { return f2_fma(b, f2(-1.0f, -1.0f), a); }
+__device__ __forceinline__ float f2_sum(F2 a) { float x, y; f2_get(a, x, y); return __fadd_rn(x, y); }
+
+// expf_near of two arguments, step by step the same operations: equal to it bit for bit.
+__device__ __forceinline__ void expf_near2(float x0, float x1, float &e0, float &e1)
+{
+    auto both = [](float v) { return f2(v, v); };
+    const F2 x = f2(x0, x1), t = f2_fma(x, both(1.44269504f), both(0x1.8p23f)), n = f2_add(t, both(-0x1.8p23f));
+    const F2 c2 = both(-3.19461849453e-05f), rh = f2_fma(n, both(-0.693115234375f), x);
+    const F2 sh = f2_fma(n, c2, rh), sl = f2_fma(n, c2, f2_sub(rh, sh));
+    F2 q = f2_fma(sh, both(1.0f / 362880.0f), both(1.0f / 40320.0f));
+    q = f2_fma(sh, q, both(1.0f / 5040.0f));
+    q = f2_fma(sh, q, both(1.0f / 720.0f));
+    q = f2_fma(sh, q, both(1.0f / 120.0f));
+    q = f2_fma(sh, q, both(1.0f / 24.0f));
+    q = f2_fma(sh, q, both(1.0f / 6.0f));
+    const F2 nsh = f2_mul(sh, both(-1.0f)), nsq = f2_mul(sh, nsh), sqe = f2_fma(sh, sh, nsq), h = f2_mul(both(-0.5f), nsq);
+    const F2 c = f2_fma(f2_mul(nsq, nsh), q, f2_fma(both(0.5f), sqe, f2_fma(sh, sl, sl)));
+    const F2 a = f2_add(h, c), ae = f2_add(f2_sub(h, a), c);
+    const F2 b = f2_add(sh, a), be = f2_add(f2_sub(sh, b), a);
+    const F2 d = f2_add(both(1.0f), b), de = f2_add(f2_sub(both(1.0f), d), b);
+    float v0, v1, t0, t1;
+    f2_get(f2_add(d, f2_add(de, f2_add(be, ae))), v0, v1);
+    f2_get(t, t0, t1);
+    e0 = exp_scaled(v0, t0, x0); e1 = exp_scaled(v1, t1, x1);
+}
+__device__ __forceinline__ void sigmoid_near2(float x0, float x1, float &s0, float &s1)
+{
+    float d0, d1;
+    expf_near2(-x0, -x1, s0, s1);
+    const F2 d = f2_add(f2(s0, s1), f2(1.0f, 1.0f)), nds = f2_mul(d, f2(-0x1p-26f, -0x1p-26f));
+    f2_get(d, d0, d1);
+    f2_get(nds, s0, s1);
+    const F2 r = f2(rcp_estimate(-s0), rcp_estimate(-s1));
+    f2_get(f2_mul(f2_fma(r, f2_fma(nds, r, f2(1.0f, 1.0f)), r), f2(0x1p-26f, 0x1p-26f)), s0, s1);
+    if (d0 == INFINITY) s0 = 0.0f;
+    if (d1 == INFINITY) s1 = 0.0f;
+}
 
 // a*b + c with two float roundings, as C compiled without FMA contraction evaluates it.
 __device__ __forceinline__ float mul_add_unfused(float a, float b, float c)

@@ -81,13 +81,15 @@ void swiglu(cudaStream_t st, float *y, const float *gu, int n, int rows, float l
     G5B_LAUNCH_PDL(swiglu_kernel, dim3((n + 255) / 256, rows), dim3(256), 0, st, y, gu, n, limit);
 }
 
-// The exponential and the sigmoid of the kernels that take millions of them (common.cuh), element by element (test aid).
+// The exponential and the sigmoid of the kernels that take millions of them (common.cuh), element by element, the sigmoid by pairs (test aid).
 __global__ void exp_near_kernel(float *e, float *sig, const float *x, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     e[i] = expf_near(x[i]);
-    sig[i] = sigmoid_near(x[i]);
+    float pair[2];
+    sigmoid_near2(x[i & ~1], x[(i | 1) < n ? i | 1 : i], pair[0], pair[1]);
+    sig[i] = pair[i & 1];
 }
 
 void exp_near(cudaStream_t st, float *e, float *sig, const float *x, int n)

@@ -154,8 +154,8 @@ __global__ void __launch_bounds__(512) kda_core_kernel(const KdaArgs a)
 // rows to PARTS lanes, in registers. Both products of a position are taken with the decayed state, o = q.(aS) + (q.k) u,
 // so that one round of shuffles serves them and the next position waits for u alone; the positions' vectors arrive by
 // asynchronous copies, 8 positions ahead. Many positions are bound by that chain and by shared-memory wavefronts (vector
-// loads and shuffles): two columns to a lane, which halves the loads per product, and one transposed sum for the four
-// values. 2048 positions of 64 heads: 5.2 ms with a thread per column, 1.7 with eight lanes to each, now 1.07. One position of
+// loads and shuffles, 48 % of what there could be): eight lanes to a column, one transposed sum for its two values. 2048 positions of
+// 64 heads: 5.2 ms with a thread per column, 1.05 with two columns to a lane of half as many warps, now 1.00. One position of
 // many sequences is bound by the state's memory traffic: four lanes to a column read it in whole 32-byte sectors.
 // The sums of a column are taken in parts with four accumulators each, products fused.
 struct KdaPrep {
@@ -164,94 +164,133 @@ struct KdaPrep {
     int heads;                              // of this launch
 };
 
-// A warp takes KDA_RUN positions of one head: the convolution weights stay in registers, the taps come as vectors.
-// Bound by its 0.5 GB of memory traffic at 2048 positions of 64 heads (82 us). KW: the width of the convolution, 0 for
-// one known at run time only.
-constexpr int KDA_RUN = 8;
+// A CTA takes KDA_TILE positions of one head, in two passes: a thread per channel of q, k, v and the gate walks the positions, four at a
+// time and two to an instruction, its weights and the last K - 1 inputs in registers; then a warp per position takes the norms of q and k
+// from shared memory. KW: the width of the convolution, 0 for one known at run time only. (q and k are wanted twice, by channel and by
+// position; a warp that kept all of a position's vectors took eight positions one after the other, each 17 KB of instructions and a chain
+// of seventeen divisions with their branches: 5 us a position however few there were.) Bound by the instructions of the exponentials and
+// reciprocals, 16 of them a channel; its memory traffic would take 10 us for 256 positions of 64 heads. With inputs that come from memory:
+// 2 positions 15 -> 5 us, 8: 41 -> 6, 50: 41 -> 12, 200: 52 -> 27, 256: 52 -> 31.
+constexpr int KDA_TILE = 16;
 template <int DS, int KW>
-__global__ void __launch_bounds__(256) kda_prep_kernel(const KdaPrep p)
+__global__ void __launch_bounds__(4 * DS) kda_prep_kernel(const KdaPrep p)
 {
     pdl_trigger();
     const KdaArgs &a = p.a;
-    constexpr int D = DS, C = DS / 32;      // channels per lane
+    constexpr int D = DS, C = DS / 32, U = 4;               // channels per lane of the second pass; positions of a step of the first
     struct alignas(4 * C) Vec { float v[C]; };
-    const int lane = threadIdx.x & 31, runs = (a.T + KDA_RUN - 1) / KDA_RUN, seq = blockIdx.y / runs, t0 = (blockIdx.y - seq * runs) * KDA_RUN;
-    const int hl = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (hl >= p.heads) { pdl_wait(); return; }
-    const int h = a.head0 + hl, P = a.H * D, K = KW ? KW : a.K, hist = K - 1, ch = h * D + lane * C;
-    const float *cs = a.state + (size_t)seq * a.seq_stride + (size_t)a.H * D * D;
-    const float *const xs[3] = {a.q, a.k, a.v}, *const ws[3] = {a.q_conv, a.k_conv, a.v_conv};
-    float w[3][C][KW ? KW : 1], dt[C];
+    __shared__ __align__(16) float xs[4][KDA_TILE][D];       // the inputs; q's and k's give way to the convolutions' results
+    const int tiles = (a.T + KDA_TILE - 1) / KDA_TILE, seq = blockIdx.y / tiles, t0 = (blockIdx.y - seq * tiles) * KDA_TILE;
+    const int h = a.head0 + blockIdx.x, P = a.H * D, K = KW ? KW : a.K, hist = K - 1, nt = a.T - t0 < KDA_TILE ? a.T - t0 : KDA_TILE;
+    const int c = threadIdx.x / D, d = threadIdx.x % D, ch = h * D + d;                 // (c: the same for a whole warp)
+    const size_t first = ((size_t)seq * a.T + t0) * P + ch;
+    const float *x = (c == 0 ? a.q : c == 1 ? a.k : c == 2 ? a.v : a.z) + first;
+    const float *wp = (c == 0 ? a.q_conv : c == 1 ? a.k_conv : a.v_conv) + (size_t)ch * K;
+    float w[KW ? KW : 1];
+    if (KW && c < 3)
 #pragma unroll
-    for (int i = 0; i < C; i++) {
-        dt[i] = a.dt_bias[ch + i];
-#pragma unroll
-        for (int c = 0; c < 3; c++)
-#pragma unroll
-            for (int j = 0; j < KW; j++) w[c][i][j] = ws[c][(size_t)(ch + i) * KW + j];
-    }
-    const float ea = expf_host(a.A_log[h]), qscale = 1.0f / sqrtf((float)D);
+        for (int j = 0; j < KW; j++) w[j] = wp[j];
+    const float dt = c == 3 ? a.dt_bias[ch] : 0.f, ea = c == 3 ? expf_host(a.A_log[h]) : 0.f;
     pdl_wait();
-    for (int t = t0; t < a.T && t < t0 + KDA_RUN; t++) {
-        const int rr = seq * a.T + t;
-        float y[3][C];
+    {
+        const float *row = x - d + d % (D / 4) * 4;            // D / 4 threads to a row of 16-byte pieces
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-            // the K - 1 inputs before position t: earlier rows of this call, or the carried history (oldest first)
-            const float *x = xs[c] + (size_t)rr * P + ch, *past = cs + (size_t)c * P * hist + (size_t)ch * hist;
-            auto tap = [&](int i, int j) { return KW ? w[c][i][KW ? j : 0] : ws[c][(size_t)(ch + i) * K + j]; };
-            const Vec now = *reinterpret_cast<const Vec *>(x);
+        for (int t = d / (D / 4); t < KDA_TILE; t += 4)
+            if (t < nt) cp_async16(&xs[c][t][d % (D / 4) * 4], row + (size_t)t * P);
+    }
+    // the input before position tt of the tile: earlier rows of this call, or the carried history (oldest first)
+    const float *cs = a.state + (size_t)seq * a.seq_stride + (size_t)a.H * D * D + (size_t)c * P * hist + (size_t)ch * hist;
+    auto before = [&](int tt) { return t0 + tt >= 0 ? x[(ptrdiff_t)tt * P] : cs[hist + t0 + tt]; };
+    float past[KW ? KW - 1 + U : 1];
+    if (c < 3)
 #pragma unroll
-            for (int i = 0; i < C; i++) y[c][i] = __fmul_rn(tap(i, hist), now.v[i]);
+        for (int j = 0; j + 1 < KW; j++) past[j] = before(j - (KW - 1));
+    cp_async_wait();
+    __syncthreads();
+    if (c == 3) {
+#pragma unroll 1
+        for (int t = 0; t < nt; t += U) {
+            float g[U];
 #pragma unroll
-            for (int j = 0; j < (KW ? KW - 1 : hist); j++) {
-                const int tt = t - hist + j;
-                Vec old;
-                if (tt >= 0) old = *reinterpret_cast<const Vec *>(x - (size_t)(hist - j) * P);
-                else
+            for (int j = 0; j < U; j++) g[j] = __fmul_rn(ea, __fadd_rn(xs[3][t + j][d], dt));
 #pragma unroll
-                    for (int i = 0; i < C; i++) old.v[i] = past[(size_t)i * hist + (hist + tt)];
-#pragma unroll
-                for (int i = 0; i < C; i++) y[c][i] = mul_add_unfused(tap(i, j), old.v[i], y[c][i]);
+            for (int j = 0; j < U; j += 2) {
+                sigmoid_near2(g[j], g[j + 1], g[j], g[j + 1]);
+                expf_near2(__fmul_rn(a.gate_lb, g[j]), __fmul_rn(a.gate_lb, g[j + 1]), g[j], g[j + 1]);
             }
 #pragma unroll
-            for (int i = 0; i < C; i++) y[c][i] = __fmul_rn(y[c][i], sigmoid_near(y[c][i]));
+            for (int j = 0; j < U; j++)
+                if (t + j < nt) p.al[first + (size_t)(t + j) * P] = g[j];
         }
-        // l2norm: divide by sqrt(sum of squares + 1e-6), sums in FP64 (glm53f_ops.c:661-667)
+    } else {
+#pragma unroll 1
+        for (int t = 0; t < nt; t += U) {
+            float y[U];
+            if constexpr (KW != 0) {
+#pragma unroll
+                for (int j = 0; j < U; j++) past[KW - 1 + j] = xs[c][t + j][d];
+#pragma unroll
+                for (int j = 0; j < U; j++) {
+                    y[j] = __fmul_rn(w[KW - 1], past[KW - 1 + j]);
+#pragma unroll
+                    for (int i = 0; i + 1 < KW; i++) y[j] = mul_add_unfused(w[i], past[j + i], y[j]);
+                }
+#pragma unroll
+                for (int j = 0; j + 1 < KW; j++) past[j] = past[j + U];
+            } else {
+                for (int j = 0; j < U; j++) {
+                    const int tt = t + j < nt ? t + j : nt - 1;
+                    float v = __fmul_rn(wp[hist], x[(size_t)tt * P]);
+                    for (int i = 0; i < hist; i++) v = mul_add_unfused(wp[i], before(tt - hist + i), v);
+                    y[j] = v;
+                }
+            }
+            float s[U];
+#pragma unroll
+            for (int j = 0; j < U; j += 2) sigmoid_near2(y[j], y[j + 1], s[j], s[j + 1]);
+#pragma unroll
+            for (int j = 0; j < U; j++)
+                if (t + j < nt) {
+                    const float v = __fmul_rn(y[j], s[j]);
+                    if (c < 2) xs[c][t + j][d] = v;
+                    else p.vn[first + (size_t)(t + j) * P] = v;
+                }
+        }
+    }
+    __syncthreads();
+    // l2norm: divide by sqrt(sum of squares + 1e-6), sums in FP64 (glm53f_ops.c:661-667); one half of the warp sums q's, the other k's
+    const int lane = threadIdx.x & 31;
+    const bool upper = lane & 16;
+    const float qscale = 1.0f / sqrtf((float)D);
+    for (int t = threadIdx.x >> 5; t < nt; t += D / 8) {
+        const size_t rr = (size_t)seq * a.T + t0 + t;
+        const float braw = a.braw[rr * a.H + h];
+        const Vec yq = *reinterpret_cast<const Vec *>(&xs[0][t][lane * C]), yk = *reinterpret_cast<const Vec *>(&xs[1][t][lane * C]);
         double qq = 0.0, kk = 0.0, qk = 0.0;
 #pragma unroll
         for (int i = 0; i < C; i++) {
-            qq += (double)y[0][i] * (double)y[0][i];
-            kk += (double)y[1][i] * (double)y[1][i];
+            qq = fma((double)yq.v[i], (double)yq.v[i], qq);
+            kk = fma((double)yk.v[i], (double)yk.v[i], kk);
         }
-        qq = warp_sum(qq); kk = warp_sum(kk);
-        const float qinv = (float)(1.0 / sqrt(qq + (double)1e-6f)), kinv = (float)(1.0 / sqrt(kk + (double)1e-6f));
-        const size_t off = (size_t)rr * P + ch;
-        const Vec z = *reinterpret_cast<const Vec *>(a.z + off);
-        Vec qn, kn, vn, al;
+        double sum = (upper ? kk : qq) + __shfl_xor_sync(0xffffffffu, upper ? qq : kk, 16);
+#pragma unroll
+        for (int m = 8; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        const float inv = (float)rsqrt_newton(sum + (double)1e-6f), other = __shfl_xor_sync(0xffffffffu, inv, 16);
+        const float qinv = upper ? other : inv, kinv = upper ? inv : other;
+        Vec qn, kn;
 #pragma unroll
         for (int i = 0; i < C; i++) {
-            qn.v[i] = __fmul_rn(__fmul_rn(y[0][i], qinv), qscale);
-            kn.v[i] = __fmul_rn(y[1][i], kinv);
-            vn.v[i] = y[2][i];
-            al.v[i] = expf_near(__fmul_rn(a.gate_lb, sigmoid_near(__fmul_rn(ea, __fadd_rn(z.v[i], dt[i])))));
-            qk += (double)qn.v[i] * (double)kn.v[i];
+            qn.v[i] = __fmul_rn(__fmul_rn(yq.v[i], qinv), qscale);
+            kn.v[i] = __fmul_rn(yk.v[i], kinv);
+            qk = fma((double)qn.v[i], (double)kn.v[i], qk);
         }
         qk = warp_sum(qk);
-        *reinterpret_cast<Vec *>(p.qn + off) = qn;
-        *reinterpret_cast<Vec *>(p.kn + off) = kn;
-        *reinterpret_cast<Vec *>(p.vn + off) = vn;
-        *reinterpret_cast<Vec *>(p.al + off) = al;
-        if (lane == 0) *reinterpret_cast<float2 *>(p.beta + ((size_t)rr * a.H + h) * 2) = make_float2(sigmoid_near(a.braw[(size_t)rr * a.H + h]), (float)qk);
+        *reinterpret_cast<Vec *>(p.qn + rr * P + h * D + lane * C) = qn;
+        *reinterpret_cast<Vec *>(p.kn + rr * P + h * D + lane * C) = kn;
+        const float beta = sigmoid_near(braw);
+        if (lane == 0) *reinterpret_cast<float2 *>(p.beta + (rr * a.H + h) * 2) = make_float2(beta, (float)qk);
     }
 }
-
-// Two floats side by side: one instruction for both (products and sums fused).
-struct F2 { unsigned long long v; };
-__device__ __forceinline__ F2 f2(float x, float y) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(x), "f"(y)); return r; }
-__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
-__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
-__device__ __forceinline__ float f2_sum(F2 a) { float x, y; asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v)); return __fadd_rn(x, y); }
 
 constexpr int KDA_TB = 8;
 template <int DS, int PARTS, int CPL, int WARPS>
@@ -334,19 +373,15 @@ __global__ void __launch_bounds__(32 * WARPS) kda_scan_kernel(const KdaPrep p)
             const float2 b = sb[buf][j];
             float *out = a.o + (size_t)(row0 + t0 + j) * P + h * D + col;
             float u[CPL];
-            if constexpr (CPL == 2) {
-                // four sums over the eight lanes of a pair of columns: half of them go on with u, half with o, then a quarter each
-                static_assert(PARTS == 8, "three halvings");
-                const float x0 = __fadd_rn(f2_sum(u0[0]), f2_sum(u1[0])), x1 = __fadd_rn(f2_sum(u0[1]), f2_sum(u1[1]));
-                const float y0 = __fadd_rn(f2_sum(o0[0]), f2_sum(o1[0])), y1 = __fadd_rn(f2_sum(o0[1]), f2_sum(o1[1]));
-                const bool is_o = lane & 16, second = lane & 8;
-                const float a0 = __fadd_rn(is_o ? y0 : x0, __shfl_xor_sync(0xffffffffu, is_o ? x0 : y0, 16));
-                const float a1 = __fadd_rn(is_o ? y1 : x1, __shfl_xor_sync(0xffffffffu, is_o ? x1 : y1, 16));
-                float v = __fadd_rn(second ? a1 : a0, __shfl_xor_sync(0xffffffffu, second ? a0 : a1, 8));
+            if constexpr (PARTS == 8) {
+                // two sums over the eight lanes of a column: half of them go on with u, half with o
+                const float x = __fadd_rn(f2_sum(u0[0]), f2_sum(u1[0])), y = __fadd_rn(f2_sum(o0[0]), f2_sum(o1[0]));
+                const bool is_o = lane & 16;
+                float v = __fadd_rn(is_o ? y : x, __shfl_xor_sync(0xffffffffu, is_o ? x : y, 16));
+                v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 8));
                 v = __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 4));
                 u[0] = __fmul_rn(__fsub_rn(sv[buf][j][cc], __shfl_sync(0xffffffffu, v, lane & 3)), b.x);
-                u[1] = __fmul_rn(__fsub_rn(sv[buf][j][cc + 1], __shfl_sync(0xffffffffu, v, (lane & 3) | 8)), b.x);
-                if ((lane & 20) == 16) out[second] = __fmaf_rn(b.y, second ? u[1] : u[0], v);
+                if ((lane & 28) == 16) *out = __fmaf_rn(b.y, u[0], v);
             } else {
                 float o = __fadd_rn(f2_sum(o0[0]), f2_sum(o1[0]));
                 u[0] = __fadd_rn(f2_sum(u0[0]), f2_sum(u1[0]));
@@ -403,7 +438,7 @@ __global__ void __launch_bounds__(256) kda_out_kernel(const KdaArgs a, int heads
 #pragma unroll
     for (int i = 0; i < C; i++) { o[i] = a.o[off + i]; oo += (double)o[i] * (double)o[i]; }
     oo = warp_sum(oo);
-    const float inv = (float)(1.0 / sqrt(oo / (double)D + (double)a.rms_eps));
+    const float inv = (float)rsqrt_newton(oo / (double)D + (double)a.rms_eps);
 #pragma unroll
     for (int i = 0; i < C; i++)
         a.o[off + i] = __fmul_rn(__fmul_rn(a.o_norm[lane * C + i], __fmul_rn(o[i], inv)), sigmoid_near(a.gb[off + i]));
@@ -719,13 +754,13 @@ template <int DS>
 static void kda_rows(cudaStream_t st, const KdaArgs &a, const KdaScratch &x, int heads, int n_seq)
 {
     KdaPrep p{a, x.qn, x.kn, x.vn, x.al, x.beta, heads};
-    const dim3 pg((heads + 7) / 8, (a.T + KDA_RUN - 1) / KDA_RUN * n_seq);
-    if (a.K == 4) G5B_LAUNCH_PDL((kda_prep_kernel<DS, 4>), pg, dim3(256), 0, st, p);
-    else          G5B_LAUNCH_PDL((kda_prep_kernel<DS, 0>), pg, dim3(256), 0, st, p);
+    const dim3 pg(heads, (a.T + KDA_TILE - 1) / KDA_TILE * n_seq);
+    if (a.K == 4) G5B_LAUNCH_PDL((kda_prep_kernel<DS, 4>), pg, dim3(4 * DS), 0, st, p);
+    else          G5B_LAUNCH_PDL((kda_prep_kernel<DS, 0>), pg, dim3(4 * DS), 0, st, p);
     // (many positions: launched the ordinary way - launched early, its few long-running CTAs crowd the SMs that the preparation
     // leaves first, seven to an SM, and the others idle)
-    if (a.T > KDA_EARLY_T) G5B_LAUNCH((kda_scan_kernel<DS, 8, 2, 2>), dim3(heads * (DS / 16), n_seq), dim3(64), 0, st, p);
-    else if (a.T > 1)      G5B_LAUNCH_PDL((kda_scan_kernel<DS, 8, 2, 2>), dim3(heads * (DS / 16), n_seq), dim3(64), 0, st, p);
+    if (a.T > KDA_EARLY_T) G5B_LAUNCH((kda_scan_kernel<DS, 8, 1, 4>), dim3(heads * (DS / 16), n_seq), dim3(128), 0, st, p);
+    else if (a.T > 1)      G5B_LAUNCH_PDL((kda_scan_kernel<DS, 8, 1, 4>), dim3(heads * (DS / 16), n_seq), dim3(128), 0, st, p);
     else                   G5B_LAUNCH_PDL((kda_scan_kernel<DS, 4, 1, 4>), dim3(heads * (DS / 32), n_seq), dim3(128), 0, st, p);
     G5B_LAUNCH_PDL(kda_out_kernel<DS>, dim3((heads + 7) / 8, a.T * n_seq), dim3(256), 0, st, a, heads);
 }
