@@ -1188,11 +1188,14 @@ static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, f
         if (!forked) mla_absorb(e->st, e->mqa, flash ? e->mqt : nullptr, mq, kvb, nt, sl);
         else if (join && cudaStreamWaitEvent(e->st, e->side_done, 0) != cudaSuccess) cudaStreamSynchronize(e->side);
         if (rc) return -1;                         // (after the join: the side stream writes buffers of the next call; the reason is in g5b_last_error)
+        int attended = 0;
         if (flash) {
-            if (mla_attend_flash(e->st, cb, e->mqt, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf)) return -1;
+            attended = mla_attend_flash(e->st, cb, e->mqt, lat, e->msel, e->mnsel, e->mpart, e->mpart_bytes, e->mdsc, nt, at, sf,
+                                        wide || sf.H != Hl ? nullptr : e->macc + (size_t)t0 * Hl * c.v_head, kvb);      // (with heads added to fill a group, kv_b has no rows for them)
+            if (attended < 0) return -1;
         } else
             mla_attend(e->st, cb, e->mqa, lat, e->msel, e->mnsel, e->mdsc, e->mpart, e->mstats, e->mcount, MLA_PART_TOKENS, nt, at, sl);
-        if (!wide) mla_vout(e->st, e->macc + (size_t)t0 * Hl * c.v_head, cb, kvb, nt, sl);
+        if (!wide && !attended) mla_vout(e->st, e->macc + (size_t)t0 * Hl * c.v_head, cb, kvb, nt, sl);
     }
     for (int h = 0; h < Hl && wide; h += GEMV_MAX_SEG) {
         GemvSeg v[GEMV_MAX_SEG];

@@ -333,10 +333,11 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
 // The same attention core on the tensor cores (BF16 latent cache, kv_lora 512): scores and weighted
 // sums as mma.sync products on exact BF16 term splits, softmax per chunk of 64 positions and a
 // rescaling reduction. part / part_bytes: scratch for the chunks' partial rows; cstat: room for
-// [T][H][ceil((topk + KP) / 64)][2] doubles. 0, or -1 where the device refuses the kernel its shared memory.
+// [T][H][ceil((topk + KP) / 64)][2] doubles. With acc_out given it may do what mla_vout does in the reduction's launch: 1 then, 0 where cb
+// is what there is, -1 where the device refuses the kernel its shared memory.
 bool mla_flash_takes(const MlaShape &s);
 int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
-                     void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s);
+                     void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s, float *acc_out, const DMat &kv_b);
 void mla_vout(cudaStream_t st, float *acc_out, const float *cb, const DMat &kv_b, int T, const MlaShape &s);
 
 }  // namespace g5b

@@ -46,8 +46,9 @@ __device__ __forceinline__ float *seq_idx(float *idx_state, const MlaShape &s, i
 // (biased variance, eps 1e-6, FP64) and gate = gate x into the indexer state.
 __device__ void dsa_pool_one(float *idx_state, const float *ape, int pool, int i, const MlaShape &s);
 
-// Blocks [0, T) do the above; blocks [T, 2T) compute the RMSNorm factor of q_a's output for the same
-// positions (it used to be a launch of its own). With one new position, the block also closes the
+// Blocks [0, T) write the latents, [T, 2T) the indexer's keys and gates, [2T, 3T) the RMSNorm factors of q_a's output: all of it waits,
+// for memory, for sums over a block, for a root, and the three need nothing from each other (one block after the other did the
+// first two: 10.0 us for one position with its inputs from memory, 7.6 so). With one new position, the second block also closes the
 // pool that position completes (otherwise dsa_pool_kernel follows).
 __global__ void __launch_bounds__(256) mla_store_kernel(
     void *latent, float *idx_state, const float *ct_raw, const float *kv_norm_w, const float *wk_raw,
@@ -57,28 +58,29 @@ __global__ void __launch_bounds__(256) mla_store_kernel(
     pdl_trigger();
     pdl_wait();
     __shared__ double red[32];
-    if ((int)blockIdx.x >= T) {
-        const int tq = blockIdx.x - T;
-        const float *row = q_raw + (size_t)tq * s.q_lora;
-        double ssq = 0.0;
-        for (int i = threadIdx.x; i < s.q_lora; i += blockDim.x) ssq += (double)row[i] * (double)row[i];
-        ssq = block_sum(ssq, red);
-        if (threadIdx.x == 0) q_inv[tq] = (float)(1.0 / sqrt(ssq / (double)s.q_lora + (double)s.rms_eps));
+    const int part = blockIdx.x / T, t = blockIdx.x - part * T, pos = pos_of(s, cached, t);
+    if (part != 1) {
+        const int n = part ? s.q_lora : s.KL;
+        const float *row = part ? q_raw + (size_t)t * n : ct_raw + (size_t)t * n;
+        double ss = 0.0;
+#pragma unroll 8
+        for (int i = threadIdx.x; i < n; i += blockDim.x) ss += (double)row[i] * (double)row[i];
+        ss = block_sum(ss, red);
+        const float inv = (float)rsqrt_newton(ss / (double)n + (double)s.rms_eps);
+        if (part) {
+            if (threadIdx.x == 0) q_inv[t] = inv;
+            return;
+        }
+        latent = const_cast<void *>(seq_latent(latent, s, t));
+#pragma unroll 2
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const float v = __fmul_rn(kv_norm_w[i], __fmul_rn(row[i], inv));
+            if (s.latent_bf16) static_cast<uint16_t *>(latent)[(size_t)pos * n + i] = __bfloat16_as_ushort(__float2bfloat16_rn(v));
+            else               static_cast<float *>(latent)[(size_t)pos * n + i] = v;
+        }
         return;
     }
-    const int t = blockIdx.x, pos = pos_of(s, cached, t);
-    latent = const_cast<void *>(seq_latent(latent, s, t));
     idx_state = seq_idx(idx_state, s, t);
-    const float *ct = ct_raw + (size_t)t * s.KL;
-    double ss = 0.0;
-    for (int i = threadIdx.x; i < s.KL; i += blockDim.x) ss += (double)ct[i] * (double)ct[i];
-    ss = block_sum(ss, red);
-    const float inv = (float)(1.0 / sqrt(ss / (double)s.KL + (double)s.rms_eps));
-    for (int i = threadIdx.x; i < s.KL; i += blockDim.x) {
-        const float v = __fmul_rn(kv_norm_w[i], __fmul_rn(ct[i], inv));
-        if (s.latent_bf16) static_cast<uint16_t *>(latent)[(size_t)pos * s.KL + i] = __bfloat16_as_ushort(__float2bfloat16_rn(v));
-        else               static_cast<float *>(latent)[(size_t)pos * s.KL + i] = v;
-    }
     const float *raw = wk_raw + (size_t)t * s.ID;
     double sum = 0.0;
     for (int i = threadIdx.x; i < s.ID; i += blockDim.x) sum += (double)raw[i];
@@ -131,7 +133,7 @@ void mla_store(cudaStream_t st, void *latent, float *idx_state, const float *ct_
     const int pool0 = cached / s.KP;                                         // pools closed before this call
     const int pool1 = (cached + (s.batch ? 1 : T)) / s.KP;                   // pools closed after this call
     const int pool_here = ((T == 1 || s.batch) && pool1 > pool0) ? pool0 : -1;
-    G5B_LAUNCH_PDL(mla_store_kernel, 2 * T, 256, 0, st, latent, idx_state, ct_raw, kv_norm_w, wk_raw, gate_raw,
+    G5B_LAUNCH_PDL(mla_store_kernel, 3 * T, 256, 0, st, latent, idx_state, ct_raw, kv_norm_w, wk_raw, gate_raw,
                k_norm_w, k_norm_b, cached, s, q_raw, q_inv, T, ape, pool_here);
     if (pool1 > pool0 && pool_here < 0)
         G5B_LAUNCH(dsa_pool_kernel, pool1 - pool0, ((s.ID + 31) / 32) * 32, 0, st, idx_state, ape, pool0, s);
@@ -309,7 +311,8 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(int *sel, int *n
     for (int k = 0; k < TOPK_KEEP; k++) own[k] = tid + k * TOPK_THREADS < np ? sc[tid + k * TOPK_THREADS] : 0.f;
 
     // the keep-th largest key, one byte at a time from the top
-    // (most scores share their upper bits: a warp counts equal digits before it touches the histogram. The search ends as
+    // (most scores share their upper bits: a warp counts equal ones before it touches the histogram. The other digits are spread, and
+    // the lanes that still count few: 8192 pools 14.3 us with warps counting everywhere, 12.0 so. The search ends as
     // soon as the digit's pools are just those still wanted, usually after the score's own four bytes: the other four
     // only tell equal scores apart)
     if (tid == 0) { prefix_s = 0ull; want_s = keep; exact_s = 0; }
@@ -322,9 +325,12 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(int *sel, int *n
         auto count = [&](int i, float v) {
             const unsigned long long k = rank_key(v, i);
             const int digit = i < np && (k & mask) == prefix ? (int)((k >> shift) & 0xff) : -1;
-            const unsigned same = __match_any_sync(0xffffffffu, digit);
-            if (digit >= 0 && (tid & 31) == __ffs(same) - 1) atomicAdd(&hist[digit], __popc(same));
-            __syncwarp();
+            if (shift == 56) {
+                const unsigned same = __match_any_sync(0xffffffffu, digit);
+                if (digit >= 0 && (tid & 31) == __ffs(same) - 1) atomicAdd(&hist[digit], __popc(same));
+                __syncwarp();
+            } else if (digit >= 0)
+                atomicAdd(&hist[digit], 1);
         };
 #pragma unroll
         for (int k = 0; k < TOPK_KEEP; k++)
@@ -1257,13 +1263,10 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, flo
 // queries in few (64 queries in five: 98 us with the registers of 48, 27 so).
 constexpr int FL_MAX_SPLITS = 64;
 template <int FL_AHEAD>
-__global__ void __launch_bounds__(FL_KL) mla_flash_reduce_kernel(float *cb, const float *part, const double *cstat, const int *nsel,
-                                                               int cached, int splits, int span, MlaShape s)
+__device__ __forceinline__ float flash_column(const float *part, const double *cstat, const int *nsel, int cached, int splits, int span, const MlaShape &s, int h, int t)
 {
-    pdl_trigger();
-    pdl_wait();
     __shared__ double s_m[FL_MAX_SPLITS], s_w[FL_MAX_SPLITS], s_z[2];
-    const int h = blockIdx.x, t = blockIdx.y, p = pos_of(s, cached, t), tid = threadIdx.x;
+    const int p = pos_of(s, cached, t), tid = threadIdx.x;
     const float *pr = part + ((size_t)t * s.H + h) * splits * FL_KL + tid;
     float v[FL_AHEAD];
 #pragma unroll
@@ -1290,7 +1293,61 @@ __global__ void __launch_bounds__(FL_KL) mla_flash_reduce_kernel(float *cb, cons
 #pragma unroll
     for (int i = 0; i < FL_AHEAD; i++) if (i < used) acc = fma(s_w[i], (double)v[i], acc);
     for (int i = FL_AHEAD; i < used; i++) acc = fma(s_w[i], (double)__ldcg(pr + (size_t)i * FL_KL), acc);
-    cb[((size_t)t * s.H + h) * FL_KL + tid] = (float)(acc / (s_z[0] + s_z[1]));
+    return (float)(acc / (s_z[0] + s_z[1]));
+}
+
+template <int FL_AHEAD>
+__global__ void __launch_bounds__(FL_KL) mla_flash_reduce_kernel(float *cb, const float *part, const double *cstat, const int *nsel,
+                                                               int cached, int splits, int span, MlaShape s)
+{
+    pdl_trigger();
+    pdl_wait();
+    cb[((size_t)blockIdx.y * s.H + blockIdx.x) * FL_KL + threadIdx.x] = flash_column<FL_AHEAD>(part, cstat, nsel, cached, splits, span, s, blockIdx.x, blockIdx.y);
+}
+
+// The same sum and, for the few queries of a decode step, the value rows of kv_b behind it: a CTA takes FL_VROWS of a head's rows, whose
+// weights are asked for with the stretches' columns, and sums the stretches for itself (88 KB out of L2, twice a head). One launch and one way to
+// memory less: reduction and mla_vout_kernel one after the other 8.2 + 7.4 us for 43 stretches, 10.8 so; the layer of one query 130.7 -> 127.2 us. (48
+// columns at a time spill beside the weights: 128.8; four rows to a warp: 131.) From four queries on mla_vout's FP64 tiles take the
+// rows of all of them at once.
+constexpr int FL_VOUT_T = 4, FL_VWARP = 8, FL_VROWS = FL_KL / 32 * FL_VWARP;
+template <int FL_AHEAD>
+__global__ void __launch_bounds__(FL_KL) mla_flash_vout_kernel(float *acc_out, const uint16_t *w, const float *part, const double *cstat, const int *nsel,
+                                                             int cached, int splits, int span, MlaShape s)
+{
+    pdl_trigger();
+    __shared__ __align__(16) float x[FL_KL];
+    const int h = blockIdx.y, t = blockIdx.z, lane = threadIdx.x & 31, r0 = blockIdx.x * FL_VROWS + (threadIdx.x >> 5) * FL_VWARP;
+    uint4 wv[FL_VWARP][2];
+#pragma unroll
+    for (int r = 0; r < FL_VWARP; r++) {
+        const uint16_t *row = w + ((size_t)h * (s.qn + s.vh) + s.qn + min(r0 + r, s.vh - 1)) * FL_KL;
+        wv[r][0] = ld_stream16(row + lane * 8);
+        wv[r][1] = ld_stream16(row + 256 + lane * 8);
+    }
+    pdl_wait();
+    x[threadIdx.x] = flash_column<FL_AHEAD>(part, cstat, nsel, cached, splits, span, s, h, t);
+    __syncthreads();
+    float acc[FL_VWARP];
+#pragma unroll
+    for (int r = 0; r < FL_VWARP; r++) acc[r] = 0.f;
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+        const float4 xa = *reinterpret_cast<const float4 *>(x + g * 256 + lane * 8), xb = *reinterpret_cast<const float4 *>(x + g * 256 + lane * 8 + 4);
+#pragma unroll
+        for (int r = 0; r < FL_VWARP; r++) {
+            float v[8];
+            bf16x2_to_f32(wv[r][g].x, v[0], v[1]); bf16x2_to_f32(wv[r][g].y, v[2], v[3]);
+            bf16x2_to_f32(wv[r][g].z, v[4], v[5]); bf16x2_to_f32(wv[r][g].w, v[6], v[7]);
+            const float s0 = fmaf(v[6], xb.z, fmaf(v[4], xb.x, fmaf(v[2], xa.z, v[0] * xa.x))), s1 = fmaf(v[7], xb.w, fmaf(v[5], xb.y, fmaf(v[3], xa.w, v[1] * xa.y)));
+            acc[r] += s0 + s1;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < FL_VWARP; r++) {
+        acc[r] = warp_sum(acc[r]);
+        if (lane == r && r0 + r < s.vh) acc_out[((size_t)t * s.H + h) * s.vh + r0 + r] = acc[r];
+    }
 }
 
 bool mla_flash_takes(const MlaShape &s)
@@ -1298,9 +1355,10 @@ bool mla_flash_takes(const MlaShape &s)
     return s.latent_bf16 && s.KL == FL_KL && s.H % FL_HEADS == 0 && (s.topk + s.KP + FL_POS - 1) / FL_POS <= FL_MAX_SPLITS;
 }
 
+// Returns 1 when the value projection into acc_out (kv_b's value rows) is done too, 0 when cb is what there is, -1 on failure.
 // scratch: `part_bytes` bytes for the stretches' rows; `cstat` room for [T][H][splits][2] doubles.
 int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
-                     void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s)
+                     void *part, size_t part_bytes, double *cstat, int T, int cached, const MlaShape &s, float *acc_out, const DMat &kv_b)
 {
     static SmemGrant grant;
     if (!dev_opt_in_smem((const void *)mla_flash_kernel, FL_SMEM, grant)) return -1;
@@ -1319,6 +1377,12 @@ int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void 
                    static_cast<const __nv_bfloat16 *>(qterms), latent, sel, nsel, cached, splits, span, s);
     // (launched the ordinary way: launched early, its CTAs crowd the SMs beside the core's, of which two fit an SM - one
     // token at 2048 / 8192 / 32768 positions: MLA layer 102.4 / 112.6 / 120.9 us, 96.3 / 106.6 / 114.8 so)
+    if (splits > 1 && acc_out && T < FL_VOUT_T && kv_b.dt == DT_BF16 && (reinterpret_cast<uintptr_t>(kv_b.w) & 15) == 0) {
+        auto sum = splits > 8 ? mla_flash_vout_kernel<24> : mla_flash_vout_kernel<8>;
+        G5B_LAUNCH(sum, dim3((s.vh + FL_VROWS - 1) / FL_VROWS, s.H, T), FL_KL, 0, st, acc_out, static_cast<const uint16_t *>(kv_b.w), static_cast<const float *>(part), cstat, nsel,
+                   cached, splits, span, s);
+        return 1;
+    }
     if (splits > 1) {
         auto reduce = splits > 8 ? mla_flash_reduce_kernel<48> : mla_flash_reduce_kernel<8>;
         G5B_LAUNCH(reduce, dim3(s.H, T), FL_KL, 0, st, cb, static_cast<const float *>(part), cstat, nsel, cached, splits, span, s);
