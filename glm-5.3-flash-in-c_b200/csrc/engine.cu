@@ -1309,7 +1309,7 @@ static int ensure_ids(g5b_engine *e, size_t n)
 
 // Layers over T positions whose ids are already on the device, then the head for positions
 // [first, T): logits of position t land in e->logits row (t - first) % CHUNK, arg-max in
-// e->am_out[t].
+// e->am_out[t] where it is wanted (argmax_host given, or need_logits = false).
 // batch: the T ids are one new token for each of sequences 0..T-1 (T <= CHUNK), all at position
 // e->cached; logits_host then receives all T rows.
 // need_logits = false (greedy decode of one token): only the arg-max is wanted, so a connected
@@ -1354,7 +1354,7 @@ static int forward_device(g5b_engine *e, const int *ids_dev, int T, bool all_pos
         }
         GemvSeg head = make_seg(e->lm_head, e->xm, E, e->logits, c.vocab, e->inv_head, e->norm);
         if (proj_batch(e, &head, 1, n, true)) return -1;
-        argmax_rows(e->st, e->am_out + t0, e->logits, c.vocab, n, e->am_v, e->am_i);
+        if (argmax_host || !need_logits) argmax_rows(e->st, e->am_out + t0, e->logits, c.vocab, n, e->am_v, e->am_i);      // (nobody else reads it)
         if (logits_host && batch)
             CU(cudaMemcpyAsync(logits_host, e->logits, (size_t)n * c.vocab * 4, cudaMemcpyDeviceToHost, e->st));
         else if (logits_host && t0 + n == T)
