@@ -1123,9 +1123,11 @@ static bool mla_heads_split(const g5b_engine *e, const Layer &w, const MlaShape 
     return true;
 }
 
-// From this many positions on W_v multiplies all of a call's positions on the tensor cores, eight heads to a launch; its
-// eight launches cost more than mla_vout's one for fewer (64 positions: 145 us there; 2048: 4.6 ms there, 0.5 here).
-constexpr int VOUT_TC_MIN_T = 75;
+// From this many positions on W_v multiplies all of a call's positions on the tensor cores, eight heads to a launch, and the attention core
+// takes MLA_STEP of them at a time; for fewer those launches cost more than the core's and mla_vout's for 64 positions each (prompts of 75 / 100 / 128 /
+// 160 / 256 / 512 tokens, eight layers, two of them MLA: 6.28 / 6.82 / 7.41 / 8.28 / 10.60 / 17.48 ms on the tensor cores, 6.19 / 6.83 / 7.36 / 8.45 / 10.87 /
+// 18.43 in groups of 64).
+constexpr int VOUT_TC_MIN_T = 129;
 
 static int run_mla(g5b_engine *e, Layer &w, const float *x, int n, int cached, float *out, bool batch = false)
 {
