@@ -144,9 +144,9 @@ __global__ void __launch_bounds__(512) kda_core_kernel(const KdaArgs a)
     }
 }
 
-// Several positions of one sequence (prompts, the two-position pass of speculative decode), or one position each of
-// many sequences. What does not depend on the previous position - three convolutions with SiLU, the gate, the
-// l2norm sums - runs for all positions at once (kda_prep_kernel, a warp per position and head); the state update
+// Several positions of one sequence (prompts, the two-position pass of speculative decode), or, with a convolution of another
+// width than four, one position each of many sequences. What does not depend on the previous position - three convolutions with SiLU, the gate, the
+// l2norm sums - runs for all positions at once (kda_prep_kernel); the state update
 // alone walks the positions (kda_scan_kernel); the output's norm and gate follow for all positions at once
 // (kda_out_kernel).
 //
