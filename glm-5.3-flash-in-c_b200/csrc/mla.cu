@@ -1033,17 +1033,22 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
 // reference, src/core/glm53f_ops.c:879-911, accumulates in FP64 and rounds the score to float).
 // A CTA takes FL_HEADS heads of one query and a stretch of its visible positions, FL_POS of them at a time: it gathers the latent
 // rows into shared memory (the DSA selection is a list of row numbers), multiplies scores, takes exponentials, multiplies the weighted
-// sum and adds it to its own, in registers. A query's reference R for the exponents is its first chunk's maximum, and a later
-// one that exceeds it by 16 (the reference takes the maximum of all scores first; e^16 more is nothing to a float's range): so the sums
-// are hardly ever rescaled. Few queries are split
+// sum and adds it to its own, in registers. Those additions are Kahan's: what one rounds away is where the next chunk's products begin
+// to be added up, so that as many chunks as there are lose no more than two roundings (plain FP32 additions let go of everything that is small
+// beside the sum: 1800 positions of 2^-22 behind one of 256 were 2e-6 of the result). It is kept to eight bits, two to a register: sums and whole
+// remainders together do not fit the registers of two CTAs per SM. (64 queries of 2051 positions, the layer: 557 us with plain
+// additions, 575 so, 604 with remainders added up by Knuth's two-sum beside the sums, 618 before the loops were cut down to the registers.)
+// A query's reference R for the exponents is its first chunk's maximum, and rises by a multiple of ln 2 when a later
+// one exceeds it by 16 (the reference takes the maximum of all scores first; e^16 more is nothing to a float's range): so the sums
+// are hardly ever rescaled, and then without rounding. Few queries are split
 // into stretches, which a second kernel puts together.
 // Bound by mma.sync (1024 products per clock and SM, measured: a quarter of the tcgen05 rate) and nearly as much by shared memory: per chunk of
 // 48 positions x 16 heads 2300 cycles of products, 2350 of ldmatrix and the rest. A CTA is a chain of phases, so two of them share an SM: rows are kept
 // without padding (16-byte pieces of row r at place piece ^ (r & 7), which ldmatrix reads without conflicts) and probabilities
 // take the place of the scores' parts, 113 KB in all. Scores are dealt out as two groups of positions x four quarters of the columns: all
 // warps at all 512 columns of eight positions each read the query's 48 KB eight times over.
-// Measured, with the reduction: 64 queries of 2051 positions 437 -> 256 us, a prompt of 2048 6.9 -> 3.2 ms a layer (a chunk of 64 positions per CTA, its
-// sums in memory, before); one query 15.6 -> 19.5. Against the FP64 core on the same cache 1.3e-6 -> 3.5e-7: fewer and better ordered
+// Measured, with the reduction: 64 queries of 2051 positions 437 -> 256 us (274 with the remainders), a prompt of 2048 6.9 -> 3.2 ms a layer (a chunk of 64
+// positions per CTA, its sums in memory, before); one query 15.6 -> 19.5. Against the FP64 core on the same cache 1.3e-6 -> 3.5e-7: fewer and better ordered
 // truncations of the tensor cores' sums.
 constexpr int FL_POS = 48, FL_HEADS = 16, FL_KL = 512, FL_PPITCH = FL_POS + 8, FL_SPITCH = FL_POS + 8;
 constexpr int FL_THREADS = 256, FL_KQ = 4;
@@ -1073,6 +1078,12 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// x and y cut off to BF16
+__device__ __forceinline__ __nv_bfloat162 upper_halves(float x, float y)
+{
+    const uint32_t v = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+    return *reinterpret_cast<const __nv_bfloat162 *>(&v);
+}
 // part: [T][H][splits][KL] floats (unnormalised rows of a stretch), cstat: [T][H][splits][2] doubles (its reference, its sum of exponentials);
 // one stretch: the finished rows go to cb. span: chunks per stretch.
 __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, float *part, double *cstat, const __nv_bfloat16 *qterms, const void *latent,
@@ -1101,12 +1112,16 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, flo
     constexpr int PIECES = FL_KL / 8, PER = FL_POS * PIECES / FL_THREADS, QPER = 3 * FL_HEADS * PIECES / FL_THREADS;
     static_assert(FL_POS * PIECES % FL_THREADS == 0 && 3 * FL_HEADS * PIECES % FL_THREADS == 0, "pieces per thread");
     auto row_of = [&](int jj) { return jj < end ? (ns < 0 ? jj : sl[jj]) : -1; };
+    // this thread's rows are grow + 4 k: every second one has its pieces four places on (fl_at)
+    static_assert(FL_THREADS == 4 * PIECES, "rows per round of the gather");
+    const int grow = tid / PIECES, gpiece = tid % PIECES, gat = fl_at(grow, gpiece);
     auto gather = [&]() {
-#pragma unroll
+#pragma unroll 6
         for (int k = 0; k < PER; k++) {
-            const int i = tid + k * FL_THREADS, row = i / PIECES, piece = i % PIECES, j = s_rows[row];
-            if (j >= 0) cp_async16(cs + fl_at(row, piece), lat + (size_t)j * FL_KL + piece * 8);
-            else        *reinterpret_cast<uint4 *>(cs + fl_at(row, piece)) = make_uint4(0u, 0u, 0u, 0u);
+            const int j = s_rows[grow + 4 * k];
+            __nv_bfloat16 *o = cs + (gat ^ ((k & 1) * 32)) + 4 * k * FL_KL;
+            if (j >= 0) cp_async16(o, lat + (size_t)j * FL_KL + gpiece * 8);
+            else        *reinterpret_cast<uint4 *>(o) = make_uint4(0u, 0u, 0u, 0u);
         }
     };
     if (tid < FL_POS) s_rows[tid] = row_of(first + tid);
@@ -1124,13 +1139,13 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, flo
     const int pg = warp >> 2, kq = warp & 3;                        // scores: positions 24 pg .., columns 128 kq ..
     const int row = 2 * warp + (lane >> 4), l16 = lane & 15;        // exponentials: this lane's head, positions l16, l16 + 16, l16 + 32
     const int arow = (lane & 7) + 8 * ((lane >> 3) & 1), ahalf = lane >> 4;
-    float ref = -INFINITY;
-    double z = 0.0;
-    float sum[8][4];                                                // weighted sums: columns 64 warp + 8 n + 2 (lane % 4), heads lane / 4 and + 8
+    double z = 0.0, ref = -INFINITY;
+    float2 sum[8][2];                                               // weighted sums: columns 64 warp + 8 n + 2 (lane % 4) and the next, heads lane / 4 and + 8
+    __nv_bfloat162 rest[8][2];                                      // what the last addition to them rounded away, to eight bits
 #pragma unroll
     for (int n = 0; n < 8; n++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) sum[n][i] = 0.f;
+        for (int i = 0; i < 2; i++) { sum[n][i] = make_float2(0.f, 0.f); rest[n][i] = __floats2bfloat162_rn(0.f, 0.f); }
 
 #pragma unroll 1
     for (int j0 = first; j0 < end; j0 += FL_POS) {
@@ -1143,7 +1158,7 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, flo
 #pragma unroll
             for (int n = 0; n < 3; n++) c[n][0] = c[n][1] = c[n][2] = c[n][3] = 0.f;
             const int b4 = pg * 24 + (lane & 7) + 8 * (lane >> 4), b2 = pg * 24 + 16 + (lane & 7), bhalf = (lane >> 3) & 1;
-#pragma unroll 2
+#pragma unroll 1
             for (int k = 0; k < 8; k++) {
                 const int piece = kq * 16 + k * 2;
                 uint32_t b[4], d[2];
@@ -1180,15 +1195,21 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, flo
             }
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if (!(m <= ref + 16.f)) {                               // (the first chunk, a score much larger, NaN)
-                const double f = exp((double)ref - (double)m);
-                scale = (float)f;
-                z *= f;
-                ref = m;
+            if (!((double)m <= ref + 16.0)) {                       // (the first chunk, a score much larger, NaN)
+                const double d = (double)m - ref;
+                if (d < 80.0) {                                     // by a power of two, which takes nothing from the sums
+                    const double k = rint(d * 1.4426950408889634);
+                    scale = __int_as_float((127 - (int)k) << 23);
+                    ref = fma(k, 0.6931471805599453, ref);
+                } else {                                            // the first chunk, whose sums are zero; or nothing of the others is left
+                    scale = ref == -INFINITY ? 1.f : 0.f;
+                    ref = (double)m;
+                }
+                z *= (double)scale;
             }
 #pragma unroll
             for (int k = 0; k < 3; k++) {
-                const double x = j0 + l16 + 16 * k < end ? exp((double)v[k] - (double)ref) : 0.0;
+                const double x = j0 + l16 + 16 * k < end ? exp((double)v[k] - ref) : 0.0;
                 z += x;
                 e[k] = (float)x;
             }
@@ -1205,32 +1226,40 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, flo
         if (__syncthreads_or(scale != 1.f)) {
             const float f0 = s_scale[lane >> 2], f1 = s_scale[(lane >> 2) + 8];
 #pragma unroll
-            for (int n = 0; n < 8; n++) { sum[n][0] *= f0; sum[n][1] *= f0; sum[n][2] *= f1; sum[n][3] *= f1; }
+            for (int n = 0; n < 8; n++) {
+                sum[n][0].x *= f0; sum[n][0].y *= f0; rest[n][0] = __hmul2(rest[n][0], __floats2bfloat162_rn(f0, f0));
+                sum[n][1].x *= f1; sum[n][1].y *= f1; rest[n][1] = __hmul2(rest[n][1], __floats2bfloat162_rn(f1, f1));
+            }
         }
-        // ---- weighted sum of the rows: this warp's 64 columns for the 16 heads
+        // ---- weighted sum of the rows: this warp's 64 columns for the 16 heads, 16 of them at a time
 #pragma unroll
-        for (int half = 0; half < 2; half++) {
-            float acc[4][4];
+        for (int quarter = 0; quarter < 4; quarter++) {
+            float acc[2][4];
 #pragma unroll
-            for (int n = 0; n < 4; n++) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
-            uint32_t b[FL_POS / 16][2][4];
+            for (int n = 0; n < 2; n++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) { const float2 r = __bfloat1622float2(rest[quarter * 2 + n][i]); acc[n][2 * i] = r.x; acc[n][2 * i + 1] = r.y; }
+            uint32_t b[FL_POS / 16][4];
 #pragma unroll
             for (int k = 0; k < FL_POS / 16; k++)
-#pragma unroll
-                for (int n = 0; n < 2; n++) ldsm_x4_trans(b[k][n], cs + fl_at(k * 16 + (lane & 15), warp * 8 + half * 4 + n * 2 + (lane >> 4)));
+                ldsm_x4_trans(b[k], cs + fl_at(k * 16 + (lane & 15), warp * 8 + quarter * 2 + (lane >> 4)));
 #pragma unroll
             for (int term = 2; term >= 0; term--)                   // (the small terms first: the tensor cores truncate to the sum's last place)
 #pragma unroll
                 for (int k = 0; k < FL_POS / 16; k++) {
                     uint32_t a[4];
                     ldsm_x4(a, ps + (size_t)(term * FL_HEADS + arow) * FL_PPITCH + k * 16 + 8 * ahalf);
-#pragma unroll
-                    for (int n = 0; n < 2; n++) { mma_bf16(acc[2 * n], a, b[k][n][0], b[k][n][1]); mma_bf16(acc[2 * n + 1], a, b[k][n][2], b[k][n][3]); }
+                    mma_bf16(acc[0], a, b[k][0], b[k][1]); mma_bf16(acc[1], a, b[k][2], b[k][3]);
                 }
 #pragma unroll
-            for (int n = 0; n < 4; n++)
+            for (int n = 0; n < 2; n++)
 #pragma unroll
-                for (int i = 0; i < 4; i++) sum[half * 4 + n][i] = __fadd_rn(sum[half * 4 + n][i], acc[n][i]);
+                for (int i = 0; i < 2; i++) {
+                    float2 &u = sum[quarter * 2 + n][i];
+                    const float x0 = acc[n][2 * i], x1 = acc[n][2 * i + 1], t0 = __fadd_rn(u.x, x0), t1 = __fadd_rn(u.y, x1), y0 = __fsub_rn(t0, u.x), y1 = __fsub_rn(t1, u.y);
+                    rest[quarter * 2 + n][i] = upper_halves(__fsub_rn(x0, y0), __fsub_rn(x1, y1));
+                    u.x = t0; u.y = t1;
+                }
         }
         __syncthreads();                                            // the rows have been read
         if (j0 + FL_POS < end) gather();
@@ -1241,19 +1270,23 @@ __global__ void __launch_bounds__(FL_THREADS, 2) mla_flash_kernel(float *cb, flo
         s_z[row] = z;
         if (splits > 1) {
             double *st = cstat + (((size_t)t * s.H + h0 + row) * splits + split) * 2;
-            st[0] = (double)ref;
+            st[0] = ref;
             st[1] = z;
         }
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 4; i += 2) {
-        const int r = (lane >> 2) + 4 * i;
+    for (int i = 0; i < 2; i++) {
+        const int r = (lane >> 2) + 8 * i;
         const double inv = splits > 1 ? 1.0 : 1.0 / s_z[r];
         float *o = (splits > 1 ? part + (((size_t)t * s.H + h0 + r) * splits + split) * FL_KL : cb + ((size_t)t * s.H + h0 + r) * FL_KL) + warp * 64 + 2 * (lane & 3);
 #pragma unroll
-        for (int n = 0; n < 8; n++)
-            *reinterpret_cast<float2 *>(o + n * 8) = make_float2((float)((double)sum[n][i] * inv), (float)((double)sum[n][i + 1] * inv));
+        for (int n = 0; n < 8; n++) {
+            const float a = sum[n][i].x, b = sum[n][i].y;
+            const float2 c = __bfloat1622float2(rest[n][i]);       // (not a number where the sum is infinite)
+            const double da = (double)a + (c.x == c.x ? (double)c.x : 0.0), db = (double)b + (c.y == c.y ? (double)c.y : 0.0);
+            *reinterpret_cast<float2 *>(o + n * 8) = make_float2((float)(da * inv), (float)(db * inv));
+        }
     }
 }
 
