@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(256) kda_out_kernel(const KdaArgs a, int heads
 // Bound by the states' way from HBM and back (64 sequences of 64 heads: 0.54 GB, 82 us). The three kernels above, of which the scan
 // read a state in pieces of 32 bytes, took 171 us a layer (27 + 139 + 5); here a thread holds two columns of 32 rows, asked for
 // before anything else, so that 128 KB are on their way to an SM while the convolutions, norms and gates of the two CTAs on it are
-// computed. Arithmetic as above: products fused, sums in parts. 64 sequences:
+// computed. Arithmetic as above: products fused, sums in parts of eight rows. 64 sequences:
 // 111 us, 7: 17.3 (34 before); a step of 64 sequences over eight layers 6.80 -> 6.39 ms.
 template <int DS>
 __global__ void __launch_bounds__(256, 2) kda_each_kernel(const KdaArgs a)
@@ -515,17 +515,21 @@ __global__ void __launch_bounds__(256, 2) kda_each_kernel(const KdaArgs a)
         if (tid < D && lane == 0) red[warp][2] = qk;
     }
     const float beta = sigmoid_near(braw);
-    F2 u = f2(0.f, 0.f), o = u;
+    F2 u[4], o[4];                                                  // four sums of eight rows each (one of 32: 1.4 times the rounding error, and no faster)
+#pragma unroll
+    for (int j = 0; j < 4; j++) u[j] = o[j] = f2(0.f, 0.f);
     const float4 *al4 = reinterpret_cast<const float4 *>(sal + rg * R), *k4 = reinterpret_cast<const float4 *>(sk + rg * R), *q4 = reinterpret_cast<const float4 *>(sq + rg * R);
 #pragma unroll
     for (int i = 0; i < R / 4; i++) {
         const float4 al = al4[i], k = k4[i], q = q4[i];
         s[4 * i] = f2_mul(s[4 * i], f2(al.x, al.x)); s[4 * i + 1] = f2_mul(s[4 * i + 1], f2(al.y, al.y));
         s[4 * i + 2] = f2_mul(s[4 * i + 2], f2(al.z, al.z)); s[4 * i + 3] = f2_mul(s[4 * i + 3], f2(al.w, al.w));
-        u = f2_fma(s[4 * i], f2(k.x, k.x), u); u = f2_fma(s[4 * i + 1], f2(k.y, k.y), u); u = f2_fma(s[4 * i + 2], f2(k.z, k.z), u); u = f2_fma(s[4 * i + 3], f2(k.w, k.w), u);
-        o = f2_fma(s[4 * i], f2(q.x, q.x), o); o = f2_fma(s[4 * i + 1], f2(q.y, q.y), o); o = f2_fma(s[4 * i + 2], f2(q.z, q.z), o); o = f2_fma(s[4 * i + 3], f2(q.w, q.w), o);
+        u[0] = f2_fma(s[4 * i], f2(k.x, k.x), u[0]); u[1] = f2_fma(s[4 * i + 1], f2(k.y, k.y), u[1]);
+        u[2] = f2_fma(s[4 * i + 2], f2(k.z, k.z), u[2]); u[3] = f2_fma(s[4 * i + 3], f2(k.w, k.w), u[3]);
+        o[0] = f2_fma(s[4 * i], f2(q.x, q.x), o[0]); o[1] = f2_fma(s[4 * i + 1], f2(q.y, q.y), o[1]);
+        o[2] = f2_fma(s[4 * i + 2], f2(q.z, q.z), o[2]); o[3] = f2_fma(s[4 * i + 3], f2(q.w, q.w), o[3]);
     }
-    us[rg][cp] = u; os[rg][cp] = o;
+    us[rg][cp] = f2_add(f2_add(u[0], u[1]), f2_add(u[2], u[3])); os[rg][cp] = f2_add(f2_add(o[0], o[1]), f2_add(o[2], o[3]));
     __syncthreads();
     float ux = 0.f, uy = 0.f, ox = 0.f, oy = 0.f;
 #pragma unroll
