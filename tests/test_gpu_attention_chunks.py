@@ -78,3 +78,22 @@ def test_several_chunks_match_the_fp64_core(gpu_lib, index_topk, cached, T, risi
     assert np.isfinite(got).all()
     assert common.rel_err(got, want) < (2e-5 if rising else 2e-6)
     eng.close()
+
+
+@pytest.mark.parametrize("index_topk,T,taken", [(3064, 1, True), (3080, 1, True), (3080, 64, True), (4092, 1, True), (4092, 5, True), (4096, 1, False)])
+def test_as_many_positions_as_the_core_takes(gpu_lib, index_topk, T, taken):
+    """Up to 4096 positions a query, 86 chunks and more than the second kernel has places for stretches; beyond, the FP64 core
+    (the same bits with and without the option). Scores below 4: the bound of the test above."""
+    cap, cached = 4608, 4500
+    eng, c = _layer(index_topk, cap)
+    rng = np.random.default_rng(10)
+    eng.state_write(0, 1, 0, synth.bf16_round(rng.standard_normal((cap, KL)).astype(np.float32)))
+    eng.state_write(0, 2, 0, rng.standard_normal(2 * cap * c.index_dim + (cap // c.index_kpool) * c.index_dim).astype(np.float32))
+    x = rng.standard_normal((T, HIDDEN)).astype(np.float32)
+    got, sel = eng.op_mla(0, x, cached)
+    eng.set_option("mla_tensor", 0)
+    want, sel64 = eng.op_mla(0, x, cached)
+    assert np.array_equal(sel, sel64) and len(sel) >= index_topk
+    assert np.array_equal(got, want) != taken
+    assert common.rel_err(got, want) < 2e-6
+    eng.close()
