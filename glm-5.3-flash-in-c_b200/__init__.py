@@ -201,7 +201,12 @@ class _ResultPool:
                 return None
             self.made[size] = self.made.get(size, 0) + 1
             self.bytes += size
-        return self.L.g5b_host_alloc(size)
+        ptr = self.L.g5b_host_alloc(size)
+        if not ptr:                                  # none to be had now: a later call may ask again
+            with self.lock:
+                self.made[size] -= 1
+                self.bytes -= size
+        return ptr
 
     def array(self, shape):
         n = 4 * math.prod(shape)

@@ -15,10 +15,13 @@ N = 1 << 16                     # floats: 256 KB
 class FakeLib:
     """g5b_host_alloc / g5b_host_free on ordinary memory, counted."""
 
-    def __init__(self):
-        self.live, self.allocs = {}, 0
+    def __init__(self, fails=0):
+        self.live, self.allocs, self.fails = {}, 0, fails
 
     def g5b_host_alloc(self, size):
+        if self.fails > 0:
+            self.fails -= 1
+            return None
         buf = ctypes.create_string_buffer(size)
         self.allocs += 1
         self.live[ctypes.addressof(buf)] = buf
@@ -71,3 +74,19 @@ def test_threads_share_a_pool():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not errors
+
+
+def test_pieces_that_could_not_be_had_are_not_counted():
+    """Memory that cannot be pinned now may be there later: as many failures as a size may have pieces do not close it."""
+    lib = FakeLib(fails=pkg._ResultPool.KEEP + 1)
+    pool = pkg._ResultPool(lib)
+    pool.reserve(4 * N, 2)
+    for _ in range(pool.KEEP - 1):
+        assert pool.array((N,)).base is None                  # an ordinary array meanwhile
+    assert pool.bytes == 0 and lib.fails == 0
+    held = [pool.array((N,)) for _ in range(pool.KEEP + 1)]
+    assert lib.allocs == len(lib.live) == pool.KEEP and pool.bytes == pool.KEEP * 4 * N
+    del held
+    gc.collect()
+    pool.close()
+    assert not lib.live
