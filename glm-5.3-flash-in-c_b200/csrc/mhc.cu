@@ -1045,9 +1045,11 @@ __global__ void __cluster_dims__(HCC_CTAS, 1, 1) __launch_bounds__(HCG_THREADS, 
     cluster_wait();
 }
 
-// From here on eight positions to a cluster are faster than one (alone, 5 us of launch included: 12 positions 26.7 against 20.5 us,
-// 16: 26.7 and 27.7, 32: 26.7 and 27.6, 40: 27.6 and 45)
-constexpr int HCG_MIN_T = 16;
+// From here on eight positions to a cluster (hc_pre_group_kernel) are as fast as a cluster for each (hc_pre_one_kernel), or faster. Alone, 5 us of launch
+// included, a site takes 24.6 us with the former at any of these sizes and with the latter 14.4 up to 15 positions, which all run at once, 24.6 from 16
+// on, 32.8 for 32, 51 for 64; with the streams' expansion 26.7 against 18.5 for 15, 26.8 for 16, 28.7 for 18, 39 for 32. A KDA + MoE layer of 12
+// sequences 280 us against 260, of 16: 292.4 and 289.8, of 18: 304 both, of 32: 347 and 366.
+constexpr int HCG_MIN_T = 17;
 
 static bool hc_pre_cluster_takes(int M, int E)
 {

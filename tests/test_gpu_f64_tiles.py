@@ -18,7 +18,7 @@ def _config(**kw):
                                 norm_topk=1, swiglu_limit=10.0, fp8_block_r=128, fp8_block_c=128), **kw})
 
 
-@pytest.mark.parametrize("hidden,T", [(512, 16), (512, 17), (640, 23), (640, 70), (4096, 31)])
+@pytest.mark.parametrize("hidden,T", [(512, 16), (512, 17), (640, 23), (512, 24), (640, 70), (4096, 31)])
 def test_mixing_sites_in_groups_of_eight(gpu_lib, binding, hidden, T):
     """Whole and ragged groups of eight; 64, 80 and 512 columns per CTA; with and without a pending stream expansion."""
     c = _config(hidden=hidden)
