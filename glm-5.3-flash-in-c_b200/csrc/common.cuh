@@ -133,7 +133,7 @@ __device__ __forceinline__ float expf_near(float x)
 
 // 1 / d rounded to nearest, d from 1 on: the estimate and one step of Newton's, whose residual is exact in a fused product, without the
 // branch that a division has for its special cases - a dozen of them in a row waited for each other. Equal to the division for every
-// mantissa (all 2^23 compared); 0 for an infinite d, NaN for NaN; from 2^126 on (subnormal results) off by less than one of their units.
+// mantissa (the test goes through all 2^23); 0 for an infinite d, NaN for NaN; from 2^126 on (subnormal results) off by less than one of their units.
 // (Taken of d / 2^26, so that neither the argument nor the estimate leaves the range of normal numbers.)
 __device__ __forceinline__ float rcp_estimate(float d)
 {

@@ -37,3 +37,17 @@ def test_sigmoid_by_pairs_is_the_rounded_quotient(gpu_lib):
     unused = np.empty_like(x)
     assert gpu_lib.g5b_debug_exp(x.ctypes.data, x.size, unused.ctypes.data, s.ctypes.data, 0) == 0
     assert np.array_equal(s, (np.float32(1) / (np.float32(1) + e)).astype(np.float32), equal_nan=True)
+
+
+def test_reciprocal_of_every_mantissa(gpu_lib):
+    """Arguments whose 1 + exp(-x) runs through all 2^23 floats from 1 to 2: x is off by half of its last place and the exponential by
+    0.53 of its own, together less than half the distance of two of these sums. Bit for bit the divided ones."""
+    n = 1 << 23
+    x = np.full(n, 200.0, np.float32)
+    x[1:] = -np.log(np.arange(1, n) / n)
+    minus, e, s, unused = -x, np.empty_like(x), np.empty_like(x), np.empty_like(x)
+    assert gpu_lib.g5b_debug_exp(minus.ctypes.data, n, e.ctypes.data, unused.ctypes.data, 0) == 0
+    assert gpu_lib.g5b_debug_exp(x.ctypes.data, n, unused.ctypes.data, s.ctypes.data, 0) == 0
+    d = np.float32(1) + e
+    assert np.array_equal(d.view(np.uint32), np.arange(n, dtype=np.uint32) + np.float32(1).view(np.uint32))
+    assert np.array_equal(s, np.float32(1) / d)
