@@ -331,9 +331,9 @@ void mla_attend(cudaStream_t st, float *cb, const double *qa, const void *latent
                 const int *nsel, double *dsc, double *part, double *stats, int *counters, int part_tokens, int T,
                 int cached, const MlaShape &s);
 // The same attention core on the tensor cores (BF16 latent cache, kv_lora 512): scores and weighted
-// sums as mma.sync products on exact BF16 term splits, softmax per chunk of 64 positions and a
-// rescaling reduction. part / part_bytes: scratch for the chunks' partial rows; cstat: room for
-// [T][H][ceil((topk + KP) / 64)][2] doubles. With acc_out given it may do what mla_vout does in the reduction's launch: 1 then, 0 where cb
+// sums as mma.sync products on exact BF16 term splits, 48 positions at a time under a running maximum; a query may be cut into
+// stretches, at most 64, whose rows a second kernel puts together. part / part_bytes: scratch for those rows, as many stretches as fit;
+// cstat: room for [T][H][stretches][2] doubles, [min(T, 64)][H][topk + KP] of them always do. With acc_out given it may do what mla_vout does in the reduction's launch: 1 then, 0 where cb
 // is what there is, -1 where the device refuses the kernel its shared memory.
 bool mla_flash_takes(const MlaShape &s);
 int mla_attend_flash(cudaStream_t st, float *cb, const void *qterms, const void *latent, const int *sel, const int *nsel,
