@@ -69,7 +69,10 @@ inline void gemv(cudaStream_t st, const DMat &m, const float *x, int ldx, float 
 // FP8 block-scaled (128 x 128 blocks) and BF16 matrices times 2 positions or more on tcgen05 tensor
 // cores, weights streamed once by TMA; activations as exact 16-bit term sums. Matrices of one format and
 // width go out in one launch. err: where a bounded wait that ran out is recorded (tc_gemm_recover after it).
-constexpr int TC_TILE_SHIFT = 5;     // log2 of the rows of one expert that a weight tile is multiplied with at once, at most (every role counts tiles)
+// Rows of one expert that a weight tile is multiplied with at once, at most, in a call of T tokens (every role counts tiles). An expert has more
+// rows than the call has tokens where places that nothing selectable is left for (scores of a NaN row) all go to expert 0.
+constexpr int TC_TILE_ROWS = 32;
+inline int tc_tile_rows(int T) { return T < TC_TILE_ROWS ? (T + 7) & ~7 : TC_TILE_ROWS; }
 struct TcGemm;
 TcGemm *tc_gemm_create(int max_c, int max_ec, int max_t, int *err);      // widest input, that of an expert, most positions
 void tc_gemm_free(TcGemm *g);
@@ -141,9 +144,10 @@ struct MoePlan {          // device arrays describing which expert multiplies wh
     int *slot_cnt;        // [max_slots] pairs of the slot
     int *pair_tok;        // [max_pairs] activation row of the pair
     int *pair_dst;        // [max_pairs] row of the contribution buffer the pair writes
-    int *slot_tile0;      // [max_slots + 1] first token tile of the slot (tiles of at most 1 << TC_TILE_SHIFT pairs)
+    int *slot_tile0;      // [max_slots + 1] first token tile of the slot (tiles of at most tile_rows pairs)
     int *n_pairs;         // [1] pairs of all slots
     int  max_slots, max_pairs;
+    int  tile_rows;       // tc_tile_rows of the call (router_plan)
 };
 struct MoeShape {
     int E, I, NE, K, br, bc, dt;       // dt of expert matrices

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     int pairs = 0, slots = 0, tiles = 0;
     for (int k = 0; k < per; k++) {
         const int le = tid * per + k;
-        if (le < a.n_local && cnt[le]) { pairs += cnt[le]; slots++; tiles += (cnt[le] + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT; }
+        if (le < a.n_local && cnt[le]) { pairs += cnt[le]; slots++; tiles += (cnt[le] + a.p.tile_rows - 1) / a.p.tile_rows; }
     }
     psum[tid] = pairs; ssum[tid] = slots; tsum[tid] = tiles;
     __syncthreads();
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
         if (cnt[le]) {
             a.p.slot_expert[sbase] = le; a.p.slot_off[sbase] = pbase; a.p.slot_cnt[sbase] = cnt[le];
             a.p.slot_tile0[sbase] = tbase;
-            pbase += cnt[le]; sbase++; tbase += (cnt[le] + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT;
+            pbase += cnt[le]; sbase++; tbase += (cnt[le] + a.p.tile_rows - 1) / a.p.tile_rows;
         }
     }
     __syncthreads();
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) router_kernel(const RouterArgs 
     }
     if (tid == 0) {
         a.p.slot_tile0[total_slots] = total_tiles;
-        if (shared) a.p.slot_tile0[total_slots + 1] = total_tiles + ((a.sh_n + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT);
+        if (shared) a.p.slot_tile0[total_slots + 1] = total_tiles + (a.sh_n + a.p.tile_rows - 1) / a.p.tile_rows;
         *a.p.n_slots = total_slots + (shared ? 1 : 0);
         *a.p.n_pairs = total_pairs + (shared ? a.sh_n : 0);
     }
@@ -252,7 +252,7 @@ __device__ __forceinline__ void group_pairs(const int *idx, int T, int K, int n_
     }
     __syncthreads();
     const int mine = tid < n_local ? cnt[tid] : 0;
-    int v[3] = {mine, mine > 0, (mine + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT}, own[3];
+    int v[3] = {mine, mine > 0, (mine + p.tile_rows - 1) / p.tile_rows}, own[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         own[k] = v[k];
@@ -291,7 +291,7 @@ __device__ __forceinline__ void group_pairs(const int *idx, int T, int K, int n_
     if (tid == 0) {
         if (shared) { p.slot_expert[total[1]] = n_local; p.slot_off[total[1]] = total[0]; p.slot_cnt[total[1]] = sh_n; }
         p.slot_tile0[total[1]] = total[2];
-        if (shared) p.slot_tile0[total[1] + 1] = total[2] + ((sh_n + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT);
+        if (shared) p.slot_tile0[total[1] + 1] = total[2] + (sh_n + p.tile_rows - 1) / p.tile_rows;
         *p.n_slots = total[1] + shared;
         *p.n_pairs = total[0] + (shared ? sh_n : 0);
     }
@@ -390,9 +390,11 @@ __global__ void __launch_bounds__(RS_THREADS) router_select_kernel(const RouterA
 constexpr int RT_TILE_MIN_T = 2, RT_TILE_CTAS = 1200, RT_MAX_PARTS = 32;
 // p may be null-planned (p.n_slots == nullptr) when only the routing is wanted.
 void router_plan(cudaStream_t st, int *idx, float *w, float *score, const float *x, int ldx, const void *gate,
-                 int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &p, int with_shared,
+                 int gate_dt, const float *bias, int T, const MoeShape &s, const MoePlan &plan, int with_shared,
                  int *counter, int shared_t0, int shared_n, double *dots)
 {
+    MoePlan p = plan;
+    p.tile_rows = tc_tile_rows(T);
     const bool one = T <= RT_MAX_TOKENS;
     // From RT_TILE_MIN_T tokens on the dot products go first, in tiles and so many stretches of the columns that there are a few
     // CTAs per SM, then the selection (7 tokens: 5.9 + 9.8 us, in one kernel 20.4; 64: 14.6 + 10.5).

@@ -92,18 +92,18 @@ struct TsArgs {
     int *err;
 };
 
-// How a slot's cnt rows are cut into tiles: equal shares of at most 1 << TC_TILE_SHIFT rows, rounded up to 8.
-__device__ __forceinline__ int ts_tile_rows(int cnt)
+// How a slot's cnt rows are cut into tiles: equal shares of at most `most` rows (a multiple of 8), rounded up to 8.
+__device__ __forceinline__ int ts_tile_rows(int cnt, int most)
 {
-    if (cnt <= 1 << TC_TILE_SHIFT) return (cnt + 7) & ~7;
-    const int k = (cnt + (1 << TC_TILE_SHIFT) - 1) >> TC_TILE_SHIFT;
+    if (cnt <= most) return (cnt + 7) & ~7;
+    const int k = (cnt + most - 1) / most;
     return ((cnt + k - 1) / k + 7) & ~7;
 }
 
 // Walks the tiles of a CTA's share in order: matrix (or expert) `which`, its row tile rt, the np activation rows from
 // row0 on, n = np rounded up to 8. An expert's row tile goes past its token tiles one after the other: its weights
 // come from L2 then.
-struct TsPlan { const int *tile0, *off, *cnt, *exp; int slots; };
+struct TsPlan { const int *tile0, *off, *cnt, *exp; int slots, rows; };
 template <int MODE>
 struct TsCursor {
     int which, rt, row0, np, n;
@@ -124,7 +124,7 @@ struct TsCursor {
     }
     __device__ __forceinline__ void enter(const TsPlan &p)
     {
-        which = p.exp[slot]; cnt = p.cnt[slot]; rows = ts_tile_rows(cnt); nt = p.tile0[slot + 1] - p.tile0[slot];
+        which = p.exp[slot]; cnt = p.cnt[slot]; rows = ts_tile_rows(cnt, p.rows); nt = p.tile0[slot + 1] - p.tile0[slot];
     }
     __device__ __forceinline__ void start(const TsArgs &a, const TsPlan &p, int tile)
     {
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_stream_fp8_kernel(const 
 // for batches of few rows per expert are no faster any more (64 tokens 327 + 168, 150: 480 + 226 against 427 + 208).
 //
 // Warps: 0-7 epilogue (two groups), 8-15 conversion, 16 weights and items, 17 terms, 18 and 19 MMA.
-constexpr int TP_ROWS = 1 << TC_TILE_SHIFT, TP_RING = 4, TP_MAX_WS = 6, TP_MAX_XS = 4, TP_PARTS = 4;
+constexpr int TP_ROWS = TC_TILE_ROWS, TP_RING = 4, TP_MAX_WS = 6, TP_MAX_XS = 4, TP_PARTS = 4;
 constexpr int TP_SLAB = TP_ROWS * 128;       // values of one quarter's sums of 128 rows of W
 constexpr int TP_DYN = 3;                    // claimed tiles at most, per CTA
 struct TpItem {
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(TS_FP8_THREADS, 1) tc_pair_kernel(const __grid
     tc_fence_before();
     pdl_wait();                                                            // (the plan, the terms, the counters)
     int n_tiles = a.tiles;
-    TsPlan plan{s_plan, s_plan + a.slots + 1, s_plan + 2 * a.slots + 1, s_plan + 3 * a.slots + 1, 0};
+    TsPlan plan{s_plan, s_plan + a.slots + 1, s_plan + 2 * a.slots + 1, s_plan + 3 * a.slots + 1, 0, a.n};
     if (MODE != TS_DENSE) {
         plan.slots = min(*a.p.n_slots, a.slots);
 #pragma unroll 1
@@ -1441,7 +1441,7 @@ bool tc_moe_takes(const TcGemm *g, const MoeShape &s, int T)
     if (!g || T < 1 || T > g->max_t || s.E > g->max_ec || s.I > g->max_ec || s.dt != DT_FP8 || s.br != 128 || s.bc != 128 || s.E % 128 || s.I % 128) return false;
     if (!(s.limit > 0.f) || s.limit * s.limit > 60000.f) return false;                  // activations must fit F16
     const int slots = (T * s.K < s.n_local ? T * s.K : s.n_local) + 1;
-    return (long)(slots + ((T * s.K + T) >> TC_TILE_SHIFT)) * (s.I / 128 > (s.E + 255) / 256 ? s.I / 128 : (s.E + 255) / 256) <= (1 << 24);
+    return (long)(slots + (T * s.K + T) / tc_tile_rows(T)) * (s.I / 128 > (s.E + 255) / 256 ? s.I / 128 : (s.E + 255) / 256) <= (1 << 24);
 }
 
 static const std::pair<CUtensorMap, CUtensorMap> *expert_maps(TcGemm *g, const ExpertSlab &w, const MoeShape &s)
@@ -1473,7 +1473,7 @@ int tc_moe_run(TcGemm *g, cudaStream_t st, float *contrib, void *act, void *xter
     G5B_LAUNCH_PDL(tc_split_kernel<true>, dim3(pairs), dim3(512), 0, st, sp);
     TsMaps m;
     TsArgs a{};
-    a.T = T; a.n = T < TP_ROWS ? (T + 7) & ~7 : TP_ROWS; a.plane = P; a.p = p; a.E = s.E; a.I = s.I; a.xinv = xinv; a.limit = s.limit; a.act_scale = act_term_scale(s.limit); a.act_inv = 1.0f / a.act_scale;
+    a.T = T; a.n = tc_tile_rows(T); a.plane = P; a.p = p; a.E = s.E; a.I = s.I; a.xinv = xinv; a.limit = s.limit; a.act_scale = act_term_scale(s.limit); a.act_inv = 1.0f / a.act_scale;
     a.slots = (T * s.K < s.n_local ? T * s.K : s.n_local) + 1;
     a.part = g->part; a.cnt = g->cnt; a.sched = g->cnt + TS_CNT; a.err = g->err;
     const size_t plan_bytes = (size_t)(4 * a.slots + 4) * sizeof(int);
