@@ -13,9 +13,13 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
 #include <string>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
+
+#include <cuda.h>
 
 #include "kernels.h"
 
@@ -281,6 +285,30 @@ static void plan_layer(g5b_engine *e, int l)
     }
 }
 
+// The driver's calls that put a device's context in place for a moment (g5b_host_alloc), looked up while an engine is created.
+struct ContextFns {
+    CUresult (*get)(CUcontext *), (*push)(CUcontext), (*pop)(CUcontext *), (*retain)(CUcontext *, CUdevice), (*release)(CUdevice);
+    bool ok;
+};
+static const ContextFns &context_fns()
+{
+    static const ContextFns fns = [] {
+        ContextFns f{};
+        auto look_up = [](const char *name, auto &fn) {
+            void *p = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) { cudaGetLastError(); return false; }
+            fn = reinterpret_cast<std::remove_reference_t<decltype(fn)>>(p);
+            return true;
+        };
+        f.ok = look_up("cuCtxGetCurrent", f.get) && look_up("cuCtxPushCurrent", f.push) && look_up("cuCtxPopCurrent", f.pop) &&
+               look_up("cuDevicePrimaryCtxRetain", f.retain) && look_up("cuDevicePrimaryCtxRelease", f.release);
+        return f;
+    }();
+    return fns;
+}
+static std::atomic<int> g_last_device{-1};               // device of the engine created last
+
 extern "C" g5b_engine *g5b_engine_create(const g5b_config *cfg, const uint8_t *is_mla,
                                          const uint8_t *is_dense, int cap, int device, int ep_rank,
                                          int ep_size)
@@ -303,6 +331,7 @@ extern "C" g5b_engine *g5b_engine_create(const g5b_config *cfg, const uint8_t *i
         return nullptr;
     }
     if (cudaSetDevice(device) != cudaSuccess) { fail("cudaSetDevice(%d) failed", device); return nullptr; }
+    if (context_fns().ok) g_last_device = device;
     g5b_engine *e = new g5b_engine();
     e->c = c;
     e->cap = cap < 1 ? 1 : cap;
@@ -1844,15 +1873,37 @@ static float *mapped_on_device(const void *p)
 }
 
 // Pinned, mapped host memory for results: a copy into it is one transfer, where ordinary memory goes through the driver's staging
-// and takes its page faults inside the copy.
+// and takes its page faults inside the copy. A thread that has not used CUDA yet (results are made before the engine's call, and given
+// back wherever the last array is dropped) would get a context on device 0, memory of a GPU that another process may own: it borrows
+// the context of the engine that was created last.
+struct BorrowedContext {
+    bool pushed = false;
+    BorrowedContext()
+    {
+        const int device = g_last_device.load();
+        if (device < 0) return;
+        const ContextFns &fn = context_fns();
+        CUcontext now = nullptr, ctx = nullptr;
+        if (!fn.ok || fn.get(&now) != CUDA_SUCCESS || now || fn.retain(&ctx, device) != CUDA_SUCCESS) return;
+        pushed = fn.push(ctx) == CUDA_SUCCESS;
+        fn.release(device);                              // (the runtime keeps it)
+    }
+    ~BorrowedContext()
+    {
+        CUcontext ctx;
+        if (pushed) context_fns().pop(&ctx);
+    }
+};
 extern "C" void *g5b_host_alloc(size_t bytes)
 {
+    BorrowedContext context;
     void *p = nullptr;
     if (bytes == 0 || cudaHostAlloc(&p, bytes, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); return nullptr; }
     return p;
 }
 extern "C" void g5b_host_free(void *p)
 {
+    BorrowedContext context;
     if (p && cudaFreeHost(p) != cudaSuccess) cudaGetLastError();
 }
 
