@@ -103,6 +103,7 @@ def lib() -> C.CDLL:
     L.g5b_engine_load_checkpoint.argtypes = [C.c_void_p, C.c_char_p, C.c_int]
     L.g5b_engine_synth_session.argtypes = [C.c_void_p, C.c_uint64, C.c_int]
     L.g5b_engine_last_picks.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]
+    L.g5b_debug_dsa_scores.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p] + [C.c_int] * 4 + [C.c_void_p, C.c_int]
     L.g5b_debug_exp.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_int]
     L.g5b_debug_moe_rows.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p]
     L.g5b_engine_decode_greedy.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_void_p]

@@ -2331,6 +2331,26 @@ extern "C" int g5b_debug_exp(const float *x, int n, float *e, float *sig, int de
     return 0;
 }
 
+extern "C" int g5b_debug_dsa_scores(const float *keys, int pools, const float *q, const float *w, int T, int heads, int dim, int tiled, float *score, int device)
+{
+    cudaStream_t st;
+    if (with_device(device, &st)) return -1;
+    if (pools < 1 || T < 1 || heads < 1 || heads > 256 || dim < 1 || dim > 512) return fail("bad indexer shape");
+    MlaShape s{};
+    s.cap = pools + T; s.ID = dim; s.IH = heads; s.KP = 1; s.topk = 0;      // pools of one position: query t sees the first pools + t
+    if (tiled && !dsa_score_tile_takes(s)) return fail("the tiled kernel does not take %d heads of %d dimensions", heads, dim);
+    const size_t ld = (size_t)s.cap + 1, keyed = (size_t)2 * s.cap * dim;
+    Tmp t;
+    float *state = (float *)t.up(nullptr, (size_t)3 * s.cap * dim * 4), *qd = (float *)t.up(q, (size_t)T * heads * dim * 4), *wd = (float *)t.up(w, (size_t)T * heads * 4);
+    float *sd = (float *)t.up(nullptr, T * ld * 4);
+    if (!state || !qd || !wd || !sd) return fail("out of device memory");
+    CU(cudaMemcpy(state + keyed, keys, (size_t)(s.cap - 1) * dim * 4, cudaMemcpyHostToDevice));
+    if (dsa_scores(st, sd, state, qd, wd, T, pools - 1, s, tiled != 0)) return -1;
+    CU(cudaMemcpy(score, sd, T * ld * 4, cudaMemcpyDeviceToHost));
+    CU(cudaGetLastError());
+    return 0;
+}
+
 extern "C" int g5b_shortconv_host(float *y, const float *x, const float *w, float *state, int channels, int k,
                                   int T, int device)
 {

@@ -323,6 +323,9 @@ void mla_store(cudaStream_t st, void *latent, float *idx_state, const float *ct_
                const float *kv_norm_w, const float *wk_raw, const float *gate_raw,
                const float *k_norm_w, const float *k_norm_b, const float *ape, const float *q_raw, float *q_inv,
                int T, int cached, const MlaShape &s);
+// Pool scores [T][cap / KP + 1] of the queries, by the tiled kernel (where it takes the shape) or the other one, bit for bit the same.
+bool dsa_score_tile_takes(const MlaShape &s);
+int dsa_scores(cudaStream_t st, float *score, const float *idx_state, const float *qidx, const float *wproj, int T, int cached, const MlaShape &s, bool tiled);
 // (0, or -1 with the reason in g5b_last_error where the device refuses a kernel its shared memory; nothing was selected then)
 int dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
                const float *wproj, float *score, int T, int cached, const MlaShape &s);

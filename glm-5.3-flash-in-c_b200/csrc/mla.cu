@@ -415,16 +415,16 @@ __global__ void __launch_bounds__(TOPK_THREADS) dsa_topk_kernel(int *sel, int *n
     if (tid == 0) nsel[t] = base + (p - np * s.KP + 1);
 }
 
-int dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
-               const float *wproj, float *score, int T, int cached, const MlaShape &s)
+bool dsa_score_tile_takes(const MlaShape &s) { return dsm_takes(s); }
+int dsa_scores(cudaStream_t st, float *score, const float *idx_state, const float *qidx, const float *wproj, int T, int cached, const MlaShape &s, bool tiled)
 {
     const int np_max = (cached + (s.batch ? 1 : T)) / s.KP;
-    if (np_max > s.topk / s.KP && dsm_takes(s)) {
+    if (tiled) {
         static SmemGrant grant;
         const size_t smem = dsm_smem(s.IH, s.ID);
         if (!dev_opt_in_smem((const void *)dsa_score_tile_kernel, smem, grant)) return -1;
         G5B_LAUNCH(dsa_score_tile_kernel, dim3((np_max + DSM_POOLS - 1) / DSM_POOLS, T), DSM_WARPS * 32, smem, st, score, idx_state, qidx, wproj, cached, s);
-    } else if (np_max > s.topk / s.KP) {
+    } else {
         const size_t smem = ((((size_t)s.ID * s.IH + 1) & ~(size_t)1) + (size_t)DSA_WARPS * DSA_POOLS * (s.IH + s.ID)) * sizeof(double);
         static SmemGrant grant;
         if (!dev_opt_in_smem((const void *)dsa_score_kernel, smem, grant)) return -1;     // (many heads of many dimensions)
@@ -433,6 +433,14 @@ int dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, con
         if (blocks > want) blocks = want;
         G5B_LAUNCH(dsa_score_kernel, dim3(blocks, T), DSA_WARPS * 32, smem, st, score, idx_state, qidx, wproj, cached, s);
     }
+    return 0;
+}
+
+int dsa_select(cudaStream_t st, int *sel, int *nsel, const float *idx_state, const float *qidx,
+               const float *wproj, float *score, int T, int cached, const MlaShape &s)
+{
+    const int np_max = (cached + (s.batch ? 1 : T)) / s.KP;
+    if (np_max > s.topk / s.KP && dsa_scores(st, score, idx_state, qidx, wproj, T, cached, s, dsm_takes(s))) return -1;
     G5B_LAUNCH_PDL(dsa_topk_kernel, T, TOPK_THREADS, 0, st, sel, nsel, score, cached, s);
     return 0;
 }

@@ -344,6 +344,10 @@ int g5b_debug_moe_rows(g5b_engine *e, int layer, const float *x, int T, float *r
 /* Test aid: the exponential and the sigmoid that the kernels over many positions use, of n host values. */
 int g5b_debug_exp(const float *x, int n, float *e, float *sig, int device);
 
+/* Test aid: the indexer's pool scores of T queries ([T][heads][dim], head weights [T][heads]) over keys [pools + T - 1][dim], of which
+ * query t sees the first pools + t, by the tiled kernel or the other one; score [T][pools + T + 1], zero beyond. */
+int g5b_debug_dsa_scores(const float *keys, int pools, const float *q, const float *w, int T, int heads, int dim, int tiled, float *score, int device);
+
 /* RMSNorm of `rows` rows of n floats on DEVICE buffers of the current CUDA device, enqueued on
  * `stream` (a cudaStream_t, NULL for the default stream) without waiting: y = w * x / sqrt(mean(x^2)
  * + eps), w may be NULL. This entry point has no counterpart in the reference. It exists for
